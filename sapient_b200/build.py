@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libsapient_cuda.so")
 SOURCES = ["kernels.cu", "attention.cu", "engine.cu", "engine_forward.cu", "engine_layers.cu", "engine_decode.cu", "gemv_imma.cu", "api.cu", "gguf.cu",
-           "attention_static.cu", "tp.cu", "gemm_tc5.cu", "gemv_ring.cu", "spec.cu", "batcher.cu", "nccl_arm.cu", "gemv_rows.cu",
+           "attention_static.cu", "tp.cu", "gemm_tc5.cu", "gemm_dq.cu", "dq_rows.cu", "gemv_ring.cu", "spec.cu", "batcher.cu", "nccl_arm.cu", "gemv_rows.cu",
            "model_plan.cu", "safetensors.cu", "engine_plan.cu", "engine_plan_post_norm.cu", "engine_plan_parallel.cu", "engine_plan_pre_norm.cu", "engine_plan_state.cu",
            "engine_plan_latent.cu", "engine_plan_grouped.cu", "mat_f32.cu", "mat_tc5.cu",
            "plan_stream.cu", "latent_attention.cu", "grouped_attention.cu", "mixed_attention.cu", "grouped_conv.cu", "state_mixer.cu", "state_chunk.cu"]

@@ -314,10 +314,15 @@ int32_t sp_cuda_matmul_nt_dev(const SpWeight* w, const float* x_dev, int64_t m, 
         const bool exact = g_tc5.load() == 2;
         SP_CUDA_TRY(wm->ws.ensure_xh((size_t)m * w->k * (exact ? 2 : 1)));
         if (exact && m > ActWorkspace::XSCALE_ROWS) { set_error("matmul: more than 4096 rows in the exact tensor-core mode"); return SP_ERR_SHAPE; }
-        if (exact) SP_CUDA_TRY(launch_x_to_f16_hilo(x_dev, (int)w->k, (int)m, (int)w->k, wm->ws.xh, wm->ws.xscale, (cudaStream_t)stream));
-        else SP_CUDA_TRY(launch_x_to_f16(x_dev, (int)w->k, (int)m, (int)w->k, wm->ws.xh, (cudaStream_t)stream));
+        if (exact) {
+            const Tc5Seg sg{w->tiled, y_dev, nullptr, w->dtype, (int)w->n};
+            SP_CUDA_TRY(launch_dq_rows(DQ_PLAIN, x_dev, (int)w->k, nullptr, nullptr, 0.f, (int)m, (int)w->k, wm->ws.dq(), (cudaStream_t)stream));
+            SP_CUDA_TRY(launch_gemm_dq(&sg, 1, (int)w->k, wm->ws.dq(), (int)m, (int)w->n, nullptr, 0, (cudaStream_t)stream));
+            return SP_OK;
+        }
+        SP_CUDA_TRY(launch_x_to_f16(x_dev, (int)w->k, (int)m, (int)w->k, wm->ws.xh, (cudaStream_t)stream));
         SP_CUDA_TRY(launch_gemm_tc5(w->tiled, w->dtype, (int)w->n, (int)w->k, wm->ws.xh, (int)m, y_dev, (int)w->n, nullptr, nullptr, 0,
-                                    (cudaStream_t)stream, &wm->ws.tc5, exact ? wm->ws.xscale : nullptr));
+                                    (cudaStream_t)stream, &wm->ws.tc5));
         return SP_OK;
     }
     if (w->tiled && g_gemv_path.load() == 0 && g_ring.load() && m >= 1 && m <= RING_MAX_M) {
@@ -364,9 +369,9 @@ int32_t sp_cuda_matmul_nt_dev(const SpWeight* w, const float* x_dev, int64_t m, 
 }
 
 static int check_kernel_flags() {
-    const int a = tc5_take_timeout(), b = imma_take_timeout();
-    if (a < 0 || b < 0) { set_error("could not read the kernels' timeout flags"); return SP_ERR_CUDA; }
-    if (a > 0) { set_error("tcgen05 GEMM: a bounded mbarrier wait expired, the outputs of that launch are not valid"); return SP_ERR_CUDA; }
+    const int a = tc5_take_timeout(), b = imma_take_timeout(), c = dq_take_timeout();
+    if (a < 0 || b < 0 || c < 0) { set_error("could not read the kernels' timeout flags"); return SP_ERR_CUDA; }
+    if (a > 0 || c > 0) { set_error("tcgen05 GEMM: a bounded mbarrier wait expired, the outputs of that launch are not valid"); return SP_ERR_CUDA; }
     if (b > 0) { set_error("streaming GEMV: a bounded mbarrier wait expired, the outputs of that launch are not valid"); return SP_ERR_CUDA; }
     return SP_OK;
 }

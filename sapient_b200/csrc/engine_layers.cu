@@ -66,7 +66,11 @@ int Engine::gemv(const float* x, int ldx, int m, int k, const DevTensor* w0, con
         for (int i = 0; i < 3 && ws[i]; ++i) ok = ok && tc5_supported(ws[i]->dtype, k);
         if (ok) {
             // many rows: dequantise each weight tile once and multiply on the 5th-generation tensor cores
-            if (tc5_exact) SP_LAUNCH(F_ELEM, launch_x_to_f16_hilo(x, ldx, m, k, ws_.xh, ws_.xscale, stream));
+            auto product = [&](const Tc5Seg* segs, int ns, int ldy, const float* r) {
+                return tc5_exact ? launch_gemm_dq(segs, ns, k, ws_.dq(), m, ldy, r, ldy, stream)
+                                 : launch_gemm_tc5_multi(segs, ns, k, ws_.xh, m, ldy, r, ldy, stream, &ws_.tc5);
+            };
+            if (tc5_exact) SP_LAUNCH(F_ELEM, launch_dq_rows(DQ_PLAIN, x, ldx, nullptr, nullptr, 0.f, m, k, ws_.dq(), stream));
             else SP_LAUNCH(F_ELEM, launch_x_to_f16(x, ldx, m, k, ws_.xh, stream));
             Tc5Seg segs[3];
             int ns = 0;
@@ -74,7 +78,7 @@ int Engine::gemv(const float* x, int ldx, int m, int k, const DevTensor* w0, con
                 // column-split matrix: this rank's partial product to scratch (the bias once, on rank 0), then to every
                 // rank's receive area (or through the library all-reduce of the comparison arm)
                 segs[ns++] = Tc5Seg{w0->tiled, h_, d.tp_rank == 0 ? b0 : nullptr, w0->dtype, (int)w0->dims[0]};
-                SP_LAUNCH(F_GEMV, launch_gemm_tc5_multi(segs, ns, k, ws_.xh, m, d.hidden, nullptr, 0, stream, &ws_.tc5, tc5_exact ? ws_.xscale : nullptr));
+                SP_LAUNCH(F_GEMV, product(segs, ns, d.hidden, nullptr));
                 if (tp_use_nccl_) {
                     SP_TRY(nccl_all_reduce(h_, (size_t)m * d.hidden));
                     SP_LAUNCH(F_ELEM, launch_add(x_, h_, x_, (int64_t)m * d.hidden, stream));
@@ -85,7 +89,7 @@ int Engine::gemv(const float* x, int ldx, int m, int k, const DevTensor* w0, con
                 return SP_OK;
             }
             for (int i = 0; i < 3 && ws[i]; ++i) segs[ns++] = Tc5Seg{ws[i]->tiled, ys[i], bs[i], ws[i]->dtype, (int)ws[i]->dims[0]};
-            SP_LAUNCH(F_GEMV, launch_gemm_tc5_multi(segs, ns, k, ws_.xh, m, ldy0, res, ldy0, stream, &ws_.tc5, tc5_exact ? ws_.xscale : nullptr));
+            SP_LAUNCH(F_GEMV, product(segs, ns, ldy0, res));
             return SP_OK;
         }
     }

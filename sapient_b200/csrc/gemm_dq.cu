@@ -1,0 +1,794 @@
+// Dequant GEMM with exact-class operands on the 5th-generation tensor cores: y[m, n] = sum_k x[m, k] * W[n, k] (+ bias,
+// + residual) from the tile-repacked ggml blocks (gemv_imma.cuh) for steps of DQ_MIN_M rows and more: batched decode,
+// mixed steps, prompts.
+//
+// What is multiplied. Activation rows are scaled by a power of two into (-1, 1) and split into an fp16 leading part and the
+// fp16 of what that rounding dropped (dq_rows.cu). Weights are never rounded:
+//   Q4_K  w = d * (sc * q) - dmin * m. sc * q <= 945 is an exact fp16 integer: ONE operand plane, two products per column
+//         (X_hi, X_lo). The minimum term is a product with the sums of 32 activations, see below.
+//   Q6_K  w = d * (sc * (q - 32)), |sc * (q - 32)| <= 4096: two planes, the integer rounded to fp16 and the exact remainder.
+//   Q8_0  w = d * q (19 bits): two planes, product rounded to fp16 and the exact remainder.
+// Two planes take three products (W_hi X_hi, W_lo X_hi, W_hi X_lo). The tensor core sums 256 columns at a time; the block scale
+// d is applied in f32 when a sum leaves tensor memory, so no f32 rounding chain is longer than that and the K-quant scales
+// cost nothing per weight.
+//
+// Why this shape. What bounded the kernel that this one replaced was not the tensor pipe (13 % busy) nor DRAM (7 %) but its
+// 16 producer warps: weights were rebuilt in f32 and split there, 376 warp instructions per 1024 weights, their raw words one
+// register set ahead. Here a pair of 4-bit weights costs a mask and one half-pair multiply-add (about 60 instructions per 1024),
+// and raw tiles arrive by bulk copies through a ring of up to 150 KB per SM, requested before the previous kernel has ended.
+// A block owns 128 weight rows x up to 128 activation rows:
+//   warp 0      one thread issues tcgen05.mma (A: weights in tensor memory, B: activations in shared memory)
+//   warp 1      bulk copies of raw weight tiles; warp 2: TMA of activation boxes (64 columns, both planes) and 32-sums
+//   warps 4-11  producers: a 16-row tile each, raw words -> fp16 planes -> tensor memory
+//   warps 12-19 drains: after 256 columns a sum is read from tensor memory (two accumulator buffers), multiplied by d and
+//               added to f32 registers; for Q4_K the minimum term m * (32-sums) is an mma.sync of 8 columns (leading parts and
+//               remainders of the sums, minima exact) times dmin, which costs a quarter instruction per element.
+// Columns are stored in the order 0 2 1 3 within groups of four, in activations and weights alike: the order in which masks
+// pick bytes out of a word, so that no weight is moved.
+// The K range of a tile is shared by the blocks of a cluster when tiles alone leave SMs idle; they meet in distributed shared
+// memory and add in part order, so results do not vary from run to run. Every wait on an mbarrier is bounded.
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <atomic>
+
+#include "gemv_imma.cuh"
+#include "kernels.h"
+#include "pdl.cuh"
+#include "plan_common.cuh"
+#include "sp_common.cuh"
+#include "tc5_ptx.cuh"
+
+namespace sp {
+
+cudaError_t count_launch_and_check();  // kernels.cu
+
+constexpr int DQ_THREADS = 640;
+constexpr int DQ_PRODUCERS = 8, DQ_FIRST_PRODUCER = 4, DQ_DRAINS = 8, DQ_FIRST_DRAIN = 12;
+constexpr int DQ_BM = 128;                 // weight rows per block
+constexpr int DQ_NB = 128;                 // activation rows per block at most
+constexpr int DQ_A_SLOTS = 4;              // weight slots in tensor memory, 64 columns each: 128 columns of K of one plane (a half);
+                                           // two planes take a pair of slots and go by the second one's barriers
+constexpr int DQ_A_COL = 2 * DQ_NB;        // tensor memory: two accumulators of DQ_NB columns, then the weight stages
+constexpr int DQ_MAX_B = 8, DQ_MAX_R = 8, DQ_X_STAGES = 3;
+constexpr int DQ_SMEM = 224 * 1024;
+constexpr int DQ_MAX_PARTS = 8;
+constexpr int DQ_P_STRIDE = DQ_BM + 4;     // floats between the columns of a partial tile: no bank conflicts
+
+__device__ int g_dq_timeout = 0;
+
+constexpr int T_Q8_0_HALF = 1000 + T_Q8_0;  // Q8_0 whose width is an odd multiple of 128: tiles of four blocks
+
+struct DqArgs {
+    Tc5Seg seg[3];
+    int nseg, k, m, ldy;
+    const float* res;      // [m][ldres] or null, added to segment 0 (may alias its y)
+    int ldres;
+    int m_tiles, nb;       // row tiles, rows per tile (a multiple of 16)
+    int items;             // tiles in all
+    int parts;             // blocks of the cluster that share a tile's K range
+    int b_stages, r_stages, r_bytes;  // depth of the activation ring, of the raw ring, bytes of a raw stage
+    const float* xscale;   // [m]
+    const __half* xsum;    // [k / 256][m][16]: sums of 32 columns as dq_rows.cu leaves them
+};
+
+__device__ __forceinline__ void dq_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// 16 lanes x 32 columns of tensor memory from a warp: words 4 i .. 4 i + 3 of lane (g, t) are columns 8 i + 2 t, + 1 of lanes g
+// (first two) and g + 8.
+__device__ __forceinline__ void dq_st(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr), "r"(v[0]),
+        "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]),
+        "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+
+// 16 lanes x 8 (16) columns, in the layout of an mma accumulator fragment.
+__device__ __forceinline__ void dq_ld8(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void dq_ld16(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+
+__device__ __forceinline__ void dq_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void dq_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void dq_init(uint64_t* bar, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(tc5_smem_u32(bar)), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ __half2 dq_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
+__device__ __forceinline__ uint32_t dq_u(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
+__device__ __forceinline__ __half2 dq_const(float f) { return __float2half2_rn(f); }
+__device__ __forceinline__ uint32_t dq_word(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+// Byte b of v twice, as the half pair (1024 + byte, 1024 + byte).
+__device__ __forceinline__ __half2 dq_twice(uint32_t v, int b) { return dq_h2(__byte_perm(v, 0x64646464u, 0x4040 | (b << 8) | b)); }
+
+// The eight 6-bit scales (minima) of a Q4_K block header, one per byte.
+__device__ __forceinline__ void q4k_scales(const uint4& hd, uint32_t& lo, uint32_t& hi) {
+    lo = hd.y & 0x3F3F3F3Fu;
+    hi = (hd.w & 0x0F0F0F0Fu) | ((hd.y >> 2) & 0x30303030u);
+}
+__device__ __forceinline__ void q4k_minima(const uint4& hd, uint32_t& lo, uint32_t& hi) {
+    lo = hd.z & 0x3F3F3F3Fu;
+    hi = ((hd.w >> 4) & 0x0F0F0F0Fu) | ((hd.z >> 2) & 0x30303030u);
+}
+
+// bytes of one 16-row tile's 256 columns
+__host__ __device__ constexpr int dq_tile_bytes(int dt) { return dt == T_Q4_K ? Q4_K_TILE_BYTES : dt == T_Q6_K ? Q6_K_TILE_BYTES : 8 * 544; }
+
+// A 16-row tile's weights, 128 columns (a half) at a time: the words of a half are read from shared memory together, then turned
+// into operands 64 columns at a time. o is the operand plane (of two planes the leading parts), ol the remainders; words
+// 4 c .. 4 c + 3 are lane (g, t)'s columns 16 c + 4 t .. + 3 of rows g and g + 8.
+template <int DT>
+struct DqTile {
+    const uint8_t* tile;   // in shared memory
+    int lane;
+    uint4 hd[2];           // Q4_K, Q6_K: headers of rows g, g + 8
+    uint4 q[4];            // the half's words: Q4_K 2, Q6_K 3, Q8_0 4 pieces
+    uint2 d8[2];           // Q8_0: the half's four scales of rows g, g + 8
+    __device__ __forceinline__ DqTile(const uint8_t* tile_, int lane_) : tile(tile_), lane(lane_) {
+        const int g = lane >> 2;
+        constexpr int AT = DT == T_Q4_K ? 2048 : 3072;
+        if (DT == T_Q4_K || DT == T_Q6_K) {
+            hd[0] = *reinterpret_cast<const uint4*>(tile + AT + g * 16);
+            hd[1] = *reinterpret_cast<const uint4*>(tile + AT + (g + 8) * 16);
+        }
+    }
+    __device__ __forceinline__ void load(int half) {
+        constexpr int N = DT == T_Q4_K ? 2 : DT == T_Q6_K ? 3 : 4;
+        const uint8_t* at = tile + (DT == T_Q8_0_HALF ? half * 2176 : half * N * 512) + lane * 16;
+#pragma unroll
+        for (int i = 0; i < N; ++i) q[i] = *reinterpret_cast<const uint4*>(at + i * 512);
+        if (DT == T_Q8_0 || DT == T_Q8_0_HALF) {
+            const uint8_t* ds = DT == T_Q8_0 ? tile + 4096 + half * 8 : tile + half * 2176 + 2048;
+            constexpr int PITCH = DT == T_Q8_0 ? 16 : 8;
+            d8[0] = *reinterpret_cast<const uint2*>(ds + (lane >> 2) * PITCH);
+            d8[1] = *reinterpret_cast<const uint2*>(ds + ((lane >> 2) + 8) * PITCH);
+        }
+    }
+    // columns 128 half + 64 e .. + 63
+    __device__ __forceinline__ void group(int half, int e, uint32_t (&o)[16], uint32_t (&ol)[16]) {
+        if (DT == T_Q4_K) {
+            const uint4 w = q[e];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                uint32_t lo, hi;
+                q4k_scales(hd[r], lo, hi);
+                const uint32_t sc = half ? hi : lo;
+                // low nibbles: (1024 + q) sc - 1024 sc; high nibbles stand 16 times higher: (1024 + 16 q) sc / 16 - 64 sc. Both exact.
+                const __half2 s0 = __hadd2(dq_twice(sc, 2 * e), dq_const(-1024.f));
+                const __half2 s1 = __hfma2(dq_twice(sc, 2 * e + 1), dq_const(0.0625f), dq_const(-64.f));
+                const __half2 c0 = __hmul2(s0, dq_const(-1024.f)), c1 = __hmul2(s1, dq_const(-1024.f));
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t v = dq_word(w, 2 * r + h), v8 = v >> 8;
+                    o[4 * h + 2 * r] = dq_u(__hfma2(dq_h2((v & 0x000F000Fu) | 0x64006400u), s0, c0));
+                    o[4 * h + 2 * r + 1] = dq_u(__hfma2(dq_h2((v8 & 0x000F000Fu) | 0x64006400u), s0, c0));
+                    o[8 + 4 * h + 2 * r] = dq_u(__hfma2(dq_h2((v & 0x00F000F0u) | 0x64006400u), s1, c1));
+                    o[8 + 4 * h + 2 * r + 1] = dq_u(__hfma2(dq_h2((v8 & 0x00F000F0u) | 0x64006400u), s1, c1));
+                }
+            }
+        } else if (DT == T_Q6_K) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const uint32_t sw = dq_word(hd[r], 2 * half + e) ^ 0x80808080u;
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    const int base = 6 * p + 3 * r;
+                    const uint32_t qh = dq_word(q[(base + 2) >> 2], (base + 2) & 3);
+#pragma unroll
+                    for (int ab = 0; ab < 2; ++ab) {
+                        const uint32_t ql = dq_word(q[(base + ab) >> 2], (base + ab) & 3);
+                        const int quarter = 2 * e + ab;
+                        const uint32_t top = quarter == 0 ? qh << 4 : quarter == 1 ? qh << 2 : quarter == 2 ? qh : qh >> 2;
+                        const uint32_t v = ((e ? ql >> 4 : ql) & 0x0F0F0F0Fu) | (top & 0xF0F0F0F0u);
+                        const __half2 sc = __hadd2(dq_twice(sw, 2 * ab + p), dq_const(-1152.f));
+                        const __half2 a = __hadd2(dq_h2((v & 0x003F003Fu) | 0x64006400u), dq_const(-1056.f));
+                        const __half2 b = __hadd2(dq_h2(((v >> 8) & 0x003F003Fu) | 0x64006400u), dq_const(-1056.f));
+                        const __half2 ah = __hmul2_rn(a, sc), bh = __hmul2_rn(b, sc);
+                        const int c = 4 * (2 * ab + p) + 2 * r;
+                        o[c] = dq_u(ah);
+                        o[c + 1] = dq_u(bh);
+                        ol[c] = dq_u(__hfma2(a, sc, __hneg2(ah)));
+                        ol[c + 1] = dq_u(__hfma2(b, sc, __hneg2(bh)));
+                    }
+                }
+            }
+        } else {
+#pragma unroll
+            for (int blk = 0; blk < 2; ++blk) {
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const uint32_t dw = e ? d8[r].y : d8[r].x;
+                    const __half2 d = dq_h2(__byte_perm(dw, 0u, blk ? 0x3232 : 0x1010));
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t v = dq_word(q[2 * e + blk], 2 * r + h);
+                        const __half2 a = __hadd2(dq_h2((v & 0x00FF00FFu) ^ 0x64806480u), dq_const(-1152.f));
+                        const __half2 b = __hadd2(dq_h2(((v >> 8) & 0x00FF00FFu) ^ 0x64806480u), dq_const(-1152.f));
+                        const __half2 ah = __hmul2_rn(a, d), bh = __hmul2_rn(b, d);
+                        const int c = 4 * (2 * blk + h) + 2 * r;
+                        o[c] = dq_u(ah);
+                        o[c + 1] = dq_u(bh);
+                        ol[c] = dq_u(__hfma2(a, d, __hneg2(ah)));
+                        ol[c + 1] = dq_u(__hfma2(b, d, __hneg2(bh)));
+                    }
+                }
+            }
+        }
+    }
+};
+
+struct DqBars {
+    uint64_t full_r[DQ_MAX_R], empty_r[DQ_MAX_R], full_a[DQ_A_SLOTS], empty_a[DQ_A_SLOTS], full_b[DQ_MAX_B], empty_b[DQ_MAX_B];
+    uint64_t full_x[DQ_X_STAGES], empty_x[DQ_X_STAGES], full_d[2], empty_d[2];
+};
+
+// Where a warp stands in a ring of `n` stages: the stage and how often the ring has wrapped. Carried from tile to tile.
+struct DqRing {
+    int st = 0;
+    uint32_t u = 0;
+    __device__ __forceinline__ void next(int n) {
+        if (++st == n) { st = 0; ++u; }
+    }
+    __device__ __forceinline__ bool full(uint64_t* bars) const { return tc5_wait(&bars[st], u & 1); }
+    __device__ __forceinline__ bool empty(uint64_t* bars) const { return u == 0 || tc5_wait(&bars[st], (u - 1) & 1); }
+};
+
+// A producer warp's walk over the block's K range, a half (128 columns) at a time; all eight warps fill a slot or a pair.
+template <int DT>
+__device__ __forceinline__ bool dq_produce(DqBars& bars, const uint8_t* raw, int r_bytes, int r_stages, int tile_w, int lane, uint32_t a_base, int n_sb,
+                                           int halves_last, DqRing& rr, DqRing& ra, bool ok) {
+    constexpr bool TWO = DT != T_Q4_K;
+    for (int sb = 0; sb < n_sb; ++sb) {
+        ok = ok && rr.full(bars.full_r);
+        DqTile<DT> t(raw + (size_t)rr.st * r_bytes + tile_w * dq_tile_bytes(DT), lane);
+        const int halves = DT == T_Q8_0_HALF && sb == n_sb - 1 ? halves_last : 2;
+        t.load(0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (DT == T_Q8_0_HALF && h >= halves) break;
+            const uint32_t at = a_base + 64u * (uint32_t)ra.st;
+            uint32_t o[16], o1[16];
+            t.group(h, 0, o, o1);
+            if (!TWO) t.group(h, 1, o1, o1);
+            if (TWO) ra.next(DQ_A_SLOTS);  // (a pair's second slot)
+            ok = ok && ra.empty(bars.empty_a);
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            dq_st(at, o);
+            dq_st(at + (TWO ? 64u : 32u), o1);
+            if (TWO) {
+                t.group(h, 1, o, o1);
+                dq_st(at + 32u, o);
+                dq_st(at + 96u, o1);
+            }
+            if (h + 1 < halves) {
+                t.load(1);
+            } else {  // the raw words have been read
+                __syncwarp();
+                if (lane == 0) tc5_arrive(&bars.empty_r[rr.st]);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                if (TWO) tc5_arrive(&bars.full_a[ra.st - 1]);
+                tc5_arrive(&bars.full_a[ra.st]);
+            }
+            ra.next(DQ_A_SLOTS);
+        }
+        rr.next(r_stages);
+    }
+    return ok;
+}
+
+// Tiles of up to 64 activation rows have both planes of the activations side by side in one product (its N is twice the rows) and
+// in the accumulator; the drain adds them. Wider tiles multiply the planes one after the other into the same columns.
+constexpr int DQ_SIDE_NJT = 4;
+
+// A drain warp's walk: acc[tile][j] holds rows 16 tile + g (+ 8) of the warp's 32, columns 8 j + 2 t (+ 1) of its NJT 8-column tiles.
+template <int DT, int NJT>
+__device__ __forceinline__ bool dq_drain(DqBars& bars, const uint8_t* raw, int r_bytes, int r_stages, const uint8_t* xs, int x_bytes, int plane, int quarter,
+                                         int half, int lane, uint32_t tmem, int n_sb, DqRing& rr, DqRing& rx, DqRing& rd, float (&acc)[2][NJT][4], bool ok) {
+    constexpr bool SIDE = NJT <= DQ_SIDE_NJT;
+    const int g = lane >> 2, t = lane & 3;
+    for (int sb = 0; sb < n_sb; ++sb) {
+        float d[2][2], dm[2][2];
+        uint32_t mn[2][2];
+        ok = ok && rr.full(bars.full_r);
+        if (DT == T_Q4_K || DT == T_Q6_K) {
+            const uint8_t* base = raw + (size_t)rr.st * r_bytes + 2 * quarter * dq_tile_bytes(DT);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const uint8_t* tile = base + i * dq_tile_bytes(DT);
+                    if (DT == T_Q4_K) {
+                        const uint4 hd = *reinterpret_cast<const uint4*>(tile + 2048 + (g + 8 * r) * 16);
+                        d[i][r] = __low2float(dq_h2(hd.x));
+                        dm[i][r] = -__high2float(dq_h2(hd.x));
+                        uint32_t lo, hi;
+                        q4k_minima(hd, lo, hi);
+                        // minima 2 t, 2 t + 1 as a half pair
+                        const uint32_t two = __byte_perm(t < 2 ? lo : hi, 0x64646464u, (t & 1) ? 0x4342 : 0x4140);
+                        mn[i][r] = dq_u(__hadd2(dq_h2(two), dq_const(-1024.f)));
+                    } else {
+                        d[i][r] = __half2float(*reinterpret_cast<const __half*>(tile + 3328 + 2 * (g + 8 * r)));
+                    }
+                }
+        }
+        __syncwarp();
+        if (lane == 0) tc5_arrive(&bars.empty_r[rr.st]);
+        rr.next(r_stages);
+        if (DT == T_Q4_K) ok = ok && rx.full(bars.full_x);
+        ok = ok && rd.full(bars.full_d);
+        ok = __all_sync(0xFFFFFFFFu, ok);
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const uint32_t from = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(rd.st * DQ_NB + half * NJT * 8);
+        const uint8_t* xrow = xs + (size_t)rx.st * x_bytes + (half * NJT * 8 + g) * 32 + t * 8;
+        // batches of two 8-column tiles, the next one requested before the current one is added
+        constexpr int NB2 = NJT >= 2 ? NJT / 2 : 1, W = NJT >= 2 ? 2 : 1, PL = SIDE ? 2 : 1;
+        uint32_t v[2][PL][4 * W];
+        auto fetch = [&](int b, uint32_t (&dst)[PL][4 * W]) {
+#pragma unroll
+            for (int p = 0; p < PL; ++p) {
+                const uint32_t a = from + ((uint32_t)(16 * (b / NB2)) << 16) + (uint32_t)((b % NB2) * 8 * W + p * plane);
+                if (W == 2) dq_ld16(a, dst[p]);
+                else dq_ld8(a, dst[p]);
+            }
+        };
+        fetch(0, v[0]);
+#pragma unroll
+        for (int b = 0; b < 2 * NB2; ++b) {
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            uint32_t(&c)[PL][4 * W] = v[b & 1];
+#pragma unroll
+            for (int e = 0; e < PL * 4 * W; ++e) asm volatile("" : "+r"(c[e / (4 * W)][e % (4 * W)]));  // not to be used before the wait
+            if (b + 1 < 2 * NB2) fetch(b + 1, v[(b + 1) & 1]);
+            const int i = b / NB2;
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                float* const a = acc[i][(b % NB2) * W + w];
+                if (DT == T_Q4_K) {
+                    const uint2 x = *reinterpret_cast<const uint2*>(xrow + ((b % NB2) * W + w) * 256);
+                    float p[4];
+                    asm volatile(
+                        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%4,%5}, {%6,%7}, {%8,%8,%8,%8};\n"
+                        : "=f"(p[0]), "=f"(p[1]), "=f"(p[2]), "=f"(p[3])
+                        : "r"(mn[i][0]), "r"(mn[i][1]), "r"(x.x), "r"(x.y), "f"(0.f));
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) a[e] = fmaf(dm[i][e >> 1], p[e], a[e]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float f = __uint_as_float(c[0][4 * w + e]);
+                    if (SIDE) f += __uint_as_float(c[PL - 1][4 * w + e]);
+                    a[e] = DT == T_Q4_K || DT == T_Q6_K ? fmaf(d[i][e >> 1], f, a[e]) : a[e] + f;
+                }
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+            tc5_arrive(&bars.empty_d[rd.st]);
+            if (DT == T_Q4_K) tc5_arrive(&bars.empty_x[rx.st]);
+        }
+        rd.next(2);
+        if (DT == T_Q4_K) rx.next(DQ_X_STAGES);
+    }
+    return ok;
+}
+
+// The MMA warp's walk, a half at a time: an activation stage is two boxes of 64 columns. The whole warp takes part and one elected thread
+// issues: control flow and operands are uniform then, as the tensor instructions want them. Issuing is the serial part of the
+// pipeline (a wait that is already over costs 100 to 250 cycles on a busy SM), so the barriers of the next half are looked at ahead of
+// a half's products and only waited for if they were not over by then.
+template <bool TWO, bool SIDE>
+__device__ __forceinline__ bool dq_issue(DqBars& bars, uint32_t tm, uint64_t bd0, uint32_t b16, int b_stages, uint32_t idesc, uint32_t idesc_side, int n_sb,
+                                         int halves_last, bool leader, DqRing& ra, DqRing& rb, DqRing& rd, bool& seen, bool ok) {
+    const uint32_t box16 = b16 >> 1, plane16 = box16 >> 1;  // a box: both planes
+    for (int sb = 0; sb < n_sb; ++sb) {
+        const int halves = sb == n_sb - 1 ? halves_last : 2;
+        for (int h = 0; h < halves; ++h) {
+            const bool first = h == 0, last = h == halves - 1;
+            const uint32_t At = tm + (uint32_t)DQ_A_COL + 64u * (uint32_t)ra.st;
+            if (TWO) ra.next(DQ_A_SLOTS);  // (a pair's second slot)
+            if (!seen && ok) {
+                bool w = true;
+                if (first) w = rd.empty(bars.empty_d);
+                w = w && ra.full(bars.full_a) && rb.full(bars.full_b);
+                ok = __all_sync(0xFFFFFFFFu, w);
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t dt = tm + (uint32_t)(rd.st * DQ_NB);
+            const uint64_t b0 = bd0 + (uint64_t)((uint32_t)rb.st * b16);  // (the address field: no carry out of the low word)
+            uint64_t* const e_b = &bars.empty_b[rb.st];
+            uint64_t* const e_a = &bars.empty_a[ra.st];
+            uint64_t* const f_d = &bars.full_d[rd.st];
+            rb.next(b_stages);
+            ra.next(DQ_A_SLOTS);
+            if (last) rd.next(2);
+            bool next = tc5_peek(&bars.full_b[rb.st], rb.u & 1);
+            // (where the next tile's format is another one, the other slot of the pair says the same: slots are filled in order)
+            next = tc5_peek(&bars.full_a[ra.st + (TWO ? 1 : 0)], ra.u & 1) && next;
+            if (last && rd.u > 0) next = tc5_peek(&bars.empty_d[rd.st], (rd.u - 1) & 1) && next;
+            if (leader) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint32_t more = i > 0 ? 1u : (uint32_t)(h > 0);
+                    const uint64_t bh = b0 + (i >> 2) * box16 + 2u * (i & 3);
+                    if (SIDE) {
+                        dq_mma(dt, At + 8u * i, bh, idesc_side, more);                  // W [X_hi | X_lo]
+                    } else {
+                        dq_mma(dt, At + 8u * i, bh + plane16, idesc, more);             // W X_lo
+                        dq_mma(dt, At + 8u * i, bh, idesc, 1u);                         // W X_hi
+                    }
+                    if (TWO) dq_mma(dt, At + 64u + 8u * i, bh, idesc, 1u);              // W_lo X_hi
+                }
+                tc5_commit(e_b);
+                if (TWO) tc5_commit(e_a - 1);
+                tc5_commit(e_a);
+                if (last) tc5_commit(f_d);
+            }
+            seen = __all_sync(0xFFFFFFFFu, next);
+        }
+    }
+    return ok;
+}
+
+// Which matrix and rows a tile is.
+struct DqItem {
+    int si, dt, n0, m0, rows;
+    __device__ __forceinline__ DqItem(const DqArgs& a, int item) {
+        int bx = item / a.m_tiles;
+        si = 0;
+        while (si < a.nseg - 1 && bx >= (a.seg[si].n + DQ_BM - 1) / DQ_BM) { bx -= (a.seg[si].n + DQ_BM - 1) / DQ_BM; ++si; }
+        dt = (a.seg[si].dtype == T_Q8_0 && (a.k & 255)) ? T_Q8_0_HALF : a.seg[si].dtype;
+        n0 = bx * DQ_BM;
+        m0 = (item % a.m_tiles) * a.nb;
+        rows = min(a.nb, a.m - m0);
+    }
+};
+
+// NJT: 8-column tiles of activation rows per drain warp; a tile's rows are at most 16 NJT. A block takes tiles blockIdx.x,
+// blockIdx.x + gridDim.x, ..; its warps run from one into the next (the epilogue of a tile under the products of the next one).
+template <int NJT>
+__global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, const __grid_constant__ CUtensorMap tmap_x) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) DqBars bars;
+    __shared__ uint32_t tmem_slot;
+    constexpr bool SIDE = NJT <= DQ_SIDE_NJT;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint8_t* smem = smem_raw + ((1024u - (tc5_smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int all_sb = (a.k + 255) / 256, part = blockIdx.z;
+    const int sb0 = part * all_sb / a.parts, n_sb = (part + 1) * all_sb / a.parts - sb0;
+    const int halves_last = min(2, (a.k - (sb0 + n_sb - 1) * 256) / 128);  // 128-column halves of this block's last 256 columns
+    const int b_bytes = 4 * a.nb * 128, x_bytes = a.nb * 32;
+    uint8_t* const xs = smem + (size_t)a.b_stages * b_bytes;
+    uint8_t* const raw = xs + DQ_X_STAGES * x_bytes;
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(tc5_smem_u32(&tmem_slot)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    if (tid == 32) {
+        tc5_prefetch_map(&tmap_x);
+        for (int s = 0; s < a.r_stages; ++s) { dq_init(&bars.full_r[s], 1); dq_init(&bars.empty_r[s], DQ_PRODUCERS + DQ_DRAINS); }
+        for (int s = 0; s < DQ_A_SLOTS; ++s) { dq_init(&bars.full_a[s], DQ_PRODUCERS); dq_init(&bars.empty_a[s], 1); }
+        for (int s = 0; s < a.b_stages; ++s) { dq_init(&bars.full_b[s], 1); dq_init(&bars.empty_b[s], 1); }
+        for (int s = 0; s < DQ_X_STAGES; ++s) { dq_init(&bars.full_x[s], 1); dq_init(&bars.empty_x[s], DQ_DRAINS); }
+        for (int s = 0; s < 2; ++s) { dq_init(&bars.full_d[s], 1); dq_init(&bars.empty_d[s], DQ_DRAINS); }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, tmem_slot, 0);
+
+    bool ok = true;
+    if (warp < DQ_FIRST_PRODUCER) {
+        if (NJT >= 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;\n");  // 128 x 32 + 256 x 96 + 256 x 128 = 640 x 96
+        if (warp == 1) {
+            if (lane == 0) {
+                // raw tiles: weights, which no kernel writes, so they are requested before the previous kernel has ended
+                DqRing r;
+                int issued = 0;
+                for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+                    const DqItem it(a, item);
+                    const int tb = dq_tile_bytes(it.dt), live = min(8, ((a.seg[it.si].n + 15) >> 4) - (it.n0 >> 4));
+                    const int64_t row_bytes = (int64_t)(a.k >> 7) * (tb >> 1);
+                    const uint8_t* src = a.seg[it.si].wt + (int64_t)(it.n0 >> 4) * row_bytes + (int64_t)sb0 * tb;
+                    for (int sb = 0; sb < n_sb; ++sb) {
+                        ok = r.empty(bars.empty_r);
+                        if (!ok) break;
+                        const uint32_t bytes = sb == n_sb - 1 ? (uint32_t)(tb / 2 * halves_last) : (uint32_t)tb;
+                        const uint32_t bar = tc5_smem_u32(&bars.full_r[r.st]), dst = tc5_smem_u32(raw + (size_t)r.st * a.r_bytes);
+                        dq_expect(bar, bytes * live);
+                        for (int i = 0; i < live; ++i) dq_bulk(dst + i * tb, src + i * row_bytes + (int64_t)sb * tb, bytes, bar);
+                        r.next(a.r_stages);
+                        ++issued;
+                    }
+                }
+                // (all copies land before the block ends, whatever became of their readers)
+                for (int i = max(0, issued - a.r_stages); i < issued && ok; ++i) ok = tc5_wait(&bars.full_r[i % a.r_stages], (uint32_t)((i / a.r_stages) & 1));
+            }
+            __syncwarp();
+            pdl_wait();
+        } else {
+            pdl_wait();
+            pdl_trigger();
+        }
+        if (warp == 2 && lane == 0) {
+            DqRing r, rx;
+            for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+                const DqItem it(a, item);
+                for (int sb = 0; sb < n_sb && ok; ++sb) {
+                    const int halves = sb == n_sb - 1 ? halves_last : 2;
+                    for (int h = 0; h < halves; ++h) {
+                        ok = r.empty(bars.empty_b);
+                        if (!ok) break;
+                        const uint32_t bar = tc5_smem_u32(&bars.full_b[r.st]), dst = tc5_smem_u32(smem + (size_t)r.st * b_bytes);
+                        dq_expect(bar, (uint32_t)b_bytes);
+                        for (int c = 0; c < 4; ++c)
+                            tc5_tma_2d(dst + c * a.nb * 128, &tmap_x, (sb0 + sb) * 256 + 128 * h + 64 * (c >> 1), (c & 1) * a.m + it.m0, bar);
+                        r.next(a.b_stages);
+                    }
+                    if (it.dt == T_Q4_K && ok) {
+                        ok = rx.empty(bars.empty_x);
+                        if (!ok) break;
+                        const uint32_t bar = tc5_smem_u32(&bars.full_x[rx.st]);
+                        dq_expect(bar, (uint32_t)(it.rows * 32));
+                        dq_bulk(tc5_smem_u32(xs + rx.st * x_bytes), a.xsum + ((int64_t)(sb0 + sb) * a.m + it.m0) * 16, (uint32_t)(it.rows * 32), bar);
+                        rx.next(DQ_X_STAGES);
+                    }
+                }
+            }
+        } else if (warp == 0) {
+            const bool leader = tc5_elect();
+            // fp16 x fp16 -> f32; N is the tile height, twice that where both planes stand side by side
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(a.nb >> 3) << 17) | ((uint32_t)(DQ_BM >> 4) << 24), idesc_side = idesc + ((uint32_t)(a.nb >> 3) << 17);
+            const uint64_t bd0 = tc5_desc(tc5_smem_u32(smem));
+            DqRing ra, rb, rd;
+            bool seen = false;
+            for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+                const DqItem it(a, item);
+#define SP_DQ_ISSUE(TWO) \
+    ok = dq_issue<TWO, SIDE>(bars, tmem, bd0, (uint32_t)b_bytes >> 4, a.b_stages, idesc, idesc_side, n_sb, halves_last, leader, ra, rb, rd, seen, ok)
+                if (it.dt == T_Q4_K) SP_DQ_ISSUE(false);
+                else SP_DQ_ISSUE(true);
+#undef SP_DQ_ISSUE
+            }
+        }
+        __syncwarp();
+        if (a.parts > 1) { cluster_sync(); cluster_sync(); }
+    } else if (warp < DQ_FIRST_DRAIN) {
+        pdl_wait();
+        const int pw = warp - DQ_FIRST_PRODUCER, tile_w = 2 * (warp & 3) + (pw >> 2);
+        const uint32_t a_base = tmem + ((uint32_t)(16 * tile_w) << 16) + (uint32_t)DQ_A_COL;
+        DqRing rr, ra;
+        for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+            const int dt = DqItem(a, item).dt;
+#define SP_DQ_PRODUCE(T) ok = dq_produce<T>(bars, raw, a.r_bytes, a.r_stages, tile_w, lane, a_base, n_sb, halves_last, rr, ra, ok)
+            if (dt == T_Q4_K) SP_DQ_PRODUCE(T_Q4_K);
+            else if (dt == T_Q6_K) SP_DQ_PRODUCE(T_Q6_K);
+            else if (dt == T_Q8_0) SP_DQ_PRODUCE(T_Q8_0);
+            else SP_DQ_PRODUCE(T_Q8_0_HALF);
+#undef SP_DQ_PRODUCE
+        }
+        __syncwarp();
+        if (a.parts > 1) { cluster_sync(); cluster_sync(); }
+    } else {
+        if (NJT >= 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 128;\n");
+        pdl_wait();
+        const int quarter = warp & 3, half = (warp - DQ_FIRST_DRAIN) >> 2, g = lane >> 2, t = lane & 3;
+        DqRing rr, rx, rd;
+        for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+            const DqItem it(a, item);
+            const Tc5Seg& sg = a.seg[it.si];
+            float acc[2][NJT][4];
+#pragma unroll
+            for (int i = 0; i < 2 * NJT * 4; ++i) acc[i / (NJT * 4)][(i / 4) % NJT][i & 3] = 0.f;
+#define SP_DQ_DRAIN(T) \
+    ok = dq_drain<T, NJT>(bars, raw, a.r_bytes, a.r_stages, xs, x_bytes, a.nb, quarter, half, lane, tmem, n_sb, rr, rx, rd, acc, ok)
+            if (it.dt == T_Q4_K) SP_DQ_DRAIN(T_Q4_K);
+            else if (it.dt == T_Q6_K) SP_DQ_DRAIN(T_Q6_K);
+            else SP_DQ_DRAIN(T_Q8_0);
+#undef SP_DQ_DRAIN
+            const float* res = it.si == 0 ? a.res : nullptr;
+            if (a.parts == 1) {
+                if (ok) {
+#pragma unroll
+                    for (int j = 0; j < NJT; ++j)
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            const int ml = (half * NJT + j) * 8 + 2 * t + c, m = it.m0 + ml;
+                            if (ml >= it.rows) continue;
+                            const float sc = a.xscale[m];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const int n = it.n0 + 32 * quarter + 16 * (i >> 1) + 8 * (i & 1) + g;
+                                if (n >= sg.n) continue;
+                                float v = fmaf(acc[i >> 1][j][2 * (i & 1) + c], sc, sg.bias ? sg.bias[n] : 0.f);
+                                if (res) v += res[(int64_t)m * a.ldres + n];
+                                sg.y[(int64_t)m * a.ldy + n] = v;
+                            }
+                        }
+                }
+                continue;
+            }
+            // (a block of a cluster takes one tile)
+            asm volatile("bar.sync 1, 256;\n" ::: "memory");  // nobody reads raw tiles or sums any more: their memory takes the partial tile
+            float* const partial = reinterpret_cast<float*>(smem);
+#pragma unroll
+            for (int j = 0; j < NJT; ++j)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const int ml = (half * NJT + j) * 8 + 2 * t + c;
+                    if (ml >= it.rows) continue;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) partial[ml * DQ_P_STRIDE + 32 * quarter + 16 * (i >> 1) + 8 * (i & 1) + g] = acc[i >> 1][j][2 * (i & 1) + c];
+                }
+            __syncwarp();
+            cluster_sync();
+            // the cluster's blocks share out the activation rows; each adds its rows' partials in part order
+            const int idx = tid - 32 * DQ_FIRST_DRAIN, nl = idx & 127, n = it.n0 + nl;
+            if (n < sg.n) {
+                const float bias = sg.bias ? sg.bias[n] : 0.f;
+                const uint32_t mine = tc5_smem_u32(partial + nl);
+                constexpr int NC = 4;
+                for (int c0 = part + a.parts * (idx >> 7); c0 < it.rows; c0 += 2 * NC * a.parts) {
+                    float f[NC], r[NC], sc[NC];
+#pragma unroll
+                    for (int j = 0; j < NC; ++j) {
+                        const int c = c0 + 2 * j * a.parts;
+                        f[j] = 0.f;
+                        sc[j] = c < it.rows ? a.xscale[it.m0 + c] : 0.f;
+                        r[j] = res && c < it.rows ? res[(int64_t)(it.m0 + c) * a.ldres + n] : 0.f;
+                    }
+                    for (int p = 0; p < a.parts; ++p) {
+                        const uint32_t peer = peer_smem(mine, p);
+#pragma unroll
+                        for (int j = 0; j < NC; ++j) {
+                            const int c = c0 + 2 * j * a.parts;
+                            if (c < it.rows) f[j] += ld_peer(peer + (uint32_t)(c * DQ_P_STRIDE) * 4);
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < NC; ++j) {
+                        const int c = c0 + 2 * j * a.parts;
+                        if (c < it.rows) sg.y[(int64_t)(it.m0 + c) * a.ldy + n] = fmaf(f[j], sc[j], bias) + r[j];
+                    }
+                }
+            }
+            __syncwarp();
+            cluster_sync();  // nobody leaves while its partials are being read
+        }
+    }
+    if (!ok) atomicExch(&g_dq_timeout, 1);
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
+}
+
+// Reads and clears the flag that a bounded wait raises when it runs out; as tc5_take_timeout.
+static std::atomic<int> g_dq_launched[SP_MAX_DEVICES];
+int dq_take_timeout() {
+    if (g_dq_launched[current_device_index()].exchange(0) == 0) return 0;
+    int flag = 0;
+    if (cudaMemcpyFromSymbol(&flag, g_dq_timeout, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return -1; }
+    if (flag) {
+        const int zero = 0;
+        cudaMemcpyToSymbol(g_dq_timeout, &zero, sizeof(int));
+    }
+    return flag ? 1 : 0;
+}
+
+// How many clusters of `parts` blocks the device holds at once (a block fills an SM, and a cluster lies within one GPC).
+static int dq_clusters(int parts) {
+    static std::atomic<int> cache[SP_MAX_DEVICES][DQ_MAX_PARTS + 1];
+    std::atomic<int>& c = cache[current_device_index()][parts];
+    int n = c.load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    n = device_sm_count() / parts;
+    if (parts > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, 1, (unsigned)parts);
+        cfg.blockDim = dim3(DQ_THREADS);
+        cfg.dynamicSmemBytes = DQ_SMEM;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = (unsigned)parts;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int got = 0;
+        if (cudaOccupancyMaxActiveClusters(&got, gemm_dq_kernel<2>, &cfg) == cudaSuccess && got > 0) n = got;
+        else cudaGetLastError();
+    }
+    n = std::max(n, 1);
+    c.store(n, std::memory_order_relaxed);
+    return n;
+}
+
+cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& in, int m, int ldy, const float* res, int ldres, cudaStream_t st) {
+    if (m <= 0 || nseg <= 0) return cudaSuccess;
+    if (nseg > 3 || k % 128 != 0) return cudaErrorInvalidValue;
+    DqArgs a{};
+    int tiles = 0, tb = 0;
+    for (int i = 0; i < nseg; ++i) {
+        if (!tc5_supported(segs[i].dtype, k) || segs[i].n <= 0) return cudaErrorInvalidValue;
+        a.seg[i] = segs[i];
+        tiles += (segs[i].n + DQ_BM - 1) / DQ_BM;
+        tb = std::max(tb, dq_tile_bytes(segs[i].dtype));
+    }
+    a.nseg = nseg; a.k = k; a.m = m; a.ldy = ldy; a.res = res; a.ldres = ldres;
+    a.xscale = in.xscale; a.xsum = in.xsum;
+    a.m_tiles = (m + DQ_NB - 1) / DQ_NB;
+    a.nb = ((m + a.m_tiles - 1) / a.m_tiles + 15) & ~15;
+    a.m_tiles = (m + a.nb - 1) / a.nb;
+    // shared memory: at most half for activations (each box serves 64 columns), the rest for raw tiles
+    const int njt = a.nb <= 16 ? 1 : a.nb <= 32 ? 2 : a.nb <= 64 ? 4 : 8;
+    const int b_bytes = 4 * a.nb * 128, x_bytes = DQ_X_STAGES * a.nb * 32;
+    a.r_bytes = 8 * tb;
+    a.b_stages = std::min(DQ_MAX_B, 128 * 1024 / b_bytes);
+    a.r_stages = std::min(DQ_MAX_R, (DQ_SMEM - 1024 - a.b_stages * b_bytes - x_bytes) / a.r_bytes);
+    static PerDeviceOnce attr_once;
+    cudaError_t le = attr_once.run([] {
+        for (auto f : {gemm_dq_kernel<1>, gemm_dq_kernel<2>, gemm_dq_kernel<4>, gemm_dq_kernel<8>}) {
+            const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    });
+    if (le != cudaSuccess) return le;
+    // parts: what makes the longest SM's share shortest, a block's start and end counted as three spans of 256 columns
+    const int items = tiles * a.m_tiles, all_sb = (k + 255) / 256;
+    int best = 1;
+    long best_cost = 0;
+    for (int p = 1; p <= std::min(DQ_MAX_PARTS, all_sb); ++p) {
+        const long waves = (items + dq_clusters(p) - 1) / dq_clusters(p), sb = (all_sb + p - 1) / p;
+        const long cost = p == 1 ? waves * sb + 3 : waves * (sb + 3) + 1;  // (a lone block runs from tile to tile)
+        if (p == 1 || cost < best_cost) { best = p; best_cost = cost; }
+    }
+    a.parts = best;
+    a.items = items;
+    const PFN_encodeTiled encode = tensor_map_encoder();
+    if (!encode) return cudaErrorNotSupported;
+    CUtensorMap tmap;
+    {
+        const cuuint64_t gdim[2] = {(cuuint64_t)k, (cuuint64_t)(2 * m)};
+        const cuuint64_t gstride[1] = {(cuuint64_t)k * sizeof(__half)};
+        const cuuint32_t box[2] = {64u, (cuuint32_t)a.nb};
+        const cuuint32_t estr[2] = {1u, 1u};
+        if (encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, in.xh, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    g_dq_launched[current_device_index()].store(1);
+    const dim3 grid((unsigned)(a.parts == 1 ? std::min(items, device_sm_count()) : items), 1, (unsigned)a.parts), block(DQ_THREADS);
+    auto kernel = njt == 1 ? gemm_dq_kernel<1> : njt == 2 ? gemm_dq_kernel<2> : njt == 4 ? gemm_dq_kernel<4> : gemm_dq_kernel<8>;
+    le = launch_pdl_cluster(kernel, grid, block, DQ_SMEM, st, a.parts, a, tmap);
+    if (le != cudaSuccess) return le;
+    return count_launch_and_check();
+}
+
+}  // namespace sp

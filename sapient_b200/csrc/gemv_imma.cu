@@ -505,17 +505,25 @@ cudaError_t ActWorkspace::ensure_xh(size_t elems) {
     if (xh) cudaFree(xh);
     xh = nullptr;
     xscale = nullptr;
+    xsum = nullptr;
     xh_elems = 0;
     const size_t bytes = (elems * sizeof(__half) + 255) / 256 * 256;
-    cudaError_t e = cudaMalloc((void**)&xh, bytes + XSCALE_ROWS * sizeof(float));
-    if (e == cudaSuccess) { xh_elems = elems; xscale = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(xh) + bytes); }
+    // sums of 32 columns, leading part and remainder, of the elems / 2 activations that an exact-class step splits
+    cudaError_t e = cudaMalloc((void**)&xh, bytes + XSCALE_ROWS * sizeof(float) + elems / 32 * sizeof(__half));
+    if (e == cudaSuccess) {
+        xh_elems = elems;
+        xscale = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(xh) + bytes);
+        xsum = reinterpret_cast<__half*>(xscale + XSCALE_ROWS);
+    }
     if (e == cudaSuccess && !tc5.buf) e = tc5.alloc();
     return e;
 }
 
+DqInput ActWorkspace::dq() const { return DqInput{xh, xscale, xsum}; }
+
 void ActWorkspace::release() {
     if (xh) cudaFree(xh);
-    xh = nullptr; xh_elems = 0; xscale = nullptr;
+    xh = nullptr; xh_elems = 0; xscale = nullptr; xsum = nullptr;
     tc5.release();
     if (xq) cudaFree(xq);
     if (colscale) cudaFree(colscale);

@@ -139,23 +139,35 @@ __global__ void __launch_bounds__(MT_THREADS, 2) mat_tc5_kernel(const MatTc5Args
     float* const partial = reinterpret_cast<float*>(smem);  // [accumulator][bn columns][128], once the ring has drained
     bool ok = true;
     if (warp == 0) {
-        if (lane == 0 && live) {
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nb >> 3) << 17) | ((uint32_t)(MT_BM >> 4) << 24);  // bf16 x bf16 -> f32
-            for (int c = 0, st = 0, u = 0; c < n_chunks; ++c, ++st) {
-                if (st == a.stages) { st = 0; ++u; }
-                ok = ok && tc5_wait(&full[st], (uint32_t)(u & 1));
+        if (__all_sync(0xFFFFFFFFu, live)) {
+            const bool leader = tc5_elect();
+            const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0), un = (uint32_t)__shfl_sync(0xFFFFFFFFu, nb >> 3, 0);
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (un << 17) | ((uint32_t)(MT_BM >> 4) << 24);  // bf16 x bf16 -> f32
+            const uint64_t ad0 = tc5_desc(tc5_smem_u32(smem));
+            const uint32_t stage16 = (uint32_t)a.stage_bytes >> 4;
+            int st = 0;
+            uint32_t u = 0;
+            const int n = __shfl_sync(0xFFFFFFFFu, n_chunks, 0);
+            for (int c = 0; c < n; ++c) {
+                if (ok) ok = __all_sync(0xFFFFFFFFu, tc5_wait(&full[st], u & 1));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint32_t base = tc5_smem_u32(smem + (size_t)st * a.stage_bytes);
-                const uint64_t ad = tc5_desc(base), ad2 = tc5_desc(base + MT_A_BYTES), bd = tc5_desc(base + a_tiles * MT_A_BYTES);
+                // (the descriptors' address field: no carry out of the low word)
+                const uint64_t ad = ad0 + (uint64_t)((uint32_t)st * stage16), ad2 = ad + (MT_A_BYTES >> 4), bd = ad + a_tiles * (MT_A_BYTES >> 4);
+                if (leader) {
 #pragma unroll
-                for (int i = 0; i < MT_BK / 16; ++i) {  // 16 columns: 32 bytes inside the swizzle row
-                    tc5_mma(tmem, ad + 2u * i, bd + 2u * i, idesc, (uint32_t)(c > 0 || i > 0));
-                    if (DUAL) tc5_mma(tmem + (uint32_t)a.bn, ad2 + 2u * i, bd + 2u * i, idesc, (uint32_t)(c > 0 || i > 0));
+                    for (int i = 0; i < MT_BK / 16; ++i) {  // 16 columns: 32 bytes inside the swizzle row
+                        const uint32_t more = i > 0 ? 1u : (uint32_t)(c > 0);
+                        tc5_mma(tm, ad + 2u * i, bd + 2u * i, idesc, more);
+                        if (DUAL) tc5_mma(tm + (uint32_t)a.bn, ad2 + 2u * i, bd + 2u * i, idesc, more);
+                    }
+                    tc5_commit(&empty[st]);
+                    if (c == n - 1) tc5_commit(&done_bar);
                 }
-                tc5_commit(&empty[st]);
+                __syncwarp();
+                if (++st == a.stages) { st = 0; ++u; }
             }
-            if (ok) tc5_commit(&done_bar);
+            if (n == 0 && leader) tc5_commit(&done_bar);  // (a short K may leave a part without chunks)
         }
     } else if (warp == 1) {
         if (lane == 0 && live) {

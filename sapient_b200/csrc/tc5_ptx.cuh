@@ -7,7 +7,8 @@
 
 namespace sp {
 
-constexpr int TC5_SPIN_LIMIT = 1 << 22;
+constexpr uint32_t TC5_WAIT_HINT_NS = 10000;
+constexpr uint32_t TC5_WAIT_LIMIT_MS = 2000;
 
 __device__ __forceinline__ uint32_t tc5_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -20,6 +21,20 @@ __device__ __forceinline__ uint64_t tc5_desc(uint32_t saddr) {
     d |= (uint64_t)1 << 46;                    // descriptor version of this architecture
     d |= (uint64_t)2 << 61;                    // 128-byte swizzle
     return d;
+}
+
+// One thread of the (converged) warp. Tensor instructions take their operands from uniform registers: a loop that the whole warp
+// walks, with this thread issuing, keeps them there; issued by a lone thread of a divergent branch an MMA took about 95 cycles.
+__device__ __forceinline__ bool tc5_elect() {
+    uint32_t one;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xFFFFFFFF;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(one));
+    return one != 0;
 }
 
 __device__ __forceinline__ void tc5_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -40,22 +55,50 @@ __device__ __forceinline__ void tc5_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc5_smem_u32(bar)) : "memory");
 }
 
-__device__ __forceinline__ bool tc5_wait(uint64_t* bar, uint32_t parity) {
-    const uint32_t a = tc5_smem_u32(bar);
-    for (int i = 0; i < TC5_SPIN_LIMIT; ++i) {
+// Whether a phase of `bar` is over, without waiting for it.
+__device__ __forceinline__ bool tc5_peek(uint64_t* bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(done)
+        : "r"(tc5_smem_u32(bar)), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
+__device__ __forceinline__ bool tc5_wait_long(uint32_t bar, uint32_t parity) {
+    // (the clock is looked at only once in 64 polls, in units of about a millisecond: one register)
+    uint32_t t0 = 0;
+    for (uint32_t i = 0;; ++i) {
         uint32_t done;
         asm volatile(
             "{\n"
             ".reg .pred p;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
             "selp.u32 %0, 1, 0, p;\n"
             "}\n"
             : "=r"(done)
-            : "r"(a), "r"(parity)
+            : "r"(bar), "r"(parity), "r"(TC5_WAIT_HINT_NS)
             : "memory");
         if (done) return true;
+        if ((i & 63u) == 63u) {
+            uint64_t now;
+            asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(now));
+            const uint32_t ms = (uint32_t)(now >> 20);
+            if (i == 63u) t0 = ms;
+            else if (ms - t0 > TC5_WAIT_LIMIT_MS) return false;
+        }
     }
-    return false;
+}
+
+// Waits for a phase of `bar`; one that is over already costs a look. The time hint lets the hardware keep the thread suspended.
+// Bounded by the global timer; false: it ran out.
+__device__ __forceinline__ bool tc5_wait(uint64_t* bar, uint32_t parity) {
+    return tc5_peek(bar, parity) || tc5_wait_long(tc5_smem_u32(bar), parity);
 }
 
 // A box of a 2-D tensor map into shared memory, counted in bytes on `bar`. x (elements) must start on 16 bytes.

@@ -129,3 +129,38 @@ def test_split_last_wave_is_reproducible_bit_for_bit(oracle, dtype, m, k, n):
     for r in runs[1:]:
         assert np.array_equal(r.view(np.uint32), runs[0].view(np.uint32))
     assert rel_l2(runs[0], oracle.matmul_nt(x, raw, dtype, n)) < 5e-4
+
+
+# edges of gemm_dq_kernel: its variants by tile height (16, 32, 64, 128 rows, the first step over each), one row tile more than fits, K
+# of one tile and of an odd number, fewer weight rows than a 16-row tile, more tiles than SMs (a block runs from one into the
+# next, the last ones short), K shared by a cluster, Q8_0 widths that are odd multiples of 128
+DQ_EDGES = [(17, 256, 7), (32, 768, 129), (33, 1280, 40), (64, 2304, 256), (65, 512, 300), (128, 256, 128), (129, 768, 136), (257, 256, 130), (40, 256, 19205),
+            (130, 512, 10250)]
+
+
+@pytest.mark.parametrize("dtype,m,k,n", [(d, *c) for d in (Q4_K, Q6_K, Q8_0) for c in DQ_EDGES] + [(Q8_0, 17, 128, 16), (Q8_0, 100, 384, 130), (Q8_0, 34, 896, 4864), (Q8_0, 200, 1152, 272)])
+def test_exact_operands_at_the_edges_of_tiles(dtype, m, k, n):
+    """Against the dequantised weights in float64. Operands keep 22 bits (2^-22 each), a sum leaves the tensor core after 256
+    columns, that is after at most 48 truncated additions of 2^-24: 4e-6 of a row's norm, twice that where Q4_K's minimum term
+    cancels most of the product."""
+    import torch
+
+    be, _ = synth.BLOCK[dtype]
+    w = ops.Weight(dtype, n, k, synth.random_bit_blocks(dtype, n * k // be, seed=m + n + dtype))
+    W = torch.from_numpy(w.dequant()).cuda().double()
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(m + k)).cuda()
+    x[2] *= 1e-30
+    x[3] = 0.0
+    y = torch.full((m, n), 7.0, device="cuda")
+    _large_m(2)
+    try:
+        w.matmul_nt_dev(x.data_ptr(), m, y.data_ptr())
+        _lib.check(_lib.lib().sp_cuda_check_kernels(0))
+    finally:
+        _large_m(1)
+        w.free()
+    want = x.double() @ W.T
+    rows = [i for i in range(m) if i != 3]
+    err = (y.double() - want)[rows].norm(dim=1) / want[rows].norm(dim=1)
+    assert torch.all(y[3] == 0.0)
+    assert float(err.max()) < 8e-6, float(err.max())

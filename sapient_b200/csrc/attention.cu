@@ -224,9 +224,13 @@ cudaError_t launch_attention(const float* q, int ldq, float* out, int ldo, int n
 // ───────────────────────────── prefill: tiled attention on tensor cores ─────────────────────────────
 // Many query tokens of ONE sequence with consecutive positions (a prefill chunk). The split kernel above re-reads the
 // whole key range once per query token; here a block takes 64 query rows of one head (4 warps x 16 rows), walks the keys
-// in tiles of 64 (4 pages) staged in shared memory, and does both contractions with mma.sync.m16n8k16 (fp16 operands —
-// K and V are fp16 in the cache already, q and the softmax weights are rounded to fp16 — f32 accumulation), with the
-// reference's online-softmax recurrence (kernels/attention.rs:98-165) applied per 64-key tile.
+// in tiles of 64 (4 pages) staged in shared memory, and does both contractions with mma.sync.m16n8k16 (K and V are fp16 in the
+// cache already, f32 accumulation), with the reference's online-softmax recurrence (kernels/attention.rs:98-165) applied per
+// 64-key tile. EXACT (engines with exact-class operands): q, scaled per row by a power of two into (-1, 1), and the softmax
+// weights each enter as an fp16 leading part plus remainder, two products each, so the result is that of the f32 kernels to
+// 2^-22 per operand; otherwise both are rounded to fp16.
+// Per query token the kernels above read every key again: 389 tokens of the Phi-2 shape (32 heads, none shared) took 325 us a
+// layer on the f32 kernel, 512 of the 8B shape 91 us on the grouped one; tiles of 64 rows take 31 and 42 us.
 namespace sp {
 
 constexpr int FA_ROWS = 64, FA_KEYS = 64, FA_WARPS = 4;
@@ -242,7 +246,7 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
 }
 
 // HD16 = head_dim / 16 (head_dim a multiple of 16, <= 128).
-template <int HD16>
+template <int HD16, bool EXACT>
 __global__ void __launch_bounds__(FA_WARPS * 32)
 attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict__ out, __half* __restrict__ out_h, int ldo, int n_tok,
                          int n_heads, int slot, int pos0, KvGeom kv, int layer, float scale) {
@@ -252,7 +256,7 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
     constexpr int TILE = FA_KEYS * LD;
     pdl_wait();
     pdl_trigger();
-    const int h = blockIdx.x, t0 = blockIdx.y * FA_ROWS;
+    const int h = blockIdx.x, t0 = (gridDim.y - 1 - blockIdx.y) * FA_ROWS;  // tiles with the longest key ranges first
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int kv_h = h / (n_heads / kv.n_kv);
     const int32_t* pt = kv.page_table + (int64_t)slot * kv.max_pages;
@@ -260,16 +264,41 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
     const int r0 = t0 + warp * 16 + g, r1 = r0 + 8;
     const int q0 = min(r0, n_tok - 1), q1 = min(r1, n_tok - 1);
     const int p0 = pos0 + q0, p1 = pos0 + q1;
-    uint32_t qa[HD16][4];
+    uint32_t qa[HD16][4], ql[EXACT ? HD16 : 1][4];
+    float sc0 = 1.f, sc1 = 1.f;  // EXACT: what a row's scores are multiplied by
     {
         const float* a = q + (int64_t)q0 * ldq + (int64_t)h * HD;
         const float* b = q + (int64_t)q1 * ldq + (int64_t)h * HD;
+        float u0 = scale, u1 = scale;
+        if (EXACT) {
+            float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+            for (int kd = 0; kd < 2 * HD16; ++kd) {
+                const float2 x0 = *reinterpret_cast<const float2*>(a + 8 * kd + 2 * t), x1 = *reinterpret_cast<const float2*>(b + 8 * kd + 2 * t);
+                a0 = fmaxf(a0, fmaxf(fabsf(x0.x), fabsf(x0.y)));
+                a1 = fmaxf(a1, fmaxf(fabsf(x1.x), fabsf(x1.y)));
+            }
+            auto unit = [&](float amax, float& up, float& down) {  // power of two that brings the row into (-1, 1), and scale times its inverse
+                amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+                amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+                const int e = amax > 0.f && amax < INFINITY ? max(-100, min(100, ilogbf(amax) + 1)) : 0;
+                up = scalbnf(1.0f, -e);
+                down = scalbnf(scale, e);
+            };
+            unit(a0, u0, sc0);
+            unit(a1, u1, sc1);
+        }
 #pragma unroll
         for (int kd = 0; kd < HD16; ++kd) {
-            const float2 x0 = *reinterpret_cast<const float2*>(a + 16 * kd + 2 * t), x1 = *reinterpret_cast<const float2*>(b + 16 * kd + 2 * t);
-            const float2 x2 = *reinterpret_cast<const float2*>(a + 16 * kd + 8 + 2 * t), x3 = *reinterpret_cast<const float2*>(b + 16 * kd + 8 + 2 * t);
-            qa[kd][0] = pack_half2(x0.x * scale, x0.y * scale); qa[kd][1] = pack_half2(x1.x * scale, x1.y * scale);
-            qa[kd][2] = pack_half2(x2.x * scale, x2.y * scale); qa[kd][3] = pack_half2(x3.x * scale, x3.y * scale);
+            float2 x[4] = {*reinterpret_cast<const float2*>(a + 16 * kd + 2 * t), *reinterpret_cast<const float2*>(b + 16 * kd + 2 * t),
+                           *reinterpret_cast<const float2*>(a + 16 * kd + 8 + 2 * t), *reinterpret_cast<const float2*>(b + 16 * kd + 8 + 2 * t)};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float u = (i & 1) ? u1 : u0;
+                const __half2 hi = __floats2half2_rn(x[i].x * u, x[i].y * u);
+                qa[kd][i] = *reinterpret_cast<const uint32_t*>(&hi);
+                if (EXACT) ql[EXACT ? kd : 0][i] = pack_half2(x[i].x * u - __low2float(hi), x[i].y * u - __high2float(hi));
+            }
         }
     }
     float o[2 * HD16][4];
@@ -315,8 +344,10 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
             for (int kd = 0; kd < HD16; ++kd) {
                 const uint32_t b0 = *reinterpret_cast<const uint32_t*>(Ks + (8 * j + g) * LD + 16 * kd + 2 * t);
                 const uint32_t b1 = *reinterpret_cast<const uint32_t*>(Ks + (8 * j + g) * LD + 16 * kd + 8 + 2 * t);
+                if (EXACT) mma_f16(s[j], ql[EXACT ? kd : 0][0], ql[EXACT ? kd : 0][1], ql[EXACT ? kd : 0][2], ql[EXACT ? kd : 0][3], b0, b1);
                 mma_f16(s[j], qa[kd][0], qa[kd][1], qa[kd][2], qa[kd][3], b0, b1);
             }
+            if (EXACT) { s[j][0] *= sc0; s[j][1] *= sc0; s[j][2] *= sc1; s[j][3] *= sc1; }
         }
         // causal mask and the tile's row maxima (row g: s[j][0..1], row g+8: s[j][2..3]; keys 8j + 2t, +1)
         float mx0 = -INFINITY, mx1 = -INFINITY;
@@ -337,15 +368,20 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
         // after the first tile every maximum is finite
         const float c0 = (n0 == -INFINITY) ? 1.f : expf(m0 - n0), c1 = (n1 == -INFINITY) ? 1.f : expf(m1 - n1);
         float sum0 = 0.f, sum1 = 0.f;
-        uint32_t pa[4][4];  // softmax weights as fp16 A fragments: k-step kk covers keys 16 kk .. + 15
+        uint32_t pa[4][4], pl[EXACT ? 4 : 1][4];  // softmax weights as fp16 A fragments: k-step kk covers keys 16 kk .. + 15
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const float e0 = (s[j][0] == -INFINITY) ? 0.f : expf(s[j][0] - n0), e1 = (s[j][1] == -INFINITY) ? 0.f : expf(s[j][1] - n0);
             const float e2 = (s[j][2] == -INFINITY) ? 0.f : expf(s[j][2] - n1), e3 = (s[j][3] == -INFINITY) ? 0.f : expf(s[j][3] - n1);
             sum0 += e0 + e1;
             sum1 += e2 + e3;
-            pa[j >> 1][(j & 1) * 2] = pack_half2(e0, e1);
-            pa[j >> 1][(j & 1) * 2 + 1] = pack_half2(e2, e3);
+            const __half2 w0 = __floats2half2_rn(e0, e1), w1 = __floats2half2_rn(e2, e3);
+            pa[j >> 1][(j & 1) * 2] = *reinterpret_cast<const uint32_t*>(&w0);
+            pa[j >> 1][(j & 1) * 2 + 1] = *reinterpret_cast<const uint32_t*>(&w1);
+            if (EXACT) {
+                pl[EXACT ? j >> 1 : 0][(j & 1) * 2] = pack_half2(e0 - __low2float(w0), e1 - __high2float(w0));
+                pl[EXACT ? j >> 1 : 0][(j & 1) * 2 + 1] = pack_half2(e2 - __low2float(w1), e3 - __high2float(w1));
+            }
         }
         sum0 += __shfl_xor_sync(0xFFFFFFFFu, sum0, 1); sum0 += __shfl_xor_sync(0xFFFFFFFFu, sum0, 2);
         sum1 += __shfl_xor_sync(0xFFFFFFFFu, sum1, 1); sum1 += __shfl_xor_sync(0xFFFFFFFFu, sum1, 2);
@@ -364,6 +400,11 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
                 asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                              : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3)
                              : "r"(addr));
+                if (EXACT) {
+                    uint32_t* const w = pl[EXACT ? kk : 0];
+                    mma_f16(o[nd], w[0], w[1], w[2], w[3], b0, b1);
+                    mma_f16(o[nd + 1], w[0], w[1], w[2], w[3], b2, b3);
+                }
                 mma_f16(o[nd], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b0, b1);
                 mma_f16(o[nd + 1], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b2, b3);
             }
@@ -574,28 +615,37 @@ cudaError_t launch_gqa_mma_phase(const float* q, int ldq, float* out, int ldo, i
     return le;
 }
 
+// A tile walks its keys alone, whatever the number of its rows; with a token per block the same keys are shared out to
+// (token, cached head) pairs -- (token, query head) where no kernel shares cached rows -- of which the device holds some 450.
+// Measured per layer: 512 tokens x 8 cached heads 91 us against 42, 389 x 32 325 against 31, but 181 x 2 17 against 17.
+bool attention_takes_tiles(int n_tok, int n_heads, int n_kv, int head_dim) {
+    return n_tok >= 16 && n_tok * (attention_gqa_mma_supported(n_heads, n_kv, head_dim) ? n_kv : n_heads) >= 600;
+}
+
 bool attention_prefill_supported(int head_dim) { return head_dim % 16 == 0 && head_dim >= 16 && head_dim <= 128; }
 
 // All n_tok tokens belong to sequence `slot` at positions pos0, pos0 + 1, ... (their keys are in the cache already).
-// out_h != null: the rows go out as fp16 to out_h (same row stride) instead of f32 to out.
+// out_h != null: the rows go out as fp16 to out_h (same row stride) instead of f32 to out. exact: operands as leading part and remainder.
 cudaError_t launch_attention_prefill(const float* q, int ldq, float* out, int ldo, int n_tok, int n_heads, int slot, int pos0, KvGeom kv,
-                                     int layer, float scale, cudaStream_t st, __half* out_h) {
+                                     int layer, float scale, cudaStream_t st, __half* out_h, bool exact) {
     if (n_tok <= 0) return cudaSuccess;
     if (!attention_prefill_supported(kv.head_dim)) return cudaErrorInvalidValue;
     const int hd16 = kv.head_dim / 16;
     const size_t smem = (size_t)4 * FA_KEYS * (kv.head_dim + 8) * sizeof(__half);  // two (K, V) tile buffers
     const dim3 grid(n_heads, (n_tok + FA_ROWS - 1) / FA_ROWS), block(FA_WARPS * 32);
     cudaError_t le = cudaErrorInvalidValue;
-#define SP_FA(N)                                                                                                        \
-    if (hd16 == N) {                                                                                                    \
+#define SP_FA(N, EX)                                                                                                    \
+    if (hd16 == N && exact == EX) {                                                                                     \
         static PerDeviceOnce big_smem;                                                                                  \
         if (smem > 48 * 1024) {                                                                                         \
-            le = big_smem.run([] { return cudaFuncSetAttribute(attention_prefill_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024); }); \
+            le = big_smem.run([] { return cudaFuncSetAttribute(attention_prefill_kernel<N, EX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024); }); \
             if (le != cudaSuccess) return le;                                                                           \
         }                                                                                                               \
-    }                                                                                                                   \
-    if (hd16 == N) le = launch_pdl(attention_prefill_kernel<N>, grid, block, smem, st, q, ldq, out, out_h, ldo, n_tok, n_heads, slot, pos0, kv, layer, scale)
-    SP_FA(1); SP_FA(2); SP_FA(3); SP_FA(4); SP_FA(5); SP_FA(6); SP_FA(7); SP_FA(8);
+        le = launch_pdl(attention_prefill_kernel<N, EX>, grid, block, smem, st, q, ldq, out, out_h, ldo, n_tok, n_heads, slot, pos0, kv, layer, scale); \
+    }
+#define SP_FA2(N) SP_FA(N, false) SP_FA(N, true)
+    SP_FA2(1) SP_FA2(2) SP_FA2(3) SP_FA2(4) SP_FA2(5) SP_FA2(6) SP_FA2(7) SP_FA2(8)
+#undef SP_FA2
 #undef SP_FA
     if (le != cudaSuccess) return le;
     return count_launch_and_check();

@@ -260,6 +260,15 @@ int Engine::step_splits(int T) const {
     return splits;
 }
 
+// Attention of the n staged tokens from t0 on, a token per block.
+int Engine::attention_tokens(int t0, int n, int l, int splits) {
+    if (n <= 0) return SP_OK;
+    const int H = d.n_heads, hd = d.head_dim, qkv_ld = (H + 2 * d.n_kv_heads) * hd;
+    SP_LAUNCH(F_ATTN, launch_attention(qkv_ + (size_t)t0 * qkv_ld, qkv_ld, attn_ + (size_t)t0 * H * hd, H * hd, n, H, d_tok_slot_ + t0, d_tok_pos_ + t0, kv_, l,
+                                       1.0f / sqrtf((float)hd), splits, att_scratch_, stream, step_ctx_));
+    return SP_OK;
+}
+
 // Attention of the T staged tokens, then the output projection added into x_ (x += W_o attn (+ b_o)).
 int Engine::attention_and_oproj(const LayerW& w, int l, int T) {
     const int H = d.n_heads, Hkv = d.n_kv_heads, hd = d.head_dim, hid = d.hidden;
@@ -296,8 +305,20 @@ int Engine::attention_and_oproj(const LayerW& w, int l, int T) {
         SP_LAUNCH(F_ATTN, launch_attention_prefill(qkv_, qkv_ld, attn_, H * hd, T, H, p_slot_[0], p_pos_[0], kv_, l, scale, stream));
         return gemv(attn_, H * hd, T, H * hd, w.o, w.ob, x_, hid, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, x_, nullptr, true);
     }
-    SP_LAUNCH(F_ATTN, launch_attention(qkv_, qkv_ld, attn_, H * hd, T, H, d_tok_slot_, d_tok_pos_, kv_, l, scale, splits, att_scratch_,
-                                       stream, step_ctx_));
+    // Exact-class operands: portions of prompts (runs of consecutive positions of one sequence) on the tiled kernel, the tokens
+    // between them on the kernels that take a token per block.
+    int done = 0;
+    if (tc5_exact && use_tc5 && !graph_step_ && attention_prefill_supported(hd)) {
+        for (int i0 = 0, i1; i0 < T; i0 = i1) {
+            for (i1 = i0 + 1; i1 < T && p_slot_[i1] == p_slot_[i0] && p_pos_[i1] == p_pos_[i1 - 1] + 1;) ++i1;
+            if (!attention_takes_tiles(i1 - i0, H, Hkv, hd)) continue;
+            SP_TRY(attention_tokens(done, i0 - done, l, splits));
+            SP_LAUNCH(F_ATTN, launch_attention_prefill(qkv_ + (size_t)i0 * qkv_ld, qkv_ld, attn_ + (size_t)i0 * H * hd, H * hd, i1 - i0, H, p_slot_[i0], p_pos_[i0],
+                                                       kv_, l, scale, stream, nullptr, true));
+            done = i1;
+        }
+    }
+    SP_TRY(attention_tokens(done, T - done, l, splits));
     return gemv(attn_, H * hd, T, H * hd, w.o, w.ob, x_, hid, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, x_, nullptr, true);
 }
 

@@ -49,3 +49,34 @@ def test_replayed_step_graphs_do_not_freeze_positions():
         e.set_kv_rounding(False)
     assert np.abs(graphs.forward_all_logits(first) - direct.forward_all_logits(first)).max() < 2e-3
     assert np.abs(graphs.forward_all_logits_cached(second) - direct.forward_all_logits_cached(second)).max() < 2e-3
+
+
+@pytest.mark.parametrize("name,n_prompt", [("tiny_phi2_wide", 75), ("tiny_phi2_wide", 129), ("tiny_phi2_wide", 191), ("tiny_llama", 300), ("tiny_llama", 321)])
+def test_tiled_attention_with_exact_operands(oracle, name, n_prompt):
+    """Engines with exact-class operands: a prompt in one chunk (tiled kernel with leading parts and remainders) against chunks of 32
+    (the f32 and grouped kernels), a second portion at a position that starts no tile, and a mixed step in which decoded tokens
+    stand before and after a prompt's portion. The two differ by f32 sums and the remainders' 2^-22, and where such a difference
+    crosses an edge of the cache's fp16 rounding a key or value moves by 2^-11 of itself: one in some thousand does, of 64 or more
+    that a score adds up, which leaves 1e-4 of logits near 1."""
+    cfg, W = tiny_model(name, max_ctx=1024)
+    rng = np.random.default_rng(n_prompt)
+    ids, more = (rng.integers(0, cfg["vocab"], n).astype(np.uint32) for n in (n_prompt, 163))
+    big = ForwardEngine.from_weights(cfg, W, max_tokens=512, max_batch=3)
+    small = ForwardEngine.from_weights(cfg, W, max_tokens=32, max_batch=3)
+    for e in (big, small):
+        e.set_kv_rounding(False)  # continuous cache rounding: this test is about the kernels
+    tol = 1e-4
+    a, b = big.forward_slot(1, ids), small.forward_slot(1, ids)
+    assert np.abs(a - b).max() < tol, np.abs(a - b).max()
+    more = np.concatenate([more, ids])
+    a, b = big.forward_slot(1, more), small.forward_slot(1, more)
+    assert np.abs(a - b).max() < tol, np.abs(a - b).max()
+    for e in (big, small):
+        e.forward_slot(0, ids[:9])
+    step = [(0, [5], [0]), (2, ids, [n_prompt - 1]), (1, [7], [0])]
+    a, b = big.forward_mixed(step), small.forward_mixed(step)
+    assert np.abs(a - b).max() < tol, np.abs(a - b).max()
+    ref = oracle_engine(oracle, cfg, W, kv_mode=1).forward_logits(ids, False)
+    assert np.abs(a[1] - ref).max() < 3e-3
+    big.close()
+    small.close()

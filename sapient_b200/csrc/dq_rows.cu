@@ -5,7 +5,8 @@
 //
 // What produces the row is part of the kernel: a norm, SwiGLU or GELU. One block per row keeps it in registers from the first
 // read to the store, so a norm reads and writes 8 bytes per value (it took two launches and 24: norm to f32, maximum, split),
-// SwiGLU 12 (28). 512 rows of the 8B shape: 26 + 22 us a layer for the norms and 31 for SwiGLU before, 9 + 9 and 14 now.
+// SwiGLU 12 (28). Norms, activations and splits of 16 layers of the 8B shape: 512 rows 1.89 ms in 114 launches before, 0.92 in
+// 66 now; 32 rows 0.47 and 0.22.
 #include <cuda_fp16.h>
 
 #include <algorithm>

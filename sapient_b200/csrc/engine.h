@@ -189,6 +189,8 @@ class Engine {
                 float* y2 = nullptr, const float* res = nullptr);
     // The same for a column-split matrix (o_proj, down_proj) whose product is added into the residual stream x_: on one
     // GPU in place; under tensor parallelism the partial product goes to scratch and is pushed to every rank.
+    cudaError_t norm_xh(int m, const float* w, const float* b);  // the block's norm of x_ into the input buffer
+    cudaError_t act_xh(int m);                                  // the activation of gu_ into it
     int gemm_xh_sum(int m, int k, const DevTensor* w, const float* b);
     size_t tp_block_bytes() const;
     int tp_alloc();

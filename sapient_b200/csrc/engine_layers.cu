@@ -198,7 +198,8 @@ int Engine::try_ring(bool* done, int m, int k, int src, const float* x, int ldx,
 }
 
 bool Engine::big_m(int m, int k, const DevTensor* w0, const DevTensor* w1, const DevTensor* w2) const {
-    if (m < TC5_MIN_M || !use_tc5 || tc5_exact || !ws_.xh || (size_t)m * k > ws_.xh_elems) return false;
+    if (m < TC5_MIN_M || !use_tc5 || !ws_.xh || (size_t)m * k * (tc5_exact ? 2 : 1) > ws_.xh_elems) return false;
+    if (tc5_exact && (m > ActWorkspace::XSCALE_ROWS || !dq_rows_fit(k))) return false;
     const DevTensor* ws[3] = {w0, w1, w2};
     for (int i = 0; i < 3 && ws[i]; ++i)
         if (!ws[i]->tiled || !tc5_supported(ws[i]->dtype, k)) return false;
@@ -213,8 +214,20 @@ int Engine::gemm_xh(int m, int k, const DevTensor* w0, const float* b0, float* y
     Tc5Seg segs[3];
     int ns = 0;
     for (int i = 0; i < 3 && ws[i]; ++i) segs[ns++] = Tc5Seg{ws[i]->tiled, ys[i], bs[i], ws[i]->dtype, (int)ws[i]->dims[0]};
-    SP_LAUNCH(F_GEMV, launch_gemm_tc5_multi(segs, ns, k, ws_.xh, m, ldy0, res, ldy0, stream, &ws_.tc5));
+    if (tc5_exact) SP_LAUNCH(F_GEMV, launch_gemm_dq(segs, ns, k, ws_.dq(), m, ldy0, res, ldy0, stream));
+    else SP_LAUNCH(F_GEMV, launch_gemm_tc5_multi(segs, ns, k, ws_.xh, m, ldy0, res, ldy0, stream, &ws_.tc5));
     return SP_OK;
+}
+
+cudaError_t Engine::norm_xh(int m, const float* w, const float* b) {
+    const int hid = d.hidden;
+    if (tc5_exact) return launch_dq_rows(d.arch == 1 ? DQ_LN : DQ_RMS, x_, hid, w, b, d.norm_eps, m, hid, ws_.dq(), stream);
+    return d.arch == 1 ? launch_layer_norm_f16(x_, w, b, m, hid, d.norm_eps, ws_.xh, stream) : launch_rms_norm_f16(x_, w, m, hid, d.norm_eps, ws_.xh, stream);
+}
+
+cudaError_t Engine::act_xh(int m) {
+    if (tc5_exact) return launch_dq_rows(d.arch == 1 ? DQ_GELU : DQ_SWIGLU, gu_, d.arch == 1 ? d.ffn : 2 * d.ffn, nullptr, nullptr, 0.f, m, d.ffn, ws_.dq(), stream);
+    return d.arch == 1 ? launch_act_f16(gu_, d.ffn, d.ffn, m, 1, ws_.xh, stream) : launch_act_f16(gu_, 2 * d.ffn, d.ffn, m, 0, ws_.xh, stream);
 }
 
 int Engine::gemm_xh_sum(int m, int k, const DevTensor* w, const float* b) {
@@ -332,7 +345,7 @@ int Engine::layer_llama(const LayerW& w, int l, int T) {
     if (ringed) {
     } else if (big_m(T, hid, w.q, w.k, w.v)) {
         SP_TRY(tp_resolve(T));
-        SP_LAUNCH(F_NORM, launch_rms_norm_f16(x_, w.n1w, T, hid, d.norm_eps, ws_.xh, stream));
+        SP_LAUNCH(F_NORM, norm_xh(T, w.n1w, nullptr));
         SP_TRY(gemm_xh(T, hid, w.q, w.qb, qkv_, qkv_ld, w.k, w.kb, qkv_ + (size_t)H * hd, w.v, w.vb, qkv_ + (size_t)(H + Hkv) * hd));
     } else if (all_tiled(w.q, w.k, w.v) && plan_digits(T, hid, ia)) {
         SP_LAUNCH(F_NORM, launch_norm_quant(x_, hid, w.n1w, nullptr, false, d.norm_eps, nullptr, 0, ia, stream, tp_take()));
@@ -350,7 +363,7 @@ int Engine::layer_llama(const LayerW& w, int l, int T) {
     if (ringed) {
     } else if (big_m(T, hid, w.gate, w.up)) {
         SP_TRY(tp_resolve(T));
-        SP_LAUNCH(F_NORM, launch_rms_norm_f16(x_, w.n2w, T, hid, d.norm_eps, ws_.xh, stream));
+        SP_LAUNCH(F_NORM, norm_xh(T, w.n2w, nullptr));
         SP_TRY(gemm_xh(T, hid, w.gate, nullptr, gu_, 2 * ffn, w.up, nullptr, gu_ + ffn));
     } else if (all_tiled(w.gate, w.up) && plan_digits(T, hid, ia)) {
         SP_LAUNCH(F_NORM, launch_norm_quant(x_, hid, w.n2w, nullptr, false, d.norm_eps, nullptr, 0, ia, stream, tp_take()));
@@ -364,7 +377,7 @@ int Engine::layer_llama(const LayerW& w, int l, int T) {
                     nullptr, x_));
     if (ringed) {
     } else if (big_m(T, ffn, w.down)) {
-        SP_LAUNCH(F_ELEM, launch_act_f16(gu_, 2 * ffn, ffn, T, 0, ws_.xh, stream));
+        SP_LAUNCH(F_ELEM, act_xh(T));
         SP_TRY(gemm_xh_sum(T, ffn, w.down, nullptr));
     } else if (all_tiled(w.down) && plan_digits(T, ffn, ia)) {
         SP_LAUNCH(F_ELEM, launch_act_fn_quant(gu_, 2 * ffn, ffn, 0, ia, stream));
@@ -392,7 +405,7 @@ int Engine::layer_phi(const LayerW& w, int l, int T) {
     }
     if (ringed) {
     } else if (big_m(T, hid, w.q, w.k, w.v) && big_m(T, hid, w.up)) {
-        SP_LAUNCH(F_NORM, launch_layer_norm_f16(x_, w.n1w, w.n1b, T, hid, d.norm_eps, ws_.xh, stream));
+        SP_LAUNCH(F_NORM, norm_xh(T, w.n1w, w.n1b));
         SP_TRY(gemm_xh(T, hid, w.q, w.qb, qkv_, qkv_ld, w.k, w.kb, qkv_ + (size_t)H * hd, w.v, w.vb, qkv_ + (size_t)(H + Hkv) * hd));
         SP_TRY(gemm_xh(T, hid, w.up, w.upb, gu_, ffn));
     } else if (all_tiled(w.q, w.k, w.v) && all_tiled(w.up) && plan_digits(T, hid, ia)) {
@@ -413,7 +426,7 @@ int Engine::layer_phi(const LayerW& w, int l, int T) {
                     nullptr, x_));
     if (ringed) {
     } else if (big_m(T, ffn, w.down)) {
-        SP_LAUNCH(F_ELEM, launch_act_f16(gu_, ffn, ffn, T, 1, ws_.xh, stream));
+        SP_LAUNCH(F_ELEM, act_xh(T));
         SP_TRY(gemm_xh(T, ffn, w.down, w.downb, x_, hid, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, x_));
     } else if (all_tiled(w.down) && plan_digits(T, ffn, ia)) {
         SP_LAUNCH(F_ELEM, launch_act_fn_quant(gu_, ffn, ffn, 1, ia, stream));

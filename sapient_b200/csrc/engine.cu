@@ -100,6 +100,8 @@ Engine::~Engine() {
     void* bufs[] = {kv_.pool, d_page_table_, x_, h_, qkv_, attn_, gu_, mid_, sel_, logits_, trace_, d_ids_, d_argmax_,
                     d_tok_slot_, d_tok_pos_, d_rows_, cos_sin_};
     for (void* p : bufs) if (p) cudaFree(p);
+    for (cudaEvent_t e : copy_done_)
+        if (e) cudaEventDestroy(e);
     void* pinned[] = {p_ids_, p_slot_, p_pos_, p_rows_, p_logits_, p_argmax_};
     for (void* p : pinned) if (p) cudaFreeHost(p);
     if (own_stream) cudaStreamDestroy(own_stream);

@@ -155,6 +155,7 @@ class Engine {
     uint64_t weight_bytes = 0, kv_bytes = 0;
 
   private:
+    int fetch_logits(float* out, size_t n);
     int run_chunk(const uint32_t* ids, int T, const std::vector<int32_t>& rows, float* logits_out, uint32_t* argmax_out);
     int enqueue_layers(int T);                       // embed + all layers for the staged token table
     // final norm is done by the caller; lm_head + argmax of rc rows (pre: digits of those rows already in the workspace)
@@ -285,6 +286,8 @@ class Engine {
     uint32_t* p_ids_ = nullptr;
     int32_t *p_slot_ = nullptr, *p_pos_ = nullptr, *p_rows_ = nullptr;
     float* p_logits_ = nullptr;
+    static constexpr int COPY_EVENTS = 32, COPY_HELPERS = 7;
+    cudaEvent_t copy_done_[COPY_EVENTS] = {};  // of fetch_logits
     uint32_t* p_argmax_ = nullptr;
     // device-resident greedy loop
     uint32_t* d_tokens_ = nullptr;

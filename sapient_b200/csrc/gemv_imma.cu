@@ -251,6 +251,8 @@ __device__ __forceinline__ void store8(float* p, const float (&v)[8]) {
 
 // Plain conversion: one warp per (256 columns, activation row).
 __global__ void __launch_bounds__(32) act_quant_kernel(const float* __restrict__ x, int ldx, QuantOut qo) {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x, m = blockIdx.y, tile = blockIdx.x;
     const int k0 = tile * 256 + lane * 8;
     const bool live = k0 < qo.k;
@@ -449,7 +451,8 @@ void imma_plan_rows(ImmaArgs& a, const ActWorkspace& ws) {
 
 cudaError_t launch_act_quant(const float* x, int ldx, const ImmaArgs& a, cudaStream_t st) {
     if (a.m <= 0) return cudaSuccess;
-    act_quant_kernel<<<dim3(a.kp / 256, a.m), 32, 0, st>>>(x, ldx, quant_out(a));
+    cudaError_t le = launch_pdl(act_quant_kernel, dim3(a.kp / 256, a.m), dim3(32), 0, st, x, ldx, quant_out(a));
+    if (le != cudaSuccess) return le;
     return count_launch_and_check();
 }
 
@@ -534,7 +537,83 @@ void ActWorkspace::release() {
 
 // ─────────────────────────────── the GEMV ────────────────────────────────────
 // (mma wrappers, tile register images and per-tile arithmetic: gemv_imma_dev.cuh)
-// ── Q8_0 with any number of blocks per tile (K not a multiple of 256) ──
+// ── Q8_0, 128 columns (four blocks) at a time: half a tile of eight blocks or a tile of four ──
+struct Q8Unit {
+    uint4 q[4];
+    uint2 d0, d1;  // f16 scales of the four blocks, rows g and g + 8
+};
+template <int BPT>
+__device__ __forceinline__ void load_q8_unit(const uint8_t* base, int u, int lane, Q8Unit& r) {
+    const int g = lane >> 2;
+    const uint8_t* tile = base + (int64_t)(BPT == 8 ? u >> 1 : u) * (BPT * 544);
+    const int half = BPT == 8 ? u & 1 : 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) r.q[j] = ldg_u4(tile + half * 2048 + j * 512 + lane * 16);
+    const uint8_t* d = tile + BPT * 512 + half * 8;
+    r.d0 = __ldg(reinterpret_cast<const uint2*>(d + g * (2 * BPT)));
+    r.d1 = __ldg(reinterpret_cast<const uint2*>(d + (g + 8) * (2 * BPT)));
+}
+// BPT 8: one digit scale per 256 columns; 4: one per 32.
+template <int NT, int BPT>
+__device__ __forceinline__ void compute_q8_unit(const ImmaArgs& a, const Q8Unit& r, int u, int lane, float (&acc)[NT][4]) {
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t e0[2] = {r.d0.x, r.d0.y}, e1[2] = {r.d1.x, r.d1.y};
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        const int col = nt * 8 + g;
+        uint4 b[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+        if (col < a.m * a.digits) {
+            const int8_t* src = a.xq + (int64_t)col * a.kp + (int64_t)(u >> 1) * 256 + t * 64 + (u & 1) * 32;
+            b[0] = ldg_u4(src);
+            b[1] = ldg_u4(src + 16);
+        }
+        float2 cs = make_float2(0.f, 0.f);
+        if (BPT == 8) cs = __ldg(reinterpret_cast<const float2*>(a.colscale + (int64_t)(u >> 1) * a.ncp + nt * 8 + 2 * t));
+        float f[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float d0 = half_bits_to_float((uint16_t)((e0[j >> 1] >> (16 * (j & 1))) & 0xFFFFu));
+            const float d1 = half_bits_to_float((uint16_t)((e1[j >> 1] >> (16 * (j & 1))) & 0xFFFFu));
+            const uint4& w = b[j >> 1];
+            int c[4];
+            imma_k32(c, r.q[j].x, r.q[j].z, r.q[j].y, r.q[j].w, (j & 1) ? w.z : w.x, (j & 1) ? w.w : w.y, 0, 0, 0, 0);
+            if (BPT == 4) {
+                cs = __ldg(reinterpret_cast<const float2*>(a.colscale + (int64_t)(4 * u + j) * a.ncp + nt * 8 + 2 * t));
+                f[0] = fmaf(cs.x * d0, (float)c[0], f[0]); f[1] = fmaf(cs.y * d0, (float)c[1], f[1]);
+                f[2] = fmaf(cs.x * d1, (float)c[2], f[2]); f[3] = fmaf(cs.y * d1, (float)c[3], f[3]);
+            } else {
+                f[0] = fmaf(d0, (float)c[0], f[0]); f[1] = fmaf(d0, (float)c[1], f[1]);
+                f[2] = fmaf(d1, (float)c[2], f[2]); f[3] = fmaf(d1, (float)c[3], f[3]);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[nt][e] = BPT == 8 ? fmaf((e & 1) ? cs.y : cs.x, f[e], acc[nt][e]) : acc[nt][e] + f[e];
+    }
+}
+// A warp's units of one tile row. DEPTH of them are in flight, the first ones from before the previous kernel has ended; read a
+// block at a time, each waited for, a Q8_0 matrix came at a third of the rate (28672 x 4096: 54 us).
+template <int NT, int BPT>
+__device__ __forceinline__ void row_q8_0(const ImmaArgs& a, const uint8_t* base, int warp, int lane, float (&acc)[NT][4]) {
+    constexpr int DEPTH = NT == 1 ? 3 : 2;
+    const int units = a.k >> 7;
+    Q8Unit r[DEPTH];
+#pragma unroll
+    for (int i = 0; i < DEPTH; ++i)
+        if (warp + i * IMMA_WARPS < units) load_q8_unit<BPT>(base, warp + i * IMMA_WARPS, lane, r[i]);
+    pdl_wait();
+    pdl_trigger();
+    for (int u0 = warp; u0 < units; u0 += DEPTH * IMMA_WARPS) {
+#pragma unroll
+        for (int i = 0; i < DEPTH; ++i) {
+            const int u = u0 + i * IMMA_WARPS, next = u + DEPTH * IMMA_WARPS;
+            if (u >= units) break;
+            compute_q8_unit<NT, BPT>(a, r[i], u, lane, acc);
+            if (next < units) load_q8_unit<BPT>(base, next, lane, r[i]);
+        }
+    }
+}
+
+// ── Q8_0 tiles of one block (K not a multiple of 128) ──
 template <int NT>
 __device__ __forceinline__ void tile_q8_0(const ImmaArgs& a, const uint8_t* tile, int kt, int bpt, int lane, float (&acc)[NT][4]) {
     const int g = lane >> 2, t = lane & 3;
@@ -590,11 +669,11 @@ __device__ __forceinline__ void reduce_store(const ImmaArgs& a, const ImmaSeg& s
 }
 
 // Kernel A (any shape): one CTA per tile row; its 8 warps split the k-tiles, operands straight from global memory.
-// FMT: 0 = segments of any format; T_Q4_K / T_Q6_K = every segment of the launch has that format — the code for the
-// other formats is left out, which lets the M <= 2 instance fit 80 registers and run three CTAs (24 warps) per SM
-// instead of two.
+// FMT: 0 = segments of any format; T_Q4_K / T_Q6_K / T_Q8_0 = every segment of the launch has that format — the code for the
+// other formats is left out, which lets the M <= 2 instance of the K-quants fit 80 registers and run three CTAs (24 warps)
+// per SM instead of two.
 template <int NT, int FMT>
-__global__ void __launch_bounds__(IMMA_WARPS * 32, (NT == 1 && FMT != 0) ? 3 : 2) gemv_imma_kernel(const ImmaArgs a) {
+__global__ void __launch_bounds__(IMMA_WARPS * 32, (NT == 1 && FMT != 0 && FMT != T_Q8_0) ? 3 : 2) gemv_imma_kernel(const ImmaArgs a) {
     __shared__ float red[IMMA_WARPS * NT * 4 * 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     int rt = blockIdx.x, s = 0;
@@ -631,22 +710,43 @@ __global__ void __launch_bounds__(IMMA_WARPS * 32, (NT == 1 && FMT != 0) ? 3 : 2
     } else if (FMT == T_Q6_K || (FMT == 0 && sg.dtype == T_Q6_K)) {
         const int kts = a.k >> 8;
         const uint8_t* base = sg.wt + (int64_t)rt * kts * Q6_K_TILE_BYTES;
-        Q6Regs ra;
+        constexpr bool TWO = NT == 1 && FMT == 0;  // (a second tile in flight where registers allow)
+        Q6Regs ra, rb;
         BFrag<NT> b;
         if (warp < kts) load_q6_k<true>(base + (int64_t)warp * Q6_K_TILE_BYTES, lane, ra);
+        if (TWO && warp + IMMA_WARPS < kts) load_q6_k<true>(base + (int64_t)(warp + IMMA_WARPS) * Q6_K_TILE_BYTES, lane, rb);
         pdl_wait();
         pdl_trigger();
-        for (int kt = warp; kt < kts; kt += IMMA_WARPS) {
-            if (kt != warp) load_q6_k<true>(base + (int64_t)kt * Q6_K_TILE_BYTES, lane, ra);
-            load_b_global<NT>(a, kt, g, t, false, true, b);
-            compute_q6_k<NT>(ra, b, lane, acc);
+        if (TWO) {
+            for (int kt = warp; kt < kts; kt += 2 * IMMA_WARPS) {
+                const int k1 = kt + IMMA_WARPS, k2 = k1 + IMMA_WARPS, k3 = k2 + IMMA_WARPS;
+                load_b_global<NT>(a, kt, g, t, false, true, b);
+                compute_q6_k<NT>(ra, b, lane, acc);
+                if (k2 < kts) load_q6_k<true>(base + (int64_t)k2 * Q6_K_TILE_BYTES, lane, ra);
+                if (k1 >= kts) break;
+                load_b_global<NT>(a, k1, g, t, false, true, b);
+                compute_q6_k<NT>(rb, b, lane, acc);
+                if (k3 < kts) load_q6_k<true>(base + (int64_t)k3 * Q6_K_TILE_BYTES, lane, rb);
+            }
+        } else {
+            for (int kt = warp; kt < kts; kt += IMMA_WARPS) {
+                if (kt != warp) load_q6_k<true>(base + (int64_t)kt * Q6_K_TILE_BYTES, lane, ra);
+                load_b_global<NT>(a, kt, g, t, false, true, b);
+                compute_q6_k<NT>(ra, b, lane, acc);
+            }
         }
-    } else if (FMT == 0) {
+    } else if (FMT == 0 || FMT == T_Q8_0) {
         const int bpt = sg.bpt, kts = (a.k >> 5) / bpt, tb = bpt * 544;
         const uint8_t* base = sg.wt + (int64_t)rt * kts * tb;
-        pdl_wait();
-        pdl_trigger();
-        for (int kt = warp; kt < kts; kt += IMMA_WARPS) tile_q8_0<NT>(a, base + (int64_t)kt * tb, kt, bpt, lane, acc);
+        if (bpt == 8) {
+            row_q8_0<NT, 8>(a, base, warp, lane, acc);
+        } else if (bpt == 4) {
+            row_q8_0<NT, 4>(a, base, warp, lane, acc);
+        } else {
+            pdl_wait();
+            pdl_trigger();
+            for (int kt = warp; kt < kts; kt += IMMA_WARPS) tile_q8_0<NT>(a, base + (int64_t)kt * tb, kt, bpt, lane, acc);
+        }
     }
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
@@ -969,10 +1069,11 @@ cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st) {
         return count_launch_and_check();
     }
     cudaError_t le;
-    bool q4_only = true, q6_only = true;
+    bool q4_only = true, q6_only = true, q8_only = true;
     for (int s = 0; s < a.nseg; ++s) {
         q4_only = q4_only && a.seg[s].dtype == T_Q4_K;
         q6_only = q6_only && a.seg[s].dtype == T_Q6_K;
+        q8_only = q8_only && a.seg[s].dtype == T_Q8_0;
     }
     // The 80-register single-format instances trade per-CTA speed for occupancy: they win once the grid is several
     // waves deep (gate|up, lm_head) and lose on grids that fit the SMs at once (o_proj, down_proj), where one CTA's
@@ -980,6 +1081,9 @@ cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st) {
     const bool deep = tiles >= 1024;
     if (nt == 1 && q4_only && deep) le = launch_pdl(gemv_imma_kernel<1, T_Q4_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
     else if (nt == 1 && q6_only && deep) le = launch_pdl(gemv_imma_kernel<1, T_Q6_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
+    else if (nt == 1 && q8_only) le = launch_pdl(gemv_imma_kernel<1, T_Q8_0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
+    else if (nt == 2 && q8_only) le = launch_pdl(gemv_imma_kernel<2, T_Q8_0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
+    else if (nt == 4 && q8_only) le = launch_pdl(gemv_imma_kernel<4, T_Q8_0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
     else if (nt == 1) le = launch_pdl(gemv_imma_kernel<1, 0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
     else if (nt == 2) le = launch_pdl(gemv_imma_kernel<2, 0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
     else if (nt == 4) le = launch_pdl(gemv_imma_kernel<4, 0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);

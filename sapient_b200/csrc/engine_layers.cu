@@ -43,7 +43,9 @@ bool Engine::plan_digits(int m, int k, ImmaArgs& ia) {
     ia = ImmaArgs{};
     ia.m = m;
     ia.k = k;
-    if (m > imma_rows_per_pass() || k > ws_.k_max) return false;
+    if (k > ws_.k_max) return false;
+    // (11 to 16 rows: one launch makes the digits of both passes; as f32 rows and a conversion per pass they took four)
+    if (m > imma_rows_per_pass()) return !use_rows && imma_plan_passes(ia, ws_);
     imma_plan(ia, ws_);
     return true;
 }
@@ -125,6 +127,7 @@ int Engine::gemv(const float* x, int ldx, int m, int k, const DevTensor* w0, con
             ImmaArgs ia{};
             if (pre) ia = *pre;
             ia.k = k; ia.m = std::min(pass, m - m0);
+            if (pre && m > pass) imma_pass(ia, m0, ia.m);
             ia.res = (res && !tp_sum) ? res + (size_t)m0 * ldy0 : nullptr;
             ia.ldres = ldy0;
             ia.tp = (tp_sum && !via_nccl) ? d_tp_ : nullptr;

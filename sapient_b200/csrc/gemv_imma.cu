@@ -441,6 +441,26 @@ void imma_plan(ImmaArgs& a, const ActWorkspace& ws) {
     a.xq = ws.xq; a.colscale = ws.colscale; a.xs32d = ws.xs32d; a.xs16d = ws.xs16d;
 }
 
+bool imma_plan_passes(ImmaArgs& a, const ActWorkspace& ws) {
+    if (!g_digit_mode.load() || a.m <= 10 || a.m > 16) return false;
+    a.digits = 3;
+    a.ncp = 64;  // a second pass looks at columns 30 .. 61
+    a.eb = (a.k % 256 == 0) ? 256 : 32;
+    a.kp = (a.k + 255) / 256 * 256;
+    a.xq = ws.xq; a.colscale = ws.colscale; a.xs32d = ws.xs32d; a.xs16d = ws.xs16d;
+    return true;
+}
+
+void imma_pass(ImmaArgs& a, int m0, int rows) {
+    const int col = m0 * a.digits, cols = rows * a.digits;
+    a.xq += (int64_t)col * a.kp;
+    a.colscale += col;
+    a.xs32d += col * 32;
+    a.xs16d += col * 32;
+    a.m = rows;
+    a.nt = cols <= 8 ? 1 : cols <= 16 ? 2 : 4;
+}
+
 void imma_plan_rows(ImmaArgs& a, const ActWorkspace& ws) {
     a.digits = 3;
     a.ncp = (a.m * 3 + 31) / 32 * 32;
@@ -1014,7 +1034,7 @@ static PerDeviceOnce g_stream_attr[3];
 // Shared-memory layout of the streaming kernel, or total == 0 when the launch does not qualify.
 static StreamPlan plan_stream(const ImmaArgs& a) {
     StreamPlan p{};
-    if (a.k % 256 != 0 || a.ncp > 16) return p;
+    if (a.k % 256 != 0 || a.ncp > 16 || a.nt) return p;
     const int kts = a.k / 256, ncols = a.m * a.digits, nt = a.ncp / 8;
     int stage = 0, tiles = 0;
     for (int s = 0; s < a.nseg; ++s) {
@@ -1049,7 +1069,7 @@ cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st) {
     int tiles = 0;
     for (int s = 0; s < a.nseg; ++s) tiles += (a.seg[s].n + 15) / 16;
     if (tiles == 0) return cudaSuccess;
-    const int nt = a.ncp / 8;
+    const int nt = a.nt ? a.nt : a.ncp / 8;
     // The persistent TMA-streaming kernel is opt-in: measured on B200 it trails the per-tile-row kernel
     // (132 vs 81 us on a 128256 x 4096 Q4_K matrix), so the default is the latter.
     const StreamPlan p = (g_imma_kernel.load() == 3 && !a.tp) ? plan_stream(a) : StreamPlan{};

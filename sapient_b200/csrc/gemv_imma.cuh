@@ -49,7 +49,8 @@ struct ImmaArgs {
     int k;
     int m;        // activation rows in this launch (<= 8 * NT / digits)
     int digits;   // 2 or 3
-    int ncp;      // padded digit columns = 8 * NT
+    int ncp;      // padded digit columns
+    int nt;       // 8-column tiles of this launch; 0: all of them
     int eb;       // columns per activation exponent block: 256 or 32
     int kp;       // k rounded up to 256: column stride of xq
     // Digits: xq[col][kp]; inside each 256-column tile the bytes are ordered [t 0..3][block 0..7][8 B], the 8 B

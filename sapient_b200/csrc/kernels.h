@@ -181,6 +181,10 @@ struct RowsScratch {
     void release();
 };
 bool rows_supported(int dtype, int64_t k);
+// Digits of 11 .. 16 rows at once (three each), for a producer that writes them in one launch; false where the mode or the count is
+// another. imma_pass makes of such a plan the launch of rows m0 .. m0 + rows - 1.
+bool imma_plan_passes(ImmaArgs& a, const ActWorkspace& ws);
+void imma_pass(ImmaArgs& a, int m0, int rows);
 void imma_plan_rows(ImmaArgs& a, const ActWorkspace& ws);  // three digits, 32-column groups (a.m <= IMMA_ROWS_MAX)
 cudaError_t launch_gemv_rows(const ImmaArgs& a, const RowsScratch& sc, cudaStream_t st);
 

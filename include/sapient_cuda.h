@@ -91,10 +91,10 @@ int32_t sp_cuda_set_activation_digits(int32_t mode);
  *      activation digits built inside the kernel) where the shape fits. */
 int32_t sp_cuda_set_gemv_path(int32_t path);
 /* Op-level matmuls with m >= 17 rows and k % 256 == 0 (Q8_0: k % 128 == 0):
- * 2 (default): the tcgen05 / TMEM dequant GEMM with exact-class operands — weights and activations each as an fp16
- *    leading part plus the fp16 of what that rounding dropped (rows scaled by a power of two first), three tensor-core
- *    products per chunk of K: ~1e-6 per product, the level of the integer-digit GEMV;
- * 1: the same GEMM with operands rounded once to fp16 (~3e-4 per product, 2x faster);
+ * 2 (default): the tcgen05 / TMEM dequant GEMM with exact-class operands — activations as an fp16 leading part plus the
+ *    fp16 of what that rounding dropped (rows scaled by a power of two first), weights unrounded (4-bit weights times their
+ *    scale as exact integers, the others in two parts): ~1e-6 per product, near the integer-digit GEMV;
+ * 1: a GEMM with operands rounded once to fp16 (~3e-4 per product);
  * 0: exact integer products on the mma.sync kernels at every row count (passes of up to 32 rows).
  * Process-wide; engines have their own switch with the same values and default. */
 int32_t sp_cuda_set_large_m_gemm(int32_t on);
@@ -315,12 +315,12 @@ int32_t sp_cuda_batcher_stats(const SpBatcher* b, uint64_t* out, int32_t cap);
 int32_t sp_cuda_engine_set_graphs(SpEngine* e, int32_t on);
 /* Steps of 17 rows and more (prefill chunks, batched decode) run on the tcgen05 GEMM: each weight tile is dequantised
  * once and multiplied with all rows on the 5th-generation tensor cores.
- * on = 2 (default): exact-class operands (leading fp16 part + remainder for weights and activations, three products per
- *    chunk of K, ~1e-6 per product); activations are converted from their f32 rows, attention stays on the f32-class
- *    kernels. Full-size models keep the 2e-2 final-logit bar (8B shape, 128-token prompt: 6.7e-3).
+ * on = 2 (default): exact-class operands (activations as a leading fp16 part + remainder, weights unrounded in one or two
+ *    operand planes, ~1e-6 per product), norms and activations fused with that split, tiled attention with the same split.
+ *    Full-size models keep the 2e-2 final-logit bar (8B shape, 128-token prompt: 6.7e-3).
  * on = 1: operands rounded once to fp16 (~3e-4 per product, inside the 1e-3 per-op bar, but the 8B shape's final logits
  *    then move by up to 4e-2), fused fp16 producers and the fp16 prefill attention: a 512-token prefill of the 8B shape
- *    takes 15 ms instead of 28 ms.
+ *    takes 15 ms instead of 23 ms.
  * on = 0: integer-digit GEMV passes of 10 rows at any row count (201 ms for that prefill).
  * Drops the captured step graphs. */
 int32_t sp_cuda_engine_set_large_m_gemm(SpEngine* e, int32_t on);

@@ -25,6 +25,9 @@
 //               remainders of the sums, minima exact) times dmin, which costs a quarter instruction per element.
 // Columns are stored in the order 0 2 1 3 within groups of four, in activations and weights alike: the order in which masks
 // pick bytes out of a word, so that no weight is moved.
+// Measured against the kernel before (matmul with its split of activations): Q4_K 28672 x 4096, 32 rows 101 -> 54 us; 4096 x 14336
+// Q6_K, 37 rows 54.6 -> 37.1; Q4_K 4096 x 4096, 512 rows 85 -> 53; 28672 x 4096, 512 rows 285 -> 286 (its 128-row tiles are bounded by
+// the shared-memory traffic of the activation boxes). Error against float64 at K = 14336: 1.3e-5 -> 5e-7.
 // The K range of a tile is shared by the blocks of a cluster when tiles alone leave SMs idle; they meet in distributed shared
 // memory and add in part order, so results do not vary from run to run. Every wait on an mbarrier is bounded.
 #include <cuda.h>

@@ -190,7 +190,9 @@ cudaError_t launch_gemv_rows(const ImmaArgs& a, const RowsScratch& sc, cudaStrea
 
 // Large-M dequant GEMM on tcgen05 / TMEM (gemm_tc5.cu): y[m, n] = x·Wᵀ (+ bias, + res) from the tiled weights and an
 // fp16 copy of the activations; k % 256 == 0, Q4_K / Q6_K / Q8_0.
-constexpr int TC5_MIN_M = 17;  // up to 16 rows one GEMV pass is faster; from 17 rows on (two passes) the tcgen05 GEMM wins (measured at 32 rows: 5.6 vs 7.1 ms per decode step of the 8B shape)
+// Up to 16 rows the integer-digit GEMV: its products are exact, 3e-7 of a result's norm against 5e-7 to 1.4e-6, although two of its
+// passes take longer from 11 rows on (Q4_K 28672 x 4096: 13 rows 96 us, 17 rows on the GEMM 54).
+constexpr int TC5_MIN_M = 17;
 bool tc5_supported(int dtype, int64_t k);
 cudaError_t launch_x_to_f16(const float* x, int ldx, int m, int k, __half* out, cudaStream_t st);
 cudaError_t launch_gemm_tc5(const uint8_t* wt, int dtype, int n, int k, const __half* xh, int m, float* y, int ldy, const float* bias,

@@ -307,6 +307,9 @@ __device__ __forceinline__ bool dq_produce(DqBars& bars, const uint8_t* raw, int
 // Tiles of up to 64 activation rows have both planes of the activations side by side in one product (its N is twice the rows) and
 // in the accumulator; the drain adds them. Wider tiles multiply the planes one after the other into the same columns.
 constexpr int DQ_SIDE_NJT = 4;
+// 64-column boxes of an activation stage: two, so that there are fewer hand-overs; one for tall tiles, whose boxes of up to 32 KB
+// would leave a ring of two stages.
+__host__ __device__ constexpr int dq_boxes(int njt) { return njt <= DQ_SIDE_NJT ? 2 : 1; }
 
 // A drain warp's walk: acc[tile][j] holds rows 16 tile + g (+ 8) of the warp's 32, columns 8 j + 2 t (+ 1) of its NJT 8-column tiles.
 template <int DT, int NJT>
@@ -401,58 +404,65 @@ __device__ __forceinline__ bool dq_drain(DqBars& bars, const uint8_t* raw, int r
     return ok;
 }
 
-// The MMA warp's walk, a half at a time: an activation stage is two boxes of 64 columns. The whole warp takes part and one elected thread
+// The MMA warp's walk, an activation stage (BOXES boxes of 64 columns) at a time. The whole warp takes part and one elected thread
 // issues: control flow and operands are uniform then, as the tensor instructions want them. Issuing is the serial part of the
 // pipeline (a wait that is already over costs 100 to 250 cycles on a busy SM), so the barriers of the next half are looked at ahead of
 // a half's products and only waited for if they were not over by then.
-template <bool TWO, bool SIDE>
+template <bool TWO, bool SIDE, int BOXES>
 __device__ __forceinline__ bool dq_issue(DqBars& bars, uint32_t tm, uint64_t bd0, uint32_t b16, int b_stages, uint32_t idesc, uint32_t idesc_side, int n_sb,
                                          int halves_last, bool leader, DqRing& ra, DqRing& rb, DqRing& rd, bool& seen, bool ok) {
-    const uint32_t box16 = b16 >> 1, plane16 = box16 >> 1;  // a box: both planes
+    constexpr int STEPS = 2 / BOXES;  // activation stages of a half
+    const uint32_t box16 = b16 / BOXES, plane16 = box16 >> 1;  // a box of 64 columns: both planes
     for (int sb = 0; sb < n_sb; ++sb) {
         const int halves = sb == n_sb - 1 ? halves_last : 2;
         for (int h = 0; h < halves; ++h) {
-            const bool first = h == 0, last = h == halves - 1;
             const uint32_t At = tm + (uint32_t)DQ_A_COL + 64u * (uint32_t)ra.st;
             if (TWO) ra.next(DQ_A_SLOTS);  // (a pair's second slot)
-            if (!seen && ok) {
-                bool w = true;
-                if (first) w = rd.empty(bars.empty_d);
-                w = w && ra.full(bars.full_a) && rb.full(bars.full_b);
-                ok = __all_sync(0xFFFFFFFFu, w);
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const uint32_t dt = tm + (uint32_t)(rd.st * DQ_NB);
-            const uint64_t b0 = bd0 + (uint64_t)((uint32_t)rb.st * b16);  // (the address field: no carry out of the low word)
-            uint64_t* const e_b = &bars.empty_b[rb.st];
-            uint64_t* const e_a = &bars.empty_a[ra.st];
-            uint64_t* const f_d = &bars.full_d[rd.st];
-            rb.next(b_stages);
-            ra.next(DQ_A_SLOTS);
-            if (last) rd.next(2);
-            bool next = tc5_peek(&bars.full_b[rb.st], rb.u & 1);
-            // (where the next tile's format is another one, the other slot of the pair says the same: slots are filled in order)
-            next = tc5_peek(&bars.full_a[ra.st + (TWO ? 1 : 0)], ra.u & 1) && next;
-            if (last && rd.u > 0) next = tc5_peek(&bars.empty_d[rd.st], (rd.u - 1) & 1) && next;
-            if (leader) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const uint32_t more = i > 0 ? 1u : (uint32_t)(h > 0);
-                    const uint64_t bh = b0 + (i >> 2) * box16 + 2u * (i & 3);
-                    if (SIDE) {
-                        dq_mma(dt, At + 8u * i, bh, idesc_side, more);                  // W [X_hi | X_lo]
-                    } else {
-                        dq_mma(dt, At + 8u * i, bh + plane16, idesc, more);             // W X_lo
-                        dq_mma(dt, At + 8u * i, bh, idesc, 1u);                         // W X_hi
-                    }
-                    if (TWO) dq_mma(dt, At + 64u + 8u * i, bh, idesc, 1u);              // W_lo X_hi
+            for (int s = 0; s < STEPS; ++s) {
+                const bool first = h == 0 && s == 0, a_last = s == STEPS - 1, last = a_last && h == halves - 1;
+                if (!seen && ok) {
+                    bool w = true;
+                    if (first) w = rd.empty(bars.empty_d);
+                    if (s == 0) w = w && ra.full(bars.full_a);
+                    w = w && rb.full(bars.full_b);
+                    ok = __all_sync(0xFFFFFFFFu, w);
                 }
-                tc5_commit(e_b);
-                if (TWO) tc5_commit(e_a - 1);
-                tc5_commit(e_a);
-                if (last) tc5_commit(f_d);
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const uint32_t dt = tm + (uint32_t)(rd.st * DQ_NB);
+                const uint64_t b0 = bd0 + (uint64_t)((uint32_t)rb.st * b16);  // (the address field: no carry out of the low word)
+                uint64_t* const e_b = &bars.empty_b[rb.st];
+                uint64_t* const e_a = &bars.empty_a[ra.st];
+                uint64_t* const f_d = &bars.full_d[rd.st];
+                rb.next(b_stages);
+                if (a_last) ra.next(DQ_A_SLOTS);
+                if (last) rd.next(2);
+                bool next = tc5_peek(&bars.full_b[rb.st], rb.u & 1);
+                // (where the next tile's format is another one, the other slot of the pair says the same: slots are filled in order)
+                if (a_last) next = tc5_peek(&bars.full_a[ra.st + (TWO ? 1 : 0)], ra.u & 1) && next;
+                if (last && rd.u > 0) next = tc5_peek(&bars.empty_d[rd.st], (rd.u - 1) & 1) && next;
+                if (leader) {
+#pragma unroll
+                    for (int i = 0; i < 4 * BOXES; ++i) {
+                        const uint32_t more = i > 0 || s > 0 ? 1u : (uint32_t)(h > 0), Ai = At + 32u * s + 8u * i;
+                        const uint64_t bh = b0 + (i >> 2) * box16 + 2u * (i & 3);
+                        if (SIDE) {
+                            dq_mma(dt, Ai, bh, idesc_side, more);                  // W [X_hi | X_lo]
+                        } else {
+                            dq_mma(dt, Ai, bh + plane16, idesc, more);             // W X_lo
+                            dq_mma(dt, Ai, bh, idesc, 1u);                         // W X_hi
+                        }
+                        if (TWO) dq_mma(dt, Ai + 64u, bh, idesc, 1u);              // W_lo X_hi
+                    }
+                    tc5_commit(e_b);
+                    if (a_last) {
+                        if (TWO) tc5_commit(e_a - 1);
+                        tc5_commit(e_a);
+                    }
+                    if (last) tc5_commit(f_d);
+                }
+                seen = __all_sync(0xFFFFFFFFu, next);
             }
-            seen = __all_sync(0xFFFFFFFFu, next);
         }
     }
     return ok;
@@ -480,12 +490,13 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
     __shared__ __align__(8) DqBars bars;
     __shared__ uint32_t tmem_slot;
     constexpr bool SIDE = NJT <= DQ_SIDE_NJT;
+    constexpr int BOXES = dq_boxes(NJT);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t* smem = smem_raw + ((1024u - (tc5_smem_u32(smem_raw) & 1023u)) & 1023u);
     const int all_sb = (a.k + 255) / 256, part = blockIdx.z;
     const int sb0 = part * all_sb / a.parts, n_sb = (part + 1) * all_sb / a.parts - sb0;
     const int halves_last = min(2, (a.k - (sb0 + n_sb - 1) * 256) / 128);  // 128-column halves of this block's last 256 columns
-    const int b_bytes = 4 * a.nb * 128, x_bytes = a.nb * 32;
+    const int b_bytes = BOXES * 2 * a.nb * 128, x_bytes = a.nb * 32;
     uint8_t* const xs = smem + (size_t)a.b_stages * b_bytes;
     uint8_t* const raw = xs + DQ_X_STAGES * x_bytes;
 
@@ -545,14 +556,14 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
             for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
                 const DqItem it(a, item);
                 for (int sb = 0; sb < n_sb && ok; ++sb) {
-                    const int halves = sb == n_sb - 1 ? halves_last : 2;
-                    for (int h = 0; h < halves; ++h) {
+                    const int steps = 2 / BOXES * (sb == n_sb - 1 ? halves_last : 2);
+                    for (int h = 0; h < steps; ++h) {
                         ok = r.empty(bars.empty_b);
                         if (!ok) break;
                         const uint32_t bar = tc5_smem_u32(&bars.full_b[r.st]), dst = tc5_smem_u32(smem + (size_t)r.st * b_bytes);
                         dq_expect(bar, (uint32_t)b_bytes);
-                        for (int c = 0; c < 4; ++c)
-                            tc5_tma_2d(dst + c * a.nb * 128, &tmap_x, (sb0 + sb) * 256 + 128 * h + 64 * (c >> 1), (c & 1) * a.m + it.m0, bar);
+                        for (int c = 0; c < 2 * BOXES; ++c)
+                            tc5_tma_2d(dst + c * a.nb * 128, &tmap_x, (sb0 + sb) * 256 + 64 * (BOXES * h + (c >> 1)), (c & 1) * a.m + it.m0, bar);
                         r.next(a.b_stages);
                     }
                     if (it.dt == T_Q4_K && ok) {
@@ -575,7 +586,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
             for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
                 const DqItem it(a, item);
 #define SP_DQ_ISSUE(TWO) \
-    ok = dq_issue<TWO, SIDE>(bars, tmem, bd0, (uint32_t)b_bytes >> 4, a.b_stages, idesc, idesc_side, n_sb, halves_last, leader, ra, rb, rd, seen, ok)
+    ok = dq_issue<TWO, SIDE, BOXES>(bars, tmem, bd0, (uint32_t)b_bytes >> 4, a.b_stages, idesc, idesc_side, n_sb, halves_last, leader, ra, rb, rd, seen, ok)
                 if (it.dt == T_Q4_K) SP_DQ_ISSUE(false);
                 else SP_DQ_ISSUE(true);
 #undef SP_DQ_ISSUE
@@ -750,7 +761,7 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
     a.m_tiles = (m + a.nb - 1) / a.nb;
     // shared memory: at most half for activations (each box serves 64 columns), the rest for raw tiles
     const int njt = a.nb <= 16 ? 1 : a.nb <= 32 ? 2 : a.nb <= 64 ? 4 : 8;
-    const int b_bytes = 4 * a.nb * 128, x_bytes = DQ_X_STAGES * a.nb * 32;
+    const int b_bytes = dq_boxes(njt) * 2 * a.nb * 128, x_bytes = DQ_X_STAGES * a.nb * 32;
     a.r_bytes = 8 * tb;
     a.b_stages = std::min(DQ_MAX_B, 128 * 1024 / b_bytes);
     a.r_stages = std::min(DQ_MAX_R, (DQ_SMEM - 1024 - a.b_stages * b_bytes - x_bytes) / a.r_bytes);
@@ -759,6 +770,13 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
         for (auto f : {gemm_dq_kernel<1>, gemm_dq_kernel<2>, gemm_dq_kernel<4>, gemm_dq_kernel<8>}) {
             const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM);
             if (e != cudaSuccess) return e;
+        }
+        // the register split of the tall variants draws on what their blocks are launched with
+        for (auto f : {gemm_dq_kernel<4>, gemm_dq_kernel<8>}) {
+            cudaFuncAttributes fa;
+            const cudaError_t e = cudaFuncGetAttributes(&fa, f);
+            if (e != cudaSuccess) return e;
+            if (fa.numRegs * DQ_THREADS < 128 * 32 + 256 * 96 + 256 * 128) return cudaErrorLaunchOutOfResources;
         }
         return cudaSuccess;
     });

@@ -26,8 +26,8 @@
 // Columns are stored in the order 0 2 1 3 within groups of four, in activations and weights alike: the order in which masks
 // pick bytes out of a word, so that no weight is moved.
 // Measured against the kernel before (matmul with its split of activations): Q4_K 28672 x 4096, 32 rows 101 -> 54 us; 4096 x 14336
-// Q6_K, 37 rows 54.6 -> 37.1; Q4_K 4096 x 4096, 512 rows 85 -> 53; 28672 x 4096, 512 rows 285 -> 286 (its 128-row tiles are bounded by
-// the shared-memory traffic of the activation boxes). Error against float64 at K = 14336: 1.3e-5 -> 5e-7.
+// Q6_K, 37 rows 54.6 -> 37.1; Q4_K 4096 x 4096, 512 rows 85 -> 49; 28672 x 4096, 512 rows 285 -> 244 (its 128-row tiles are bounded by
+// the shared-memory traffic of the activation boxes). Short K is where it loses: Q8_0 17920 x 1536, 192 rows 33.9 -> 42.8. Error against float64 at K = 14336: 1.3e-5 -> 5e-7.
 // The K range of a tile is shared by the blocks of a cluster when tiles alone leave SMs idle; they meet in distributed shared
 // memory and add in part order, so results do not vary from run to run. Every wait on an mbarrier is bounded.
 #include <cuda.h>
@@ -69,7 +69,7 @@ struct DqArgs {
     const float* res;      // [m][ldres] or null, added to segment 0 (may alias its y)
     int ldres;
     int m_tiles, nb;       // row tiles, rows per tile (a multiple of 16)
-    int items;             // tiles in all
+    int item0, items;      // tiles of this launch: item0 .. items - 1
     int parts;             // blocks of the cluster that share a tile's K range
     int b_stages, r_stages, r_bytes;  // depth of the activation ring, of the raw ring, bytes of a raw stage
     const float* xscale;   // [m]
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
                 // raw tiles: weights, which no kernel writes, so they are requested before the previous kernel has ended
                 DqRing r;
                 int issued = 0;
-                for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+                for (int item = a.item0 + blockIdx.x; item < a.items && ok; item += gridDim.x) {
                     const DqItem it(a, item);
                     const int tb = dq_tile_bytes(it.dt), live = min(8, ((a.seg[it.si].n + 15) >> 4) - (it.n0 >> 4));
                     const int64_t row_bytes = (int64_t)(a.k >> 7) * (tb >> 1);
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
         }
         if (warp == 2 && lane == 0) {
             DqRing r, rx;
-            for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+            for (int item = a.item0 + blockIdx.x; item < a.items && ok; item += gridDim.x) {
                 const DqItem it(a, item);
                 for (int sb = 0; sb < n_sb && ok; ++sb) {
                     const int steps = 2 / BOXES * (sb == n_sb - 1 ? halves_last : 2);
@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
             const uint64_t bd0 = tc5_desc(tc5_smem_u32(smem));
             DqRing ra, rb, rd;
             bool seen = false;
-            for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+            for (int item = a.item0 + blockIdx.x; item < a.items; item += gridDim.x) {
                 const DqItem it(a, item);
 #define SP_DQ_ISSUE(TWO) \
     ok = dq_issue<TWO, SIDE, BOXES>(bars, tmem, bd0, (uint32_t)b_bytes >> 4, a.b_stages, idesc, idesc_side, n_sb, halves_last, leader, ra, rb, rd, seen, ok)
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
         const int pw = warp - DQ_FIRST_PRODUCER, tile_w = 2 * (warp & 3) + (pw >> 2);
         const uint32_t a_base = tmem + ((uint32_t)(16 * tile_w) << 16) + (uint32_t)DQ_A_COL;
         DqRing rr, ra;
-        for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+        for (int item = a.item0 + blockIdx.x; item < a.items; item += gridDim.x) {
             const int dt = DqItem(a, item).dt;
 #define SP_DQ_PRODUCE(T) ok = dq_produce<T>(bars, raw, a.r_bytes, a.r_stages, tile_w, lane, a_base, n_sb, halves_last, rr, ra, ok)
             if (dt == T_Q4_K) SP_DQ_PRODUCE(T_Q4_K);
@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
         pdl_wait();
         const int quarter = warp & 3, half = (warp - DQ_FIRST_DRAIN) >> 2, g = lane >> 2, t = lane & 3;
         DqRing rr, rx, rd;
-        for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+        for (int item = a.item0 + blockIdx.x; item < a.items; item += gridDim.x) {
             const DqItem it(a, item);
             const Tc5Seg& sg = a.seg[it.si];
             float acc[2][NJT][4];
@@ -783,15 +783,28 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
     if (le != cudaSuccess) return le;
     // parts: what makes the longest SM's share shortest, a block's start and end counted as three spans of 256 columns
     const int items = tiles * a.m_tiles, all_sb = (k + 255) / 256;
-    int best = 1;
-    long best_cost = 0;
-    for (int p = 1; p <= std::min(DQ_MAX_PARTS, all_sb); ++p) {
-        const long waves = (items + dq_clusters(p) - 1) / dq_clusters(p), sb = (all_sb + p - 1) / p;
-        const long cost = p == 1 ? waves * sb + 3 : waves * (sb + 3) + 1;  // (a lone block runs from tile to tile)
-        if (p == 1 || cost < best_cost) { best = p; best_cost = cost; }
-    }
-    a.parts = best;
+    auto best_split = [&](int n, long& cost, bool lone) {
+        int best = 1;
+        for (int p = 1; p <= std::min(DQ_MAX_PARTS, all_sb); ++p) {
+            const long waves = (n + dq_clusters(p) - 1) / dq_clusters(p), sb = (all_sb + p - 1) / p;
+            const long c = p == 1 && lone ? waves * sb + 3 : waves * (sb + 3) + 1;  // (a lone block runs from tile to tile)
+            if (p == 1 || c < cost) { best = p; cost = c; }
+        }
+        return best;
+    };
+    long cost = 0;
+    a.parts = best_split(items, cost, true);
     a.items = items;
+    // A few tiles over whole rounds of the SMs (28672 rows in tiles of 128, 512 activation rows: 896 = 6 x 148 + 8) would take a round
+    // of their own: they get a second launch that shares out their K range where that is shorter, its own start counted as two spans
+    // more. Measured there: Q4_K, K = 4096 270 -> 244 us, and 145 -> 121 at 192 rows (448 = 3 x 148 + 4).
+    const int sms = device_sm_count(), over = items % sms;
+    int tail_parts = 0;
+    if (a.parts == 1 && items > sms && over > 0) {
+        long tail = 0;
+        tail_parts = best_split(over, tail, false);
+        if (tail + 2 >= all_sb) tail_parts = 0;
+    }
     const PFN_encodeTiled encode = tensor_map_encoder();
     if (!encode) return cudaErrorNotSupported;
     CUtensorMap tmap;
@@ -805,11 +818,17 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
             return cudaErrorInvalidValue;
     }
     g_dq_launched[current_device_index()].store(1);
-    const dim3 grid((unsigned)(a.parts == 1 ? std::min(items, device_sm_count()) : items), 1, (unsigned)a.parts), block(DQ_THREADS);
     auto kernel = njt == 1 ? gemm_dq_kernel<1> : njt == 2 ? gemm_dq_kernel<2> : njt == 4 ? gemm_dq_kernel<4> : gemm_dq_kernel<8>;
-    le = launch_pdl_cluster(kernel, grid, block, DQ_SMEM, st, a.parts, a, tmap);
-    if (le != cudaSuccess) return le;
-    return count_launch_and_check();
+    auto launch = [&](int from, int to, int parts) {
+        a.item0 = from; a.items = to; a.parts = parts;
+        const int n = to - from;
+        const dim3 grid((unsigned)(parts == 1 ? std::min(n, sms) : n), 1, (unsigned)parts);
+        const cudaError_t e = launch_pdl_cluster(kernel, grid, dim3(DQ_THREADS), DQ_SMEM, st, parts, a, tmap);
+        return e != cudaSuccess ? e : count_launch_and_check();
+    };
+    if (!tail_parts) return launch(0, items, a.parts);
+    le = launch(0, items - over, 1);
+    return le != cudaSuccess ? le : launch(items - over, items, tail_parts);
 }
 
 }  // namespace sp

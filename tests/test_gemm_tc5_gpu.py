@@ -133,9 +133,9 @@ def test_split_last_wave_is_reproducible_bit_for_bit(oracle, dtype, m, k, n):
 
 # edges of gemm_dq_kernel: its variants by tile height (16, 32, 64, 128 rows, the first step over each), one row tile more than fits, K
 # of one tile and of an odd number, fewer weight rows than a 16-row tile, more tiles than SMs (a block runs from one into the
-# next, the last ones short), K shared by a cluster, rows longer than a block keeps in registers, Q8_0 widths that are odd multiples of 128
+# next, the last ones short), K shared by a cluster, rows longer than a block keeps in registers, two tiles over a round of the SMs (a launch of their own), Q8_0 widths that are odd multiples of 128
 DQ_EDGES = [(17, 256, 7), (32, 768, 129), (33, 1280, 40), (64, 2304, 256), (65, 512, 300), (128, 256, 128), (129, 768, 136), (257, 256, 130), (40, 256, 19205),
-            (130, 512, 10250), (20, 16640, 40)]
+            (130, 512, 10250), (20, 16640, 40), (20, 4096, 19074)]
 
 
 @pytest.mark.parametrize("dtype,m,k,n", [(d, *c) for d in (Q4_K, Q6_K, Q8_0) for c in DQ_EDGES] + [(Q8_0, 17, 128, 16), (Q8_0, 100, 384, 130), (Q8_0, 34, 896, 4864), (Q8_0, 200, 1152, 272)])

@@ -45,6 +45,7 @@ SIGNATURES = {
     "sp_cuda_matmul_nt": (_i32, [_vp, _vp, _i64, _vp]),
     "sp_cuda_matmul_nt_dev": (_i32, [_vp, _vp, _i64, _vp, _vp]),
     "sp_cuda_check_kernels": (_i32, [_i32]),
+    "sp_cuda_report_wait": (_i32, [_vp, _i32, _i32]),
     "sp_cuda_set_gemv_path": (_i32, [_i32]),
     "sp_cuda_set_activation_digits": (_i32, [_i32]),
     "sp_cuda_weight_info": (_i32, [_vp, C.POINTER(_i32), C.POINTER(_i64), C.POINTER(_i64), C.POINTER(_sz)]),

@@ -253,7 +253,8 @@ int32_t sp_cuda_upload_weight(int32_t device, int32_t dtype, int64_t n, int64_t 
         if (ce == cudaSuccess) ce = launch_repack(dtype, w->d, n, k, w->tiled, 0);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(0);
         if (ce == cudaSuccess) ce = w->ws.alloc((int)k);
-        if (ce == cudaSuccess) ce = ring_device_init();
+        if (ce == cudaSuccess) ce = device_wait_flags().alloc();
+        w->ws.waits = w->ring.waits = device_wait_flags().dev;
         if (ce == cudaSuccess) ce = w->ring.alloc((int)((n + 15) / 16));
         if (ce == cudaSuccess) ce = w->rows.alloc();
     }
@@ -322,7 +323,7 @@ int32_t sp_cuda_matmul_nt_dev(const SpWeight* w, const float* x_dev, int64_t m, 
         }
         SP_CUDA_TRY(launch_x_to_f16(x_dev, (int)w->k, (int)m, (int)w->k, wm->ws.xh, (cudaStream_t)stream));
         SP_CUDA_TRY(launch_gemm_tc5(w->tiled, w->dtype, (int)w->n, (int)w->k, wm->ws.xh, (int)m, y_dev, (int)w->n, nullptr, nullptr, 0,
-                                    (cudaStream_t)stream, &wm->ws.tc5));
+                                    (cudaStream_t)stream, &wm->ws.tc5, wm->ws.waits));
         return SP_OK;
     }
     if (w->tiled && g_gemv_path.load() == 0 && g_ring.load() && m >= 1 && m <= RING_MAX_M) {
@@ -369,11 +370,19 @@ int32_t sp_cuda_matmul_nt_dev(const SpWeight* w, const float* x_dev, int64_t m, 
 }
 
 static int check_kernel_flags() {
-    const int a = tc5_take_timeout(), b = imma_take_timeout(), c = dq_take_timeout();
-    if (a < 0 || b < 0 || c < 0) { set_error("could not read the kernels' timeout flags"); return SP_ERR_CUDA; }
-    if (a > 0 || c > 0) { set_error("tcgen05 GEMM: a bounded mbarrier wait expired, the outputs of that launch are not valid"); return SP_ERR_CUDA; }
-    if (b > 0) { set_error("streaming GEMV: a bounded mbarrier wait expired, the outputs of that launch are not valid"); return SP_ERR_CUDA; }
+    if (const char* what = device_wait_flags().take()) { set_error(what); return SP_ERR_CUDA; }
     return SP_OK;
+}
+
+int32_t sp_cuda_report_wait(SpEngine* e, int32_t device, int32_t kind) {
+    API_BEGIN
+    if (kind < 0 || kind >= WAIT_KINDS) { set_error("no such kind of wait"); return SP_ERR_ARG; }
+    if (e) return e->e->report_wait(kind);
+    SP_CUDA_TRY(cudaSetDevice(device));
+    SP_CUDA_TRY(device_wait_flags().alloc());
+    SP_CUDA_TRY(launch_report_wait(device_wait_flags().dev, kind, nullptr));
+    return SP_OK;
+    API_END
 }
 
 int32_t sp_cuda_check_kernels(int32_t device) {

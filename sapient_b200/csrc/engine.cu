@@ -96,6 +96,7 @@ Engine::~Engine() {
     if (argmax_scratch_) cudaFree(argmax_scratch_);
     ring_.release();
     rows_.release();
+    waits_.release();
     for (void* p : owned_) cudaFree(p);
     void* bufs[] = {kv_.pool, d_page_table_, x_, h_, qkv_, attn_, gu_, mid_, sel_, logits_, trace_, d_ids_, d_argmax_,
                     d_tok_slot_, d_tok_pos_, d_rows_, cos_sin_};
@@ -326,7 +327,6 @@ int Engine::repack_weights() {
     {
         // tile rows of the widest launch: q|k|v, gate|up (two segments), lm_head
         const int64_t widest = std::max<int64_t>({(int64_t)d.vocab, 2 * (int64_t)d.ffn, (int64_t)(d.n_heads + 2 * d.n_kv_heads) * d.head_dim, (int64_t)d.hidden});
-        SP_CUDA_TRY(ring_device_init());
         SP_CUDA_TRY(ring_.alloc((int)(widest / 16 + 8)));
     }
     if (d.max_tokens > imma_rows_per_pass()) SP_CUDA_TRY(rows_.alloc());
@@ -336,6 +336,8 @@ int Engine::repack_weights() {
 int Engine::finalize() {
     if (finalized) return SP_OK;
     SP_CUDA_TRY(cudaSetDevice(d.device));
+    SP_CUDA_TRY(waits_.alloc());
+    ws_.waits = ring_.waits = waits_.dev;
     if (load_stream_) SP_CUDA_TRY(cudaStreamSynchronize(load_stream_));  // every weight has landed
     release_staging();
     if (plan_) {

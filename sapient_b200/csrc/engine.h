@@ -117,6 +117,7 @@ class Engine {
     int tp_set_allreduce(int mode);                 // 0: fused peer push (default); 1: library all-reduce
     // After a stream synchronise: SP_ERR_CUDA if a bounded mbarrier wait of one of this device's kernels ran out since
     // the last check (the kernel's outputs are then stale), else tp_check().
+    int report_wait(int kind);  // as a kernel of this engine does whose wait ran out
     int device_check();
     void drop_graphs();                             // forget the captured step graphs (a launch parameter changed)
     int vocab_local() const { return vocab_l_; }
@@ -181,6 +182,7 @@ class Engine {
     int try_ring(bool* done, int m, int k, int src, const float* x, int ldx, const float* nw, const float* nb, const DevTensor* w0,
                  const float* b0, float* y0, int ldy, const DevTensor* w1 = nullptr, const float* b1 = nullptr, float* y1 = nullptr,
                  const DevTensor* w2 = nullptr, const float* b2 = nullptr, float* y2 = nullptr, const float* res = nullptr);
+    WaitFlags waits_;   // of this engine's launches
     RingScratch ring_;
     RowsScratch rows_;         // K-split partials of the one-pass many-row GEMV
     bool big_m(int m, int k, const DevTensor* w0, const DevTensor* w1 = nullptr, const DevTensor* w2 = nullptr) const;
@@ -260,7 +262,7 @@ class Engine {
     int plan_dense(int layer, int T);
     int plan_rollback(int slot, int n, int* kept);
     int plan_mat(const PlanMat& w, const void* x, int ldx, int m, void* y, int ldy, bool out_f32);
-    int plan_product(const MatArgs& a, int max_tiles);
+    int plan_product(MatArgs a, int max_tiles);
     int plan_head(const int32_t* rows, int n);
     int plan_ctx_bucket() const;
     int plan_privatise_copy(int from, int to);

@@ -70,7 +70,7 @@ int Engine::gemv(const float* x, int ldx, int m, int k, const DevTensor* w0, con
             // many rows: dequantise each weight tile once and multiply on the 5th-generation tensor cores
             auto product = [&](const Tc5Seg* segs, int ns, int ldy, const float* r) {
                 return tc5_exact ? launch_gemm_dq(segs, ns, k, ws_.dq(), m, ldy, r, ldy, stream)
-                                 : launch_gemm_tc5_multi(segs, ns, k, ws_.xh, m, ldy, r, ldy, stream, &ws_.tc5);
+                                 : launch_gemm_tc5_multi(segs, ns, k, ws_.xh, m, ldy, r, ldy, stream, &ws_.tc5, ws_.waits);
             };
             if (tc5_exact) SP_LAUNCH(F_ELEM, launch_dq_rows(DQ_PLAIN, x, ldx, nullptr, nullptr, 0.f, m, k, ws_.dq(), stream));
             else SP_LAUNCH(F_ELEM, launch_x_to_f16(x, ldx, m, k, ws_.xh, stream));
@@ -218,7 +218,7 @@ int Engine::gemm_xh(int m, int k, const DevTensor* w0, const float* b0, float* y
     int ns = 0;
     for (int i = 0; i < 3 && ws[i]; ++i) segs[ns++] = Tc5Seg{ws[i]->tiled, ys[i], bs[i], ws[i]->dtype, (int)ws[i]->dims[0]};
     if (tc5_exact) SP_LAUNCH(F_GEMV, launch_gemm_dq(segs, ns, k, ws_.dq(), m, ldy0, res, ldy0, stream));
-    else SP_LAUNCH(F_GEMV, launch_gemm_tc5_multi(segs, ns, k, ws_.xh, m, ldy0, res, ldy0, stream, &ws_.tc5));
+    else SP_LAUNCH(F_GEMV, launch_gemm_tc5_multi(segs, ns, k, ws_.xh, m, ldy0, res, ldy0, stream, &ws_.tc5, ws_.waits));
     return SP_OK;
 }
 

@@ -374,7 +374,8 @@ int Engine::plan_stage(int T) {
     return SP_OK;
 }
 
-int Engine::plan_product(const MatArgs& a, int max_tiles) {
+int Engine::plan_product(MatArgs a, int max_tiles) {
+    a.waits = waits_.dev;
     SP_LAUNCH(F_GEMV, a.f32 ? launch_mat_f32(a, stream) : launch_mat_tc5(a, max_tiles, stream));
     return SP_OK;
 }

@@ -59,8 +59,6 @@ constexpr int DQ_SMEM = 224 * 1024;
 constexpr int DQ_MAX_PARTS = 8;
 constexpr int DQ_P_STRIDE = DQ_BM + 4;     // floats between the columns of a partial tile: no bank conflicts
 
-__device__ int g_dq_timeout = 0;
-
 constexpr int T_Q8_0_HALF = 1000 + T_Q8_0;  // Q8_0 whose width is an odd multiple of 128: tiles of four blocks
 
 struct DqArgs {
@@ -74,6 +72,7 @@ struct DqArgs {
     int b_stages, r_stages, r_bytes;  // depth of the activation ring, of the raw ring, bytes of a raw stage
     const float* xscale;   // [m]
     const __half* xsum;    // [k / 256][m][16]: sums of 32 columns as dq_rows.cu leaves them
+    int* waits;            // WaitFlags of the launch's owner
 };
 
 __device__ __forceinline__ void dq_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -697,23 +696,10 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
             cluster_sync();  // nobody leaves while its partials are being read
         }
     }
-    if (!ok) atomicExch(&g_dq_timeout, 1);
+    if (!ok) report_wait(a.waits, WAIT_GEMM);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
-}
-
-// Reads and clears the flag that a bounded wait raises when it runs out; as tc5_take_timeout.
-static std::atomic<int> g_dq_launched[SP_MAX_DEVICES];
-int dq_take_timeout() {
-    if (g_dq_launched[current_device_index()].exchange(0) == 0) return 0;
-    int flag = 0;
-    if (cudaMemcpyFromSymbol(&flag, g_dq_timeout, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return -1; }
-    if (flag) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(g_dq_timeout, &zero, sizeof(int));
-    }
-    return flag ? 1 : 0;
 }
 
 // How many clusters of `parts` blocks the device holds at once (a block fills an SM, and a cluster lies within one GPC).
@@ -745,7 +731,7 @@ static int dq_clusters(int parts) {
 
 cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& in, int m, int ldy, const float* res, int ldres, cudaStream_t st) {
     if (m <= 0 || nseg <= 0) return cudaSuccess;
-    if (nseg > 3 || k % 128 != 0) return cudaErrorInvalidValue;
+    if (nseg > 3 || k % 128 != 0 || !in.waits) return cudaErrorInvalidValue;
     DqArgs a{};
     int tiles = 0, tb = 0;
     for (int i = 0; i < nseg; ++i) {
@@ -755,7 +741,7 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
         tb = std::max(tb, dq_tile_bytes(segs[i].dtype));
     }
     a.nseg = nseg; a.k = k; a.m = m; a.ldy = ldy; a.res = res; a.ldres = ldres;
-    a.xscale = in.xscale; a.xsum = in.xsum;
+    a.xscale = in.xscale; a.xsum = in.xsum; a.waits = in.waits;
     a.m_tiles = (m + DQ_NB - 1) / DQ_NB;
     a.nb = ((m + a.m_tiles - 1) / a.m_tiles + 15) & ~15;
     a.m_tiles = (m + a.nb - 1) / a.nb;
@@ -817,7 +803,6 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
-    g_dq_launched[current_device_index()].store(1);
     auto kernel = njt == 1 ? gemm_dq_kernel<1> : njt == 2 ? gemm_dq_kernel<2> : njt == 4 ? gemm_dq_kernel<4> : gemm_dq_kernel<8>;
     auto launch = [&](int from, int to, int parts) {
         a.item0 = from; a.items = to; a.parts = parts;

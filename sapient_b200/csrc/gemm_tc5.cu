@@ -23,7 +23,7 @@
 // ~2e-4 relative L2 of the f32 reference (bf16 would sit at ~2e-3, above the 1e-3 parity bar). Each weight is computed
 // in f32 from exact operands and rounded to fp16 once (Q8_0: the exact product of int8 and f16 scale, in half2).
 // (Exact-class operands, the default of the callers: gemm_dq.cu.)
-// Every wait on an mbarrier is bounded; on expiry the kernel raises g_tc5_timeout, still frees its tensor memory
+// Every wait on an mbarrier is bounded; on expiry the kernel reports it (kernels.h: WaitFlags), still frees its tensor memory
 // and returns.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -54,7 +54,6 @@ constexpr int TC5_NB_MAX = 256;                // activation rows per CTA
 constexpr int TC5_SMEM_LIMIT = 192 * 1024;
 constexpr int TC5_SMEM_MIN = 120 * 1024;       // more than half an SM's shared memory: one CTA per SM, which owns all of its tensor memory
 
-__device__ int g_tc5_timeout = 0;
 
 // Instruction descriptor, kind::f16: fp16 A and B, fp32 D, both K-major, M = 128, N = nb.
 __device__ __forceinline__ uint32_t tc5_idesc(int nb) {
@@ -336,6 +335,7 @@ struct Tc5Args {
     unsigned* split_cnt;
     int stage_bytes;    // 256 * (widest activation tile of the launch, rounded to 16): two boxes of 64 columns
     int stages;         // depth of the activation ring that fits shared memory (3..8)
+    int* waits;         // WaitFlags of the launch's owner
 };
 
 __global__ void __launch_bounds__(TC5_THREADS, 1) gemm_tc5_kernel(const Tc5Args a, const __grid_constant__ CUtensorMap tmap_x) {
@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(TC5_THREADS, 1) gemm_tc5_kernel(const Tc5Args 
             }
         }
     }
-    if (!ok) atomicExch(&g_tc5_timeout, 1);
+    if (!ok) report_wait(a.waits, WAIT_GEMM);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     if (warp == TC5_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TC5_TMEM_COLS) : "memory");
@@ -540,21 +540,6 @@ __global__ void x_to_f16_kernel(const float* __restrict__ x, int ldx, int k, __h
     const float4 p0 = *reinterpret_cast<const float4*>(x + m * ldx + c), p1 = *reinterpret_cast<const float4*>(x + m * ldx + c + 4);
     *reinterpret_cast<uint4*>(out + m * k + c) =
         make_uint4(pack_h2(p0.x, p0.y), pack_h2(p0.z, p0.w), pack_h2(p1.x, p1.y), pack_h2(p1.z, p1.w));
-}
-
-// Reads and clears the flag a bounded mbarrier wait of gemm_tc5_kernel raises when it runs out (the kernel then skips
-// its epilogue, so y is stale). Synchronous copy from the device the calling thread has current: call it only where
-// the stream has been synchronised already. 1 = a wait expired since the last call, 0 = none, -1 = CUDA error.
-static std::atomic<int> g_tc5_launched[SP_MAX_DEVICES];  // per device: a launch has happened since the flag was last read
-int tc5_take_timeout() {
-    if (g_tc5_launched[current_device_index()].exchange(0) == 0) return 0;
-    int flag = 0;
-    if (cudaMemcpyFromSymbol(&flag, g_tc5_timeout, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return -1; }
-    if (flag) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(g_tc5_timeout, &zero, sizeof(int));
-    }
-    return flag ? 1 : 0;
 }
 
 bool tc5_supported(int dtype, int64_t k) {
@@ -591,7 +576,7 @@ void Tc5Scratch::release() {
 }
 
 cudaError_t launch_gemm_tc5_multi(const Tc5Seg* segs, int nseg, int k, const __half* xh, int m, int ldy, const float* res, int ldres,
-                                  cudaStream_t st, const Tc5Scratch* scratch) {
+                                  cudaStream_t st, const Tc5Scratch* scratch, int* waits) {
     if (m <= 0 || nseg <= 0) return cudaSuccess;
     if (nseg > 3 || k % 128 != 0) return cudaErrorInvalidValue;
     Tc5Args a{};
@@ -635,23 +620,22 @@ cudaError_t launch_gemm_tc5_multi(const Tc5Seg* segs, int nseg, int k, const __h
     }
     a.nseg = nseg; a.k = k; a.xh = xh; a.m = m; a.ldy = ldy; a.res = res; a.ldres = ldres;
     a.m_tiles = m_tiles; a.full_items = full_items; a.tail_split = tail_split;
-    a.stage_bytes = stage_bytes; a.stages = stages;
+    a.stage_bytes = stage_bytes; a.stages = stages; a.waits = waits;
     constexpr int SMEM_CAP = TC5_SMEM_LIMIT + 1024;
     cudaError_t le;
     le = attr_once.run([] { return cudaFuncSetAttribute(gemm_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP); });
     if (le != cudaSuccess) return le;
     if (tail_split > 1) { a.split_buf = scratch->buf; a.split_cnt = scratch->cnt; }
     const int grid = full_items + (items - full_items) * tail_split;
-    g_tc5_launched[current_device_index()].store(1);
     le = launch_pdl(gemm_tc5_kernel, dim3((unsigned)grid), dim3(TC5_THREADS), smem_bytes, st, a, tmap);
     if (le != cudaSuccess) return le;
     return count_launch_and_check();
 }
 
 cudaError_t launch_gemm_tc5(const uint8_t* wt, int dtype, int n, int k, const __half* xh, int m, float* y, int ldy, const float* bias,
-                            const float* res, int ldres, cudaStream_t st, const Tc5Scratch* scratch) {
+                            const float* res, int ldres, cudaStream_t st, const Tc5Scratch* scratch, int* waits) {
     Tc5Seg sg{wt, y, bias, dtype, n};
-    return launch_gemm_tc5_multi(&sg, 1, k, xh, m, ldy, res, ldres, st, scratch);
+    return launch_gemm_tc5_multi(&sg, 1, k, xh, m, ldy, res, ldres, st, scratch, waits);
 }
 
 }  // namespace sp

@@ -438,7 +438,7 @@ void imma_plan(ImmaArgs& a, const ActWorkspace& ws) {
     a.ncp = cols <= 8 ? 8 : cols <= 16 ? 16 : 32;
     a.eb = (a.k % 256 == 0) ? 256 : 32;
     a.kp = (a.k + 255) / 256 * 256;
-    a.xq = ws.xq; a.colscale = ws.colscale; a.xs32d = ws.xs32d; a.xs16d = ws.xs16d;
+    a.xq = ws.xq; a.colscale = ws.colscale; a.xs32d = ws.xs32d; a.xs16d = ws.xs16d; a.waits = ws.waits;
 }
 
 bool imma_plan_passes(ImmaArgs& a, const ActWorkspace& ws) {
@@ -447,7 +447,7 @@ bool imma_plan_passes(ImmaArgs& a, const ActWorkspace& ws) {
     a.ncp = 64;  // a second pass looks at columns 30 .. 61
     a.eb = (a.k % 256 == 0) ? 256 : 32;
     a.kp = (a.k + 255) / 256 * 256;
-    a.xq = ws.xq; a.colscale = ws.colscale; a.xs32d = ws.xs32d; a.xs16d = ws.xs16d;
+    a.xq = ws.xq; a.colscale = ws.colscale; a.xs32d = ws.xs32d; a.xs16d = ws.xs16d; a.waits = ws.waits;
     return true;
 }
 
@@ -466,7 +466,7 @@ void imma_plan_rows(ImmaArgs& a, const ActWorkspace& ws) {
     a.ncp = (a.m * 3 + 31) / 32 * 32;
     a.eb = (a.k % 256 == 0) ? 256 : 32;
     a.kp = (a.k + 255) / 256 * 256;
-    a.xq = ws.xq; a.colscale = ws.colscale; a.xs32d = ws.xs32d; a.xs16d = ws.xs16d;
+    a.xq = ws.xq; a.colscale = ws.colscale; a.xs32d = ws.xs32d; a.xs16d = ws.xs16d; a.waits = ws.waits;
 }
 
 cudaError_t launch_act_quant(const float* x, int ldx, const ImmaArgs& a, cudaStream_t st) {
@@ -542,7 +542,7 @@ cudaError_t ActWorkspace::ensure_xh(size_t elems) {
     return e;
 }
 
-DqInput ActWorkspace::dq() const { return DqInput{xh, xscale, xsum}; }
+DqInput ActWorkspace::dq() const { return DqInput{xh, xscale, xsum, waits}; }
 
 void ActWorkspace::release() {
     if (xh) cudaFree(xh);
@@ -790,7 +790,6 @@ constexpr int STREAM_SMEM_LIMIT = 220 * 1024;
 constexpr int STREAM_SPIN_LIMIT = 1 << 16;  // polls of up to ~20 us each (the try_wait time hint) before a wait gives up: about a second
 
 // Set when a bounded wait in a kernel of this file ran out; host code reads and clears it.
-__device__ int g_imma_timeout = 0;
 
 struct StreamPlan {
     int stage_bytes;   // ring slot size: largest tile among the segments, multiple of 128
@@ -983,50 +982,7 @@ __global__ void __launch_bounds__(STREAM_WARPS * 32, 1) gemv_imma_stream_kernel(
         rt += gridDim.x;
         while (s < a.nseg - 1 && rt >= seg_tiles(s)) { rt -= seg_tiles(s); ++s; }
     }
-    if (!ok && lane == 0) atomicExch(&g_imma_timeout, 1);
-}
-
-// Reads and clears g_imma_timeout (device the calling thread has current; call after a stream synchronise).
-// 1 = a bounded wait of the streaming kernel expired since the last call, 0 = none, -1 = CUDA error.
-// The ring GEMV (gemv_ring.cu) reports through a host-mapped flag per device, so that checking it costs no CUDA call.
-static std::atomic<int*> g_ring_flag_host[SP_MAX_DEVICES];
-static std::atomic<int*> g_ring_flag_dev[SP_MAX_DEVICES];
-cudaError_t ring_device_init() {
-    const int di = current_device_index();
-    if (g_ring_flag_host[di].load()) return cudaSuccess;
-    int* h = nullptr;
-    cudaError_t e = cudaHostAlloc((void**)&h, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
-    if (e != cudaSuccess) return e;
-    *h = 0;
-    int* d = nullptr;
-    e = cudaHostGetDevicePointer((void**)&d, h, 0);
-    if (e != cudaSuccess) { cudaFreeHost(h); return e; }
-    int* expected = nullptr;
-    if (g_ring_flag_host[di].compare_exchange_strong(expected, h)) g_ring_flag_dev[di].store(d);
-    else cudaFreeHost(h);  // another thread was first
-    return cudaSuccess;
-}
-int* imma_timeout_flag() {
-    const int di = current_device_index();
-    while (g_ring_flag_host[di].load() && !g_ring_flag_dev[di].load()) {}  // the winner of the race publishes the device pointer last
-    return g_ring_flag_dev[di].load();
-}
-void imma_note_ring_launch() {}
-
-static std::atomic<int> g_stream_launched[SP_MAX_DEVICES];  // per device: the streaming kernel has been launched since the flag was last read
-int imma_take_timeout() {
-    if (int* h = g_ring_flag_host[current_device_index()].load()) {
-        volatile int* vh = h;
-        if (*vh) { *vh = 0; return 1; }
-    }
-    if (g_stream_launched[current_device_index()].exchange(0) == 0) return 0;
-    int flag = 0;
-    if (cudaMemcpyFromSymbol(&flag, g_imma_timeout, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return -1; }
-    if (flag) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(g_imma_timeout, &zero, sizeof(int));
-    }
-    return flag ? 1 : 0;
+    if (!ok && lane == 0) report_wait(a.waits, WAIT_GEMV);
 }
 
 static PerDeviceOnce g_stream_attr[3];
@@ -1083,7 +1039,6 @@ cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st) {
             });
             if (e != cudaSuccess) return e;
         }
-        g_stream_launched[current_device_index()].store(1);
         if (nt == 1) gemv_imma_stream_kernel<1><<<grid, STREAM_WARPS * 32, p.total, st>>>(a, p);
         else gemv_imma_stream_kernel<2><<<grid, STREAM_WARPS * 32, p.total, st>>>(a, p);
         return count_launch_and_check();

@@ -50,6 +50,7 @@ struct ImmaArgs {
     int m;        // activation rows in this launch (<= 8 * NT / digits)
     int digits;   // 2 or 3
     int ncp;      // padded digit columns
+    int* waits;   // WaitFlags of the launch's owner
     int nt;       // 8-column tiles of this launch; 0: all of them
     int eb;       // columns per activation exponent block: 256 or 32
     int kp;       // k rounded up to 256: column stride of xq

@@ -28,7 +28,7 @@
 //     tile row, re-arms the slot with the next bulk copy, and writes finished rows: digit columns summed, bias,
 //     residual, store (or the cross-CTA hand-over above). Consumers never wait for anything but data.
 // Every mbarrier wait is bounded; after an expired wait the CTA stops consuming, raises the error flag the host reads
-// (imma_take_timeout), waits — bounded again — for its copies in flight and returns.
+// (kernels.h: WaitFlags), waits — bounded again — for its copies in flight and returns.
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -42,8 +42,6 @@
 namespace sp {
 
 cudaError_t count_launch_and_check();  // kernels.cu
-void imma_note_ring_launch();          // gemv_imma.cu: arms imma_take_timeout
-int* imma_timeout_flag();              // gemv_imma.cu: device address of the flag on the current device
 
 // Consumer warps = tiles per ring slot. 15 (16 warps with the service warp: four per scheduler, up to 128 registers per
 // thread) for launches that mix weight formats; 23 (24 warps, 80 registers) when every segment has one K-quant format
@@ -408,7 +406,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) gemv_ring_kernel(const __gri
         }
         if (ok && cur_row >= 0) ring_row_out<R>(ro, cur_seg, cur_row, racc);
         if (!ok) {
-            if (lane == 0) *reinterpret_cast<volatile int*>(a.err) = 1;  // host-mapped flag: a plain store
+            if (lane == 0) report_wait(a.waits, WAIT_GEMV);
             // copies still in flight write into this CTA's shared memory: wait for them (bounded) before leaving
             for (int i = retired; i < issued; ++i) {
                 const int s = i % a.stages;
@@ -543,7 +541,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) gemv_ring_kernel(const __gri
             ct += len;
             if (++slot == a.stages) { slot = 0; par ^= 1u; }
         }
-        if (!ok && lane == 0) *reinterpret_cast<volatile int*>(a.err) = 1;
+        if (!ok && lane == 0) report_wait(a.waits, WAIT_GEMV);
     }
 }
 
@@ -630,8 +628,7 @@ cudaError_t launch_gemv_ring(RingArgs& a, cudaStream_t st) {
     const int sms = device_sm_count();
     // at least one full ring slot of work per CTA
     const int grid = std::min(sms, std::max(1, a.total_tiles / a.cw));
-    a.err = imma_timeout_flag();
-    if (!a.err) return cudaErrorInvalidValue;
+    if (!a.waits) return cudaErrorInvalidValue;
     cudaError_t e;
     if (nt == 2) e = ring_launch_instance<2, RING_CW_MIXED, 0>(a, grid, st);
     else if (a.cw == RING_CW_SINGLE && a.fmt == T_Q4_K) e = ring_launch_instance<1, RING_CW_SINGLE, T_Q4_K>(a, grid, st);

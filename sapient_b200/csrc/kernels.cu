@@ -17,6 +17,7 @@
 
 #include <atomic>
 #include <cstdlib>
+#include <mutex>
 
 #include "pdl.cuh"
 
@@ -779,6 +780,50 @@ cudaError_t launch_gather_rows(const float* src, int ld, const int32_t* rows, in
     if (n_rows == 0) return cudaSuccess;
     gather_rows_kernel<<<n_rows, 256, 0, st>>>(src, ld, rows, dim, dst);
     return finish_launch();
+}
+
+// ── waits that ran out ──
+__global__ void report_wait_kernel(int* waits, int kind) { report_wait(waits, kind); }
+
+cudaError_t launch_report_wait(int* waits, int kind, cudaStream_t st) {
+    if (!waits || kind < 0 || kind >= WAIT_KINDS) return cudaErrorInvalidValue;
+    report_wait_kernel<<<1, 1, 0, st>>>(waits, kind);
+    return count_launch_and_check();
+}
+
+cudaError_t WaitFlags::alloc() {
+    static std::mutex one;  // (two threads may upload a device's first weight)
+    std::lock_guard<std::mutex> lock(one);
+    if (host) return cudaSuccess;
+    int *h = nullptr, *d = nullptr;
+    cudaError_t e = cudaHostAlloc((void**)&h, WAIT_KINDS * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e != cudaSuccess) return e;
+    for (int i = 0; i < WAIT_KINDS; ++i) h[i] = 0;
+    if ((e = cudaHostGetDevicePointer((void**)&d, h, 0)) != cudaSuccess) { cudaFreeHost(h); return e; }
+    dev = d;
+    host = h;
+    return cudaSuccess;
+}
+
+void WaitFlags::release() {
+    if (int* h = host.exchange(nullptr)) cudaFreeHost(h);
+    dev = nullptr;
+}
+
+const char* WaitFlags::take() {
+    static const char* const what[WAIT_KINDS] = {"tcgen05 GEMM: a bounded mbarrier wait expired, the outputs of that launch are not valid",
+                                                 "tcgen05 GEMM on bf16 weights: a bounded mbarrier wait expired, the outputs of that launch are not valid",
+                                                 "streaming GEMV: a bounded mbarrier wait expired, the outputs of that launch are not valid"};
+    const char* said = nullptr;
+    int* const h = host;
+    for (int i = 0; h && i < WAIT_KINDS; ++i)
+        if (__atomic_exchange_n(&h[i], 0, __ATOMIC_ACQ_REL) && !said) said = what[i];
+    return said;
+}
+
+WaitFlags& device_wait_flags() {
+    static WaitFlags flags[SP_MAX_DEVICES];
+    return flags[current_device_index()];
 }
 
 }  // namespace sp

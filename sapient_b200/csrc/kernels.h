@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "gemv_imma.cuh"
 
 namespace sp {
@@ -61,10 +63,19 @@ void imma_select_kernel(int which);
 // pass) above; 1 = 3 digits always (10 rows per pass). imma_rows_per_pass() is the pass size that follows.
 void imma_set_digit_mode(int mode);
 int imma_rows_per_pass();
-// Bounded device-side waits (mbarrier waits of the streaming GEMV and of the tcgen05 GEMM) raise a per-device flag when
-// they run out. These read and clear it on the current device: 1 = expired since the last call, 0 = none, -1 = CUDA error.
-int imma_take_timeout();
-int tc5_take_timeout();
+// A device-side wait that runs out is reported to flags in mapped host memory, a kernel's plain store; whoever owns the launch (an
+// engine; for op-level calls the device) owns the flags, and its launches carry their device address. Looking costs no CUDA call, so
+// it is done after every synchronisation: a mark of what has been launched would miss the replays of a captured step.
+enum WaitKind : int { WAIT_GEMM = 0, WAIT_MAT, WAIT_GEMV, WAIT_KINDS };
+struct WaitFlags {
+    std::atomic<int*> host{nullptr};
+    int* dev = nullptr;
+    cudaError_t alloc();        // on the current device, once; not during stream capture
+    void release();
+    const char* take();         // clears the flags; what to say if one was up, else null. After a synchronisation
+};
+WaitFlags& device_wait_flags();         // of op-level calls on the current device; alloc() is up to the caller
+cudaError_t launch_report_wait(int* waits, int kind, cudaStream_t st);  // reports as a kernel does whose wait ran out
 // ── Persistent ring GEMV for steps of 1-5 rows (gemv_ring.cu) ──
 // Where the activations of a launch come from: f32 rows as they are, or through the operation that precedes the matrix
 // in the layer, applied by every CTA on its own copy.
@@ -77,6 +88,7 @@ struct RingScratch {
     float* part = nullptr;
     unsigned* cnt = nullptr;   // zero between launches
     int rows_cap = 0, ctas_cap = 0;
+    int* waits = nullptr;      // WaitFlags of the owner
     cudaError_t alloc(int max_rows);  // on the current device; not during stream capture
     void release();
 };
@@ -100,11 +112,8 @@ struct RingArgs {
     int off_bar, off_flush, off_cs, off_rec32, off_rec16, off_xq, off_stage;
     float* fix_part;
     unsigned* fix_cnt;
-    int* err;
+    int* waits;           // WaitFlags of the launch's owner
 };
-// One-time per-device set-up of the ring kernel's error flag (host-mapped memory): call before the first launch on a
-// device, outside stream capture (engine finalize and weight upload do).
-cudaError_t ring_device_init();
 // share_sm: size the ring so that two CTAs fit an SM (this kernel's and the next kernel's prologue under programmatic
 // dependent launch). False when the launch cannot use this kernel (shape, formats, shared memory, scratch size).
 bool ring_plan(RingArgs& a, const RingScratch& sc, bool share_sm = false);
@@ -158,6 +167,7 @@ struct ActWorkspace {
     __half* xsum = nullptr;
     static constexpr int XSCALE_ROWS = 4096;
     DqInput dq() const;
+    int* waits = nullptr;      // WaitFlags of the owner
     Tc5Scratch tc5;            // allocated with xh
     cudaError_t ensure_xh(size_t elems);  // grows the buffer (allocates: not during stream capture)
     static constexpr int NCP_MAX = 96;  // digit columns: 32 rows x 3 digits (gemv_rows.cu); the tile-row kernel uses up to 32
@@ -196,7 +206,7 @@ constexpr int TC5_MIN_M = 17;
 bool tc5_supported(int dtype, int64_t k);
 cudaError_t launch_x_to_f16(const float* x, int ldx, int m, int k, __half* out, cudaStream_t st);
 cudaError_t launch_gemm_tc5(const uint8_t* wt, int dtype, int n, int k, const __half* xh, int m, float* y, int ldy, const float* bias,
-                            const float* res, int ldres, cudaStream_t st, const Tc5Scratch* scratch = nullptr);
+                            const float* res, int ldres, cudaStream_t st, const Tc5Scratch* scratch, int* waits);
 struct Tc5Seg {
     const uint8_t* wt;  // tiled weights
     float* y;           // output base: element (m, r) at y[m * ldy + r]
@@ -205,7 +215,7 @@ struct Tc5Seg {
 };
 // Up to three matrices sharing the activations in ONE launch (q|k|v, gate|up); res is added to segment 0.
 cudaError_t launch_gemm_tc5_multi(const Tc5Seg* segs, int nseg, int k, const __half* xh, int m, int ldy, const float* res, int ldres,
-                                  cudaStream_t st, const Tc5Scratch* scratch = nullptr);
+                                  cudaStream_t st, const Tc5Scratch* scratch, int* waits);
 
 // The same with exact-class operands (gemm_dq.cu), from activations in this form: every row scaled by a
 // power of two to (-1, 1) (xscale[m] receives the inverse), so that remainders stay inside the fp16 range whatever the row's
@@ -215,6 +225,7 @@ struct DqInput {
     __half* xh;
     float* xscale;
     __half* xsum;
+    int* waits;  // WaitFlags of the launch's owner
 };
 // Rows of x[m, ldx] to that form (dq_rows.cu), as they are or through what produces them: RMS / LayerNorm with weight w and bias b,
 // SwiGLU of (x[0 .. k), x[k .. 2k)), tanh-GELU. All but DQ_PLAIN: k as dq_rows_fit allows.
@@ -222,7 +233,6 @@ enum DqSource { DQ_PLAIN, DQ_RMS, DQ_LN, DQ_SWIGLU, DQ_GELU };
 bool dq_rows_fit(int k);
 cudaError_t launch_dq_rows(int src, const float* x, int ldx, const float* w, const float* b, float eps, int m, int k, const DqInput& in, cudaStream_t st);
 cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& in, int m, int ldy, const float* res, int ldres, cudaStream_t st);
-int dq_take_timeout();  // as tc5_take_timeout
 
 cudaError_t launch_dequant(int dtype, const uint8_t* w, int64_t n, int64_t k, float* out, cudaStream_t st);
 cudaError_t launch_gemv(const GemvArgs& a, cudaStream_t st);

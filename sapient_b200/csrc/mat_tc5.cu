@@ -35,7 +35,6 @@ constexpr int MT_A_BYTES = MT_BM * MT_BK * 2;
 constexpr int MT_SMEM = 108 * 1024;        // per CTA, two of which share an SM
 constexpr int MT_MAX_PARTS = 8;
 
-__device__ int g_mat_tc5_timeout = 0;
 
 struct MatTc5Seg {
     void* y;
@@ -59,6 +58,7 @@ struct MatTc5Args {
     MatOut outs[MAT_MAX_OUTS];
     float arg[2];
     MatNorm norm;
+    int* waits;
 };
 
 // OUTS: a plain product whose weight rows go where a.outs says (OUT_F32 then has no meaning). NORM: it adds into the stream and
@@ -332,22 +332,10 @@ __global__ void __launch_bounds__(MT_THREADS, 2) mat_tc5_kernel(const MatTc5Args
         if (warp < 2) { __syncwarp(); cluster_sync(); }  // the service warps' share of the cluster's first barrier
         cluster_sync();                                  // nobody leaves while its partials are being read
     }
-    if (!ok) atomicExch(&g_mat_tc5_timeout, 1);
+    if (!ok) report_wait(a.waits, WAIT_MAT);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
-}
-
-static std::atomic<int> g_mat_tc5_launched[SP_MAX_DEVICES];
-int mat_tc5_take_timeout() {
-    if (g_mat_tc5_launched[current_device_index()].exchange(0) == 0) return 0;
-    int flag = 0;
-    if (cudaMemcpyFromSymbol(&flag, g_mat_tc5_timeout, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return -1; }
-    if (flag) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(g_mat_tc5_timeout, &zero, sizeof(int));
-    }
-    return flag ? 1 : 0;
 }
 
 // [rows][cols] bf16 with a row stride of ld elements, boxes of 64 columns x box_rows.
@@ -399,7 +387,7 @@ cudaError_t launch_mat_tc5(const MatArgs& a, int max_tiles, cudaStream_t st) {
     k.slots0 = a.moe ? max_tiles : groups * k.row_tiles;
     const int slots = k.slots0 + (a.nseg == 2 ? k.row_tiles : 0);
     k.moe = a.moe; k.gather = a.gather; k.rows = a.rows; k.gate = a.gate; k.ldgate = a.ldgate;
-    k.n_outs = a.n_outs; k.norm = a.norm;
+    k.n_outs = a.n_outs; k.norm = a.norm; k.waits = a.waits;
     std::copy(a.arg, a.arg + 2, k.arg);
     std::copy(a.outs, a.outs + MAT_MAX_OUTS, k.outs);
     const int acc = a.dual ? 2 : 1;
@@ -427,7 +415,6 @@ cudaError_t launch_mat_tc5(const MatArgs& a, int max_tiles, cudaStream_t st) {
         return cudaSuccess;
     });
     if (le != cudaSuccess) return le;
-    g_mat_tc5_launched[current_device_index()].store(1);
     const dim3 grid((unsigned)row_blocks, (unsigned)slots, (unsigned)k.parts), block(MT_THREADS);
     const size_t smem = (size_t)(k.stages * k.stage_bytes + 1024);
 #define SP_MT(DUAL, F32) le = launch_pdl_cluster(mat_tc5_kernel<DUAL, F32>, grid, block, smem, st, k.parts, k, mw[0], mx[0], mw[1], mx[1])

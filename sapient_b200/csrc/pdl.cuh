@@ -53,6 +53,9 @@ struct PerDeviceOnce {
     }
 };
 
+// A wait ran out (kernels.h: WaitFlags).
+__device__ __forceinline__ void report_wait(int* waits, int kind) { *reinterpret_cast<volatile int*>(waits + kind) = 1; }
+
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::); }
 

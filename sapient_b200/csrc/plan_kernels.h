@@ -87,6 +87,7 @@ struct MatArgs {
     MatOut outs[MAT_MAX_OUTS];
     float arg[2];              // of the activation
     MatNorm norm;              // null w: none; else one range that adds
+    int* waits;                // WaitFlags of the launch's owner (bf16)
 };
 
 // The ranges cover the matrix, and the product is a plain one.
@@ -110,7 +111,6 @@ cudaError_t launch_mat_f32(const MatArgs& a, cudaStream_t st);
 // rows. max_tiles: upper bound of the row tiles of a grouped launch.
 constexpr int MAT_GATHER_ROWS = 32;
 cudaError_t launch_mat_tc5(const MatArgs& a, int max_tiles, cudaStream_t st);
-int mat_tc5_take_timeout();    // as tc5_take_timeout (kernels.h)
 
 // ── the stream between the products ──
 // x0[t] = table[ids[t]] * scale (+ pos_table[tok_pos[t]], or null) (f32), xb (or null) = the same, or its norm (norm.w), in the

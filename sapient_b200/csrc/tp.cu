@@ -277,12 +277,17 @@ int Engine::tp_reset() {
     return SP_OK;
 }
 
+int Engine::report_wait(int kind) {
+    if (!finalized) { set_error("the engine has no stream yet"); return SP_ERR_STATE; }
+    SP_CUDA_TRY(cudaSetDevice(d.device));
+    SP_CUDA_TRY(launch_report_wait(waits_.dev, kind, stream));
+    return SP_OK;
+}
+
 int Engine::device_check() {
-    const int a = tc5_take_timeout(), b = imma_take_timeout(), c = mat_tc5_take_timeout(), q = dq_take_timeout();
-    if (a < 0 || b < 0 || c < 0 || q < 0) { set_error("could not read the kernels' timeout flags"); return SP_ERR_CUDA; }
-    if (a > 0 || q > 0) { set_error("tcgen05 GEMM: a bounded mbarrier wait expired, the outputs of that launch are not valid"); return SP_ERR_CUDA; }
-    if (c > 0) { set_error("tcgen05 GEMM on bf16 weights: a bounded mbarrier wait expired, the outputs of that launch are not valid"); return SP_ERR_CUDA; }
-    if (b > 0) { set_error("streaming GEMV: a bounded mbarrier wait expired, the outputs of that launch are not valid"); return SP_ERR_CUDA; }
+    // its own flags, and those of op-level calls on its device, which have no other call that waits for them
+    for (WaitFlags* f : {&waits_, &device_wait_flags()})
+        if (const char* what = f->take()) { set_error(what); return SP_ERR_CUDA; }
     return tp_check();
 }
 

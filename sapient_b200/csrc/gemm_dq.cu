@@ -25,9 +25,10 @@
 //               remainders of the sums, minima exact) times dmin, which costs a quarter instruction per element.
 // Columns are stored in the order 0 2 1 3 within groups of four, in activations and weights alike: the order in which masks
 // pick bytes out of a word, so that no weight is moved.
-// Measured against the kernel before (matmul with its split of activations): Q4_K 28672 x 4096, 32 rows 101 -> 54 us; 4096 x 14336
-// Q6_K, 37 rows 54.6 -> 37.1; Q4_K 4096 x 4096, 512 rows 85 -> 49; 28672 x 4096, 512 rows 285 -> 244 (its 128-row tiles are bounded by
-// the shared-memory traffic of the activation boxes). Short K is where it loses: Q8_0 17920 x 1536, 192 rows 33.9 -> 42.8. Error against float64 at K = 14336: 1.3e-5 -> 5e-7.
+// Measured against the kernel before (matmul with its split of activations), us: Q4_K 28672 x 4096, 32 rows 101 -> 51, 512 rows 285 -> 230;
+// 4096 x 14336 Q6_K, 37 rows 54.6 -> 35; Q4_K 4096 x 4096, 512 rows 85 -> 44; Q8_0 17920 x 1536, 192 rows 32.5 -> 33.5, 512 rows 71.7 ->
+// 68. That kernel took 256 activation rows per tile, one pass over the weights where two are made here, which still tells at the
+// largest products: Q6_K 20000 x 14336, 192 rows 268 -> 282. Error against float64 at K = 14336: 1.3e-5 -> 5e-7.
 // The K range of a tile is shared by the blocks of a cluster when tiles alone leave SMs idle; they meet in distributed shared
 // memory and add in part order, so results do not vary from run to run. Every wait on an mbarrier is bounded.
 #include <cuda.h>
@@ -405,8 +406,9 @@ __device__ __forceinline__ bool dq_drain(DqBars& bars, const uint8_t* raw, int r
 
 // The MMA warp's walk, an activation stage (BOXES boxes of 64 columns) at a time. The whole warp takes part and one elected thread
 // issues: control flow and operands are uniform then, as the tensor instructions want them. Issuing is the serial part of the
-// pipeline (a wait that is already over costs 100 to 250 cycles on a busy SM), so the barriers of the next half are looked at ahead of
-// a half's products and only waited for if they were not over by then.
+// pipeline (a wait that is already over costs 100 to 250 cycles on a busy SM), so the barriers of the next stage are looked at ahead of
+// a stage's products and only waited for if they were not over by then; with two weight planes half of the products go first, so
+// that the tensor pipe has work under the looks (Q8_0 28672 x 4096, 96 rows 84 -> 79 us; with one plane it costs 2 %).
 template <bool TWO, bool SIDE, int BOXES>
 __device__ __forceinline__ bool dq_issue(DqBars& bars, uint32_t tm, uint64_t bd0, uint32_t b16, int b_stages, uint32_t idesc, uint32_t idesc_side, int n_sb,
                                          int halves_last, bool leader, DqRing& ra, DqRing& rb, DqRing& rd, bool& seen, bool ok) {
@@ -436,13 +438,9 @@ __device__ __forceinline__ bool dq_issue(DqBars& bars, uint32_t tm, uint64_t bd0
                 rb.next(b_stages);
                 if (a_last) ra.next(DQ_A_SLOTS);
                 if (last) rd.next(2);
-                bool next = tc5_peek(&bars.full_b[rb.st], rb.u & 1);
-                // (where the next tile's format is another one, the other slot of the pair says the same: slots are filled in order)
-                if (a_last) next = tc5_peek(&bars.full_a[ra.st + (TWO ? 1 : 0)], ra.u & 1) && next;
-                if (last && rd.u > 0) next = tc5_peek(&bars.empty_d[rd.st], (rd.u - 1) & 1) && next;
-                if (leader) {
+                auto multiply = [&](int from, int to) {
 #pragma unroll
-                    for (int i = 0; i < 4 * BOXES; ++i) {
+                    for (int i = from; i < to; ++i) {
                         const uint32_t more = i > 0 || s > 0 ? 1u : (uint32_t)(h > 0), Ai = At + 32u * s + 8u * i;
                         const uint64_t bh = b0 + (i >> 2) * box16 + 2u * (i & 3);
                         if (SIDE) {
@@ -453,6 +451,15 @@ __device__ __forceinline__ bool dq_issue(DqBars& bars, uint32_t tm, uint64_t bd0
                         }
                         if (TWO) dq_mma(dt, Ai + 64u, bh, idesc, 1u);              // W_lo X_hi
                     }
+                };
+                constexpr int AHEAD = TWO ? 2 * BOXES : 0;  // columns / 16 multiplied before the looks
+                if (AHEAD > 0 && leader) multiply(0, AHEAD);
+                bool next = tc5_peek(&bars.full_b[rb.st], rb.u & 1);
+                // (where the next tile's format is another one, the other slot of the pair says the same: slots are filled in order)
+                if (a_last) next = tc5_peek(&bars.full_a[ra.st + (TWO ? 1 : 0)], ra.u & 1) && next;
+                if (last && rd.u > 0) next = tc5_peek(&bars.empty_d[rd.st], (rd.u - 1) & 1) && next;
+                if (leader) {
+                    multiply(AHEAD, 4 * BOXES);
                     tc5_commit(e_b);
                     if (a_last) {
                         if (TWO) tc5_commit(e_a - 1);
@@ -465,6 +472,39 @@ __device__ __forceinline__ bool dq_issue(DqBars& bars, uint32_t tm, uint64_t bd0
         }
     }
     return ok;
+}
+
+// The end of a tile: a lane's rows of y (row0, + 1, + 8, ..; left of them are there) at the columns n, + 8, + 16, + 24. Short straight
+// code: all that a warp does once per tile is fetched from far away, an instruction in some ten cycles, and with an address and
+// two bounds for each value a tile's end took 10 000 cycles (96 rows), twice what the two accumulators bridge (in shared memory first,
+// for stores of 128 bytes, it took as long). Q8_0 17920 x 1536, 192 rows 41.4 -> 33.7 us, 512 rows 80 -> 68.
+template <int NJT, bool WHOLE, bool RES>
+__device__ __forceinline__ void dq_store(const float (&acc)[2][NJT][4], const DqArgs& a, const Tc5Seg& sg, int64_t row0, int left, int n) {
+    float bias[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) bias[i] = sg.bias && (WHOLE || n + 8 * i < sg.n) ? sg.bias[n + 8 * i] : 0.f;
+    const float* xs = a.xscale + row0;
+    float sc[2 * NJT];  // (ahead of the stores, which the compiler takes for possible changes of them)
+#pragma unroll
+    for (int j = 0; j < 2 * NJT; ++j) sc[j] = (j >> 1) * 8 + (j & 1) < left ? xs[(j >> 1) * 8 + (j & 1)] : 0.f;
+    float* y = sg.y + row0 * a.ldy + n;
+    const float* r = RES ? a.res + row0 * a.ldres + n : nullptr;
+#pragma unroll
+    for (int j = 0; j < 2 * NJT; ++j) {
+        if ((j >> 1) * 8 + (j & 1) < left) {
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = fmaf(acc[i >> 1][j >> 1][2 * (i & 1) + (j & 1)], sc[j], bias[i]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (RES && (WHOLE || n + 8 * i < sg.n)) v[i] += r[8 * i];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (WHOLE || n + 8 * i < sg.n) y[8 * i] = v[i];
+        }
+        y += (j & 1) ? 7 * (int64_t)a.ldy : (int64_t)a.ldy;
+        if (RES) r += (j & 1) ? 7 * (int64_t)a.ldres : (int64_t)a.ldres;
+    }
 }
 
 // Which matrix and rows a tile is.
@@ -629,37 +669,27 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
             const float* res = it.si == 0 ? a.res : nullptr;
             if (a.parts == 1) {
                 if (ok) {
-#pragma unroll
-                    for (int j = 0; j < NJT; ++j)
-#pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            const int ml = (half * NJT + j) * 8 + 2 * t + c, m = it.m0 + ml;
-                            if (ml >= it.rows) continue;
-                            const float sc = a.xscale[m];
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const int n = it.n0 + 32 * quarter + 16 * (i >> 1) + 8 * (i & 1) + g;
-                                if (n >= sg.n) continue;
-                                float v = fmaf(acc[i >> 1][j][2 * (i & 1) + c], sc, sg.bias ? sg.bias[n] : 0.f);
-                                if (res) v += res[(int64_t)m * a.ldres + n];
-                                sg.y[(int64_t)m * a.ldy + n] = v;
-                            }
-                        }
+                    const int left = it.rows - half * NJT * 8 - 2 * t, n = it.n0 + 32 * quarter + g;
+                    const bool whole = it.n0 + 32 * quarter + 32 <= sg.n;
+                    const int64_t row0 = it.m0 + half * NJT * 8 + 2 * t;
+                    if (whole && res) dq_store<NJT, true, true>(acc, a, sg, row0, left, n);
+                    else if (whole) dq_store<NJT, true, false>(acc, a, sg, row0, left, n);
+                    else if (res) dq_store<NJT, false, true>(acc, a, sg, row0, left, n);
+                    else dq_store<NJT, false, false>(acc, a, sg, row0, left, n);
                 }
                 continue;
             }
             // (a block of a cluster takes one tile)
             asm volatile("bar.sync 1, 256;\n" ::: "memory");  // nobody reads raw tiles or sums any more: their memory takes the partial tile
             float* const partial = reinterpret_cast<float*>(smem);
+            static_assert(DQ_NB * DQ_P_STRIDE * 4 <= DQ_SMEM - 1024, "a partial tile of any height");
+            // (rows that are not there too: nobody reads them)
+            float* const mine_at = partial + (half * NJT * 8 + 2 * t) * DQ_P_STRIDE + 32 * quarter + g;
 #pragma unroll
-            for (int j = 0; j < NJT; ++j)
+            for (int j = 0; j < 2 * NJT; ++j)
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const int ml = (half * NJT + j) * 8 + 2 * t + c;
-                    if (ml >= it.rows) continue;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) partial[ml * DQ_P_STRIDE + 32 * quarter + 16 * (i >> 1) + 8 * (i & 1) + g] = acc[i >> 1][j][2 * (i & 1) + c];
-                }
+                for (int i = 0; i < 4; ++i)
+                    mine_at[((j >> 1) * 8 + (j & 1)) * DQ_P_STRIDE + 16 * (i >> 1) + 8 * (i & 1)] = acc[i >> 1][j >> 1][2 * (i & 1) + (j & 1)];
             __syncwarp();
             cluster_sync();
             // the cluster's blocks share out the activation rows; each adds its rows' partials in part order
@@ -767,29 +797,30 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
         return cudaSuccess;
     });
     if (le != cudaSuccess) return le;
-    // parts: what makes the longest SM's share shortest, a block's start and end counted as three spans of 256 columns
-    const int items = tiles * a.m_tiles, all_sb = (k + 255) / 256;
-    auto best_split = [&](int n, long& cost, bool lone) {
-        int best = 1;
+    // How the tiles are dealt out, by the longest SM's time in tenths of a span of 256 columns. One block per SM that walks over tiles:
+    // a tile is its spans and 3, the walk's start 10. Clusters that share a tile's K range: every wave of them is its spans and 45 (5
+    // less for the first, whose start lies under the kernel before). Where tiles go over whole rounds of the SMs, those that do may
+    // have a launch of their own, 30 for the launch. Fitted to forced choices over 13 shapes x 6 row counts x 3 formats, of which the
+    // rule takes the fastest or one within 4 %. In us: Q4_K 6144 x 4096, 512 rows (192 tiles) walked 74.7, clusters of two 84.5, a walk
+    // and 44 tiles shared by two 70.6; 20000 x 14336, 20 rows (157 tiles) 160, clusters of four 121, nine tiles shared by eight 97;
+    // 8960 x 1536, 300 rows (210 tiles) 37 walked, 39 in two launches.
+    const int items = tiles * a.m_tiles, all_sb = (k + 255) / 256, sms = device_sm_count();
+    auto shared = [&](int n, int& parts) {
+        long cost = 0;
         for (int p = 1; p <= std::min(DQ_MAX_PARTS, all_sb); ++p) {
-            const long waves = (n + dq_clusters(p) - 1) / dq_clusters(p), sb = (all_sb + p - 1) / p;
-            const long c = p == 1 && lone ? waves * sb + 3 : waves * (sb + 3) + 1;  // (a lone block runs from tile to tile)
-            if (p == 1 || c < cost) { best = p; cost = c; }
+            const long waves = (n + dq_clusters(p) - 1) / dq_clusters(p), c = waves * (10 * ((all_sb + p - 1) / p) + 45) - 5;
+            if (p == 1 || c < cost) { parts = p; cost = c; }
         }
-        return best;
+        return cost;
     };
-    long cost = 0;
-    a.parts = best_split(items, cost, true);
-    a.items = items;
-    // A few tiles over whole rounds of the SMs (28672 rows in tiles of 128, 512 activation rows: 896 = 6 x 148 + 8) would take a round
-    // of their own: they get a second launch that shares out their K range where that is shorter, its own start counted as two spans
-    // more. Measured there: Q4_K, K = 4096 270 -> 244 us, and 145 -> 121 at 192 rows (448 = 3 x 148 + 4).
-    const int sms = device_sm_count(), over = items % sms;
-    int tail_parts = 0;
-    if (a.parts == 1 && items > sms && over > 0) {
-        long tail = 0;
-        tail_parts = best_split(over, tail, false);
-        if (tail + 2 >= all_sb) tail_parts = 0;
+    auto walked = [&](int n) { return (long)((n + sms - 1) / sms) * (10 * all_sb + 3) + 10; };
+    int walk = items, parts = 1;  // tiles that are walked over; the rest is shared by `parts` blocks each
+    long cost = walked(items);
+    for (const int first : {0, items / sms * sms}) {
+        int p = 1;
+        if (first == items) continue;
+        const long c = shared(items - first, p) + (first > 0 ? walked(first) + 30 : 0);
+        if (c < cost) { cost = c; walk = first; parts = p; }
     }
     const PFN_encodeTiled encode = tensor_map_encoder();
     if (!encode) return cudaErrorNotSupported;
@@ -807,13 +838,13 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
     auto launch = [&](int from, int to, int parts) {
         a.item0 = from; a.items = to; a.parts = parts;
         const int n = to - from;
+        if (n == 0) return cudaSuccess;
         const dim3 grid((unsigned)(parts == 1 ? std::min(n, sms) : n), 1, (unsigned)parts);
         const cudaError_t e = launch_pdl_cluster(kernel, grid, dim3(DQ_THREADS), DQ_SMEM, st, parts, a, tmap);
         return e != cudaSuccess ? e : count_launch_and_check();
     };
-    if (!tail_parts) return launch(0, items, a.parts);
-    le = launch(0, items - over, 1);
-    return le != cudaSuccess ? le : launch(items - over, items, tail_parts);
+    le = launch(0, walk, 1);
+    return le != cudaSuccess ? le : launch(walk, items, parts);
 }
 
 }  // namespace sp

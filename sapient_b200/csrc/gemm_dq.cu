@@ -30,7 +30,8 @@
 // 68. That kernel took 256 activation rows per tile, one pass over the weights where two are made here, which still tells at the
 // largest products: Q6_K 20000 x 14336, 192 rows 268 -> 282. Error against float64 at K = 14336: 1.3e-5 -> 5e-7.
 // The K range of a tile is shared by the blocks of a cluster when tiles alone leave SMs idle; they meet in distributed shared
-// memory and add in part order, so results do not vary from run to run. Every wait on an mbarrier is bounded.
+// memory and add in part order, so results do not vary from run to run. Every wait on an mbarrier is bounded; after one that ran out
+// nothing more is issued, the warps that did issue wait (bounded) for their copies and products in flight, y is left alone.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -243,7 +244,7 @@ struct DqTile {
 
 struct DqBars {
     uint64_t full_r[DQ_MAX_R], empty_r[DQ_MAX_R], full_a[DQ_A_SLOTS], empty_a[DQ_A_SLOTS], full_b[DQ_MAX_B], empty_b[DQ_MAX_B];
-    uint64_t full_x[DQ_X_STAGES], empty_x[DQ_X_STAGES], full_d[2], empty_d[2];
+    uint64_t full_x[DQ_X_STAGES], empty_x[DQ_X_STAGES], full_d[2], empty_d[2], idle;
 };
 
 // Where a warp stands in a ring of `n` stages: the stage and how often the ring has wrapped. Carried from tile to tile.
@@ -453,12 +454,12 @@ __device__ __forceinline__ bool dq_issue(DqBars& bars, uint32_t tm, uint64_t bd0
                     }
                 };
                 constexpr int AHEAD = TWO ? 2 * BOXES : 0;  // columns / 16 multiplied before the looks
-                if (AHEAD > 0 && leader) multiply(0, AHEAD);
+                if (AHEAD > 0 && leader && ok) multiply(0, AHEAD);
                 bool next = tc5_peek(&bars.full_b[rb.st], rb.u & 1);
                 // (where the next tile's format is another one, the other slot of the pair says the same: slots are filled in order)
                 if (a_last) next = tc5_peek(&bars.full_a[ra.st + (TWO ? 1 : 0)], ra.u & 1) && next;
                 if (last && rd.u > 0) next = tc5_peek(&bars.empty_d[rd.st], (rd.u - 1) & 1) && next;
-                if (leader) {
+                if (leader && ok) {
                     multiply(AHEAD, 4 * BOXES);
                     tc5_commit(e_b);
                     if (a_last) {
@@ -550,6 +551,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
         for (int s = 0; s < a.b_stages; ++s) { dq_init(&bars.full_b[s], 1); dq_init(&bars.empty_b[s], 1); }
         for (int s = 0; s < DQ_X_STAGES; ++s) { dq_init(&bars.full_x[s], 1); dq_init(&bars.empty_x[s], DQ_DRAINS); }
         for (int s = 0; s < 2; ++s) { dq_init(&bars.full_d[s], 1); dq_init(&bars.empty_d[s], DQ_DRAINS); }
+        dq_init(&bars.idle, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -582,7 +584,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
                     }
                 }
                 // (all copies land before the block ends, whatever became of their readers)
-                for (int i = max(0, issued - a.r_stages); i < issued && ok; ++i) ok = tc5_wait(&bars.full_r[i % a.r_stages], (uint32_t)((i / a.r_stages) & 1));
+                for (int i = max(0, issued - a.r_stages); i < issued; ++i) ok = tc5_wait(&bars.full_r[i % a.r_stages], (uint32_t)((i / a.r_stages) & 1)) && ok;
             }
             __syncwarp();
             pdl_wait();
@@ -592,6 +594,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
         }
         if (warp == 2 && lane == 0) {
             DqRing r, rx;
+            int boxes = 0, sums = 0;
             for (int item = a.item0 + blockIdx.x; item < a.items && ok; item += gridDim.x) {
                 const DqItem it(a, item);
                 for (int sb = 0; sb < n_sb && ok; ++sb) {
@@ -604,6 +607,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
                         for (int c = 0; c < 2 * BOXES; ++c)
                             tc5_tma_2d(dst + c * a.nb * 128, &tmap_x, (sb0 + sb) * 256 + 64 * (BOXES * h + (c >> 1)), (c & 1) * a.m + it.m0, bar);
                         r.next(a.b_stages);
+                        ++boxes;
                     }
                     if (it.dt == T_Q4_K && ok) {
                         ok = rx.empty(bars.empty_x);
@@ -612,9 +616,12 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
                         dq_expect(bar, (uint32_t)(it.rows * 32));
                         dq_bulk(tc5_smem_u32(xs + rx.st * x_bytes), a.xsum + ((int64_t)(sb0 + sb) * a.m + it.m0) * 16, (uint32_t)(it.rows * 32), bar);
                         rx.next(DQ_X_STAGES);
+                        ++sums;
                     }
                 }
             }
+            for (int i = max(0, boxes - a.b_stages); i < boxes; ++i) ok = tc5_wait(&bars.full_b[i % a.b_stages], (uint32_t)((i / a.b_stages) & 1)) && ok;
+            for (int i = max(0, sums - DQ_X_STAGES); i < sums; ++i) ok = tc5_wait(&bars.full_x[i % DQ_X_STAGES], (uint32_t)((i / DQ_X_STAGES) & 1)) && ok;
         } else if (warp == 0) {
             const bool leader = tc5_elect();
             // fp16 x fp16 -> f32; N is the tile height, twice that where both planes stand side by side
@@ -629,6 +636,10 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
                 if (it.dt == T_Q4_K) SP_DQ_ISSUE(false);
                 else SP_DQ_ISSUE(true);
 #undef SP_DQ_ISSUE
+            }
+            if (!ok && leader) {  // what has been issued reads shared and writes tensor memory
+                tc5_commit(&bars.idle);
+                tc5_wait(&bars.idle, 0);
             }
         }
         __syncwarp();
@@ -694,7 +705,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
             cluster_sync();
             // the cluster's blocks share out the activation rows; each adds its rows' partials in part order
             const int idx = tid - 32 * DQ_FIRST_DRAIN, nl = idx & 127, n = it.n0 + nl;
-            if (n < sg.n) {
+            if (n < sg.n && ok) {
                 const float bias = sg.bias ? sg.bias[n] : 0.f;
                 const uint32_t mine = tc5_smem_u32(partial + nl);
                 constexpr int NC = 4;

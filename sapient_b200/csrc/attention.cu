@@ -226,9 +226,11 @@ cudaError_t launch_attention(const float* q, int ldq, float* out, int ldo, int n
 // whole key range once per query token; here a block takes 64 query rows of one head (4 warps x 16 rows), walks the keys
 // in tiles of 64 (4 pages) staged in shared memory, and does both contractions with mma.sync.m16n8k16 (K and V are fp16 in the
 // cache already, f32 accumulation), with the reference's online-softmax recurrence (kernels/attention.rs:98-165) applied per
-// 64-key tile. EXACT (engines with exact-class operands): q, scaled per row by a power of two into (-1, 1), and the softmax
-// weights each enter as an fp16 leading part plus remainder, two products each, so the result is that of the f32 kernels to
-// 2^-22 per operand; otherwise both are rounded to fp16.
+// 64-key tile. EXACT (engines with exact-class operands): q, scaled per row by a power of two into (-2^15, 2^15), and the softmax
+// weights times 2^14 each enter as an fp16 leading part plus remainder, two products each: 22 bits of every query coordinate down to
+// 2^-18 of the row's largest and of every weight down to 2^-17; smaller ones to 2^-40 of the largest, 2^-39 of the largest weight,
+// where a remainder becomes one of fp16's subnormal numbers. (Unscaled those begin at 2^-14, and weights under 2^-25 were missing
+// from the sum but not from its denominator.) Otherwise both are rounded to fp16.
 // Per query token the kernels above read every key again: 389 tokens of the Phi-2 shape (32 heads, none shared) took 325 us a
 // layer on the f32 kernel, 512 of the 8B shape 91 us on the grouped one; tiles of 64 rows take 31 and 42 us.
 namespace sp {
@@ -251,6 +253,7 @@ __global__ void __launch_bounds__(FA_WARPS * 32)
 attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict__ out, __half* __restrict__ out_h, int ldo, int n_tok,
                          int n_heads, int slot, int pos0, KvGeom kv, int layer, float scale) {
     constexpr int HD = HD16 * 16, LD = HD + 8;  // padded row of the shared tiles (halves): conflict-free fragment loads
+    constexpr float WEIGHT_UP = EXACT ? 16384.f : 1.f;
     extern __shared__ __align__(16) __half fa_smem[];
     // two (K, V) tile buffers: cp.async fills one while the tensor cores work on the other
     constexpr int TILE = FA_KEYS * LD;
@@ -278,12 +281,12 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
                 a0 = fmaxf(a0, fmaxf(fabsf(x0.x), fabsf(x0.y)));
                 a1 = fmaxf(a1, fmaxf(fabsf(x1.x), fabsf(x1.y)));
             }
-            auto unit = [&](float amax, float& up, float& down) {  // power of two that brings the row into (-1, 1), and scale times its inverse
+            auto unit = [&](float amax, float& up, float& down) {  // power of two that brings the row into (-2^15, 2^15), and scale times its inverse
                 amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
                 amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
                 const int e = amax > 0.f && amax < INFINITY ? max(-100, min(100, ilogbf(amax) + 1)) : 0;
-                up = scalbnf(1.0f, -e);
-                down = scalbnf(scale, e);
+                up = scalbnf(1.0f, 15 - e);
+                down = scalbnf(scale, e - 15);
             };
             unit(a0, u0, sc0);
             unit(a1, u1, sc1);
@@ -375,12 +378,13 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
             const float e2 = (s[j][2] == -INFINITY) ? 0.f : expf(s[j][2] - n1), e3 = (s[j][3] == -INFINITY) ? 0.f : expf(s[j][3] - n1);
             sum0 += e0 + e1;
             sum1 += e2 + e3;
-            const __half2 w0 = __floats2half2_rn(e0, e1), w1 = __floats2half2_rn(e2, e3);
+            const float g0 = e0 * WEIGHT_UP, g1 = e1 * WEIGHT_UP, g2 = e2 * WEIGHT_UP, g3 = e3 * WEIGHT_UP;
+            const __half2 w0 = __floats2half2_rn(g0, g1), w1 = __floats2half2_rn(g2, g3);
             pa[j >> 1][(j & 1) * 2] = *reinterpret_cast<const uint32_t*>(&w0);
             pa[j >> 1][(j & 1) * 2 + 1] = *reinterpret_cast<const uint32_t*>(&w1);
             if (EXACT) {
-                pl[EXACT ? j >> 1 : 0][(j & 1) * 2] = pack_half2(e0 - __low2float(w0), e1 - __high2float(w0));
-                pl[EXACT ? j >> 1 : 0][(j & 1) * 2 + 1] = pack_half2(e2 - __low2float(w1), e3 - __high2float(w1));
+                pl[EXACT ? j >> 1 : 0][(j & 1) * 2] = pack_half2(g0 - __low2float(w0), g1 - __high2float(w0));
+                pl[EXACT ? j >> 1 : 0][(j & 1) * 2 + 1] = pack_half2(g2 - __low2float(w1), g3 - __high2float(w1));
             }
         }
         sum0 += __shfl_xor_sync(0xFFFFFFFFu, sum0, 1); sum0 += __shfl_xor_sync(0xFFFFFFFFu, sum0, 2);
@@ -411,7 +415,7 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
         }
         __syncthreads();  // this tile's buffer may be refilled from the next iteration on
     }
-    const float i0 = (l0 == 0.f) ? 0.f : 1.0f / l0, i1 = (l1 == 0.f) ? 0.f : 1.0f / l1;
+    const float i0 = (l0 == 0.f) ? 0.f : 1.0f / l0 / WEIGHT_UP, i1 = (l1 == 0.f) ? 0.f : 1.0f / l1 / WEIGHT_UP;
 #pragma unroll
     for (int nd = 0; nd < 2 * HD16; ++nd) {
         const int64_t c = (int64_t)h * HD + 8 * nd + 2 * t;

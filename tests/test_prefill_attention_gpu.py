@@ -5,7 +5,8 @@ and against the oracle."""
 import numpy as np
 import pytest
 
-from helpers import oracle_engine, tiny_model
+from helpers import oracle_engine, rel_l2, tiny_model
+from sapient_b200 import ops, synth
 from sapient_b200.engine import ForwardEngine
 
 pytestmark = pytest.mark.gpu
@@ -80,3 +81,49 @@ def test_tiled_attention_with_exact_operands(oracle, name, n_prompt):
     assert np.abs(a[1] - ref).max() < 3e-3
     big.close()
     small.close()
+
+
+@pytest.mark.parametrize("heads,depth", [(8, 18.4), (8, 16.0), (4, 12.0)])
+def test_long_flat_tails_keep_their_weight(oracle, heads, depth):
+    """The first token has all of the weight but e^-depth per other token, and a value of zero: what comes out of the attention is the sum
+    of up to 900 weights far below fp16's range (e^-18.4 = 2^-26.5). Queries and keys are one coordinate each, of a pair that the
+    rotation leaves where it is (base 1e30). Scores of size depth in f32: 2^-23 depth per weight and the same in the reference, 1e-5;
+    remainders of small weights are whole multiples of 2^-38 of the largest weight, so each may be 2^-39 off."""
+    import torch
+
+    hid = 256
+    shape = dict(arch="qwen2", n_layers=1, hidden=hid, n_heads=heads, n_kv_heads=heads, head_dim=64, ffn=256, vocab=320, norm_eps=1e-5, rope_theta=1e30,
+                 tied=False, qkv_bias=True)
+    cfg, W = synth.build_model(shape, seed=5, device="cpu", max_ctx=1024)
+
+    def put(name, m):
+        dt, dims, _ = W[name]
+        W[name] = (dt, dims, synth.quantize(dt, m).reshape(-1) if dt != synth.F32 else m.contiguous().view(torch.uint8).reshape(-1))
+
+    n, p = heads * 64, "model.layers.0."
+    embed = torch.randn(320, hid, generator=torch.Generator().manual_seed(1)) * 0.02
+    embed[:2] = 0.0
+    embed[0, 0] = embed[1, 1] = 1.0  # after the norm: 16 in this column
+    put("model.embed_tokens.weight", embed)
+    put(p + "input_layernorm.weight", torch.ones(hid))
+    k, v, at = torch.zeros(n, hid), torch.zeros(n, hid), torch.arange(20, n, 64)
+    k[at, 0] = depth / 16
+    v[:, 1] = 30000.0 / 16
+    qb = torch.zeros(n)
+    qb[at] = 8.0
+    put(p + "self_attn.q_proj.weight", torch.zeros(n, hid))
+    put(p + "self_attn.k_proj.weight", k)
+    put(p + "self_attn.v_proj.weight", v)
+    put(p + "self_attn.q_proj.bias", qb)
+    for name in ("self_attn.k_proj.bias", "self_attn.v_proj.bias"):
+        put(p + name, torch.zeros(n))
+    W = synth.weights_to_numpy(W)
+    dt, dims, raw = W[p + "self_attn.k_proj.weight"]
+    depth = 16.0 * float(ops.Weight(dt, *dims, raw).dequant().max())  # as quantised
+    ids = np.array([0] + [1] * 899, np.uint32)
+    eng = ForwardEngine.from_weights(cfg, W, max_tokens=1024)
+    eng.set_kv_rounding(False)
+    got = eng.forward_logits(ids, False)
+    ref = oracle_engine(oracle, cfg, W, kv_mode=1).forward_logits(ids, True)  # (from the cache, with its fp16 rounding)
+    assert rel_l2(got, ref) < 3e-5 + 2.0 ** -39 * np.exp(depth), rel_l2(got, ref)
+    eng.close()

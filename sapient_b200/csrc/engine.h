@@ -14,6 +14,7 @@
 #include <string>
 #include <vector>
 
+#include "copy_pool.h"
 #include "../../include/sapient_cuda.h"
 #include "kernels.h"
 #include "page_pool.h"
@@ -289,6 +290,7 @@ class Engine {
     float* p_logits_ = nullptr;
     static constexpr int COPY_EVENTS = 32, COPY_HELPERS = 7;
     cudaEvent_t copy_done_[COPY_EVENTS] = {};  // of fetch_logits
+    CopyPool copy_pool_;
     uint32_t* p_argmax_ = nullptr;
     // device-resident greedy loop
     uint32_t* d_tokens_ = nullptr;

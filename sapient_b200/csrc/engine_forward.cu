@@ -5,8 +5,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
-#include <system_error>
-#include <thread>
 
 #include "engine.h"
 #include "engine_plan.h"
@@ -144,9 +142,10 @@ int Engine::enqueue_decode_step(int T) {
     return enqueue_head(0, T);
 }
 
-// The first n floats of logits_ to host memory of the caller's, through the pinned buffer. Beyond four megabytes that is several
-// copies in flight on the device and on the host: a lone thread takes longer to write a caller's fresh pages (32 rows of 128256
-// logits: 1.6 ms) than the device to make them. Returns with the stream's work done.
+// The first n floats of logits_ to host memory of the caller's, through the pinned buffer. From eight slices (four megabytes) on that is
+// several copies in flight on the device and on the host: a lone thread takes longer to write a caller's fresh pages (32 rows of
+// 128256 logits: 1.6 ms) than the device to make them. This thread waits for the first copy alone; the engine's helpers, which
+// sleep until then, are woken for what is left. Returns with the stream's work done.
 int Engine::fetch_logits(float* out, size_t n) {
     constexpr size_t SLICE = (size_t)1 << 17;  // floats
     const int slices = (int)((n + SLICE - 1) / SLICE);
@@ -163,26 +162,15 @@ int Engine::fetch_logits(float* out, size_t n) {
         SP_CUDA_TRY(cudaMemcpyAsync(p_logits_ + first(g), logits_ + first(g), (first(g + 1) - first(g)) * 4, cudaMemcpyDeviceToHost, stream));
         SP_CUDA_TRY(cudaEventRecord(copy_done_[g], stream));
     }
+    SP_CUDA_TRY(cudaEventSynchronize(copy_done_[0]));
     std::atomic<int> next{0}, failed{0};
-    auto work = [&] {
+    copy_pool_.run(std::min(COPY_HELPERS, slices / 2), [&] {
         cudaSetDevice(d.device);
         for (int g; (g = next.fetch_add(1)) < groups;) {
             if (cudaEventSynchronize(copy_done_[g]) != cudaSuccess) { failed.store(1); return; }
             std::memcpy(out + first(g), p_logits_ + first(g), (first(g + 1) - first(g)) * 4);
         }
-    };
-    std::thread helpers[COPY_HELPERS];
-    const int want = std::min(COPY_HELPERS, slices / 2);
-    for (int i = 0; i < want; ++i) {
-        try {
-            helpers[i] = std::thread(work);
-        } catch (const std::system_error&) {
-            break;  // those that run, and this thread, do it all
-        }
-    }
-    work();
-    for (std::thread& t : helpers)
-        if (t.joinable()) t.join();
+    });
     SP_CUDA_TRY(cudaStreamSynchronize(stream));
     if (failed.load()) { set_error("copy of the logits failed"); return SP_ERR_CUDA; }
     return SP_OK;

@@ -321,6 +321,9 @@ int32_t sp_cuda_matmul_nt_dev(const SpWeight* w, const float* x_dev, int64_t m, 
             SP_CUDA_TRY(launch_gemm_dq(&sg, 1, (int)w->k, wm->ws.dq(), (int)m, (int)w->n, nullptr, 0, (cudaStream_t)stream));
             return SP_OK;
         }
+        cudaStreamCaptureStatus capturing;
+        SP_CUDA_TRY(cudaStreamIsCapturing((cudaStream_t)stream, &capturing));
+        if (capturing == cudaStreamCaptureStatusNone) SP_CUDA_TRY(wm->ws.ensure_split());  // else, on a first call, no wave is split
         SP_CUDA_TRY(launch_x_to_f16(x_dev, (int)w->k, (int)m, (int)w->k, wm->ws.xh, (cudaStream_t)stream));
         SP_CUDA_TRY(launch_gemm_tc5(w->tiled, w->dtype, (int)w->n, (int)w->k, wm->ws.xh, (int)m, y_dev, (int)w->n, nullptr, nullptr, 0,
                                     (cudaStream_t)stream, &wm->ws.tc5, wm->ws.waits));
@@ -929,10 +932,7 @@ int32_t sp_cuda_engine_set_large_m_gemm(SpEngine* e, int32_t on) {
     if (!e) { set_error("null engine"); return SP_ERR_ARG; }
     SP_CUDA_TRY(cudaSetDevice(e->e->d.device));
     if (on < 0 || on > 2) { set_error("large-M mode must be 0, 1 or 2"); return SP_ERR_ARG; }
-    e->e->use_tc5 = on != 0;
-    e->e->tc5_exact = on == 2;
-    e->e->drop_graphs();
-    return SP_OK;
+    return e->e->set_large_m_gemm(on);
     API_END
 }
 

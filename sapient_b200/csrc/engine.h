@@ -147,6 +147,7 @@ class Engine {
     // 10 rows at any row count (7x slower on a 512-token prompt). sp_cuda_engine_set_large_m_gemm chooses.
     bool use_tc5 = true;
     bool tc5_exact = true;
+    int set_large_m_gemm(int mode);                 // 2 exact class, 1 fp16-rounded, 0 integer passes
     bool graph_step_ = false;  // a step is being captured: its kernels may take positions only from device memory
     // 1 (default): new K / V rows get the reference's Q8_0 cache rounding before they are stored as fp16 (head_dim % 32
     // == 0, where the reference keeps a Q8_0 cache); 0: plain fp16 rounding. Change only while the caches are empty.

@@ -89,6 +89,14 @@ void Engine::drop_graphs() {
     step_graph_kernels_.clear();
 }
 
+int Engine::set_large_m_gemm(int mode) {
+    if (mode == 1 && ws_.xh) SP_CUDA_TRY(ws_.ensure_split());
+    use_tc5 = mode != 0;
+    tc5_exact = mode == 2;
+    drop_graphs();
+    return SP_OK;
+}
+
 int Engine::drain_async() {
     if (!async_pending_) return SP_OK;
     async_pending_ = false;

@@ -565,6 +565,7 @@ cudaError_t Tc5Scratch::alloc() {
     cudaError_t e = cudaMalloc((void**)&buf, parts_cap * TC5_NB_MAX * TC5_BM * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void**)&cnt, TC5_SPLIT_MAX_ITEMS * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(cnt, 0, TC5_SPLIT_MAX_ITEMS * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // the launches may go to a stream that does not wait for this one
     if (e != cudaSuccess) release();
     return e;
 }

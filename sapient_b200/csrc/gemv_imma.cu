@@ -538,9 +538,10 @@ cudaError_t ActWorkspace::ensure_xh(size_t elems) {
         xscale = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(xh) + bytes);
         xsum = reinterpret_cast<__half*>(xscale + XSCALE_ROWS);
     }
-    if (e == cudaSuccess && !tc5.buf) e = tc5.alloc();
     return e;
 }
+
+cudaError_t ActWorkspace::ensure_split() { return tc5.buf ? cudaSuccess : tc5.alloc(); }
 
 DqInput ActWorkspace::dq() const { return DqInput{xh, xscale, xsum, waits}; }
 

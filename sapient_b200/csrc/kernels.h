@@ -168,8 +168,9 @@ struct ActWorkspace {
     static constexpr int XSCALE_ROWS = 4096;
     DqInput dq() const;
     int* waits = nullptr;      // WaitFlags of the owner
-    Tc5Scratch tc5;            // allocated with xh
+    Tc5Scratch tc5;            // only where the GEMM with fp16-rounded operands was chosen
     cudaError_t ensure_xh(size_t elems);  // grows the buffer (allocates: not during stream capture)
+    cudaError_t ensure_split();           // makes tc5 (allocates: not during stream capture)
     static constexpr int NCP_MAX = 96;  // digit columns: 32 rows x 3 digits (gemv_rows.cu); the tile-row kernel uses up to 32
     cudaError_t alloc(int k_max_);
     void release();

@@ -59,7 +59,7 @@ def test_large_m_gemm_matches_oracle_and_gemv(oracle, dtype, m, k, n):
 @pytest.mark.parametrize("dtype", [Q4_K, Q6_K, Q8_0])
 @pytest.mark.parametrize("m,k,n", CASES + [(32, 4096, 1024), (64, 2048, 640), (200, 4096, 300), (128, 14336, 256)])
 def test_exact_operand_mode_is_at_the_level_of_the_integer_path(oracle, dtype, m, k, n):
-    """Mode 2: weights and activations each as an fp16 leading part plus remainder, three products per chunk of K. The
+    """Mode 2: activations as an fp16 leading part plus remainder, weights unrounded in one or two operand planes. The
     result must sit where the exact integer-digit GEMV sits (2e-5 of the oracle, whose own f32 sums differ by that much
     between summation orders), two hundred times below the fp16-operand mode."""
     be, _ = synth.BLOCK[dtype]
@@ -164,3 +164,32 @@ def test_exact_operands_at_the_edges_of_tiles(dtype, m, k, n):
     err = (y.double() - want)[rows].norm(dim=1) / want[rows].norm(dim=1)
     assert torch.all(y[3] == 0.0)
     assert float(err.max()) < 8e-6, float(err.max())
+
+
+def test_only_rounded_operands_hold_a_buffer_for_shared_tiles():
+    """19 MB on 148 SMs for each weight (or engine) whose steps may split their last tiles over several blocks, which the exact-class
+    kernel does without memory."""
+    import torch
+
+    raw = synth.random_bit_blocks(Q4_K, 256 * 256 // 256, seed=5)
+    x, y = torch.randn(17, 256, device="cuda"), torch.empty(17, 256, device="cuda")
+
+    def used(mode):
+        _large_m(mode)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        for w in weights:
+            w.matmul_nt_dev(x.data_ptr(), 17, y.data_ptr())
+        torch.cuda.synchronize()
+        return before - torch.cuda.mem_get_info()[0]
+
+    weights = [ops.Weight(Q4_K, 256, 256, raw) for _ in range(9)]
+    first = weights.pop()
+    for mode in (1, 2):  # what the process allocates once
+        _large_m(mode)
+        first.matmul_nt_dev(x.data_ptr(), 17, y.data_ptr())
+    # 17 x 256 split activations and their sums are 20 KB a weight; allocations come out of blocks of 2 MB
+    assert used(2) <= 8 * (2 << 20)
+    assert used(1) >= 8 * 148 * 128 * 256 * 4 * 0.9 or torch.cuda.get_device_properties(0).multi_processor_count != 148
+    for w in weights + [first]:
+        w.free()

@@ -158,7 +158,7 @@ B32_BATCH, B32_PROMPT, B32_WARM, B32_STEPS = 32, 1024, 4, 24
 def batch32_section(cfg, W, wbytes: int, local: int, rank: int, world: int, stream, barrier, peaks) -> dict:
     """The other half of the metric: 32 sequences with 1024-token prompts decoded together over the paged fp16 KV cache
     (the tensor-parallel configuration of the benchmark at its own sizes; one GPU holds it whole, N GPUs split it).
-    Three timings of the same step at context ~1024: the default (tcgen05 GEMM with exact-class operands), the same GEMM
+    Three timings of the same step at context ~1024: the default (tcgen05 GEMM with exact-class operands), the GEMM
     with operands rounded to fp16 (opt-in) and integer-digit GEMV passes of 10 rows (opt-in). Prompts are prefilled
     untimed on the fastest path in every case."""
     import torch
@@ -212,7 +212,7 @@ def batch32_section(cfg, W, wbytes: int, local: int, rank: int, world: int, stre
         out[tag] = {"tokens_per_s": B32_BATCH * B32_STEPS / (ms / 1e3), "ms_per_step": ms / B32_STEPS, "context": ctx_mid,
                     "bytes_per_step_per_gpu": int(step_bytes), "achieved_gbs_per_gpu": gbs, "frac_of_measured_peak": gbs / peaks["hbm_gbs"],
                     "frac_of_8TBs": gbs / 8000.0}
-    out["exact"]["path"] = "tcgen05 / TMEM dequant GEMM, exact-class operands (fp16 leading part + remainder of weights and activations), the default"
+    out["exact"]["path"] = "tcgen05 / TMEM dequant GEMM, exact-class operands (activations as fp16 leading part + remainder, weights unrounded), the default"
     out["tcgen05"]["path"] = "tcgen05 / TMEM dequant GEMM, operands rounded to fp16 (opt-in)"
     out["integer_passes"]["path"] = "integer-digit mma.sync GEMV passes of 10 rows (opt-in)"
     eng.close()
@@ -223,7 +223,8 @@ def sweep_section() -> list:
     """Operator sweep of the standalone dequant-matmul for the four benchmark shapes and the three block formats (weights
     rotated through more than twice the L2, CUDA events on the launching stream): achieved GB/s at M = 1 (tensor-core GEMV)
     and at M = 32 (the default for 17 rows and more: tcgen05 GEMM with exact-class operands) and TFLOP/s at M = 512 on the
-    tcgen05 GEMM in both modes (useful flops; the exact-class mode issues three products per useful one)."""
+    tcgen05 GEMM in both modes (useful flops; the exact-class mode issues two products per useful one
+    for Q4_K, three for Q6_K and Q8_0)."""
     from sapient_b200 import sweep
 
     rows = []
@@ -240,7 +241,7 @@ def sweep_section() -> list:
                          "m512_us": round(r512x["us"], 1), "m512_tflops": round(r512x["tflops"], 1),
                          "m512_fp16_operands_us": round(r512["us"], 1), "m512_fp16_operands_tflops": round(r512["tflops"], 1),
                          "paths": "m1: integer-digit GEMV; m32, m512: tcgen05 GEMM, exact-class operands (default); "
-                                  "m512_fp16_operands: the same GEMM with operands rounded to fp16 (opt-in)"})
+                                  "m512_fp16_operands: tcgen05 GEMM, operands rounded to fp16 (opt-in)"})
     return rows
 
 

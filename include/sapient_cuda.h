@@ -311,11 +311,11 @@ int32_t sp_cuda_batcher_forget(SpBatcher* b, uint64_t id);
  * index pages held, free pool pages. */
 #define SP_BATCHER_STATS 9
 int32_t sp_cuda_batcher_stats(const SpBatcher* b, uint64_t* out, int32_t cap);
-/* Replay decode steps as CUDA graphs (default on). */
 /* For tests of what follows a wait that ran out: a kernel reports one of `kind` (0: GEMM on quantised weights, 1: product
  * on bf16 weights, 2: streaming GEMV) as those kernels do, on the engine's stream in the engine's name, or (engine null)
  * for `device`'s op-level calls. The owner's next call that waits for the device fails with SP_ERR_CUDA, once. */
 int32_t sp_cuda_report_wait(SpEngine* engine, int32_t device, int32_t kind);
+/* Replay decode steps as CUDA graphs (default on). */
 int32_t sp_cuda_engine_set_graphs(SpEngine* e, int32_t on);
 /* Steps of 17 rows and more (prefill chunks, batched decode) run on the tcgen05 GEMM: each weight tile is dequantised
  * once and multiplied with all rows on the 5th-generation tensor cores.

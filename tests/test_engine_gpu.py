@@ -339,3 +339,21 @@ def test_float_linears_are_quantised_to_q8_0_at_load_like_the_reference(oracle, 
     ref.forward_logits(ids, True)
     assert np.abs(a.forward_logits([4], True) - ref.forward_logits([3, 4], True)).max() < LOGIT_BAR
     a.close(); b.close()
+
+
+@pytest.mark.parametrize("vocab,tokens", [(150001, 33), (65537, 19), (32779, 32)])
+def test_logits_copied_in_pieces_are_those_of_rows_copied_alone(vocab, tokens):
+    """35, 10 and 9 pieces of up to 2^17 floats in up to 32 copies, none of them whole rows, against single rows (one copy). The head's
+    kernel differs with the number of rows, so rows agree to the activations' digits (2^-15 at worst, 3e-5 of a row) and not to the
+    bit; of a piece out of place most values are off by as much as they are large."""
+    cfg, W = synth.build_model(dict(synth.CONFIGS["tiny_llama"], vocab=vocab), seed=5, device="cpu", max_ctx=64)
+    eng = ForwardEngine.from_weights(cfg, synth.weights_to_numpy(W), max_batch=1, max_tokens=64)
+    ids = np.random.default_rng(vocab).integers(0, vocab, tokens).astype(np.uint32)
+    for _ in range(2):
+        eng.reset_cache()
+        got = eng.forward_all_logits(ids)
+    for row in sorted({0, 1, tokens // 2, min(31, tokens - 1), tokens - 1}):
+        eng.reset_cache()
+        want = eng.forward_mixed([(0, ids, [row])])[0]
+        assert np.abs(got[row] - want).max() < 1e-3 * np.linalg.norm(want) / np.sqrt(vocab)
+    eng.close()

@@ -619,11 +619,26 @@ cudaError_t launch_gqa_mma_phase(const float* q, int ldq, float* out, int ldo, i
     return le;
 }
 
-// A tile walks its keys alone, whatever the number of its rows; with a token per block the same keys are shared out to
-// (token, cached head) pairs -- (token, query head) where no kernel shares cached rows -- of which the device holds some 450.
-// Measured per layer: 512 tokens x 8 cached heads 91 us against 42, 389 x 32 325 against 31, but 181 x 2 17 against 17.
-bool attention_takes_tiles(int n_tok, int n_heads, int n_kv, int head_dim) {
-    return n_tok >= 16 && n_tok * (attention_gqa_mma_supported(n_heads, n_kv, head_dim) ? n_kv : n_heads) >= 600;
+// A tile walks all its keys alone, at 50 to 76 ns each whatever the number of its rows, and up to two blocks per SM take no longer
+// than one. With a token per block the same keys cost every (token, cached head) pair -- (token, query head) where no kernel
+// shares cached rows -- its own pass: so tiles are for many pairs, and the later a portion of a prompt stands in its
+// context the more pairs it takes. Whole steps of four-layer models, us, a token per block / tiles:
+//   32 heads on 8 cached, 128 coordinates   128 tokens at position 0: 874 / 849, at 1000: 1085 / 1164, at 8000: 2558 / 3284
+//                                           300 tokens at position 0: 1849 / 1782, at 1000: 2283 / 2099, at 8000: 5279 / 4252
+//   12 on 2, 128                            300 tokens at position 0: 662 / 675, at 8000: 1795 / 2459
+//   14 on 2, 64                             300 tokens at position 0: 412 / 445, at 8000: 1022 / 2196
+//   32 unshared, 80                         24 tokens at position 0: 369 / 373, at 200: 468 / 407; 300 at 8000: 39048 / 3018
+// Both times are lines through 168 such pairs (these models, 17 to 300 tokens, positions 0 to 8000). The choice is the faster side's in
+// all but a few, by up to 8 us a layer; more than 600 pairs at any position, the rule before, cost up to 180.
+bool attention_takes_tiles(int n_tok, int pos0, int n_heads, int n_kv, int head_dim) {
+    if (n_tok < 16) return false;
+    const bool shared = attention_gqa_mma_supported(n_heads, n_kv, head_dim);
+    const double keys = pos0 + 0.5 * n_tok, last = pos0 + n_tok;  // a token's on average, the last tile's
+    const double pairs = (double)n_tok * (shared ? n_kv : n_heads);
+    const double by_token = pairs * (shared ? 10.0 + keys * (0.014 + 0.00028 * head_dim) : 2.2 + keys * (0.005 + 0.0015 * head_dim));
+    const double blocks = (double)n_heads * ((n_tok + FA_ROWS - 1) / FA_ROWS);
+    const double by_tile = 2000.0 + last * (25.0 + 0.4 * head_dim) * fmax(1.0, blocks / (2.0 * device_sm_count()));
+    return by_tile < by_token;  // ns, on 148 SMs
 }
 
 bool attention_prefill_supported(int head_dim) { return head_dim % 16 == 0 && head_dim >= 16 && head_dim <= 128; }

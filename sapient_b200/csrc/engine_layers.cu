@@ -327,7 +327,7 @@ int Engine::attention_and_oproj(const LayerW& w, int l, int T) {
     if (tc5_exact && use_tc5 && !graph_step_ && attention_prefill_supported(hd)) {
         for (int i0 = 0, i1; i0 < T; i0 = i1) {
             for (i1 = i0 + 1; i1 < T && p_slot_[i1] == p_slot_[i0] && p_pos_[i1] == p_pos_[i1 - 1] + 1;) ++i1;
-            if (!attention_takes_tiles(i1 - i0, H, Hkv, hd)) continue;
+            if (!attention_takes_tiles(i1 - i0, p_pos_[i0], H, Hkv, hd)) continue;
             SP_TRY(attention_tokens(done, i0 - done, l, splits));
             SP_LAUNCH(F_ATTN, launch_attention_prefill(qkv_ + (size_t)i0 * qkv_ld, qkv_ld, attn_ + (size_t)i0 * H * hd, H * hd, i1 - i0, H, p_slot_[i0], p_pos_[i0],
                                                        kv_, l, scale, stream, nullptr, true));

@@ -136,8 +136,8 @@ cudaError_t launch_attention_split(const float* q, int ldq, int n_tok, int n_hea
 
 // Prefill attention on tensor cores: n_tok tokens of one sequence at consecutive positions pos0.. (keys already cached).
 bool attention_prefill_supported(int head_dim);
-// Whether a run of n_tok consecutive positions is better off on the tiled kernel than with a token per block.
-bool attention_takes_tiles(int n_tok, int n_heads, int n_kv, int head_dim);
+// Whether a run of n_tok consecutive positions from pos0 on is better off on the tiled kernel than with a token per block.
+bool attention_takes_tiles(int n_tok, int pos0, int n_heads, int n_kv, int head_dim);
 cudaError_t launch_attention_prefill(const float* q, int ldq, float* out, int ldo, int n_tok, int n_heads, int slot, int pos0, KvGeom kv,
                                      int layer, float scale, cudaStream_t st, __half* out_h = nullptr, bool exact = false);
 

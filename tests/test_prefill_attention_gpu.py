@@ -127,3 +127,26 @@ def test_long_flat_tails_keep_their_weight(oracle, heads, depth):
     ref = oracle_engine(oracle, cfg, W, kv_mode=1).forward_logits(ids, True)  # (from the cache, with its fp16 rounding)
     assert rel_l2(got, ref) < 3e-5 + 2.0 ** -39 * np.exp(depth), rel_l2(got, ref)
     eng.close()
+
+
+@pytest.mark.parametrize("later", [40, 300])
+def test_portions_on_either_kernel_by_their_position(oracle, later):
+    """Shared heads: 300 tokens from position 0 on take tiles, 40 from 300 on a token per block, 300 from 300 on tiles again; decoded tokens
+    read what they left. Against chunks of 32, which never take tiles; the tolerance is that of the test above."""
+    shape = dict(synth.CONFIGS["tiny_llama"], hidden=512, n_heads=16, n_kv_heads=8, head_dim=64)
+    cfg, W = synth.build_model(shape, seed=6, device="cpu", max_ctx=1024)
+    W = synth.weights_to_numpy(W)
+    rng = np.random.default_rng(later)
+    ids, more = (rng.integers(0, cfg["vocab"], n).astype(np.uint32) for n in (300, later))
+    big, small = (ForwardEngine.from_weights(cfg, W, max_tokens=n) for n in (512, 32))
+    for e in (big, small):
+        e.set_kv_rounding(False)
+    for step in (ids, more, [3], [4]):
+        a, b = big.forward_logits(step, True), small.forward_logits(step, True)
+        assert np.abs(a - b).max() < 1e-4, np.abs(a - b).max()
+    ref = oracle_engine(oracle, cfg, W, kv_mode=1)
+    for step in (ids, more, [3], [4]):
+        want = ref.forward_logits(np.asarray(step, np.uint32), True)
+    assert np.abs(a - want).max() < 3e-3
+    big.close()
+    small.close()

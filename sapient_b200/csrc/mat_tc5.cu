@@ -364,23 +364,32 @@ cudaError_t launch_mat_tc5(const MatArgs& a, int max_tiles, cudaStream_t st) {
     const int groups = a.moe ? 1 : a.seg[0].groups;
     // activation rows per tile: all of a small step, else as many as keep the SMs busy
     int bn = a.m <= 16 ? 16 : a.m <= 32 ? 32 : a.moe ? MOE_TILE : a.dual ? 128 : 256;
-    // K split over the CTAs of a cluster until every SM has one, but no part shorter than four chunks
-    auto split = [&](int64_t tiles) {
-        int parts = 1;
-        while (parts < MT_MAX_PARTS && tiles * parts < sms && kp_max / MT_BK >= 8 * parts) parts *= 2;
-        return parts;
-    };
-    // Fewer tiles than SMs: from the height on whose partial sums fit shared memory, K is split where that fills the SMs; only
-    // otherwise are tiles made lower, which fetches every weight once more per halving and leaves the tensor pipe waiting (40 of its
-    // cycles for 32 rows, 64 for 128). Four prompts of 301 tokens and eight steps of Tedelix at width 2048: 7.87 -> 7.41 ms.
-    bool by_k = a.m <= 32;
     if (!a.moe)
-        while (bn > 32) {
-            const int64_t tiles = (int64_t)row_blocks * groups * ((a.m + bn - 1) / bn);
-            if (bn < 2 * a.m && tiles >= sms) break;
-            if (bn < 2 * a.m && a.nseg == 1 && bn <= (a.dual ? 64 : 128) && tiles * split(tiles) >= sms) { by_k = true; break; }
-            bn >>= 1;
-        }
+        while (bn > 32 && ((int64_t)row_blocks * groups * ((a.m + bn - 1) / bn) < sms || bn >= 2 * a.m)) bn >>= 1;
+    const int acc = a.dual ? 2 : 1;
+    // More than 32 rows: low tiles fetch every weight once more per halving; a shared K range pays for partial sums that cross the
+    // cluster. It is shared where that takes less time in the model below: with a long K and few tiles (2048 x 9216, 96 rows: 41.6 ->
+    // 15.9 us), not where a part is over before its sums are added (2048 x 512, 512 rows: 6.1, shared 11.9). Constants fitted to 3400
+    // times of 24 matrices at 33 to 2000 rows, at every height and number of parts, 10 % off on average; its choices took 0.82 of
+    // low tiles' time on average and 1.06 at worst.
+    k.parts = 1;
+    if (!a.moe && a.nseg == 1 && a.m > 32) {
+        auto time = [&](int h, int p) {  // us
+            // 64 columns of K, heights 32 to 256, for a CTA alone on its SM and for two; clusters of four and eight leave SMs over
+            static constexpr double CHUNK[2][2][4] = {{{0.287, 0.303, 0.358, 0.539}, {0.315, 0.331, 0.385, 0.634}},
+                                                      {{0.436, 0.685, 0.767, 0.0}, {0.491, 0.607, 0.843, 0.0}}};
+            const double ctas = (double)row_blocks * groups * ((a.m + h - 1) / h) * p, values = (double)h * acc;
+            const double waves = ceil(ctas / ((p == 8 ? 0.865 : p == 4 ? 0.946 : 1.0) * 2.0 * sms));
+            const bool two = ctas > sms;
+            const double chunks = waves * (kp_max / MT_BK) / p * CHUNK[a.dual][two][h <= 32 ? 0 : h <= 64 ? 1 : h <= 128 ? 2 : 3];
+            return 2.52 + chunks + 0.0168 * std::max(1.0, ctas / sms) * values +
+                   (p > 1 ? waves * (2.79 + 0.127 * p) + (two ? 2.0 * waves : 1.0) * values * 0.0589 / p : 0.0);
+        };
+        double best = time(bn, 1);
+        for (int h = 32; h <= (a.dual ? 64 : 128) && h < 2 * a.m; h *= 2)
+            for (int p = 2; p <= MT_MAX_PARTS && kp_max / MT_BK >= 4 * p; p *= 2)
+                if (const double t = time(h, p); t < best) { best = t; bn = h; k.parts = p; }
+    }
     k.bn = bn;
     k.m = a.m;
     k.row_tiles = (a.m + bn - 1) / bn;
@@ -390,13 +399,14 @@ cudaError_t launch_mat_tc5(const MatArgs& a, int max_tiles, cudaStream_t st) {
     k.n_outs = a.n_outs; k.norm = a.norm; k.waits = a.waits;
     std::copy(a.arg, a.arg + 2, k.arg);
     std::copy(a.outs, a.outs + MAT_MAX_OUTS, k.outs);
-    const int acc = a.dual ? 2 : 1;
     k.stage_bytes = acc * MT_A_BYTES + bn * MT_BK * 2;
     k.tmem_cols = std::max(32, acc * bn);
     k.stages = std::min(MT_MAX_STAGES, MT_SMEM / k.stage_bytes);
     int64_t busy = 0;  // tiles that exist
     for (int i = 0; i < a.nseg; ++i) busy += (int64_t)((a.seg[i].n + MT_BM - 1) / MT_BM) * (i ? k.row_tiles : k.slots0);
-    k.parts = by_k ? split(busy) : 1;
+    // up to 32 rows: a CTA per SM, but no part shorter than four chunks of K
+    if (a.m <= 32)
+        while (k.parts < MT_MAX_PARTS && busy * k.parts < sms && kp_max / MT_BK >= 8 * k.parts) k.parts *= 2;
     CUtensorMap mw[2], mx[2];
     for (int i = 0; i < a.nseg; ++i) {
         const MatSeg& s = a.seg[i];

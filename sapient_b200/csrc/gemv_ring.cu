@@ -610,6 +610,7 @@ bool ring_plan(RingArgs& a, const RingScratch& sc, bool share_sm) {
         a.smem_total = off + a.stages * a.stage_bytes;
         a.fix_part = sc.part;
         a.fix_cnt = sc.cnt;
+        a.waits = sc.waits;
         return true;
     }
     return false;

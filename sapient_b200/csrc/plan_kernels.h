@@ -105,8 +105,8 @@ inline bool mat_outs_valid(const MatArgs& a) {
 // f32: plain fused multiply-adds on 32 x 32 tiles, any shape and row count.
 cudaError_t launch_mat_f32(const MatArgs& a, cudaStream_t st);
 
-// bf16: tcgen05 / TMEM, both operands staged by TMA, any shape and row count. Launches whose tiles leave SMs idle split K
-// over several CTAs through `sc` (partial tiles, summed in order by the last to arrive). Grouped by expert: with `gather`
+// bf16: tcgen05 / TMEM, both operands staged by TMA, any shape and row count. Where that takes less time the CTAs of a cluster
+// share a tile's K range (partial tiles meet in distributed shared memory, added in part order). Grouped by expert: with `gather`
 // (at most MAT_GATHER_ROWS rows) every expert multiplies all rows and keeps its own; otherwise the x rows are the sorted
 // rows. max_tiles: upper bound of the row tiles of a grouped launch.
 constexpr int MAT_GATHER_ROWS = 32;

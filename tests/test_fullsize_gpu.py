@@ -24,8 +24,8 @@ Per model, two comparisons, both with the bars of the task written out and no pe
     oracle's greedy pick at least as often as the reordered oracle does, or on 99 % of the steps.
 
 The engines run in their default configuration: decode steps on exact integer products with three-digit activations,
-prompts (steps of 17 rows and more) on the tcgen05 GEMM with exact-class operands (fp16 leading part + remainder of weights
-and activations, ~1e-6 per product). The same GEMM with operands rounded once to fp16 (~3e-4 per product, twice as fast)
+prompts (steps of 17 rows and more) on the tcgen05 GEMM with exact-class operands (activations as fp16 leading part +
+remainder, weights unrounded, ~1e-6 per product). The GEMM with operands rounded once to fp16 (~3e-4 per product)
 is measured by a further test on the same inputs: its prompt leaves the 2e-2 bar on the largest model (that is why it is
 not the default); what is asserted for it is that the deviation stays of the order of the fp16
 roundings it introduces — an O(1) fault (a misplaced tile) would be hundreds of times larger — and that greedy decoding

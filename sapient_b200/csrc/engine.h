@@ -141,7 +141,7 @@ class Engine {
     bool use_ring = false;     // steps of 1-5 rows on the bulk-copy ring GEMV (opt-in: measured slower than the tile-row kernels)
     // Steps of TC5_MIN_M rows and more (prompts, batches) run on a tcgen05 GEMM. tc5_exact (the default): exact-class operands
     // (gemm_dq.cu, dq_rows.cu), ~1e-6 per product, and tiled attention with operands split alike. Full-size models keep the
-    // 2e-2 final-logit bar (8B shape, 128-token prompt: 6.7e-3).
+    // 2e-2 final-logit bar (tests/test_fullsize_gpu.py).
     // tc5_exact == false: operands rounded once to fp16 (gemm_tc5.cu; ~3e-4 per product; the 8B shape's logits then move by up
     // to 4e-2), with the fused fp16 producers and the fp16 prefill attention. use_tc5 == false: integer-digit GEMV passes of
     // 10 rows at any row count (7x slower on a 512-token prompt). sp_cuda_engine_set_large_m_gemm chooses.

@@ -374,8 +374,8 @@ class ForwardEngine:
 
     def set_large_m_gemm(self, on) -> None:
         """Steps of 17 rows and more: 2 (default) the tcgen05 GEMM with exact-class operands (activations as leading
-        fp16 part + remainder, weights unrounded); True / 1 the one with operands rounded to fp16 (up to twice as fast
-        from some 100 rows on, no faster at 32; final logits of full-size models may leave the 2e-2 bar); False / 0 integer-digit GEMV passes of 10 rows."""
+        fp16 part + remainder, weights unrounded); True / 1 the one with operands rounded to fp16 (1 to 2.4 times
+        as fast per product of 512 rows; final logits of full-size models may leave the 2e-2 bar); False / 0 integer-digit GEMV passes of 10 rows."""
         check(lib().sp_cuda_engine_set_large_m_gemm(self._h, int(on)))
 
     def set_many_row_gemv(self, on: bool) -> None:

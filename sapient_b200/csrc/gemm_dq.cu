@@ -25,6 +25,13 @@
 //               remainders of the sums, minima exact) times dmin, which costs a quarter instruction per element.
 // Columns are stored in the order 0 2 1 3 within groups of four, in activations and weights alike: the order in which masks
 // pick bytes out of a word, so that no weight is moved.
+// What holds it is the serial work of its single warps -- the one that issues the products, the one that asks for activations -- whose
+// instructions wait for those of 16 busy others: copies of activations are one box for both planes and all columns of a stage (four at
+// 32 rows before), roles branch on a warp number that is uniform to the compiler, and drains take the minimum term before
+// they wait for the sums. Q4_K 28672 x 4096 32 rows 48.5 -> 39.5 us, 128 rows 70.5 -> 67.3, 512 rows 214 -> 208; Q6_K 4096 x 14336 37 rows
+// 31.0 -> 29.3; Q4_K 17920 x 1536 192 rows 29.7 -> 28.0; Q8_0 28672 x 4096 32 rows 49.8 -> 48.5, 10240 x 2560 389 rows 60.2 -> 60.0.
+// Without effect: a second group of eight producers, two warps that issue products for accumulators in turn, a ring of 3 or 5
+// activation stages instead of 4, waits that ask without looking first.
 // Measured against the kernel before (matmul with its split of activations), us: Q4_K 28672 x 4096, 32 rows 101 -> 51, 512 rows 285 -> 230;
 // 4096 x 14336 Q6_K, 37 rows 54.6 -> 35; Q4_K 4096 x 4096, 512 rows 85 -> 44; Q8_0 17920 x 1536, 192 rows 32.5 -> 33.5, 512 rows 71.7 ->
 // 68. That kernel took 256 activation rows per tile, one pass over the weights where two are made here, which still tells at the
@@ -112,6 +119,13 @@ __device__ __forceinline__ void dq_ld16(uint32_t taddr, uint32_t* r) {
 __device__ __forceinline__ void dq_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
+}
+// Boxes of 64 columns, leading parts and remainders of the rows from m0 on, one after the other: [box][plane][row][64].
+__device__ __forceinline__ void dq_box(uint32_t dst, const CUtensorMap* map, int m0, int box, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %2, %4}], [%5];\n" ::"r"(dst), "l"(map), "r"(0),
+        "r"(m0), "r"(box), "r"(bar)
+        : "memory");
 }
 __device__ __forceinline__ void dq_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
@@ -348,11 +362,26 @@ __device__ __forceinline__ bool dq_drain(DqBars& bars, const uint8_t* raw, int r
         if (lane == 0) tc5_arrive(&bars.empty_r[rr.st]);
         rr.next(r_stages);
         if (DT == T_Q4_K) ok = ok && rx.full(bars.full_x);
+        const uint8_t* xrow = xs + (size_t)rx.st * x_bytes + (half * NJT * 8 + g) * 32 + t * 8;
+        if (DT == T_Q4_K && ok) {
+#pragma unroll
+            for (int j = 0; j < NJT; ++j) {
+                const uint2 x = *reinterpret_cast<const uint2*>(xrow + j * 256);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    float p[4];
+                    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%4,%5}, {%6,%7}, {%8,%8,%8,%8};\n"
+                        : "=f"(p[0]), "=f"(p[1]), "=f"(p[2]), "=f"(p[3])
+                        : "r"(mn[i][0]), "r"(mn[i][1]), "r"(x.x), "r"(x.y), "f"(0.f));
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[i][j][e] = fmaf(dm[i][e >> 1], p[e], acc[i][j][e]);
+                }
+            }
+        }
         ok = ok && rd.full(bars.full_d);
         ok = __all_sync(0xFFFFFFFFu, ok);
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t from = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(rd.st * DQ_NB + half * NJT * 8);
-        const uint8_t* xrow = xs + (size_t)rx.st * x_bytes + (half * NJT * 8 + g) * 32 + t * 8;
         // batches of two 8-column tiles, the next one requested before the current one is added
         constexpr int NB2 = NJT >= 2 ? NJT / 2 : 1, W = NJT >= 2 ? 2 : 1, PL = SIDE ? 2 : 1;
         uint32_t v[2][PL][4 * W];
@@ -376,16 +405,6 @@ __device__ __forceinline__ bool dq_drain(DqBars& bars, const uint8_t* raw, int r
 #pragma unroll
             for (int w = 0; w < W; ++w) {
                 float* const a = acc[i][(b % NB2) * W + w];
-                if (DT == T_Q4_K) {
-                    const uint2 x = *reinterpret_cast<const uint2*>(xrow + ((b % NB2) * W + w) * 256);
-                    float p[4];
-                    asm volatile(
-                        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%4,%5}, {%6,%7}, {%8,%8,%8,%8};\n"
-                        : "=f"(p[0]), "=f"(p[1]), "=f"(p[2]), "=f"(p[3])
-                        : "r"(mn[i][0]), "r"(mn[i][1]), "r"(x.x), "r"(x.y), "f"(0.f));
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) a[e] = fmaf(dm[i][e >> 1], p[e], a[e]);
-                }
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     float f = __uint_as_float(c[0][4 * w + e]);
@@ -532,7 +551,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
     __shared__ uint32_t tmem_slot;
     constexpr bool SIDE = NJT <= DQ_SIDE_NJT;
     constexpr int BOXES = dq_boxes(NJT);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
     uint8_t* smem = smem_raw + ((1024u - (tc5_smem_u32(smem_raw) & 1023u)) & 1023u);
     const int all_sb = (a.k + 255) / 256, part = blockIdx.z;
     const int sb0 = part * all_sb / a.parts, n_sb = (part + 1) * all_sb / a.parts - sb0;
@@ -605,8 +624,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
                         if (!ok) break;
                         const uint32_t bar = tc5_smem_u32(&bars.full_b[r.st]), dst = tc5_smem_u32(smem + (size_t)r.st * b_bytes);
                         dq_expect(bar, (uint32_t)b_bytes);
-                        for (int c = 0; c < 2 * BOXES; ++c)
-                            tc5_tma_2d(dst + c * a.nb * 128, &tmap_x, (sb0 + sb) * 256 + 64 * (BOXES * h + (c >> 1)), (c & 1) * a.m + it.m0, bar);
+                        dq_box(dst, &tmap_x, it.m0, (sb0 + sb) * 4 + BOXES * h, bar);
                         r.next(a.b_stages);
                         ++boxes;
                     }
@@ -645,8 +663,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
         }
         __syncwarp();
         if (a.parts > 1) { cluster_sync(); cluster_sync(); }
-    } else if (warp < DQ_FIRST_DRAIN) {
-        pdl_wait();
+    } else if (warp < DQ_FIRST_DRAIN) {  // (reads and writes nothing of another kernel: its first slots are made before that has ended)
         const int pw = warp - DQ_FIRST_PRODUCER, tile_w = 2 * (warp & 3) + (pw >> 2);
         const uint32_t a_base = tmem + ((uint32_t)(16 * tile_w) << 16) + (uint32_t)DQ_A_COL;
         DqRing rr, ra;
@@ -838,11 +855,11 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
     if (!encode) return cudaErrorNotSupported;
     CUtensorMap tmap;
     {
-        const cuuint64_t gdim[2] = {(cuuint64_t)k, (cuuint64_t)(2 * m)};
-        const cuuint64_t gstride[1] = {(cuuint64_t)k * sizeof(__half)};
-        const cuuint32_t box[2] = {64u, (cuuint32_t)a.nb};
-        const cuuint32_t estr[2] = {1u, 1u};
-        if (encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, in.xh, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+        const cuuint64_t gdim[4] = {64u, (cuuint64_t)m, 2u, (cuuint64_t)(k / 64)};
+        const cuuint64_t gstride[3] = {(cuuint64_t)k * sizeof(__half), (cuuint64_t)m * k * sizeof(__half), 64 * sizeof(__half)};
+        const cuuint32_t box[4] = {64u, (cuuint32_t)a.nb, 2u, (cuuint32_t)dq_boxes(njt)};
+        const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
+        if (encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, in.xh, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }

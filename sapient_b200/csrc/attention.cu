@@ -10,71 +10,89 @@
 #include "kernels.h"
 #include "pdl.cuh"
 #include "sp_common.cuh"
+#include "splits.cuh"
 
 namespace sp {
 
 cudaError_t count_launch_and_check();  // kernels.cu
 
 constexpr int ATT_WARPS = 4;
-constexpr int ATT_MAX_PAIRS = 4;  // head_dim <= 256
-constexpr int ATT_KEYS = 4;       // keys per warp iteration
+constexpr int ATT_KEYS = 4;  // keys of a warp's round
 
 __device__ __forceinline__ int64_t kv_off(const KvGeom& kv, int layer, int page, int which, int head) {
     return ((((int64_t)layer * kv.n_pages + page) * 2 + which) * kv.n_kv + head) * (int64_t)(KV_PAGE * kv.head_dim);
 }
 
 // part: [n_tok][n_heads][n_splits][head_dim + 2] = (m, l, o[head_dim]); unused when n_splits == 1.
+// PAIRS: coordinate pairs of a lane (head_dim <= 64 PAIRS). A round's rows are requested a round ahead, those of the first one before
+// the previous kernel has ended: it only appends the last `fresh` positions or fewer. What a launch takes is the chain of loads --
+// position, page, rows. Requested as they were needed, all by size of the largest head, it was 6.1 us of a layer of the 8B shape at
+// context 517 (33 keys a block), 6.4 of Phi-2's at 645, 6.6 for 5 rows of the 1.5B shape; now 4.5, 5.0, 4.4. (Eight keys a round: 3.8,
+// 4.8, 6.3, and 3.7 against 2.5 for the 9 keys a block of the 0.5B shape at 130, where the sums over lanes of keys that are not
+// there count.)
+template <int PAIRS>
 __global__ void __launch_bounds__(ATT_WARPS * 32)
 attention_split_kernel(const float* __restrict__ q, int ldq, float* __restrict__ out, int ldo, int n_heads,
                        const int32_t* __restrict__ tok_slot, const int32_t* __restrict__ tok_pos, KvGeom kv, int layer,
-                       float scale, int n_splits, float* __restrict__ part) {
+                       float scale, int n_splits, float* __restrict__ part, int fresh) {
     __shared__ float sh_m[ATT_WARPS], sh_l[ATT_WARPS];
-    __shared__ float sh_o[ATT_WARPS][256];
-    pdl_wait();
-    pdl_trigger();
+    __shared__ float sh_o[ATT_WARPS][64 * PAIRS];
     const int h = blockIdx.x, t = blockIdx.y, sp = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int hd = kv.head_dim, npairs = hd >> 1;
+    const int kv_h = h / (n_heads / kv.n_kv);
+    if (fresh < 0) pdl_wait();  // nothing is known about the previous kernel
     const int slot = tok_slot[t], n_keys = tok_pos[t] + 1;
     // this split's key range
     const int per = (n_keys + n_splits - 1) / n_splits;
     const int k_begin = sp * per, k_end = min(n_keys, k_begin + per);
-    const int kv_h = h / (n_heads / kv.n_kv);
-    const float* qrow = q + (int64_t)t * ldq + (int64_t)h * hd;
-    float2 qv[ATT_MAX_PAIRS], o[ATT_MAX_PAIRS];
+    const int32_t* pt = kv.page_table + (int64_t)slot * kv.max_pages;
+    // all K and V fragments of a round are requested before any arithmetic, so the V loads do not wait for the scores
+    struct Round { __half2 k[ATT_KEYS][PAIRS], v[ATT_KEYS][PAIRS]; };
+    auto load = [&](int key0, Round& r) {
+        const int last = min(key0 + ATT_KEYS, k_end) - 1;  // tail keys repeat the last one and get weight 0
+        const int page0 = pt[key0 / KV_PAGE], page1 = pt[last / KV_PAGE];
 #pragma unroll
-    for (int i = 0; i < ATT_MAX_PAIRS; ++i) {
+        for (int j = 0; j < ATT_KEYS; ++j) {
+            const int key = min(key0 + j, last);
+            const int page = key / KV_PAGE == key0 / KV_PAGE ? page0 : page1;
+            const __half2* kp = reinterpret_cast<const __half2*>(kv.pool + kv_off(kv, layer, page, 0, kv_h) + (int64_t)(key % KV_PAGE) * hd);
+            const __half2* vp = reinterpret_cast<const __half2*>(kv.pool + kv_off(kv, layer, page, 1, kv_h) + (int64_t)(key % KV_PAGE) * hd);
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) {
+                const int p = lane + 32 * i;
+                r.k[j][i] = (p < npairs) ? kp[p] : __half2();
+                r.v[j][i] = (p < npairs) ? vp[p] : __half2();
+            }
+        }
+    };
+    static_assert(ATT_KEYS <= KV_PAGE, "a round lies within two pages");
+    constexpr int STRIDE = ATT_WARPS * ATT_KEYS;
+    int key0 = k_begin + warp * ATT_KEYS;
+    Round ra, rb;
+    const bool early = fresh >= 0 && key0 < k_end && min(key0 + ATT_KEYS, k_end) <= n_keys - fresh;
+    if (early) load(key0, ra);
+    if (fresh >= 0) pdl_wait();
+    pdl_trigger();
+    const float* qrow = q + (int64_t)t * ldq + (int64_t)h * hd;
+    float2 qv[PAIRS], o[PAIRS];
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) {
         const int p = lane + 32 * i;
         qv[i] = (p < npairs) ? make_float2(qrow[2 * p], qrow[2 * p + 1]) : make_float2(0.f, 0.f);
         o[i] = make_float2(0.f, 0.f);
     }
+    if (!early && key0 < k_end) load(key0, ra);
     float m = -INFINITY, l = 0.f;
-    const int32_t* pt = kv.page_table + (int64_t)slot * kv.max_pages;
-    for (int key0 = k_begin + warp * ATT_KEYS; key0 < k_end; key0 += ATT_WARPS * ATT_KEYS) {
-        // all K and V fragments of the four keys are requested before any arithmetic, so the V loads do not wait
-        // for the scores
-        __half2 kr[ATT_KEYS][ATT_MAX_PAIRS], vr[ATT_KEYS][ATT_MAX_PAIRS];
+    auto round = [&](int k0, const Round& r) {
         float s[ATT_KEYS];
-#pragma unroll
-        for (int j = 0; j < ATT_KEYS; ++j) {
-            const int key = min(key0 + j, k_end - 1);  // tail keys repeat the last one and get weight 0
-            const int page = pt[key / KV_PAGE];
-            const __half2* kp = reinterpret_cast<const __half2*>(kv.pool + kv_off(kv, layer, page, 0, kv_h) + (int64_t)(key % KV_PAGE) * hd);
-            const __half2* vp = reinterpret_cast<const __half2*>(kv.pool + kv_off(kv, layer, page, 1, kv_h) + (int64_t)(key % KV_PAGE) * hd);
-#pragma unroll
-            for (int i = 0; i < ATT_MAX_PAIRS; ++i) {
-                const int p = lane + 32 * i;
-                kr[j][i] = (p < npairs) ? kp[p] : __half2();
-                vr[j][i] = (p < npairs) ? vp[p] : __half2();
-            }
-        }
 #pragma unroll
         for (int j = 0; j < ATT_KEYS; ++j) {
             float part_dot = 0.f;
 #pragma unroll
-            for (int i = 0; i < ATT_MAX_PAIRS; ++i) {
+            for (int i = 0; i < PAIRS; ++i) {
                 if (lane + 32 * i < npairs) {
-                    const float2 kf = __half22float2(kr[j][i]);
+                    const float2 kf = __half22float2(r.k[j][i]);
                     part_dot = fmaf(qv[i].x, kf.x, part_dot);
                     part_dot = fmaf(qv[i].y, kf.y, part_dot);
                 }
@@ -88,7 +106,7 @@ attention_split_kernel(const float* __restrict__ q, int ldq, float* __restrict__
         float m_new = m;
 #pragma unroll
         for (int j = 0; j < ATT_KEYS; ++j) {
-            s[j] = (key0 + j < k_end) ? s[j] * scale : -INFINITY;
+            s[j] = (k0 + j < k_end) ? s[j] * scale : -INFINITY;
             m_new = fmaxf(m_new, s[j]);
         }
         const float corr = expf(m - m_new);  // the first key of the range is always live, so m_new is finite
@@ -96,12 +114,12 @@ attention_split_kernel(const float* __restrict__ q, int ldq, float* __restrict__
 #pragma unroll
         for (int j = 0; j < ATT_KEYS; ++j) { pw[j] = expf(s[j] - m_new); psum += pw[j]; }
 #pragma unroll
-        for (int i = 0; i < ATT_MAX_PAIRS; ++i) {
+        for (int i = 0; i < PAIRS; ++i) {
             if (lane + 32 * i < npairs) {
                 float ox = corr * o[i].x, oy = corr * o[i].y;
 #pragma unroll
                 for (int j = 0; j < ATT_KEYS; ++j) {
-                    const float2 vf = __half22float2(vr[j][i]);
+                    const float2 vf = __half22float2(r.v[j][i]);
                     ox = fmaf(pw[j], vf.x, ox);
                     oy = fmaf(pw[j], vf.y, oy);
                 }
@@ -110,10 +128,17 @@ attention_split_kernel(const float* __restrict__ q, int ldq, float* __restrict__
         }
         l = fmaf(corr, l, psum);
         m = m_new;
+    };
+    for (; key0 < k_end; key0 += 2 * STRIDE) {
+        if (key0 + STRIDE < k_end) load(key0 + STRIDE, rb);
+        round(key0, ra);
+        if (key0 + STRIDE >= k_end) break;
+        if (key0 + 2 * STRIDE < k_end) load(key0 + 2 * STRIDE, ra);
+        round(key0 + STRIDE, rb);
     }
     if (lane == 0) { sh_m[warp] = m; sh_l[warp] = l; }
 #pragma unroll
-    for (int i = 0; i < ATT_MAX_PAIRS; ++i) {
+    for (int i = 0; i < PAIRS; ++i) {
         const int p = lane + 32 * i;
         if (p < npairs) { sh_o[warp][2 * p] = o[i].x; sh_o[warp][2 * p + 1] = o[i].y; }
     }
@@ -152,7 +177,7 @@ bool attention_takes_mma(int n_tok, int ctx_hint, int n_heads, int n_kv, int hea
     return (int64_t)n_tok * ctx_hint >= 4096 && attention_gqa_mma_supported(n_heads, n_kv, head_dim);
 }
 cudaError_t launch_gqa_mma_phase(const float* q, int ldq, float* out, int ldo, int n_tok, int n_heads, const int32_t* tok_slot,
-                                 const int32_t* tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st);
+                                 const int32_t* tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st, int fresh);
 
 // Which kernel a launch takes. ctx_hint: an upper bound of the longest context among the tokens (0: unknown). Short work
 // is latency-bound and runs on the f32 kernel, a block per (head, token, split); from a few thousand (token, key) pairs
@@ -161,35 +186,23 @@ cudaError_t launch_gqa_mma_phase(const float* q, int ldq, float* out, int ldo, i
 // on 4.4 GB of KV; the tensor-core kernel 1.5 ms).
 static cudaError_t launch_split_phase(const float* q, int ldq, float* out, int ldo, int n_tok, int n_heads, const int32_t* tok_slot,
                                       const int32_t* tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st,
-                                      int ctx_hint) {
+                                      int ctx_hint, int fresh) {
     if (attention_takes_mma(n_tok, ctx_hint, n_heads, kv.n_kv, kv.head_dim))
-        return launch_gqa_mma_phase(q, ldq, out, ldo, n_tok, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, st);
-    return launch_pdl(attention_split_kernel, dim3(n_heads, n_tok, n_splits), dim3(ATT_WARPS * 32), 0, st, q, ldq, out, ldo, n_heads, tok_slot,
-                      tok_pos, kv, layer, scale, n_splits, scratch);
+        return launch_gqa_mma_phase(q, ldq, out, ldo, n_tok, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, st, fresh);
+    auto kernel = kv.head_dim <= 64 ? attention_split_kernel<1> : kv.head_dim <= 128 ? attention_split_kernel<2> : attention_split_kernel<4>;
+    return launch_pdl(kernel, dim3(n_heads, n_tok, n_splits), dim3(ATT_WARPS * 32), 0, st, q, ldq, out, ldo, n_heads, tok_slot,
+                      tok_pos, kv, layer, scale, n_splits, scratch, fresh);
 }
 
+// Merge of the splits (splits.cuh); one thread per coordinate.
+template <int NS>
 __global__ void attention_merge_kernel(const float* __restrict__ part, int n_heads, int n_splits, int hd, float* __restrict__ out,
                                        int ldo) {
     pdl_wait();
     pdl_trigger();
     const int h = blockIdx.x, t = blockIdx.y;
     const float* src = part + ((int64_t)t * n_heads + h) * n_splits * (hd + 2);
-    float M = -INFINITY;
-    for (int s = 0; s < n_splits; ++s) M = fmaxf(M, src[(int64_t)s * (hd + 2)]);
-    float L = 0.f;
-    for (int s = 0; s < n_splits; ++s) {
-        const float ms = src[(int64_t)s * (hd + 2)];
-        if (ms != -INFINITY) L = fmaf(expf(ms - M), src[(int64_t)s * (hd + 2) + 1], L);
-    }
-    const float inv = (L == 0.f) ? 0.f : 1.0f / L;
-    for (int e = threadIdx.x; e < hd; e += blockDim.x) {
-        float acc = 0.f;
-        for (int s = 0; s < n_splits; ++s) {
-            const float ms = src[(int64_t)s * (hd + 2)];
-            if (ms != -INFINITY) acc = fmaf(expf(ms - M), src[(int64_t)s * (hd + 2) + 2 + e], acc);
-        }
-        out[(int64_t)t * ldo + (int64_t)h * hd + e] = acc * inv;
-    }
+    for (int e = threadIdx.x; e < hd; e += blockDim.x) out[(int64_t)t * ldo + (int64_t)h * hd + e] = merge_splits<NS>(src, n_splits, hd, e);
 }
 
 size_t attention_scratch_floats(int n_tok, int n_heads, int n_splits, int head_dim) {
@@ -197,24 +210,26 @@ size_t attention_scratch_floats(int n_tok, int n_heads, int n_splits, int head_d
 }
 
 cudaError_t launch_attention_split(const float* q, int ldq, int n_tok, int n_heads, const int32_t* tok_slot, const int32_t* tok_pos,
-                                   KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st, int ctx_hint) {
+                                   KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st, int ctx_hint, int fresh) {
     if (n_tok == 0) return cudaSuccess;
     if (n_splits < 2 || !scratch) return cudaErrorInvalidValue;
-    cudaError_t le = launch_split_phase(q, ldq, nullptr, 0, n_tok, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, st, ctx_hint);
+    cudaError_t le = launch_split_phase(q, ldq, nullptr, 0, n_tok, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, st, ctx_hint, fresh);
     if (le != cudaSuccess) return le;
     return count_launch_and_check();
 }
 
 cudaError_t launch_attention(const float* q, int ldq, float* out, int ldo, int n_tok, int n_heads, const int32_t* tok_slot,
                              const int32_t* tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* scratch,
-                             cudaStream_t st, int ctx_hint) {
+                             cudaStream_t st, int ctx_hint, int fresh) {
     if (n_tok == 0) return cudaSuccess;
     if (n_splits < 1 || (n_splits > 1 && !scratch)) return cudaErrorInvalidValue;
-    cudaError_t le = launch_split_phase(q, ldq, out, ldo, n_tok, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, st, ctx_hint);
+    cudaError_t le = launch_split_phase(q, ldq, out, ldo, n_tok, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, st, ctx_hint, fresh);
     if (le != cudaSuccess) return le;
     cudaError_t e = count_launch_and_check();
     if (e != cudaSuccess || n_splits == 1) return e;
-    le = launch_pdl(attention_merge_kernel, dim3(n_heads, n_tok), dim3(128), 0, st, (const float*)scratch, n_heads, n_splits, kv.head_dim, out, ldo);
+    if (n_splits > MERGE_MAX_SPLITS) return cudaErrorInvalidValue;
+    auto merge = n_splits <= 4 ? attention_merge_kernel<4> : n_splits <= 16 ? attention_merge_kernel<16> : attention_merge_kernel<MERGE_MAX_SPLITS>;
+    le = launch_pdl(merge, dim3(n_heads, n_tok), dim3(128), 0, st, (const float*)scratch, n_heads, n_splits, kv.head_dim, out, ldo);
     if (le != cudaSuccess) return le;
     return count_launch_and_check();
 }
@@ -443,11 +458,11 @@ constexpr int GM_WARPS = 4;
 template <int HD16>
 __global__ void __launch_bounds__(GM_WARPS * 32)
 attention_gqa_mma_kernel(const float* __restrict__ q, int ldq, float* __restrict__ out, int ldo, int n_heads, const int32_t* __restrict__ tok_slot,
-                         const int32_t* __restrict__ tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* __restrict__ part) {
+                         const int32_t* __restrict__ tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* __restrict__ part,
+                         int fresh) {
     constexpr int HD = HD16 * 16, LD = HD + 8, TILE = KV_PAGE * LD;
     extern __shared__ __align__(16) __half gm_smem[];
-    pdl_wait();
-    pdl_trigger();
+    if (fresh < 0) pdl_wait();  // nothing is known about the previous kernel
     const int kv_h = blockIdx.x, tok = blockIdx.y, sp = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int group = n_heads / kv.n_kv;
@@ -457,6 +472,29 @@ attention_gqa_mma_kernel(const float* __restrict__ q, int ldq, float* __restrict
     const int p_begin = sp * per, p_end = min(n_pg, p_begin + per);
     const int32_t* pt = kv.page_table + (int64_t)slot * kv.max_pages;
     __half* my = gm_smem + (size_t)warp * 4 * TILE;  // [buffer][K | V][16][LD]
+    auto fetch = [&](int pg, int buf) {  // keys 16 pg .. 16 pg + 15 of this KV head; keys past the sequence arrive as zeros
+        const int page = pt[pg];
+        const __half* ksrc = kv.pool + kv_off(kv, layer, page, 0, kv_h);
+        const __half* vsrc = kv.pool + kv_off(kv, layer, page, 1, kv_h);
+        __half* Kd = my + (size_t)buf * 2 * TILE;
+        __half* Vd = Kd + TILE;
+#pragma unroll
+        for (int it = 0; it < (KV_PAGE * HD / 8) / 32; ++it) {
+            const int idx = it * 32 + lane, kr = idx / (HD / 8), pc = idx - kr * (HD / 8);
+            const int bytes = (pg * KV_PAGE + kr < n_keys) ? 16 : 0;
+            const uint32_t kd = (uint32_t)__cvta_generic_to_shared(Kd + kr * LD + pc * 8), vd = (uint32_t)__cvta_generic_to_shared(Vd + kr * LD + pc * 8);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(kd), "l"(ksrc + kr * HD + pc * 8), "r"(bytes) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(vd), "l"(vsrc + kr * HD + pc * 8), "r"(bytes) : "memory");
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    // the first page is requested before the previous kernel has ended: it only appends the last `fresh` positions or fewer
+    int pg = p_begin + warp;
+    const bool early = fresh >= 0 && pg < p_end && (pg + 1) * KV_PAGE <= n_keys - fresh;
+    if (early) fetch(pg, 0);
+    if (fresh >= 0) pdl_wait();
+    pdl_trigger();
+    if (!early && pg < p_end) fetch(pg, 0);
     // query fragments: rows g (leading fp16 part) and g + 8 (remainder) of head kv_h * group + g
     uint32_t qa[HD16][4];
     {
@@ -474,28 +512,10 @@ attention_gqa_mma_kernel(const float* __restrict__ q, int ldq, float* __restrict
             qa[kd][3] = pack_half2(x2.x - f2.x, x2.y - f2.y);
         }
     }
-    auto fetch = [&](int pg, int buf) {  // keys 16 pg .. 16 pg + 15 of this KV head; keys past the sequence arrive as zeros
-        const int page = pt[pg];
-        const __half* ksrc = kv.pool + kv_off(kv, layer, page, 0, kv_h);
-        const __half* vsrc = kv.pool + kv_off(kv, layer, page, 1, kv_h);
-        __half* Kd = my + (size_t)buf * 2 * TILE;
-        __half* Vd = Kd + TILE;
-#pragma unroll
-        for (int it = 0; it < (KV_PAGE * HD / 8) / 32; ++it) {
-            const int idx = it * 32 + lane, kr = idx / (HD / 8), pc = idx - kr * (HD / 8);
-            const int bytes = (pg * KV_PAGE + kr < n_keys) ? 16 : 0;
-            const uint32_t kd = (uint32_t)__cvta_generic_to_shared(Kd + kr * LD + pc * 8), vd = (uint32_t)__cvta_generic_to_shared(Vd + kr * LD + pc * 8);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(kd), "l"(ksrc + kr * HD + pc * 8), "r"(bytes) : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(vd), "l"(vsrc + kr * HD + pc * 8), "r"(bytes) : "memory");
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
     float o[2 * HD16][4];
 #pragma unroll
     for (int i = 0; i < 2 * HD16; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
     float m = -INFINITY, l = 0.f;  // head g's running maximum (the same in its four lanes) and this lane's share of the denominator
-    int pg = p_begin + warp;
-    if (pg < p_end) fetch(pg, 0);
     for (int buf = 0; pg < p_end; pg += GM_WARPS, buf ^= 1) {
         if (pg + GM_WARPS < p_end) {
             fetch(pg + GM_WARPS, buf ^ 1);  // that buffer was consumed before the __syncwarp that ended the last iteration
@@ -600,7 +620,7 @@ bool attention_gqa_mma_supported(int n_heads, int n_kv, int head_dim) {
 }
 
 cudaError_t launch_gqa_mma_phase(const float* q, int ldq, float* out, int ldo, int n_tok, int n_heads, const int32_t* tok_slot,
-                                 const int32_t* tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st) {
+                                 const int32_t* tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st, int fresh) {
     const int hd16 = kv.head_dim / 16;
     const size_t smem = (size_t)GM_WARPS * 4 * KV_PAGE * (kv.head_dim + 8) * sizeof(__half);
     const dim3 grid(kv.n_kv, n_tok, n_splits), block(GM_WARPS * 32);
@@ -612,7 +632,7 @@ cudaError_t launch_gqa_mma_phase(const float* q, int ldq, float* out, int ldo, i
             le = big_smem.run([] { return cudaFuncSetAttribute(attention_gqa_mma_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024); }); \
             if (le != cudaSuccess) return le;                                                                           \
         }                                                                                                               \
-        le = launch_pdl(attention_gqa_mma_kernel<N>, grid, block, smem, st, q, ldq, out, ldo, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch); \
+        le = launch_pdl(attention_gqa_mma_kernel<N>, grid, block, smem, st, q, ldq, out, ldo, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, fresh); \
     }
     SP_GM(1) SP_GM(2) SP_GM(3) SP_GM(4) SP_GM(5) SP_GM(6) SP_GM(7) SP_GM(8)
 #undef SP_GM

@@ -219,7 +219,7 @@ class Engine {
     int vocab_l_ = 0, vocab_off_ = 0;
     DevTensor head_view_;           // lm_head restricted to the rows this engine computes
     bool plan_digits(int m, int k, ImmaArgs& ia);
-    int attention_tokens(int t0, int n, int l, int splits);
+    int attention_tokens(int t0, int n, int l, int splits, int fresh);
     int attention_and_oproj(const LayerW& w, int l, int T);
 
     // Weight upload: two pinned staging buffers, copies enqueued on a dedicated stream; the host fills one buffer while the

@@ -276,12 +276,12 @@ int Engine::step_splits(int T) const {
     return splits;
 }
 
-// Attention of the n staged tokens from t0 on, a token per block.
-int Engine::attention_tokens(int t0, int n, int l, int splits) {
+// Attention of the n staged tokens from t0 on, a token per block. fresh: rows of the step, whose keys were just appended.
+int Engine::attention_tokens(int t0, int n, int l, int splits, int fresh) {
     if (n <= 0) return SP_OK;
     const int H = d.n_heads, hd = d.head_dim, qkv_ld = (H + 2 * d.n_kv_heads) * hd;
     SP_LAUNCH(F_ATTN, launch_attention(qkv_ + (size_t)t0 * qkv_ld, qkv_ld, attn_ + (size_t)t0 * H * hd, H * hd, n, H, d_tok_slot_ + t0, d_tok_pos_ + t0, kv_, l,
-                                       1.0f / sqrtf((float)hd), splits, att_scratch_, stream, step_ctx_));
+                                       1.0f / sqrtf((float)hd), splits, att_scratch_, stream, step_ctx_, fresh));
     return SP_OK;
 }
 
@@ -297,7 +297,7 @@ int Engine::attention_and_oproj(const LayerW& w, int l, int T) {
     ImmaArgs ia;
     if (splits > 1 && use_ring && d.tp_size == 1 && !trace_on && T <= RING_MAX_M && all_tiled(w.o)) {
         // split-K attention merged to f32 rows; the output projection quantises them itself
-        SP_LAUNCH(F_ATTN, launch_attention(qkv_, qkv_ld, attn_, H * hd, T, H, d_tok_slot_, d_tok_pos_, kv_, l, scale, splits, att_scratch_, stream, step_ctx_));
+        SP_LAUNCH(F_ATTN, launch_attention(qkv_, qkv_ld, attn_, H * hd, T, H, d_tok_slot_, d_tok_pos_, kv_, l, scale, splits, att_scratch_, stream, step_ctx_, T));
         bool done = false;
         SP_TRY(try_ring(&done, T, H * hd, RING_SRC_PLAIN, attn_, H * hd, nullptr, nullptr, w.o, w.ob, x_, hid, nullptr, nullptr, nullptr, nullptr,
                         nullptr, nullptr, x_));
@@ -305,7 +305,7 @@ int Engine::attention_and_oproj(const LayerW& w, int l, int T) {
         return gemv(attn_, H * hd, T, H * hd, w.o, w.ob, x_, hid, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, x_, nullptr, true);
     }
     if (splits > 1 && !trace_on && all_tiled(w.o) && plan_digits(T, H * hd, ia)) {
-        SP_LAUNCH(F_ATTN, launch_attention_split(qkv_, qkv_ld, T, H, d_tok_slot_, d_tok_pos_, kv_, l, scale, splits, att_scratch_, stream, step_ctx_));
+        SP_LAUNCH(F_ATTN, launch_attention_split(qkv_, qkv_ld, T, H, d_tok_slot_, d_tok_pos_, kv_, l, scale, splits, att_scratch_, stream, step_ctx_, T));
         SP_LAUNCH(F_ATTN, launch_attn_merge_quant(att_scratch_, H, splits, hd, nullptr, 0, ia, stream));
         return gemv(attn_, H * hd, T, H * hd, w.o, w.ob, x_, hid, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, x_, &ia, true);
     }
@@ -328,13 +328,13 @@ int Engine::attention_and_oproj(const LayerW& w, int l, int T) {
         for (int i0 = 0, i1; i0 < T; i0 = i1) {
             for (i1 = i0 + 1; i1 < T && p_slot_[i1] == p_slot_[i0] && p_pos_[i1] == p_pos_[i1 - 1] + 1;) ++i1;
             if (!attention_takes_tiles(i1 - i0, p_pos_[i0], H, Hkv, hd)) continue;
-            SP_TRY(attention_tokens(done, i0 - done, l, splits));
+            SP_TRY(attention_tokens(done, i0 - done, l, splits, T));
             SP_LAUNCH(F_ATTN, launch_attention_prefill(qkv_ + (size_t)i0 * qkv_ld, qkv_ld, attn_ + (size_t)i0 * H * hd, H * hd, i1 - i0, H, p_slot_[i0], p_pos_[i0],
                                                        kv_, l, scale, stream, nullptr, true));
             done = i1;
         }
     }
-    SP_TRY(attention_tokens(done, T - done, l, splits));
+    SP_TRY(attention_tokens(done, T - done, l, splits, T));
     return gemv(attn_, H * hd, T, H * hd, w.o, w.ob, x_, hid, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, x_, nullptr, true);
 }
 

@@ -19,6 +19,7 @@
 #include "kernels.h"
 #include "pdl.cuh"
 #include "sp_common.cuh"
+#include "splits.cuh"
 #include "tp.cuh"
 
 namespace sp {
@@ -383,35 +384,18 @@ __global__ void __launch_bounds__(32) act_fn_quant_kernel(const float* __restric
 // Merge of the split-K attention partials (see attention.cu) emitting the digits of the attention output row;
 // one block per (256 columns of the [n_heads * hd] row, token), one thread per column, warp 0 converts the
 // merged 256 values to digits. part: [tok][head][split][hd + 2]. Splits without keys carry m = -inf, l = 0, o = 0.
-constexpr int MERGE_MAX_SPLITS = 32;
+template <int NS>
 __global__ void __launch_bounds__(256) attn_merge_quant_kernel(const float* __restrict__ part, int n_heads, int n_splits, int hd,
                                                                float* __restrict__ out, int ldo, QuantOut qo) {
     __shared__ __align__(16) float sv[256];
-    pdl_wait();
-    pdl_trigger();
     const int m = blockIdx.y, tile = blockIdx.x;
     const int col = tile * 256 + threadIdx.x;
+    const int h = col / hd, e = col - h * hd;
+    pdl_wait();
+    pdl_trigger();
     float v = 0.f;
     if (col < qo.k) {
-        const int h = col / hd, e = col - h * hd;
-        const float* src = part + ((int64_t)m * n_heads + h) * n_splits * (hd + 2);
-        float ms[MERGE_MAX_SPLITS];
-        float M = -INFINITY;
-#pragma unroll
-        for (int s = 0; s < MERGE_MAX_SPLITS; ++s) {
-            ms[s] = s < n_splits ? src[(int64_t)s * (hd + 2)] : -INFINITY;
-            M = fmaxf(M, ms[s]);
-        }
-        float L = 0.f;
-#pragma unroll
-        for (int s = 0; s < MERGE_MAX_SPLITS; ++s) {
-            if (s < n_splits) {
-                const float c = (ms[s] == -INFINITY) ? 0.f : expf(ms[s] - M);
-                L = fmaf(c, src[(int64_t)s * (hd + 2) + 1], L);
-                v = fmaf(c, src[(int64_t)s * (hd + 2) + 2 + e], v);
-            }
-        }
-        v *= (L == 0.f) ? 0.f : 1.0f / L;
+        v = merge_splits<NS>(part + ((int64_t)m * n_heads + h) * n_splits * (hd + 2), n_splits, hd, e);
         if (out) out[(int64_t)m * ldo + col] = v;
     }
     sv[threadIdx.x] = v;
@@ -499,7 +483,8 @@ cudaError_t launch_attn_merge_quant(const float* part, int n_heads, int n_splits
                                     cudaStream_t st) {
     if (a.m <= 0) return cudaSuccess;
     if (n_splits > MERGE_MAX_SPLITS) return cudaErrorInvalidValue;
-    cudaError_t le = launch_pdl(attn_merge_quant_kernel, dim3(a.kp / 256, a.m), dim3(256), 0, st, part, n_heads, n_splits, hd, out, ldo,
+    auto kernel = n_splits <= 4 ? attn_merge_quant_kernel<4> : n_splits <= 16 ? attn_merge_quant_kernel<16> : attn_merge_quant_kernel<MERGE_MAX_SPLITS>;
+    cudaError_t le = launch_pdl(kernel, dim3(a.kp / 256, a.m), dim3(256), 0, st, part, n_heads, n_splits, hd, out, ldo,
                                 quant_out(a));
     if (le != cudaSuccess) return le;
     return count_launch_and_check();

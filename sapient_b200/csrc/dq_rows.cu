@@ -56,8 +56,8 @@ __device__ __forceinline__ float dr_block(float v, float* sh) {
 // Power of two that brings a row of this maximum into (-1, 1), and its inverse.
 __device__ __forceinline__ float2 dr_scale(float amax) {
     if (!(amax > 0.f && amax < INFINITY)) return make_float2(1.f, 1.f);
-    const int e = max(-100, min(100, ilogbf(amax) + 1));  // amax < 2^e
-    return make_float2(scalbnf(1.0f, -e), scalbnf(1.0f, e));
+    const int e = max(-100, min(100, (__float_as_int(amax) >> 23) - 126));  // amax < 2^e (subnormal maxima end at -100)
+    return make_float2(__int_as_float((127 - e) << 23), __int_as_float((127 + e) << 23));
 }
 
 // Columns c .. c + 7 (v, in their order) of row m; every lane of the warp calls.
@@ -93,10 +93,17 @@ __device__ __forceinline__ void dr_split(const DqRowsArgs& a, int m, int c, bool
 template <int SRC, int NC>
 __global__ void __launch_bounds__(DR_THREADS) dq_rows_kernel(const DqRowsArgs a) {
     __shared__ float sh[DR_THREADS / 32];
-    pdl_wait();
-    pdl_trigger();
     const int m = blockIdx.x;
     const float* row = a.x + (int64_t)m * a.ldx;
+    // (a short row's norm weights, which no kernel writes, are here when the row comes)
+    constexpr bool AHEAD = NC == 1 && (SRC == DQ_RMS || SRC == DQ_LN);
+    float wa[8], ba[8];
+    if (AHEAD && threadIdx.x * 8 < a.k) {
+        if (a.w) dr_load8(a.w + threadIdx.x * 8, wa);
+        if (SRC == DQ_LN && a.b) dr_load8(a.b + threadIdx.x * 8, ba);
+    }
+    pdl_wait();
+    pdl_trigger();
     float v[NC][8];
     float amax = 0.f;
     auto each = [&](auto f) {
@@ -138,10 +145,11 @@ __global__ void __launch_bounds__(DR_THREADS) dq_rows_kernel(const DqRowsArgs a)
         const float inv = 1.0f / sqrtf(dr_block<false>(s, sh) / (float)a.k + a.eps);
         each([&](float (&x)[8], int c) {
             float w[8], b[8];
-            if (a.w) dr_load8(a.w + c, w);
-            if (SRC == DQ_LN && a.b) dr_load8(a.b + c, b);
+            if (!AHEAD && a.w) dr_load8(a.w + c, w);
+            if (!AHEAD && SRC == DQ_LN && a.b) dr_load8(a.b + c, b);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
+                if (AHEAD) { w[i] = wa[i]; b[i] = ba[i]; }
                 x[i] = __fmul_rn(x[i] - mean, inv);
                 if (a.w) x[i] = __fmul_rn(x[i], w[i]);
                 if (SRC == DQ_LN && a.b) x[i] = __fadd_rn(x[i], b[i]);

@@ -183,10 +183,10 @@ __device__ __forceinline__ void quantize_chunk(const float (&v)[8], bool live, i
     const int digits = qo.digits, P = 8 * digits - 2;
     float up = 0.f, down = 0.f;  // x * up -> fixed point; digit 0 scale = down
     if (amax > 0.f && amax < INFINITY) {
-        int e = ilogbf(amax) + 1;          // amax < 2^e
-        e = max(e, -100);                  // keep 2^(P-e) finite
-        up = scalbnf(1.0f, P - e);         // exact powers of two
-        down = scalbnf(1.0f, e - P);
+        // amax < 2^e; e >= -100 keeps 2^(P-e) finite (zero exponent fields, subnormal maxima, end there too)
+        const int e = max((__float_as_int(amax) >> 23) - 126, -100);
+        up = __int_as_float((127 + P - e) << 23);  // exact powers of two
+        down = __int_as_float((127 + e - P) << 23);
     }
     // balanced base-256 digits, least significant first
     uint32_t w0[3] = {0u, 0u, 0u}, w1[3] = {0u, 0u, 0u};
@@ -270,9 +270,15 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_quant_kernel(float* x, i
                                                                      const float* __restrict__ b, float eps, float* __restrict__ y, int ldy,
                                                                      QuantOut qo, const TpDev* tp) {
     __shared__ float sh[NORM_WARPS];
+    const int m = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (weights of the warp's first tile: no kernel writes them, so they are here when the row comes)
+    float wf[8], bf[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (warp * 256 + lane * 8 < qo.k) {
+        load8(w + warp * 256 + lane * 8, wf);
+        if (LAYER_NORM && b) load8(b + warp * 256 + lane * 8, bf);
+    }
     pdl_wait();
     pdl_trigger();
-    const int m = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // tensor parallel: the row still lacks the sum of the ranks' partial products (o_proj / down_proj); add it first
     uint32_t tp_epoch = 0;
     if (tp) tp_epoch = tp_consume_row(*tp, x, (int64_t)m * ldx, m, qo.k);
@@ -329,19 +335,18 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_quant_kernel(float* x, i
         const bool live = k0 < k;
         float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (live) {
-            float xv[8], wv[8];
+            float xv[8], wv[8], bv[8];
             if (tile == warp) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) xv[i] = xf[i];
+                for (int i = 0; i < 8; ++i) { xv[i] = xf[i]; wv[i] = wf[i]; bv[i] = bf[i]; }
             } else {
                 load8(row + k0, xv);
+                load8(w + k0, wv);
+                if (LAYER_NORM && b) load8(b + k0, bv);
             }
-            load8(w + k0, wv);
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(__fmul_rn(xv[i] - mean, inv), wv[i]);
             if (LAYER_NORM && b) {
-                float bv[8];
-                load8(b + k0, bv);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] = __fadd_rn(v[i], bv[i]);
             }

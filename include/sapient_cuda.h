@@ -77,14 +77,14 @@ int32_t sp_cuda_check_kernels(int32_t device);
 /* Precision of the activations in the tensor-core GEMV passes. The reference multiplies f32 activations
  * (kernels/matmul.rs:862-943); this backend splits each activation into int8 digits with one power-of-two scale per 256
  * (Q8_0: 32) columns, so that the products with the integer weights are exact. 1 (default): three digits (2^-23 of the
- * block maximum) at every row count, 10 rows per pass. 0: three digits for steps of 1-2 rows, two digits (2^-15) and 16
- * rows per pass above — fewer passes for batched steps at ~1e-4 relative error per product. Process-wide; engines drop
+ * block maximum) at every row count. 0: three digits for steps of 1-2 rows, two digits (2^-15) above — a third fewer
+ * digit columns for batched steps at ~1e-4 relative error per product. Process-wide; engines drop
  * their captured step graphs when it changes (sp_cuda_engine_set_graphs off/on). */
 int32_t sp_cuda_set_activation_digits(int32_t mode);
 /* Which GEMV kernel runs (process-wide; op-level calls — engines have sp_cuda_engine_set_ring):
- *   0 (default): the tensor-core GEMV — one CTA per 16-row tile row for up to 10 activation rows, the one-pass many-row
- *      kernel (a CTA per eight tile rows, digits of a k-tile shared in shared memory) for passes of 11 to 32 rows;
- *   2: the tile-row kernel only (passes of 10 rows at any row count);
+ *   0 (default): the tensor-core GEMV — one CTA per 16-row tile row for up to 16 activation rows, the one-pass many-row
+ *      kernel (a CTA per eight tile rows, digits of a k-tile shared in shared memory) for passes of 17 to 32 rows;
+ *   2: the tile-row kernel only (passes of 16 rows at any row count);
  *   1: the CUDA-core GEMV on the raw blocks (an independent second implementation for cross-checks);
  *   3: the per-warp streaming variant of the tile-row kernel where the shape qualifies;
  *   4: calls of 1-5 rows take the bulk-copy ring GEMV (persistent CTAs, shared-memory ring fed by cp.async.bulk,
@@ -326,7 +326,7 @@ int32_t sp_cuda_engine_set_graphs(SpEngine* e, int32_t on);
  * on = 1: operands rounded once to fp16 (~3e-4 per product, inside the 1e-3 per-op bar, but the 8B shape's final logits
  *    then move by up to 4e-2), fused fp16 producers and the fp16 prefill attention: a 512-token prefill of the 8B shape
  *    takes 15 ms; products of 512 rows are 1 (Q8_0 4096 x 4096) to 2.4 times (128256 x 4096) as fast as with on = 2.
- * on = 0: integer-digit GEMV passes of 10 rows at any row count (201 ms for that prefill).
+ * on = 0: integer-digit GEMV passes of 16 rows at any row count.
  * Drops the captured step graphs. */
 int32_t sp_cuda_engine_set_large_m_gemm(SpEngine* e, int32_t on);
 /* Steps of 1-5 rows on the bulk-copy ring GEMV with the preceding norm / activation fused into it (default off: it
@@ -334,7 +334,7 @@ int32_t sp_cuda_engine_set_large_m_gemm(SpEngine* e, int32_t on);
 int32_t sp_cuda_engine_set_ring(SpEngine* e, int32_t on);
 /* For the steps that do not go to the tcgen05 GEMM (11-16 rows; every step of 11 rows and more when
  * sp_cuda_engine_set_large_m_gemm is 0): 1 = passes of up to 32 rows on the one-pass many-row GEMV, weights read once per
- * 32 rows; 0 (default) = passes of 10 rows on the tile-row kernel. The same exact integer products, another order of the
+ * 32 rows; 0 (default) = passes of 16 rows on the tile-row kernel. The same exact integer products, another order of the
  * f32 additions over k. */
 int32_t sp_cuda_engine_set_many_row_gemv(SpEngine* e, int32_t on);
 /* Per-kernel-family device timing (CUDA events around every launch; disables graphs while on). Families, in order:

@@ -42,7 +42,7 @@ int spec_greedy(Engine* target, Engine* draft, const uint32_t* prompt, size_t n_
 namespace {
 
 std::atomic<int> g_gemv_path{0};  // 0: tensor-core GEMV on tiled weights; 1: CUDA-core GEMV on raw blocks
-std::atomic<int> g_rows{1};       // calls of 11 rows and more on the one-pass many-row GEMV (path 2 turns it off: passes of 10 rows)
+std::atomic<int> g_rows{1};       // calls of 17 rows and more that are not on tcgen05: the many-row GEMV (path 2 turns it off: passes of 16 rows)
 std::atomic<int> g_ring{0};       // calls of 1-5 rows on the bulk-copy ring GEMV where it fits (path 4)
 
 #define API_BEGIN try {
@@ -341,7 +341,7 @@ int32_t sp_cuda_matmul_nt_dev(const SpWeight* w, const float* x_dev, int64_t m, 
     }
     if (w->tiled && g_gemv_path.load() == 0 && g_rows.load() && m > imma_rows_per_pass() && rows_supported(w->dtype, w->k) &&
         (w->dtype != T_Q8_0 || imma_q8_bpt(w->k) == 8)) {
-        // 11 rows and more: passes of up to 32 rows, each reading the weights once
+        // passes of up to 32 rows, each reading the weights once
         for (int64_t m0 = 0; m0 < m; m0 += IMMA_ROWS_MAX) {
             ImmaArgs ia{};
             ia.k = (int)w->k; ia.m = (int)std::min<int64_t>(IMMA_ROWS_MAX, m - m0); ia.nseg = 1;

@@ -133,10 +133,9 @@ class Engine {
     bool trace_on = false;
     bool use_graphs = true;
     // Steps of 11 rows and more that do not take the tcgen05 GEMM (11-16 rows, or use_tc5 off) as passes of up to 32 rows on
-    // the one-pass kernel (gemv_rows.cu) instead of passes of 10 on the tile-row kernel. Off by default: inside a step the
-    // two cost the same (32-row step of the 8B shape: 15.97 vs 15.50 ms) — the one-pass kernel reads the weights once but
-    // launches per segment and cannot take digits written by the fused producers; as a stand-alone matmul it is 1.3x
-    // faster (the op-level choice for 11-16 rows).
+    // the one-pass kernel (gemv_rows.cu) instead of passes of 16 on the tile-row kernel. Off by default: it launches per
+    // segment and cannot take digits written by the fused producers, and 13 rows of Q4_K 28672 x 4096 take 95 us on it, 41 on
+    // the other.
     bool use_rows = false;
     bool use_ring = false;     // steps of 1-5 rows on the bulk-copy ring GEMV (opt-in: measured slower than the tile-row kernels)
     // Steps of TC5_MIN_M rows and more (prompts, batches) run on a tcgen05 GEMM. tc5_exact (the default): exact-class operands
@@ -144,7 +143,7 @@ class Engine {
     // 2e-2 final-logit bar (tests/test_fullsize_gpu.py).
     // tc5_exact == false: operands rounded once to fp16 (gemm_tc5.cu; ~3e-4 per product; the 8B shape's logits then move by up
     // to 4e-2), with the fused fp16 producers and the fp16 prefill attention. use_tc5 == false: integer-digit GEMV passes of
-    // 10 rows at any row count (7x slower on a 512-token prompt). sp_cuda_engine_set_large_m_gemm chooses.
+    // 16 rows at any row count. sp_cuda_engine_set_large_m_gemm chooses.
     bool use_tc5 = true;
     bool tc5_exact = true;
     int set_large_m_gemm(int mode);                 // 2 exact class, 1 fp16-rounded, 0 integer passes

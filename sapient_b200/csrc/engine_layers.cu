@@ -44,8 +44,7 @@ bool Engine::plan_digits(int m, int k, ImmaArgs& ia) {
     ia.m = m;
     ia.k = k;
     if (k > ws_.k_max) return false;
-    // (11 to 16 rows: one launch makes the digits of both passes; as f32 rows and a conversion per pass they took four)
-    if (m > imma_rows_per_pass()) return !use_rows && imma_plan_passes(ia, ws_);
+    if (m > imma_rows_per_pass() || (use_rows && m >= ROWS_MIN_M)) return false;
     imma_plan(ia, ws_);
     return true;
 }
@@ -95,8 +94,8 @@ int Engine::gemv(const float* x, int ldx, int m, int k, const DevTensor* w0, con
             return SP_OK;
         }
     }
-    // 11 rows and more on one GPU: passes of up to 32 rows, each reading the weights once (gemv_rows.cu)
-    if (tiled && !tp_sum && !pre && use_rows && m > imma_rows_per_pass() && k % 256 == 0 && k <= ws_.k_max) {
+    // 11 rows and more on one GPU, where chosen: passes of up to 32 rows, each reading the weights once (gemv_rows.cu)
+    if (tiled && !tp_sum && !pre && use_rows && m >= ROWS_MIN_M && k % 256 == 0 && k <= ws_.k_max) {
         bool ok = true;
         for (int i = 0; i < 3 && ws[i]; ++i) ok = ok && rows_supported(ws[i]->dtype, k);
         if (ok) {
@@ -127,7 +126,6 @@ int Engine::gemv(const float* x, int ldx, int m, int k, const DevTensor* w0, con
             ImmaArgs ia{};
             if (pre) ia = *pre;
             ia.k = k; ia.m = std::min(pass, m - m0);
-            if (pre && m > pass) imma_pass(ia, m0, ia.m);
             ia.res = (res && !tp_sum) ? res + (size_t)m0 * ldy0 : nullptr;
             ia.ldres = ldy0;
             ia.tp = (tp_sum && !via_nccl) ? d_tp_ : nullptr;
@@ -267,7 +265,7 @@ int Engine::step_splits(int T) const {
         return std::min(want, limit);
     }
     int splits = 1;
-    if (T <= imma_rows_per_pass()) splits = d.n_heads * T <= 64 ? ATT_SPLITS : d.n_heads * T <= 128 ? 8 : 4;
+    if (T < ROWS_MIN_M) splits = d.n_heads * T <= 64 ? ATT_SPLITS : d.n_heads * T <= 128 ? 8 : 4;
     if (T <= ATT_SPLIT_TOKENS) {
         int by_ctx = 1;
         while (by_ctx < ATT_SPLITS && by_ctx * 128 < step_ctx_) by_ctx <<= 1;

@@ -152,7 +152,7 @@ cudaError_t launch_repack(int dtype, const uint8_t* raw, int64_t n, int64_t k, u
 // ─────────────────────────── activation digits ───────────────────────────────
 // Where the digits of one GEMV input go (see gemv_imma.cuh for the layouts).
 struct QuantOut {
-    int k, kp, digits, eb, ncp;
+    int k, kp, digits, eb, ncp, linear;
     int8_t* xq;
     float* colscale;
     int8_t* xs32d;
@@ -160,7 +160,7 @@ struct QuantOut {
 };
 __host__ inline QuantOut quant_out(const ImmaArgs& a) {
     QuantOut q;
-    q.k = a.k; q.kp = a.kp; q.digits = a.digits; q.eb = a.eb; q.ncp = a.ncp;
+    q.k = a.k; q.kp = a.kp; q.digits = a.digits; q.eb = a.eb; q.ncp = a.ncp; q.linear = a.linear;
     q.xq = const_cast<int8_t*>(a.xq); q.colscale = const_cast<float*>(a.colscale);
     q.xs32d = const_cast<int8_t*>(a.xs32d); q.xs16d = const_cast<int8_t*>(a.xs16d);
     return q;
@@ -213,9 +213,10 @@ __device__ __forceinline__ void quantize_chunk(const float (&v)[8], bool live, i
         const int s32 = s16 + __shfl_xor_sync(0xFFFFFFFFu, s16, 2);
         if (d < digits && live) {
             const int col = m * digits + d;
-            int8_t* dst = qo.xq + (int64_t)col * qo.kp + (int64_t)tile * 256 + blk * 8 + 4 * h;
-            *reinterpret_cast<uint32_t*>(dst + t0 * 64) = w0[d];
-            *reinterpret_cast<uint32_t*>(dst + (t0 + 1) * 64) = w1[d];
+            int8_t* dst = qo.linear ? qo.xq + (int64_t)col * qo.kp + (int64_t)tile * 256 + blk * 8 + 4 * h + t0 * 64
+                                    : qo.xq + (((int64_t)tile * qo.ncp + (col & ~7)) * 256 + (blk >> 1) * 512 + ((col & 7) * 4 + t0) * 16 + (blk & 1) * 8 + 4 * h);
+            *reinterpret_cast<uint32_t*>(dst) = w0[d];
+            *reinterpret_cast<uint32_t*>(dst + (qo.linear ? 64 : 16)) = w1[d];
             int8_t* r32 = qo.xs32d + ((int64_t)tile * qo.ncp + col) * 32;
             int8_t* r16 = qo.xs16d + ((int64_t)tile * qo.ncp + col) * 32;
             if ((lane & 1) == 0) {
@@ -413,45 +414,25 @@ __global__ void __launch_bounds__(256) attn_merge_quant_kernel(const float* __re
     }
 }
 
-// 1 (default): 3 digits for every pass (10 rows per pass): activations held to 2^-23 of each block's maximum at any row
-//    count — the setting under which full-size models stay within the final-logit bar of the reference's f32 path.
-// 0: 3 digits while they fit one 8-column n-tile (m <= 2), else 2 digits (2^-15) and 16 rows per pass: fewer passes for
-//    batched steps, at ~1e-4 relative error per product.
+// 1 (default): 3 digits at any row count: activations held to 2^-23 of each block's maximum, the setting under which full-size models
+//    stay within the final-logit bar of the reference's f32 path.
+// 0: 3 digits while they fit one 8-column n-tile (m <= 2), else 2 digits (2^-15): fewer n-tiles, at ~1e-4 relative error per product.
 static std::atomic<int> g_digit_mode{1};
 void imma_set_digit_mode(int mode) { g_digit_mode.store(mode ? 1 : 0); }
-int imma_rows_per_pass() { return g_digit_mode.load() ? 10 : 16; }
+int imma_rows_per_pass() { return 16; }
 
 void imma_plan(ImmaArgs& a, const ActWorkspace& ws) {
-    a.digits = (a.m <= 2 || (g_digit_mode.load() && a.m <= 10)) ? 3 : 2;
-    const int cols = a.m * a.digits;
-    a.ncp = cols <= 8 ? 8 : cols <= 16 ? 16 : 32;
+    a.digits = (a.m <= 2 || g_digit_mode.load()) ? 3 : 2;
+    a.ncp = (a.m * a.digits + 7) / 8 * 8;
     a.eb = (a.k % 256 == 0) ? 256 : 32;
     a.kp = (a.k + 255) / 256 * 256;
+    a.linear = 0;
     a.xq = ws.xq; a.colscale = ws.colscale; a.xs32d = ws.xs32d; a.xs16d = ws.xs16d; a.waits = ws.waits;
-}
-
-bool imma_plan_passes(ImmaArgs& a, const ActWorkspace& ws) {
-    if (!g_digit_mode.load() || a.m <= 10 || a.m > 16) return false;
-    a.digits = 3;
-    a.ncp = 64;  // a second pass looks at columns 30 .. 61
-    a.eb = (a.k % 256 == 0) ? 256 : 32;
-    a.kp = (a.k + 255) / 256 * 256;
-    a.xq = ws.xq; a.colscale = ws.colscale; a.xs32d = ws.xs32d; a.xs16d = ws.xs16d; a.waits = ws.waits;
-    return true;
-}
-
-void imma_pass(ImmaArgs& a, int m0, int rows) {
-    const int col = m0 * a.digits, cols = rows * a.digits;
-    a.xq += (int64_t)col * a.kp;
-    a.colscale += col;
-    a.xs32d += col * 32;
-    a.xs16d += col * 32;
-    a.m = rows;
-    a.nt = cols <= 8 ? 1 : cols <= 16 ? 2 : 4;
 }
 
 void imma_plan_rows(ImmaArgs& a, const ActWorkspace& ws) {
     a.digits = 3;
+    a.linear = 1;
     a.ncp = (a.m * 3 + 31) / 32 * 32;
     a.eb = (a.k % 256 == 0) ? 256 : 32;
     a.kp = (a.k + 255) / 256 * 256;
@@ -559,7 +540,7 @@ __device__ __forceinline__ void load_q8_unit(const uint8_t* base, int u, int lan
     const uint8_t* tile = base + (int64_t)(BPT == 8 ? u >> 1 : u) * (BPT * 544);
     const int half = BPT == 8 ? u & 1 : 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) r.q[j] = ldg_u4(tile + half * 2048 + j * 512 + lane * 16);
+    for (int j = 0; j < 4; ++j) r.q[j] = ldw_u4(tile + half * 2048 + j * 512 + lane * 16);
     const uint8_t* d = tile + BPT * 512 + half * 8;
     r.d0 = __ldg(reinterpret_cast<const uint2*>(d + g * (2 * BPT)));
     r.d1 = __ldg(reinterpret_cast<const uint2*>(d + (g + 8) * (2 * BPT)));
@@ -569,15 +550,20 @@ template <int NT, int BPT>
 __device__ __forceinline__ void compute_q8_unit(const ImmaArgs& a, const Q8Unit& r, int u, int lane, float (&acc)[NT][4]) {
     const int g = lane >> 2, t = lane & 3;
     const uint32_t e0[2] = {r.d0.x, r.d0.y}, e1[2] = {r.d1.x, r.d1.y};
+    const int8_t* src = a.xq + (int64_t)(u >> 1) * a.ncp * 256 + (u & 1) * 1024 + lane * 16;
+    auto digits = [&](int nt, uint4 (&b)[2]) {
+        b[0] = b[1] = make_uint4(0u, 0u, 0u, 0u);
+        if (NT > 2 || nt * 8 + g < a.m * a.digits) {
+            b[0] = ldg_u4(src + nt * 2048);
+            b[1] = ldg_u4(src + nt * 2048 + 512);
+        }
+    };
+    uint4 next[2];
+    digits(0, next);
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-        const int col = nt * 8 + g;
-        uint4 b[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-        if (col < a.m * a.digits) {
-            const int8_t* src = a.xq + (int64_t)col * a.kp + (int64_t)(u >> 1) * 256 + t * 64 + (u & 1) * 32;
-            b[0] = ldg_u4(src);
-            b[1] = ldg_u4(src + 16);
-        }
+        const uint4 b[2] = {next[0], next[1]};
+        if (nt + 1 < NT) digits(nt + 1, next);
         float2 cs = make_float2(0.f, 0.f);
         if (BPT == 8) cs = __ldg(reinterpret_cast<const float2*>(a.colscale + (int64_t)(u >> 1) * a.ncp + nt * 8 + 2 * t));
         float f[4] = {0.f, 0.f, 0.f, 0.f};
@@ -603,20 +589,20 @@ __device__ __forceinline__ void compute_q8_unit(const ImmaArgs& a, const Q8Unit&
 }
 // A warp's units of one tile row. DEPTH of them are in flight, the first ones from before the previous kernel has ended; read a
 // block at a time, each waited for, a Q8_0 matrix came at a third of the rate (28672 x 4096: 54 us).
-template <int NT, int BPT>
+template <int NT, int BPT, int WARPS>
 __device__ __forceinline__ void row_q8_0(const ImmaArgs& a, const uint8_t* base, int warp, int lane, float (&acc)[NT][4]) {
     constexpr int DEPTH = NT == 1 ? 3 : 2;
     const int units = a.k >> 7;
     Q8Unit r[DEPTH];
 #pragma unroll
     for (int i = 0; i < DEPTH; ++i)
-        if (warp + i * IMMA_WARPS < units) load_q8_unit<BPT>(base, warp + i * IMMA_WARPS, lane, r[i]);
+        if (warp + i * WARPS < units) load_q8_unit<BPT>(base, warp + i * WARPS, lane, r[i]);
     pdl_wait();
     pdl_trigger();
-    for (int u0 = warp; u0 < units; u0 += DEPTH * IMMA_WARPS) {
+    for (int u0 = warp; u0 < units; u0 += DEPTH * WARPS) {
 #pragma unroll
         for (int i = 0; i < DEPTH; ++i) {
-            const int u = u0 + i * IMMA_WARPS, next = u + DEPTH * IMMA_WARPS;
+            const int u = u0 + i * WARPS, next = u + DEPTH * WARPS;
             if (u >= units) break;
             compute_q8_unit<NT, BPT>(a, r[i], u, lane, acc);
             if (next < units) load_q8_unit<BPT>(base, next, lane, r[i]);
@@ -630,7 +616,7 @@ __device__ __forceinline__ void tile_q8_0(const ImmaArgs& a, const uint8_t* tile
     const int g = lane >> 2, t = lane & 3;
     const uint16_t* dh = reinterpret_cast<const uint16_t*>(tile + bpt * 512);
     for (int bb = 0; bb < bpt; ++bb) {
-        const uint4 q = ldg_u4(tile + bb * 512 + lane * 16);
+        const uint4 q = ldw_u4(tile + bb * 512 + lane * 16);
         const float d0 = half_bits_to_float(__ldg(dh + g * bpt + bb)), d1 = half_bits_to_float(__ldg(dh + (g + 8) * bpt + bb));
         const int blk32 = kt * bpt + bb;
 #pragma unroll
@@ -638,7 +624,7 @@ __device__ __forceinline__ void tile_q8_0(const ImmaArgs& a, const uint8_t* tile
             const int col = nt * 8 + g;
             uint2 b = make_uint2(0u, 0u);
             if (col < a.m * a.digits)
-                b = __ldg(reinterpret_cast<const uint2*>(a.xq + (int64_t)col * a.kp + (int64_t)(blk32 >> 3) * 256 + t * 64 + (blk32 & 7) * 8));
+                b = __ldg(reinterpret_cast<const uint2*>(a.xq + ((int64_t)(blk32 >> 3) * a.ncp + nt * 8) * 256 + ((blk32 >> 1) & 3) * 512 + lane * 16 + (blk32 & 1) * 8));
             int c[4];
             imma_k32(c, q.x, q.z, q.y, q.w, b.x, b.y, 0, 0, 0, 0);
             const float2 cs = __ldg(reinterpret_cast<const float2*>(a.colscale + (int64_t)(blk32 * 32 / a.eb) * a.ncp + nt * 8 + 2 * t));
@@ -679,14 +665,19 @@ __device__ __forceinline__ void reduce_store(const ImmaArgs& a, const ImmaSeg& s
     }
 }
 
-// Kernel A (any shape): one CTA per tile row; its 8 warps split the k-tiles, operands straight from global memory.
+// Kernel A (any shape): one CTA per tile row; its warps split the k-tiles, operands straight from global memory. What bounds it is
+// latency: of 16 warps an SM most wait for weights from DRAM or digits from L1. So weights do not go through L1 (half of the digits'
+// loads missed there), digits come in fragments, and from three n-tiles on a chunk of them is requested while the one before is
+// multiplied. Up to 16 rows in one pass (two of 10 rows read and unpacked every weight twice). Q4_K 28672 x 4096, us: 5 rows 31.2 -> 23.4,
+// 10 rows 43 -> 36, 13 rows 95 -> 41; Q6_K 5 rows 37.7 -> 31.0, 13 rows 128 -> 55; Q8_0 1 row 28.6 -> 26.4, 5 rows 35.1 -> 29.4, 13 rows
+// 90 -> 47.
 // FMT: 0 = segments of any format; T_Q4_K / T_Q6_K / T_Q8_0 = every segment of the launch has that format — the code for the
 // other formats is left out, which lets the M <= 2 instance of the K-quants fit 80 registers and run three CTAs (24 warps)
 // per SM instead of two.
-template <int NT, int FMT>
-__global__ void __launch_bounds__(IMMA_WARPS * 32, (NT == 1 && FMT != 0 && FMT != T_Q8_0) ? 3 : 2) gemv_imma_kernel(const ImmaArgs a) {
-    __shared__ float red[IMMA_WARPS * NT * 4 * 32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+template <int NT, int FMT, int WARPS = IMMA_WARPS>
+__global__ void __launch_bounds__(WARPS * 32, (NT == 1 && FMT != 0 && FMT != T_Q8_0) ? 3 : 16 / WARPS) gemv_imma_kernel(const ImmaArgs a) {
+    __shared__ float red[WARPS * NT * 4 * 32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int rt = blockIdx.x, s = 0;
     while (s < a.nseg - 1 && rt >= (a.seg[s].n + 15) / 16) { rt -= (a.seg[s].n + 15) / 16; ++s; }
     const ImmaSeg& sg = a.seg[s];
@@ -699,64 +690,83 @@ __global__ void __launch_bounds__(IMMA_WARPS * 32, (NT == 1 && FMT != 0 && FMT !
         const int kts = a.k >> 8;
         const uint8_t* base = sg.wt + (int64_t)rt * kts * Q4_K_TILE_BYTES;
         Q4Regs ra, rb;
-        BFrag<NT> b;
+        auto tile_q4 = [&](int at, const Q4Regs& w) {
+            if constexpr (NT <= 2) {
+                BFrag<NT> b;
+                load_b_global<NT>(a, at, lane, true, false, b);
+                compute_q4_k<NT>(w, b, lane, acc);
+            } else {
+                compute_q4_k<NT>(w, BGlobal<NT>(a, at, lane), lane, acc);
+            }
+        };
+        constexpr bool TWO = NT <= 3;  // (a second tile in flight where registers allow)
         int kt = warp;
         if (kt < kts) load_q4_k<true>(base + (int64_t)kt * Q4_K_TILE_BYTES, lane, ra);
-        if (kt + IMMA_WARPS < kts) load_q4_k<true>(base + (int64_t)(kt + IMMA_WARPS) * Q4_K_TILE_BYTES, lane, rb);
+        if (TWO && kt + WARPS < kts) load_q4_k<true>(base + (int64_t)(kt + WARPS) * Q4_K_TILE_BYTES, lane, rb);
         pdl_wait();  // the weight tiles above are in flight while the producer of the activations finishes
         pdl_trigger();
-        bool first = true;
-        while (kt < kts) {
-            const int k1 = kt + IMMA_WARPS, k2 = kt + 2 * IMMA_WARPS;
-            if (!first && k1 < kts) load_q4_k<true>(base + (int64_t)k1 * Q4_K_TILE_BYTES, lane, rb);
-            first = false;
-            load_b_global<NT>(a, kt, g, t, true, false, b);
-            compute_q4_k<NT>(ra, b, lane, acc);
-            if (k1 >= kts) break;
-            if (k2 < kts) load_q4_k<true>(base + (int64_t)k2 * Q4_K_TILE_BYTES, lane, ra);
-            load_b_global<NT>(a, k1, g, t, true, false, b);
-            compute_q4_k<NT>(rb, b, lane, acc);
-            kt = k2;
+        if (TWO) {
+            bool first = true;
+            while (kt < kts) {
+                const int k1 = kt + WARPS, k2 = kt + 2 * WARPS;
+                if (!first && k1 < kts) load_q4_k<true>(base + (int64_t)k1 * Q4_K_TILE_BYTES, lane, rb);
+                first = false;
+                tile_q4(kt, ra);
+                if (k1 >= kts) break;
+                if (k2 < kts) load_q4_k<true>(base + (int64_t)k2 * Q4_K_TILE_BYTES, lane, ra);
+                tile_q4(k1, rb);
+                kt = k2;
+            }
+        } else {
+            for (; kt < kts; kt += WARPS) {
+                tile_q4(kt, ra);
+                if (kt + WARPS < kts) load_q4_k<true>(base + (int64_t)(kt + WARPS) * Q4_K_TILE_BYTES, lane, ra);
+            }
         }
     } else if (FMT == T_Q6_K || (FMT == 0 && sg.dtype == T_Q6_K)) {
         const int kts = a.k >> 8;
         const uint8_t* base = sg.wt + (int64_t)rt * kts * Q6_K_TILE_BYTES;
         constexpr bool TWO = NT == 1 && FMT == 0;  // (a second tile in flight where registers allow)
         Q6Regs ra, rb;
-        BFrag<NT> b;
+        auto tile_q6 = [&](int at, const Q6Regs& w) {
+            if constexpr (NT <= 2) {
+                BFrag<NT> b;
+                load_b_global<NT>(a, at, lane, false, true, b);
+                compute_q6_k<NT>(w, b, lane, acc);
+            } else {
+                compute_q6_k<NT>(w, BGlobal<NT>(a, at, lane), lane, acc);
+            }
+        };
         if (warp < kts) load_q6_k<true>(base + (int64_t)warp * Q6_K_TILE_BYTES, lane, ra);
-        if (TWO && warp + IMMA_WARPS < kts) load_q6_k<true>(base + (int64_t)(warp + IMMA_WARPS) * Q6_K_TILE_BYTES, lane, rb);
+        if (TWO && warp + WARPS < kts) load_q6_k<true>(base + (int64_t)(warp + WARPS) * Q6_K_TILE_BYTES, lane, rb);
         pdl_wait();
         pdl_trigger();
         if (TWO) {
-            for (int kt = warp; kt < kts; kt += 2 * IMMA_WARPS) {
-                const int k1 = kt + IMMA_WARPS, k2 = k1 + IMMA_WARPS, k3 = k2 + IMMA_WARPS;
-                load_b_global<NT>(a, kt, g, t, false, true, b);
-                compute_q6_k<NT>(ra, b, lane, acc);
+            for (int kt = warp; kt < kts; kt += 2 * WARPS) {
+                const int k1 = kt + WARPS, k2 = k1 + WARPS, k3 = k2 + WARPS;
+                tile_q6(kt, ra);
                 if (k2 < kts) load_q6_k<true>(base + (int64_t)k2 * Q6_K_TILE_BYTES, lane, ra);
                 if (k1 >= kts) break;
-                load_b_global<NT>(a, k1, g, t, false, true, b);
-                compute_q6_k<NT>(rb, b, lane, acc);
+                tile_q6(k1, rb);
                 if (k3 < kts) load_q6_k<true>(base + (int64_t)k3 * Q6_K_TILE_BYTES, lane, rb);
             }
         } else {
-            for (int kt = warp; kt < kts; kt += IMMA_WARPS) {
+            for (int kt = warp; kt < kts; kt += WARPS) {
                 if (kt != warp) load_q6_k<true>(base + (int64_t)kt * Q6_K_TILE_BYTES, lane, ra);
-                load_b_global<NT>(a, kt, g, t, false, true, b);
-                compute_q6_k<NT>(ra, b, lane, acc);
+                tile_q6(kt, ra);
             }
         }
     } else if (FMT == 0 || FMT == T_Q8_0) {
         const int bpt = sg.bpt, kts = (a.k >> 5) / bpt, tb = bpt * 544;
         const uint8_t* base = sg.wt + (int64_t)rt * kts * tb;
         if (bpt == 8) {
-            row_q8_0<NT, 8>(a, base, warp, lane, acc);
+            row_q8_0<NT, 8, WARPS>(a, base, warp, lane, acc);
         } else if (bpt == 4) {
-            row_q8_0<NT, 4>(a, base, warp, lane, acc);
+            row_q8_0<NT, 4, WARPS>(a, base, warp, lane, acc);
         } else {
             pdl_wait();
             pdl_trigger();
-            for (int kt = warp; kt < kts; kt += IMMA_WARPS) tile_q8_0<NT>(a, base + (int64_t)kt * tb, kt, bpt, lane, acc);
+            for (int kt = warp; kt < kts; kt += WARPS) tile_q8_0<NT>(a, base + (int64_t)kt * tb, kt, bpt, lane, acc);
         }
     }
 #pragma unroll
@@ -764,7 +774,7 @@ __global__ void __launch_bounds__(IMMA_WARPS * 32, (NT == 1 && FMT != 0 && FMT !
 #pragma unroll
         for (int e = 0; e < 4; ++e) red[((warp * NT + nt) * 4 + e) * 32 + lane] = acc[nt][e];
     __syncthreads();
-    reduce_store<NT, IMMA_WARPS>(a, sg, s == 0, rt, red);
+    reduce_store<NT, WARPS>(a, sg, s == 0, rt, red);
 }
 
 // ── Kernel B (k % 256 == 0, digits fit shared memory): persistent streaming kernel ──
@@ -860,12 +870,8 @@ __global__ void __launch_bounds__(STREAM_WARPS * 32, 1) gemv_imma_stream_kernel(
     asm volatile("griddepcontrol.launch_dependents;\n" ::);
     const int ncols = a.m * a.digits;
     {
-        int8_t* xs = reinterpret_cast<int8_t*>(smem + p.xq_off);
-        const int vec_per_col = a.kp / 16;
-        for (int i = threadIdx.x; i < ncols * vec_per_col; i += blockDim.x) {
-            const int c = i / vec_per_col, v = i - c * vec_per_col;
-            reinterpret_cast<uint4*>(xs)[i] = ldg_u4(a.xq + (int64_t)c * a.kp + (int64_t)v * 16);
-        }
+        uint4* xs = reinterpret_cast<uint4*>(smem + p.xq_off);
+        for (int i = threadIdx.x; i < kts * a.ncp * 16; i += blockDim.x) xs[i] = ldg_u4(a.xq + (int64_t)i * 16);
         // records [kt][col][32 B] -> shared [kt][ncols][32 B]; scales [kt][ncp] -> shared [kt][ncp]
         uint4* r32 = reinterpret_cast<uint4*>(smem + p.rec32_off);
         uint4* r16 = reinterpret_cast<uint4*>(smem + p.rec16_off);
@@ -907,10 +913,10 @@ __global__ void __launch_bounds__(STREAM_WARPS * 32, 1) gemv_imma_stream_kernel(
             for (int nt = 0; nt < NT; ++nt) {
                 const int col = nt * 8 + g;
                 if (col < ncols) {
-                    const int8_t* base = xs + (size_t)col * a.kp + (size_t)kt * 256 + t * 64;
+                    const int8_t* base = xs + ((size_t)kt * a.ncp + nt * 8) * 256 + lane * 16;
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        const uint4 v = ld_u4(base + 16 * q);
+                        const uint4 v = ld_u4(base + 512 * q);
                         b.w[nt][4 * q] = v.x; b.w[nt][4 * q + 1] = v.y; b.w[nt][4 * q + 2] = v.z; b.w[nt][4 * q + 3] = v.w;
                     }
                     const size_t rec = ((size_t)kt * ncols + col) * 32 + 4 * t;
@@ -981,7 +987,7 @@ static PerDeviceOnce g_stream_attr[3];
 // Shared-memory layout of the streaming kernel, or total == 0 when the launch does not qualify.
 static StreamPlan plan_stream(const ImmaArgs& a) {
     StreamPlan p{};
-    if (a.k % 256 != 0 || a.ncp > 16 || a.nt) return p;
+    if (a.k % 256 != 0 || a.ncp > 16) return p;
     const int kts = a.k / 256, ncols = a.m * a.digits, nt = a.ncp / 8;
     int stage = 0, tiles = 0;
     for (int s = 0; s < a.nseg; ++s) {
@@ -997,7 +1003,7 @@ static StreamPlan plan_stream(const ImmaArgs& a) {
         int off = STREAM_WARPS * stages * stage;
         p.stages = stages;
         p.bar_off = off; off += STREAM_WARPS * STREAM_MAX_STAGES * 8;
-        p.xq_off = off; off += ncols * a.kp;
+        p.xq_off = off; off += kts * a.ncp * 256;
         p.rec32_off = off; off += kts * ncols * 32;
         p.rec16_off = off; off += kts * ncols * 32;
         p.cs_off = off; off += kts * a.ncp * 4;
@@ -1016,7 +1022,7 @@ cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st) {
     int tiles = 0;
     for (int s = 0; s < a.nseg; ++s) tiles += (a.seg[s].n + 15) / 16;
     if (tiles == 0) return cudaSuccess;
-    const int nt = a.nt ? a.nt : a.ncp / 8;
+    const int nt = a.ncp / 8;
     // The persistent TMA-streaming kernel is opt-in: measured on B200 it trails the per-tile-row kernel
     // (132 vs 81 us on a 128256 x 4096 Q4_K matrix), so the default is the latter.
     const StreamPlan p = (g_imma_kernel.load() == 3 && !a.tp) ? plan_stream(a) : StreamPlan{};
@@ -1041,18 +1047,22 @@ cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st) {
         q6_only = q6_only && a.seg[s].dtype == T_Q6_K;
         q8_only = q8_only && a.seg[s].dtype == T_Q8_0;
     }
-    // The 80-register single-format instances trade per-CTA speed for occupancy: they win once the grid is several
-    // waves deep (gate|up, lm_head) and lose on grids that fit the SMs at once (o_proj, down_proj), where one CTA's
-    // latency is the kernel's.
-    const bool deep = tiles >= 1024;
-    if (nt == 1 && q4_only && deep) le = launch_pdl(gemv_imma_kernel<1, T_Q4_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
-    else if (nt == 1 && q6_only && deep) le = launch_pdl(gemv_imma_kernel<1, T_Q6_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
-    else if (nt == 1 && q8_only) le = launch_pdl(gemv_imma_kernel<1, T_Q8_0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
-    else if (nt == 2 && q8_only) le = launch_pdl(gemv_imma_kernel<2, T_Q8_0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
-    else if (nt == 4 && q8_only) le = launch_pdl(gemv_imma_kernel<4, T_Q8_0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
-    else if (nt == 1) le = launch_pdl(gemv_imma_kernel<1, 0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
-    else if (nt == 2) le = launch_pdl(gemv_imma_kernel<2, 0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
-    else if (nt == 4) le = launch_pdl(gemv_imma_kernel<4, 0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
+    // One or two rows: the 80-register single-format instances trade per-block speed for a third block per SM. Q6_K 17920 x 1536 (1120
+    // tile rows) 11.1 -> 9.7 us, 128256 x 4096 99 -> 81; with grids that fit the SMs at once a block's latency is the kernel's. Q4_K has two
+    // tiles per warp in flight without them, and few waves are worth more evenly filled: 18944 x 3584 13.6 us with two blocks, 15.4
+    // with three, 28672 x 4096 19.4 and 20.9, but 128256 x 4096 71.9 and 66.6, 151936 x 1536 58.0 and 49.8.
+    const bool deep_q4 = tiles >= 4096, deep_q6 = tiles >= 1024;
+    // Fewer tile rows than SMs: 16 warps share a row's columns, where there is a piece for more than eight. Q4_K 1536 x 8960 1 row 6.3
+    // -> 5.6 us, 13 rows 14.7 -> 10.9; Q8_0 896 x 4864 5.6 -> 4.6, 13 rows 9.5 -> 7.4. (With eight pieces or fewer 2 % slower.)
+    const bool wide = tiles <= device_sm_count() && a.k / (q8_only && a.seg[0].bpt > 1 ? 128 : 256) > IMMA_WARPS;
+    if (nt == 1 && q4_only && deep_q4) le = launch_pdl(gemv_imma_kernel<1, T_Q4_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
+    else if (nt == 1 && q6_only && deep_q6) le = launch_pdl(gemv_imma_kernel<1, T_Q6_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
+#define SP_GEMV(N)                                                                                                                   \
+    else if (nt == N)                                                                                                                \
+        le = !wide ? launch_pdl(q8_only ? gemv_imma_kernel<N, T_Q8_0> : gemv_imma_kernel<N, 0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a) \
+                   : launch_pdl(q8_only ? gemv_imma_kernel<N, T_Q8_0, 16> : gemv_imma_kernel<N, 0, 16>, dim3(tiles), dim3(512), 0, st, a);
+    SP_GEMV(1) SP_GEMV(2) SP_GEMV(3) SP_GEMV(4) SP_GEMV(5) SP_GEMV(6)
+#undef SP_GEMV
     else return cudaErrorInvalidValue;
     if (le != cudaSuccess) return le;
     return count_launch_and_check();

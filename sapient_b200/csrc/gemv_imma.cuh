@@ -31,7 +31,7 @@ namespace sp {
 constexpr int TILE_ROWS = 16;
 constexpr int Q4_K_TILE_BYTES = 16 * 144;  // 2304
 constexpr int Q6_K_TILE_BYTES = 16 * 210;  // 3360
-constexpr int IMMA_MAX_NT = 4;             // n-tiles of 8 digit columns per launch (<= 16 activation rows)
+constexpr int IMMA_MAX_NT = 6;             // n-tiles of 8 digit columns per launch (<= 16 activation rows of 3 digits)
 
 struct ImmaSeg {
     const uint8_t* wt;  // tiled weights
@@ -51,11 +51,13 @@ struct ImmaArgs {
     int digits;   // 2 or 3
     int ncp;      // padded digit columns
     int* waits;   // WaitFlags of the launch's owner
-    int nt;       // 8-column tiles of this launch; 0: all of them
+    int linear;   // digits one column after the other (gemv_rows.cu stages them so) instead of in fragments
     int eb;       // columns per activation exponent block: 256 or 32
     int kp;       // k rounded up to 256: column stride of xq
-    // Digits: xq[col][kp]; inside each 256-column tile the bytes are ordered [t 0..3][block 0..7][8 B], the 8 B
-    // of (t, block) being columns 4t..4t+3 and 16+4t..16+4t+3 of that 32-block (one lane's B fragment).
+    // Digits in B fragments: [k / 256][ncp / 8][chunk 0..3][lane 0..31][16 B], lane (g, t)'s 16 B being columns 4t..4t+3 and
+    // 16+4t..16+4t+3 of the 32-blocks 2 chunk and 2 chunk + 1 of digit column 8 nt + g: a warp's load is 512 bytes in a row. (A column
+    // after the other it touched 64 separate pieces: 10 rows took 16 wavefronts a load and four times as long as its products.)
+    // linear: xq[col][kp], the bytes of a tile ordered [t 0..3][block 0..7][8 B].
     const int8_t* xq;
     const float* colscale;  // [k / eb][ncp]
     // Digit sums S of every 32-block (xs32d) and 16-block (xs16d) of a tile, split as S = a + 64 b with a in

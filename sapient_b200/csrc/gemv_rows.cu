@@ -1,8 +1,7 @@
 // Tensor-core GEMV for 11 to 32 activation rows in ONE pass over the weights (exact integer products, three digits).
 //
 // The tile-row kernel (gemv_imma.cu) gives a CTA one 16-row tile row and lets its warps split the k-tiles, so every warp
-// needs its own activation digits and fetches them from L2 into registers: fine for a few rows, but at 10 rows per pass
-// a 32-row step streams the weights four times and waits on ~90 dependent L2 loads per tile. Here the roles are turned
+// needs its own activation digits and fetches them into registers, and takes 16 rows a pass. Here the roles are turned
 // round: a CTA owns EIGHT tile rows (128 weight rows, one per warp) and walks the k-tiles of its K range together, so
 // the digits of a k-tile — up to 96 columns x 256 bytes — are staged once per CTA in shared memory (cp.async, double
 // buffered) and read by all eight warps, while each warp keeps its weight tile in registers (the next one prefetched)

@@ -59,8 +59,8 @@ cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st);
 // 0: the one-CTA-per-tile-row kernel; 3: the persistent TMA-streaming kernel when k % 256 == 0 and the digits fit
 // shared memory.
 void imma_select_kernel(int which);
-// Activation precision of the tensor-core GEMV passes (process-wide): 0 = 3 digits for 1-2 rows, 2 digits (16 rows per
-// pass) above; 1 = 3 digits always (10 rows per pass). imma_rows_per_pass() is the pass size that follows.
+// Activation precision of the tensor-core GEMV passes (process-wide): 0 = 3 digits for 1-2 rows, 2 digits above; 1 = 3 digits
+// always. imma_rows_per_pass(): rows of one pass.
 void imma_set_digit_mode(int mode);
 int imma_rows_per_pass();
 // A device-side wait that runs out is reported to flags in mapped host memory, a kernel's plain store; whoever owns the launch (an
@@ -171,7 +171,7 @@ struct ActWorkspace {
     Tc5Scratch tc5;            // only where the GEMM with fp16-rounded operands was chosen
     cudaError_t ensure_xh(size_t elems);  // grows the buffer (allocates: not during stream capture)
     cudaError_t ensure_split();           // makes tc5 (allocates: not during stream capture)
-    static constexpr int NCP_MAX = 96;  // digit columns: 32 rows x 3 digits (gemv_rows.cu); the tile-row kernel uses up to 32
+    static constexpr int NCP_MAX = 96;  // digit columns: 32 rows x 3 digits (gemv_rows.cu); the tile-row kernel uses up to 48
     cudaError_t alloc(int k_max_);
     void release();
 };
@@ -191,18 +191,15 @@ struct RowsScratch {
     cudaError_t alloc();
     void release();
 };
+constexpr int ROWS_MIN_M = 11;  // rows from which an engine that has chosen it takes this kernel
 bool rows_supported(int dtype, int64_t k);
-// Digits of 11 .. 16 rows at once (three each), for a producer that writes them in one launch; false where the mode or the count is
-// another. imma_pass makes of such a plan the launch of rows m0 .. m0 + rows - 1.
-bool imma_plan_passes(ImmaArgs& a, const ActWorkspace& ws);
-void imma_pass(ImmaArgs& a, int m0, int rows);
 void imma_plan_rows(ImmaArgs& a, const ActWorkspace& ws);  // three digits, 32-column groups (a.m <= IMMA_ROWS_MAX)
 cudaError_t launch_gemv_rows(const ImmaArgs& a, const RowsScratch& sc, cudaStream_t st);
 
 // Large-M dequant GEMM on tcgen05 / TMEM (gemm_tc5.cu): y[m, n] = x·Wᵀ (+ bias, + res) from the tiled weights and an
 // fp16 copy of the activations; k % 256 == 0, Q4_K / Q6_K / Q8_0.
-// Up to 16 rows the integer-digit GEMV: its products are exact, 3e-7 of a result's norm against 5e-7 to 1.4e-6, although two of its
-// passes take longer from 11 rows on (Q4_K 28672 x 4096: 13 rows 96 us, 17 rows on the GEMM 54).
+// Up to 16 rows the integer-digit GEMV: its products are exact, 3e-7 of a result's norm against 5e-7 to 1.4e-6, and it takes little
+// longer even where the GEMM is best (Q4_K 28672 x 4096: 16 rows 46 us, 17 rows on the GEMM 42).
 constexpr int TC5_MIN_M = 17;
 bool tc5_supported(int dtype, int64_t k);
 cudaError_t launch_x_to_f16(const float* x, int ldx, int m, int k, __half* out, cudaStream_t st);

@@ -375,12 +375,12 @@ class ForwardEngine:
     def set_large_m_gemm(self, on) -> None:
         """Steps of 17 rows and more: 2 (default) the tcgen05 GEMM with exact-class operands (activations as leading
         fp16 part + remainder, weights unrounded); True / 1 the one with operands rounded to fp16 (1 to 2.4 times
-        as fast per product of 512 rows; final logits of full-size models may leave the 2e-2 bar); False / 0 integer-digit GEMV passes of 10 rows."""
+        as fast per product of 512 rows; final logits of full-size models may leave the 2e-2 bar); False / 0 integer-digit GEMV passes of 16 rows."""
         check(lib().sp_cuda_engine_set_large_m_gemm(self._h, int(on)))
 
     def set_many_row_gemv(self, on: bool) -> None:
         """Steps of 11 rows and more as passes of up to 32 rows on the one-pass GEMV (exact integer products, weights read
-        once per pass) instead of passes of 10 rows — for the steps that do not go to the tcgen05 GEMM (11-16 rows, or
+        once per pass) instead of passes of 16 rows — for the steps that do not go to the tcgen05 GEMM (11-16 rows, or
         set_large_m_gemm(0))."""
         check(lib().sp_cuda_engine_set_many_row_gemv(self._h, int(on)))
 

@@ -288,7 +288,7 @@ class Engine {
     uint32_t* p_ids_ = nullptr;
     int32_t *p_slot_ = nullptr, *p_pos_ = nullptr, *p_rows_ = nullptr;
     float* p_logits_ = nullptr;
-    static constexpr int COPY_EVENTS = 32, COPY_HELPERS = 7;
+    static constexpr int COPY_EVENTS = 8, COPY_HELPERS = 7;
     cudaEvent_t copy_done_[COPY_EVENTS] = {};  // of fetch_logits
     CopyPool copy_pool_;
     uint32_t* p_argmax_ = nullptr;

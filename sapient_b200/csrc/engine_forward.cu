@@ -142,33 +142,39 @@ int Engine::enqueue_decode_step(int T) {
     return enqueue_head(0, T);
 }
 
-// The first n floats of logits_ to host memory of the caller's, through the pinned buffer. From eight slices (four megabytes) on that is
-// several copies in flight on the device and on the host: a lone thread takes longer to write a caller's fresh pages (32 rows of
-// 128256 logits: 1.6 ms) than the device to make them. This thread waits for the first copy alone; the engine's helpers, which
-// sleep until then, are woken for what is left. Returns with the stream's work done.
+// The first n floats of logits_ to host memory of the caller's, through the pinned buffer. From four megabytes on several threads
+// copy out of it while the device still fills it: a lone one takes longer to write a caller's fresh pages (32 rows of 128256 logits:
+// 1.6 ms) than the device to make them. (Five rows of 151936, three megabytes, take 100 us longer so: threads wake slowly.) The device's copies are few, for each costs it three microseconds and
+// a short one runs slower (16.4 MB: one copy 293 us, 8 318, 32 404, with their events 496); threads take a quarter of a
+// megabyte at a time of what has arrived. This thread waits for the first copy alone; the engine's helpers, which sleep until then, are
+// woken for what is left. Returns with the stream's work done.
 int Engine::fetch_logits(float* out, size_t n) {
-    constexpr size_t SLICE = (size_t)1 << 17;  // floats
+    constexpr size_t SLICE = (size_t)1 << 16;  // floats that a thread takes
     const int slices = (int)((n + SLICE - 1) / SLICE);
-    if (slices < 8) {
+    if (slices < 16) {
         SP_CUDA_TRY(cudaMemcpyAsync(p_logits_, logits_, n * 4, cudaMemcpyDeviceToHost, stream));
         SP_CUDA_TRY(cudaStreamSynchronize(stream));
         std::memcpy(out, p_logits_, n * 4);
         return SP_OK;
     }
-    const int groups = std::min(slices, COPY_EVENTS);  // slices that share an event
-    auto first = [&](int g) { return std::min(n, (size_t)((int64_t)g * slices / groups) * SLICE); };
+    const int groups = std::min(slices / 4, COPY_EVENTS);  // the device's copies
+    auto first = [&](int g) { return (int)((int64_t)g * slices / groups); };
+    auto at = [&](int slice) { return std::min(n, slice * SLICE); };
     for (int g = 0; g < groups; ++g) {
         if (!copy_done_[g]) SP_CUDA_TRY(cudaEventCreateWithFlags(&copy_done_[g], cudaEventDisableTiming));
-        SP_CUDA_TRY(cudaMemcpyAsync(p_logits_ + first(g), logits_ + first(g), (first(g + 1) - first(g)) * 4, cudaMemcpyDeviceToHost, stream));
+        const size_t a = at(first(g)), b = at(first(g + 1));
+        SP_CUDA_TRY(cudaMemcpyAsync(p_logits_ + a, logits_ + a, (b - a) * 4, cudaMemcpyDeviceToHost, stream));
         SP_CUDA_TRY(cudaEventRecord(copy_done_[g], stream));
     }
     SP_CUDA_TRY(cudaEventSynchronize(copy_done_[0]));
     std::atomic<int> next{0}, failed{0};
     copy_pool_.run(std::min(COPY_HELPERS, slices / 2), [&] {
         cudaSetDevice(d.device);
-        for (int g; (g = next.fetch_add(1)) < groups;) {
+        int g = 0;  // (slices are dealt out in order)
+        for (int s; (s = next.fetch_add(1)) < slices;) {
+            while (s >= first(g + 1)) ++g;
             if (cudaEventSynchronize(copy_done_[g]) != cudaSuccess) { failed.store(1); return; }
-            std::memcpy(out + first(g), p_logits_ + first(g), (first(g + 1) - first(g)) * 4);
+            std::memcpy(out + at(s), p_logits_ + at(s), (at(s + 1) - at(s)) * 4);
         }
     });
     SP_CUDA_TRY(cudaStreamSynchronize(stream));

@@ -529,6 +529,35 @@ void ActWorkspace::release() {
 
 // ─────────────────────────────── the GEMV ────────────────────────────────────
 // (mma wrappers, tile register images and per-tile arithmetic: gemv_imma_dev.cuh)
+// A warp's own digits of one tile of one activation row (a.x): the layouts of gemv_imma.cuh for a tile of eight columns.
+struct __align__(16) OwnDigits {
+    int8_t xq[2048], r32[256], r16[256];
+    float cs[64];
+    struct View {
+        const OwnDigits* d;
+        int lane;
+        __device__ __forceinline__ uint4 chunk(int, int i) const { return ld_u4(d->xq + i * 512 + lane * 16); }
+        __device__ __forceinline__ void rec32(int, uint32_t& a, uint32_t& b) const { word(d->r32, a, b); }
+        __device__ __forceinline__ void rec16(int, uint32_t& a, uint32_t& b) const { word(d->r16, a, b); }
+        __device__ __forceinline__ float2 scale(int) const { return *reinterpret_cast<const float2*>(d->cs + 2 * (lane & 3)); }
+        __device__ __forceinline__ void word(const int8_t* rec, uint32_t& a, uint32_t& b) const {
+            a = *reinterpret_cast<const uint32_t*>(rec + (lane >> 2) * 32 + 4 * (lane & 3));
+            b = *reinterpret_cast<const uint32_t*>(rec + (lane >> 2) * 32 + 4 * (lane & 3) + 16);
+        }
+    };
+    __device__ __forceinline__ View view(int lane) const { return View{this, lane}; }
+    // (columns past the row's three hold whatever was there: nobody reads their sums)
+    __device__ __forceinline__ void make(const ImmaArgs& a, int tile, int lane) {
+        const QuantOut q{a.k, 256, 3, 256, 8, 0, xq, cs, r32, r16};
+        float v[8];
+        load8(a.x + tile * 256 + lane * 8, v);
+        *reinterpret_cast<uint2*>(r32 + lane * 8) = make_uint2(0u, 0u);  // (bytes of a record that stand for no block)
+        __syncwarp();
+        quantize_chunk(v, true, lane, 0, 0, q);
+        __syncwarp();
+    }
+};
+
 // ── Q8_0, 128 columns (four blocks) at a time: half a tile of eight blocks or a tile of four ──
 struct Q8Unit {
     uint4 q[4];
@@ -674,13 +703,22 @@ __device__ __forceinline__ void reduce_store(const ImmaArgs& a, const ImmaSeg& s
 // FMT: 0 = segments of any format; T_Q4_K / T_Q6_K / T_Q8_0 = every segment of the launch has that format — the code for the
 // other formats is left out, which lets the M <= 2 instance of the K-quants fit 80 registers and run three CTAs (24 warps)
 // per SM instead of two.
-template <int NT, int FMT, int WARPS = IMMA_WARPS>
+template <int NT, int FMT, int WARPS = IMMA_WARPS, int OWN = 0>
 __global__ void __launch_bounds__(WARPS * 32, (NT == 1 && FMT != 0 && FMT != T_Q8_0) ? 3 : 16 / WARPS) gemv_imma_kernel(const ImmaArgs a) {
-    __shared__ float red[WARPS * NT * 4 * 32];
+    __shared__ float sums[OWN ? 1 : WARPS * NT * 4 * 32];
+    __shared__ OwnDigits own_digits[OWN ? WARPS : 1][OWN ? OWN : 1];
+    float* const red = OWN ? reinterpret_cast<float*>(own_digits) : sums;
+    static_assert(sizeof(OwnDigits) >= 4 * 32 * sizeof(float), "the digits' memory takes the sums");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int rt = blockIdx.x, s = 0;
     while (s < a.nseg - 1 && rt >= (a.seg[s].n + 15) / 16) { rt -= (a.seg[s].n + 15) / 16; ++s; }
     const ImmaSeg& sg = a.seg[s];
+    // (while the first weights are on their way)
+    auto make_own = [&] {
+#pragma unroll
+        for (int i = 0; i < OWN; ++i)
+            if (warp + i * WARPS < (a.k >> 8)) own_digits[warp][i].make(a, warp + i * WARPS, lane);
+    };
     float acc[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
@@ -691,7 +729,9 @@ __global__ void __launch_bounds__(WARPS * 32, (NT == 1 && FMT != 0 && FMT != T_Q
         const uint8_t* base = sg.wt + (int64_t)rt * kts * Q4_K_TILE_BYTES;
         Q4Regs ra, rb;
         auto tile_q4 = [&](int at, const Q4Regs& w) {
-            if constexpr (NT <= 2) {
+            if constexpr (OWN) {
+                compute_q4_k<NT>(w, own_digits[warp][at / WARPS].view(lane), lane, acc);
+            } else if constexpr (NT <= 2) {
                 BFrag<NT> b;
                 load_b_global<NT>(a, at, lane, true, false, b);
                 compute_q4_k<NT>(w, b, lane, acc);
@@ -705,6 +745,7 @@ __global__ void __launch_bounds__(WARPS * 32, (NT == 1 && FMT != 0 && FMT != T_Q
         if (TWO && kt + WARPS < kts) load_q4_k<true>(base + (int64_t)(kt + WARPS) * Q4_K_TILE_BYTES, lane, rb);
         pdl_wait();  // the weight tiles above are in flight while the producer of the activations finishes
         pdl_trigger();
+        make_own();
         if (TWO) {
             bool first = true;
             while (kt < kts) {
@@ -729,7 +770,9 @@ __global__ void __launch_bounds__(WARPS * 32, (NT == 1 && FMT != 0 && FMT != T_Q
         constexpr bool TWO = NT == 1 && FMT == 0;  // (a second tile in flight where registers allow)
         Q6Regs ra, rb;
         auto tile_q6 = [&](int at, const Q6Regs& w) {
-            if constexpr (NT <= 2) {
+            if constexpr (OWN) {
+                compute_q6_k<NT>(w, own_digits[warp][at / WARPS].view(lane), lane, acc);
+            } else if constexpr (NT <= 2) {
                 BFrag<NT> b;
                 load_b_global<NT>(a, at, lane, false, true, b);
                 compute_q6_k<NT>(w, b, lane, acc);
@@ -741,6 +784,7 @@ __global__ void __launch_bounds__(WARPS * 32, (NT == 1 && FMT != 0 && FMT != T_Q
         if (TWO && warp + WARPS < kts) load_q6_k<true>(base + (int64_t)(warp + WARPS) * Q6_K_TILE_BYTES, lane, rb);
         pdl_wait();
         pdl_trigger();
+        make_own();
         if (TWO) {
             for (int kt = warp; kt < kts; kt += 2 * WARPS) {
                 const int k1 = kt + WARPS, k2 = k1 + WARPS, k3 = k2 + WARPS;
@@ -769,6 +813,7 @@ __global__ void __launch_bounds__(WARPS * 32, (NT == 1 && FMT != 0 && FMT != T_Q
             for (int kt = warp; kt < kts; kt += WARPS) tile_q8_0<NT>(a, base + (int64_t)kt * tb, kt, bpt, lane, acc);
         }
     }
+    if (OWN) __syncthreads();
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -1017,6 +1062,20 @@ static StreamPlan plan_stream(const ImmaArgs& a) {
     return p;
 }
 
+// Whether the warps of a GEMV on one row of f32 make the digits that they multiply: one launch for two. A warp has at most two tiles of
+// columns then, and makes their digits while its weights are on their way; every block does, so the grid is at most two blocks
+// per SM. On the device (one call after the other in a graph) Q4_K 4096 x 4096 5.0 -> 4.7 us, 2048 x 1536 3.4 -> 2.4, Q6_K 4096 x 4096 6.4 -> 5.5;
+// enqueued call by call 10.0 -> 7.6. With two rows, or digits made tile by tile inside the loop, it takes longer than the launch that it
+// saves (4096 x 4096 8.1 and 5.7 us), and so do Q8_0's pieces, two of which share a tile.
+static bool imma_makes_digits(const ImmaArgs& a) {
+    int tiles = 0;
+    for (int s = 0; s < a.nseg; ++s) {
+        if (a.seg[s].dtype != T_Q4_K && a.seg[s].dtype != T_Q6_K) return false;
+        tiles += (a.seg[s].n + 15) / 16;
+    }
+    return a.m == 1 && !a.tp && g_imma_kernel.load() == 0 && a.k <= 4096 && tiles <= 2 * device_sm_count();
+}
+
 cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st) {
     if (a.m <= 0) return cudaSuccess;
     int tiles = 0;
@@ -1040,7 +1099,7 @@ cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st) {
         else gemv_imma_stream_kernel<2><<<grid, STREAM_WARPS * 32, p.total, st>>>(a, p);
         return count_launch_and_check();
     }
-    cudaError_t le;
+    cudaError_t le = cudaErrorInvalidValue;
     bool q4_only = true, q6_only = true, q8_only = true;
     for (int s = 0; s < a.nseg; ++s) {
         q4_only = q4_only && a.seg[s].dtype == T_Q4_K;
@@ -1055,7 +1114,11 @@ cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st) {
     // Fewer tile rows than SMs: 16 warps share a row's columns, where there is a piece for more than eight. Q4_K 1536 x 8960 1 row 6.3
     // -> 5.6 us, 13 rows 14.7 -> 10.9; Q8_0 896 x 4864 5.6 -> 4.6, 13 rows 9.5 -> 7.4. (With eight pieces or fewer 2 % slower.)
     const bool wide = tiles <= device_sm_count() && a.k / (q8_only && a.seg[0].bpt > 1 ? 128 : 256) > IMMA_WARPS;
-    if (nt == 1 && q4_only && deep_q4) le = launch_pdl(gemv_imma_kernel<1, T_Q4_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
+    if (a.x) {
+        if (!imma_makes_digits(a)) return cudaErrorInvalidValue;
+        le = !wide ? launch_pdl(gemv_imma_kernel<1, 0, 8, 2>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a)
+                   : launch_pdl(gemv_imma_kernel<1, 0, 16, 1>, dim3(tiles), dim3(512), 0, st, a);
+    } else if (nt == 1 && q4_only && deep_q4) le = launch_pdl(gemv_imma_kernel<1, T_Q4_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
     else if (nt == 1 && q6_only && deep_q6) le = launch_pdl(gemv_imma_kernel<1, T_Q6_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
 #define SP_GEMV(N)                                                                                                                   \
     else if (nt == N)                                                                                                                \
@@ -1074,6 +1137,10 @@ cudaError_t launch_quant_gemv(const float* x, int ldx, ImmaArgs& a, const ActWor
     if (a.m <= 0) return cudaSuccess;
     if (a.m > imma_rows_per_pass() || a.k > ws.k_max) return cudaErrorInvalidValue;
     imma_plan(a, ws);
+    if (requantize && imma_makes_digits(a)) {
+        a.x = x;
+        return launch_gemv_imma(a, st);
+    }
     if (requantize) {
         cudaError_t e = launch_act_quant(x, ldx, a, st);
         if (e != cudaSuccess) return e;

@@ -65,6 +65,7 @@ struct ImmaArgs {
     // They feed one extra mma per tile for the Q4_K minimum term and the Q6_K zero point.
     const int8_t* xs32d;
     const int8_t* xs16d;
+    const float* x;         // the one activation row itself, or null: the warps make its digits (xq .. xs16d are not used)
     const float* res;       // optional residual for segment 0 (may alias its y)
     int ldres;
     // Tensor-parallel column-split matrix (tp != null): segment 0's outputs are not stored to y but pushed, as partial

@@ -8,7 +8,7 @@ from sapient_b200 import ops, synth
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("dtype,n,k", [(synth.Q4_K, 40, 2048), (synth.Q4_K, 72, 2304), (synth.Q4_K, 40, 4352), (synth.Q4_K, 2384, 2304),
+@pytest.mark.parametrize("dtype,n,k", [(synth.Q4_K, 40, 256), (synth.Q4_K, 40, 2048), (synth.Q4_K, 2400, 4096), (synth.Q6_K, 40, 4096), (synth.Q4_K, 72, 2304), (synth.Q4_K, 40, 4352), (synth.Q4_K, 2384, 2304),
                                        (synth.Q6_K, 40, 2304), (synth.Q6_K, 24, 4608), (synth.Q8_0, 40, 1024), (synth.Q8_0, 40, 1152),
                                        (synth.Q8_0, 72, 2304), (synth.Q8_0, 40, 96), (synth.Q8_0, 2384, 1152)])
 def test_every_row_count_of_a_pass(dtype, n, k):
@@ -24,6 +24,8 @@ def test_every_row_count_of_a_pass(dtype, n, k):
         for m in range(1, 18):
             got, want = w.matmul_nt(x[:m]).astype(np.float64), x[:m].astype(np.float64) @ values
             assert np.all(np.linalg.norm(got - want, axis=1) < 2e-6 * np.linalg.norm(want, axis=1)), m
+        # one row may make its digits itself, two never: the same digits, products and sums
+        assert np.array_equal(w.matmul_nt(x[3:4]), w.matmul_nt(x[3:5])[:1])
     finally:
         ops.set_large_m_gemm(2)
         w.free()

@@ -792,25 +792,17 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
     if (m <= 0 || nseg <= 0) return cudaSuccess;
     if (nseg > 3 || k % 128 != 0 || !in.waits) return cudaErrorInvalidValue;
     DqArgs a{};
-    int tiles = 0, tb = 0;
+    int tiles = 0, one_plane = 0, tb = 0;
     for (int i = 0; i < nseg; ++i) {
         if (!tc5_supported(segs[i].dtype, k) || segs[i].n <= 0) return cudaErrorInvalidValue;
         a.seg[i] = segs[i];
         tiles += (segs[i].n + DQ_BM - 1) / DQ_BM;
+        if (segs[i].dtype == T_Q4_K) one_plane += (segs[i].n + DQ_BM - 1) / DQ_BM;
         tb = std::max(tb, dq_tile_bytes(segs[i].dtype));
     }
     a.nseg = nseg; a.k = k; a.m = m; a.ldy = ldy; a.res = res; a.ldres = ldres;
     a.xscale = in.xscale; a.xsum = in.xsum; a.waits = in.waits;
-    a.m_tiles = (m + DQ_NB - 1) / DQ_NB;
-    a.nb = ((m + a.m_tiles - 1) / a.m_tiles + 15) & ~15;
-    a.m_tiles = (m + a.nb - 1) / a.nb;
-    // shared memory: at most half for activations (each box serves 64 columns), the rest for raw tiles
-    const int njt = a.nb <= 16 ? 1 : a.nb <= 32 ? 2 : a.nb <= 64 ? 4 : 8;
-    const int b_bytes = dq_boxes(njt) * 2 * a.nb * 128, x_bytes = DQ_X_STAGES * a.nb * 32;
-    a.r_bytes = 8 * tb;
-    a.b_stages = std::min(DQ_MAX_B, 128 * 1024 / b_bytes);
-    a.r_stages = std::min(DQ_MAX_R, (DQ_SMEM - 1024 - a.b_stages * b_bytes - x_bytes) / a.r_bytes);
-    static PerDeviceOnce attr_once;
+    static PerDeviceOnce attr_once;  // (ahead of the plan, which asks how many clusters fit)
     cudaError_t le = attr_once.run([] {
         for (auto f : {gemm_dq_kernel<1>, gemm_dq_kernel<2>, gemm_dq_kernel<4>, gemm_dq_kernel<8>}) {
             const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM);
@@ -826,14 +818,18 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
         return cudaSuccess;
     });
     if (le != cudaSuccess) return le;
-    // How the tiles are dealt out, by the longest SM's time in tenths of a span of 256 columns. One block per SM that walks over tiles:
-    // a tile is its spans and 3, the walk's start 10. Clusters that share a tile's K range: every wave of them is its spans and 45 (5
-    // less for the first, whose start lies under the kernel before). Where tiles go over whole rounds of the SMs, those that do may
-    // have a launch of their own, 30 for the launch. Fitted to forced choices over 13 shapes x 6 row counts x 3 formats, of which the
-    // rule takes the fastest or one within 4 %. In us: Q4_K 6144 x 4096, 512 rows (192 tiles) walked 74.7, clusters of two 84.5, a walk
-    // and 44 tiles shared by two 70.6; 20000 x 14336, 20 rows (157 tiles) 160, clusters of four 121, nine tiles shared by eight 97;
-    // 8960 x 1536, 300 rows (210 tiles) 37 walked, 39 in two launches.
-    const int items = tiles * a.m_tiles, all_sb = (k + 255) / 256, sms = device_sm_count();
+    // How high the tiles are and how they are dealt out, by the longest SM's time. One block per SM that walks over tiles: in tenths of
+    // a span of 256 columns, a tile is its spans and 3, the walk's start 10. Clusters that share a tile's K range: every wave of them is
+    // its spans and 45 (5 less for the first, whose start lies under the kernel before). Where tiles go over whole rounds of the SMs,
+    // those that do may have a launch of their own, 30 for the launch. Fitted to forced choices over 13 shapes x 6 row counts x 3 formats,
+    // of which the rule takes the fastest or one within 4 %. In us: Q4_K 6144 x 4096, 512 rows (192 tiles) walked 74.7, clusters of two
+    // 84.5, a walk and 44 tiles shared by two 70.6; 20000 x 14336, 20 rows (157 tiles) 160, clusters of four 121, nine tiles shared by
+    // eight 97; 8960 x 1536, 300 rows (210 tiles) 37 walked, 39 in two launches.
+    // A span of a low tile takes less time, if more for each row (SPAN: us, measured with one tile per SM): lower ones than need be are
+    // for SMs that would be idle, and taken where they promise a seventh (of less than that nothing was left). Q8_0, 389 rows: 2560 x 2560
+    // 80 tiles of 112 rows 25.4 us, 140 of 64 21.1; 2560 x 10240 71.9 and 66.1; 1152 x 896, 300 rows 10.9 and 8.6; Q4_K 2048 x 1536, 192
+    // rows 12.0 and 11.0.
+    const int all_sb = (k + 255) / 256, sms = device_sm_count();
     auto shared = [&](int n, int& parts) {
         long cost = 0;
         for (int p = 1; p <= std::min(DQ_MAX_PARTS, all_sb); ++p) {
@@ -843,14 +839,32 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
         return cost;
     };
     auto walked = [&](int n) { return (long)((n + sms - 1) / sms) * (10 * all_sb + 3) + 10; };
-    int walk = items, parts = 1;  // tiles that are walked over; the rest is shared by `parts` blocks each
-    long cost = walked(items);
-    for (const int first : {0, items / sms * sms}) {
-        int p = 1;
-        if (first == items) continue;
-        const long c = shared(items - first, p) + (first > 0 ? walked(first) + 30 : 0);
-        if (c < cost) { cost = c; walk = first; parts = p; }
+    int items = 0, walk = 0, parts = 1;  // tiles; those that are walked over; the rest is shared by `parts` blocks each
+    double best = 0.0;
+    const int fewest = (m + DQ_NB - 1) / DQ_NB;
+    for (int low = fewest, last = 0; last != 16; ++low) {
+        const int h = ((m + low - 1) / low + 15) & ~15, m_tiles = (m + h - 1) / h, n = tiles * m_tiles;
+        if (h == last) continue;
+        last = h;
+        static constexpr double SPAN[2][8] = {{1.30, 1.39, 1.50, 1.67, 1.98, 2.18, 2.33, 2.53}, {1.04, 1.13, 1.26, 1.27, 1.70, 1.77, 1.94, 2.03}};
+        const double span = (low > fewest ? 1.16 : 1.0) * (SPAN[0][h / 16 - 1] * (tiles - one_plane) + SPAN[1][h / 16 - 1] * one_plane) / tiles;
+        auto take = [&](long tenths, int w, int p) {
+            if (best == 0.0 || span * tenths < best) { best = span * tenths; a.nb = h; a.m_tiles = m_tiles; items = n; walk = w; parts = p; }
+        };
+        take(walked(n), n, 1);
+        for (const int first : {0, n / sms * sms}) {
+            int p = 1;
+            if (first == n) continue;
+            const long c = shared(n - first, p) + (first > 0 ? walked(first) + 30 : 0);
+            take(c, first, p);
+        }
     }
+    // shared memory: at most half for activations (each box serves 64 columns), the rest for raw tiles
+    const int njt = a.nb <= 16 ? 1 : a.nb <= 32 ? 2 : a.nb <= 64 ? 4 : 8;
+    const int b_bytes = dq_boxes(njt) * 2 * a.nb * 128, x_bytes = DQ_X_STAGES * a.nb * 32;
+    a.r_bytes = 8 * tb;
+    a.b_stages = std::min(DQ_MAX_B, 128 * 1024 / b_bytes);
+    a.r_stages = std::min(DQ_MAX_R, (DQ_SMEM - 1024 - a.b_stages * b_bytes - x_bytes) / a.r_bytes);
     const PFN_encodeTiled encode = tensor_map_encoder();
     if (!encode) return cudaErrorNotSupported;
     CUtensorMap tmap;

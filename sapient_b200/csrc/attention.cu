@@ -454,8 +454,7 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
 // softmax weights are split the same way for the second contraction. K and V are fp16 in the cache, hence exact.
 // Online softmax per page with the reference's recurrence (kernels/attention.rs:98-165); the warps' states are merged
 // through shared memory, and the block writes either the output rows (one split) or the split partials.
-constexpr int GM_WARPS = 4;
-template <int HD16>
+template <int HD16, int GM_WARPS>
 __global__ void __launch_bounds__(GM_WARPS * 32)
 attention_gqa_mma_kernel(const float* __restrict__ q, int ldq, float* __restrict__ out, int ldo, int n_heads, const int32_t* __restrict__ tok_slot,
                          const int32_t* __restrict__ tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* __restrict__ part,
@@ -622,17 +621,25 @@ bool attention_gqa_mma_supported(int n_heads, int n_kv, int head_dim) {
 cudaError_t launch_gqa_mma_phase(const float* q, int ldq, float* out, int ldo, int n_tok, int n_heads, const int32_t* tok_slot,
                                  const int32_t* tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st, int fresh) {
     const int hd16 = kv.head_dim / 16;
-    const size_t smem = (size_t)GM_WARPS * 4 * KV_PAGE * (kv.head_dim + 8) * sizeof(__half);
-    const dim3 grid(kv.n_kv, n_tok, n_splits), block(GM_WARPS * 32);
+    const dim3 grid(kv.n_kv, n_tok, n_splits);
+    // Four warps a block while few blocks share an SM; three where they would not all fit at once (70 KB each with 128 coordinates; four blocks
+    // of three warps do): 32 sequences of the 8B shape, 512 blocks, 23.2 -> 20.4 us a layer, but 104 blocks of the 1.5B shape 6.0 -> 6.5.
+    const bool narrow = (int64_t)kv.n_kv * n_tok * n_splits > 2 * device_sm_count();
+    const int warps = narrow ? 3 : 4;
+    const size_t smem = (size_t)warps * 4 * KV_PAGE * (kv.head_dim + 8) * sizeof(__half);
+    const dim3 block(32 * warps);
     cudaError_t le = cudaErrorInvalidValue;
 #define SP_GM(N)                                                                                                        \
     if (hd16 == N) {                                                                                                    \
         static PerDeviceOnce big_smem;                                                                                  \
         if (smem > 48 * 1024) {                                                                                         \
-            le = big_smem.run([] { return cudaFuncSetAttribute(attention_gqa_mma_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024); }); \
+            le = big_smem.run([] {                                                                                      \
+                const cudaError_t e = cudaFuncSetAttribute(attention_gqa_mma_kernel<N, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024); \
+                return e != cudaSuccess ? e : cudaFuncSetAttribute(attention_gqa_mma_kernel<N, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024); \
+            });                                                                                                         \
             if (le != cudaSuccess) return le;                                                                           \
         }                                                                                                               \
-        le = launch_pdl(attention_gqa_mma_kernel<N>, grid, block, smem, st, q, ldq, out, ldo, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, fresh); \
+        le = launch_pdl(narrow ? attention_gqa_mma_kernel<N, 3> : attention_gqa_mma_kernel<N, 4>, grid, block, smem, st, q, ldq, out, ldo, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, fresh); \
     }
     SP_GM(1) SP_GM(2) SP_GM(3) SP_GM(4) SP_GM(5) SP_GM(6) SP_GM(7) SP_GM(8)
 #undef SP_GM

@@ -258,10 +258,11 @@ int Engine::step_splits(int T) const {
     if (plan_) return plan_ctx_bucket();
     if (T <= ATT_SPLIT_TOKENS && attention_takes_mma(T, step_ctx_, d.n_heads, d.n_kv_heads, d.head_dim)) {
         // tensor-core kernel, a block per (KV head, token, split): enough blocks to fill the SMs three deep, but no range
-        // shorter than 256 keys (4 pages per warp) — its fixed cost per block (query fragments, warp merge) is larger
+        // shorter than 128 keys (2 pages per warp): its fixed cost per block (query fragments, warp merge) is larger. 13 sequences of
+        // the 1.5B shape at 700 keys, us a layer: 256 keys 8.2, 128 6.0, 64 6.0 and a merge that takes 0.8 longer
         int want = 1, limit = 1;
         while (want < ATT_SPLITS && d.n_kv_heads * T * want < 444) want <<= 1;
-        while (limit < ATT_SPLITS && limit * 2 * 256 <= step_ctx_) limit <<= 1;
+        while (limit < ATT_SPLITS && limit * 2 * 128 <= step_ctx_) limit <<= 1;
         return std::min(want, limit);
     }
     int splits = 1;

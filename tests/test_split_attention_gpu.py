@@ -20,6 +20,17 @@ def test_key_counts(oracle, hd, sq, sk):
     assert rel_l2(ops.gqa_attention(q, k, v), oracle.attention(q, k, v, oracle.causal_mask(sq, sk))) < 1e-5
 
 
+@pytest.mark.parametrize("hd,H,Hkv", [(64, 8, 2), (128, 16, 8), (80, 6, 3)])
+@pytest.mark.parametrize("sq,sk", [(16, 257), (16, 400), (40, 161), (111, 130), (160, 170)])
+def test_grouped_kernel_with_few_and_many_blocks(oracle, hd, H, Hkv, sq, sk):
+    """(Query rows, cached heads) below and above two blocks per SM: four and three warps a block, which share the pages out differently."""
+    rng = np.random.default_rng(hd + sk)
+    q = rng.standard_normal((H, sq, hd)).astype(np.float32)
+    k, v = (f16_round(rng.standard_normal((Hkv, sk, hd))) for _ in range(2))
+    # queries and weights in two fp16 parts (2^-22), f32 sums
+    assert rel_l2(ops.gqa_attention(q, k, v), oracle.attention(q, k, v, oracle.causal_mask(sq, sk))) < 1e-5
+
+
 @pytest.mark.parametrize("name", ["tiny_llama", "tiny_phi2"])
 def test_rows_of_a_step_see_each_other(name):
     """Five rows at once and one after the other, from lengths around pages and rounds: the rows of a step are keys of the later ones."""

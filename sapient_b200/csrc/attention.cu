@@ -9,6 +9,7 @@
 // With one split the block writes the output row directly.
 #include "kernels.h"
 #include "pdl.cuh"
+#include "plan_common.cuh"
 #include "sp_common.cuh"
 #include "splits.cuh"
 
@@ -263,8 +264,9 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
 }
 
 // HD16 = head_dim / 16 (head_dim a multiple of 16, <= 128).
+// (Three blocks an SM up to 80 coordinates, two above, by registers: with 172 instead of 168 Phi-2's took 27.0 us a layer for 22.7.)
 template <int HD16, bool EXACT>
-__global__ void __launch_bounds__(FA_WARPS * 32)
+__global__ void __launch_bounds__(FA_WARPS * 32, HD16 <= 5 ? 3 : 2)
 attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict__ out, __half* __restrict__ out_h, int ldo, int n_tok,
                          int n_heads, int slot, int pos0, KvGeom kv, int layer, float scale) {
     constexpr int HD = HD16 * 16, LD = HD + 8;  // padded row of the shared tiles (halves): conflict-free fragment loads
@@ -324,30 +326,44 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
     for (int i = 0; i < 2 * HD16; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
     const int last_pos = pos0 + min(t0 + FA_ROWS, n_tok) - 1;  // newest key any row of the block may see
-    auto fetch_tile = [&](int k0, int buf) {  // asynchronous copy of keys k0 .. k0 + 63 (zeros past the newest visible key)
+    // pages of a tile's keys (past the newest visible key: the last page, of which nothing is read)
+    auto pages_of = [&](int k0) {
+        int4 p;
+        const int last = last_pos / KV_PAGE, first = k0 / KV_PAGE;
+        p.x = pt[min(first, last)];
+        p.y = pt[min(first + 1, last)];
+        p.z = pt[min(first + 2, last)];
+        p.w = pt[min(first + 3, last)];
+        return p;
+    };
+    auto fetch_tile = [&](int k0, int buf, const int4& pages) {  // asynchronous copy of keys k0 .. k0 + 63 (zeros past the newest visible key)
         __half* Kd = fa_smem + (2 * buf) * TILE;
         __half* Vd = Kd + TILE;
-        for (int idx = threadIdx.x; idx < FA_KEYS * (HD / 8); idx += FA_WARPS * 32) {
-            const int kr = idx / (HD / 8), pc = idx - kr * (HD / 8);
-            const int key = k0 + kr;
-            const bool live = key <= last_pos;
-            const int page = live ? pt[key / KV_PAGE] : 0;
-            const int64_t in_page = (int64_t)((live ? key : 0) % KV_PAGE) * HD + pc * 8;
+        static_assert(FA_KEYS == 4 * KV_PAGE, "four pages a tile");
+#pragma unroll
+        for (int i = 0; i < FA_KEYS * (HD / 8) / (FA_WARPS * 32); ++i) {
+            const int idx = threadIdx.x + i * FA_WARPS * 32, kr = idx / (HD / 8), pc = idx - kr * (HD / 8);
+            const int page = kr < KV_PAGE ? pages.x : kr < 2 * KV_PAGE ? pages.y : kr < 3 * KV_PAGE ? pages.z : pages.w;
+            const int64_t in_page = (int64_t)(kr % KV_PAGE) * HD + pc * 8;
             const __half* ksrc = kv.pool + kv_off(kv, layer, page, 0, kv_h) + in_page;
             const __half* vsrc = kv.pool + kv_off(kv, layer, page, 1, kv_h) + in_page;
             const uint32_t kd = (uint32_t)__cvta_generic_to_shared(Kd + kr * LD + pc * 8), vd = (uint32_t)__cvta_generic_to_shared(Vd + kr * LD + pc * 8);
-            const int bytes = live ? 16 : 0;  // 0: nothing is read, the 16 bytes are zero-filled
+            const int bytes = k0 + kr <= last_pos ? 16 : 0;  // 0: nothing is read, the 16 bytes are zero-filled
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(kd), "l"(ksrc), "r"(bytes) : "memory");
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(vd), "l"(vsrc), "r"(bytes) : "memory");
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    fetch_tile(0, 0);
-    for (int k0 = 0, buf = 0; k0 <= last_pos; k0 += FA_KEYS, buf ^= 1) {
+    // of a cluster of two blocks each takes every other tile of keys
+    const int step = FA_KEYS * (int)gridDim.z, part = blockIdx.z, k_first = part * FA_KEYS;
+    if (k_first <= last_pos) fetch_tile(k_first, 0, pages_of(k_first));
+    int4 pages = pages_of(k_first + step);  // a tile ahead of its copies
+    for (int k0 = k_first, buf = 0; k0 <= last_pos; k0 += step, buf ^= 1) {
         const __half* Ks = fa_smem + (2 * buf) * TILE;
         const __half* Vs = Ks + TILE;
-        if (k0 + FA_KEYS <= last_pos) {
-            fetch_tile(k0 + FA_KEYS, buf ^ 1);  // that buffer's previous tile was consumed before the barrier that ended the last iteration
+        if (k0 + step <= last_pos) {
+            fetch_tile(k0 + step, buf ^ 1, pages);  // that buffer's previous tile was consumed before the barrier that ended the last iteration
+            pages = pages_of(k0 + 2 * step);
             asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         } else {
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -430,18 +446,55 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
         }
         __syncthreads();  // this tile's buffer may be refilled from the next iteration on
     }
-    const float i0 = (l0 == 0.f) ? 0.f : 1.0f / l0 / WEIGHT_UP, i1 = (l1 == 0.f) ? 0.f : 1.0f / l1 / WEIGHT_UP;
-#pragma unroll
-    for (int nd = 0; nd < 2 * HD16; ++nd) {
+    auto put = [&](int nd, const float (&v)[4], float i0, float i1) {
         const int64_t c = (int64_t)h * HD + 8 * nd + 2 * t;
         if (out_h) {  // fp16 rows for the tensor-core output projection
-            if (r0 < n_tok) *reinterpret_cast<__half2*>(out_h + (int64_t)r0 * ldo + c) = __floats2half2_rn(o[nd][0] * i0, o[nd][1] * i0);
-            if (r1 < n_tok) *reinterpret_cast<__half2*>(out_h + (int64_t)r1 * ldo + c) = __floats2half2_rn(o[nd][2] * i1, o[nd][3] * i1);
+            if (r0 < n_tok) *reinterpret_cast<__half2*>(out_h + (int64_t)r0 * ldo + c) = __floats2half2_rn(v[0] * i0, v[1] * i0);
+            if (r1 < n_tok) *reinterpret_cast<__half2*>(out_h + (int64_t)r1 * ldo + c) = __floats2half2_rn(v[2] * i1, v[3] * i1);
         } else {
-            if (r0 < n_tok) *reinterpret_cast<float2*>(out + (int64_t)r0 * ldo + c) = make_float2(o[nd][0] * i0, o[nd][1] * i0);
-            if (r1 < n_tok) *reinterpret_cast<float2*>(out + (int64_t)r1 * ldo + c) = make_float2(o[nd][2] * i1, o[nd][3] * i1);
+            if (r0 < n_tok) *reinterpret_cast<float2*>(out + (int64_t)r0 * ldo + c) = make_float2(v[0] * i0, v[1] * i0);
+            if (r1 < n_tok) *reinterpret_cast<float2*>(out + (int64_t)r1 * ldo + c) = make_float2(v[2] * i1, v[3] * i1);
+        }
+    };
+    auto share = [](float l) { return (l == 0.f) ? 0.f : 1.0f / l / WEIGHT_UP; };
+    if (gridDim.z == 1) {
+        const float i0 = share(l0), i1 = share(l1);
+#pragma unroll
+        for (int nd = 0; nd < 2 * HD16; ++nd) put(nd, o[nd], i0, i1);
+        return;
+    }
+    // each block finishes half of the coordinates: the other half goes to the peer, by thread (the tile buffers are free: the loop ends
+    // with a barrier)
+    float4* const sent = reinterpret_cast<float4*>(fa_smem) + threadIdx.x;
+    constexpr int PITCH = FA_WARPS * 32;
+    static_assert((HD16 + 1) * PITCH * 16 <= 4 * TILE * 2, "the tile buffers take what is sent");
+#pragma unroll
+    for (int i = 0; i < HD16; ++i) {
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = part == 0 ? o[HD16 + i][e] : o[i][e];
+        sent[i * PITCH] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+    sent[HD16 * PITCH] = make_float4(m0, l0, m1, l1);
+    cluster_sync();
+    {
+        const uint32_t peer = peer_smem(smem_addr(sent), part ^ 1);
+        const float2 s0 = ld_peer2(peer + HD16 * PITCH * 16), s1 = ld_peer2(peer + HD16 * PITCH * 16 + 8);
+        const float M0 = fmaxf(m0, s0.x), M1 = fmaxf(m1, s1.x);  // (finite: one of the two has seen key 0)
+        const float a0 = m0 == -INFINITY ? 0.f : expf(m0 - M0), b0 = s0.x == -INFINITY ? 0.f : expf(s0.x - M0);
+        const float a1 = m1 == -INFINITY ? 0.f : expf(m1 - M1), b1 = s1.x == -INFINITY ? 0.f : expf(s1.x - M1);
+        const float i0 = share(fmaf(a0, l0, b0 * s0.y)), i1 = share(fmaf(a1, l1, b1 * s1.y));
+#pragma unroll
+        for (int i = 0; i < HD16; ++i) {
+            const float2 u = ld_peer2(peer + i * PITCH * 16), w = ld_peer2(peer + i * PITCH * 16 + 8);
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = part == 0 ? o[i][e] : o[HD16 + i][e];
+            const float sum[4] = {fmaf(a0, v[0], b0 * u.x), fmaf(a0, v[1], b0 * u.y), fmaf(a1, v[2], b1 * w.x), fmaf(a1, v[3], b1 * w.y)};
+            put(part * HD16 + i, sum, i0, i1);
         }
     }
+    cluster_sync();  // nobody leaves while its sums are being read
 }
 
 // ───────────────── decode-shaped attention on tensor cores: the query heads of a GQA group as one tile ─────────────────
@@ -678,7 +731,11 @@ cudaError_t launch_attention_prefill(const float* q, int ldq, float* out, int ld
     if (!attention_prefill_supported(kv.head_dim)) return cudaErrorInvalidValue;
     const int hd16 = kv.head_dim / 16;
     const size_t smem = (size_t)4 * FA_KEYS * (kv.head_dim + 8) * sizeof(__half);  // two (K, V) tile buffers
-    const dim3 grid(n_heads, (n_tok + FA_ROWS - 1) / FA_ROWS), block(FA_WARPS * 32);
+    // The longest tile's chain of keys is what a launch takes, some 4 us for 64 of them: two blocks share it while SMs have room for them
+    // (389 tokens of Phi-2 29.6 -> 22.7 us a layer, 512 of the 8B shape 39.2 -> 36.5, most of it from pages that are looked up a tile ahead).
+    const int row_tiles = (n_tok + FA_ROWS - 1) / FA_ROWS;
+    const int parts = pos0 + n_tok > 2 * FA_KEYS && (int64_t)n_heads * row_tiles <= 2 * device_sm_count() ? 2 : 1;
+    const dim3 grid(n_heads, row_tiles, parts), block(FA_WARPS * 32);
     cudaError_t le = cudaErrorInvalidValue;
 #define SP_FA(N, EX)                                                                                                    \
     if (hd16 == N && exact == EX) {                                                                                     \
@@ -687,7 +744,7 @@ cudaError_t launch_attention_prefill(const float* q, int ldq, float* out, int ld
             le = big_smem.run([] { return cudaFuncSetAttribute(attention_prefill_kernel<N, EX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024); }); \
             if (le != cudaSuccess) return le;                                                                           \
         }                                                                                                               \
-        le = launch_pdl(attention_prefill_kernel<N, EX>, grid, block, smem, st, q, ldq, out, out_h, ldo, n_tok, n_heads, slot, pos0, kv, layer, scale); \
+        le = launch_pdl_cluster(attention_prefill_kernel<N, EX>, grid, block, smem, st, parts, q, ldq, out, out_h, ldo, n_tok, n_heads, slot, pos0, kv, layer, scale); \
     }
 #define SP_FA2(N) SP_FA(N, false) SP_FA(N, true)
     SP_FA2(1) SP_FA2(2) SP_FA2(3) SP_FA2(4) SP_FA2(5) SP_FA2(6) SP_FA2(7) SP_FA2(8)

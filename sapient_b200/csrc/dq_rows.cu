@@ -20,6 +20,8 @@ namespace sp {
 cudaError_t count_launch_and_check();  // kernels.cu
 
 constexpr int DR_THREADS = 512;
+// Threads of a row's block, at most: twice as many where they have two pieces of eight columns.
+__host__ __device__ constexpr int dr_threads(int nc) { return nc == 2 ? 2 * DR_THREADS : DR_THREADS; }
 
 struct DqRowsArgs {
     const float* x;
@@ -91,8 +93,8 @@ __device__ __forceinline__ void dr_split(const DqRowsArgs& a, int m, int c, bool
 
 // One row per block, up to 8 NC columns per thread in registers. Formulas: kernels/layernorm.rs:17-105, elementwise.rs:120-143.
 template <int SRC, int NC>
-__global__ void __launch_bounds__(DR_THREADS) dq_rows_kernel(const DqRowsArgs a) {
-    __shared__ float sh[DR_THREADS / 32];
+__global__ void __launch_bounds__(dr_threads(NC)) dq_rows_kernel(const DqRowsArgs a) {
+    __shared__ float sh[dr_threads(NC) / 32];
     const int m = blockIdx.x;
     const float* row = a.x + (int64_t)m * a.ldx;
     // (a short row's norm weights, which no kernel writes, are here when the row comes)
@@ -202,9 +204,12 @@ cudaError_t launch_dq_rows(int src, const float* x, int ldx, const float* w, con
     DqRowsArgs a{};
     a.x = x; a.ldx = ldx; a.k = k; a.m_rows = m; a.w = w; a.b = b; a.eps = eps; a.up = k;
     a.xh = in.xh; a.xscale = in.xscale; a.xsum = in.xsum;
-    // threads for eight columns each, at most DR_THREADS of them with one, two or four such pieces
-    const int pieces = k / 8, nc = pieces <= DR_THREADS ? 1 : pieces <= 2 * DR_THREADS ? 2 : 4;
-    const dim3 grid((unsigned)m), block((unsigned)std::min(DR_THREADS, (pieces + 31) / 32 * 32));
+    // Threads for eight columns each, or, above 4096 columns, for two or four such pieces. While rows are few a block has an SM nearly for
+    // itself, and with more warps hides its loads better: SwiGLU of 32 rows of 14336, two pieces 5.4 us and four 8.4, of 192 rows of 8960 6.3
+    // and 7.0, GELU of 389 rows of 10240 8.3 and 10.0; but 512 rows of 14336 23.5 and 18.3.
+    const int pieces = k / 8, nc = pieces <= DR_THREADS ? 1 : pieces <= 2 * DR_THREADS || m <= 3 * device_sm_count() ? 2 : 4;
+    const int threads = std::min(dr_threads(nc), ((pieces + nc - 1) / nc + 31) / 32 * 32);
+    const dim3 grid((unsigned)m), block((unsigned)(dq_rows_fit(k) ? threads : DR_THREADS));
     cudaError_t le = cudaErrorInvalidValue;
 #define SP_DR(S)                                                                                  \
     if (src == S) {                                                                               \

@@ -329,7 +329,7 @@ int Engine::repack_weights() {
         const int64_t widest = std::max<int64_t>({(int64_t)d.vocab, 2 * (int64_t)d.ffn, (int64_t)(d.n_heads + 2 * d.n_kv_heads) * d.head_dim, (int64_t)d.hidden});
         SP_CUDA_TRY(ring_.alloc((int)(widest / 16 + 8)));
     }
-    if (d.max_tokens > imma_rows_per_pass()) SP_CUDA_TRY(rows_.alloc());
+    if (d.max_tokens >= ROWS_MIN_M) SP_CUDA_TRY(rows_.alloc());
     return SP_OK;
 }
 

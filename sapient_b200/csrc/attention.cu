@@ -195,7 +195,7 @@ static cudaError_t launch_split_phase(const float* q, int ldq, float* out, int l
                       tok_pos, kv, layer, scale, n_splits, scratch, fresh);
 }
 
-// Merge of the splits (splits.cuh); one thread per coordinate.
+// Merge of the splits (splits.cuh); one thread per coordinate. NS: at most so many splits, 0: any number.
 template <int NS>
 __global__ void attention_merge_kernel(const float* __restrict__ part, int n_heads, int n_splits, int hd, float* __restrict__ out,
                                        int ldo) {
@@ -203,7 +203,12 @@ __global__ void attention_merge_kernel(const float* __restrict__ part, int n_hea
     pdl_trigger();
     const int h = blockIdx.x, t = blockIdx.y;
     const float* src = part + ((int64_t)t * n_heads + h) * n_splits * (hd + 2);
-    for (int e = threadIdx.x; e < hd; e += blockDim.x) out[(int64_t)t * ldo + (int64_t)h * hd + e] = merge_splits<NS>(src, n_splits, hd, e);
+    for (int e = threadIdx.x; e < hd; e += blockDim.x) {
+        float v;
+        if constexpr (NS > 0) v = merge_splits<NS>(src, n_splits, hd, e);
+        else v = merge_many_splits(src, n_splits, hd, e);
+        out[(int64_t)t * ldo + (int64_t)h * hd + e] = v;
+    }
 }
 
 size_t attention_scratch_floats(int n_tok, int n_heads, int n_splits, int head_dim) {
@@ -228,8 +233,8 @@ cudaError_t launch_attention(const float* q, int ldq, float* out, int ldo, int n
     if (le != cudaSuccess) return le;
     cudaError_t e = count_launch_and_check();
     if (e != cudaSuccess || n_splits == 1) return e;
-    if (n_splits > MERGE_MAX_SPLITS) return cudaErrorInvalidValue;
-    auto merge = n_splits <= 4 ? attention_merge_kernel<4> : n_splits <= 16 ? attention_merge_kernel<16> : attention_merge_kernel<MERGE_MAX_SPLITS>;
+    auto merge = n_splits <= 4 ? attention_merge_kernel<4> : n_splits <= 16 ? attention_merge_kernel<16>
+                 : n_splits <= MERGE_MAX_SPLITS ? attention_merge_kernel<MERGE_MAX_SPLITS> : attention_merge_kernel<0>;
     le = launch_pdl(merge, dim3(n_heads, n_tok), dim3(128), 0, st, (const float*)scratch, n_heads, n_splits, kv.head_dim, out, ldo);
     if (le != cudaSuccess) return le;
     return count_launch_and_check();

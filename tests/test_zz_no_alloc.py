@@ -5,6 +5,7 @@ calls in a row that share the library's fixed scratch array, whether this file r
 import numpy as np
 import pytest
 
+from helpers import rel_l2
 from sapient_b200 import _lib, ops
 
 pytestmark = pytest.mark.gpu
@@ -87,3 +88,15 @@ def test_static_scratch_rejects_oversized_request():
     q, k, v = _rand(4, H, Hkv, sq, sk, hd)
     with pytest.raises(_lib.SapientCudaError, match="static buffer"):
         _static_attention(torch, q, k, v, n_splits=n_splits)
+
+
+@pytest.mark.parametrize("hd", [32, 80, 128])
+@pytest.mark.parametrize("n_splits", [16, 17, 32, 33, 48, 64])
+def test_every_number_of_splits(hd, n_splits):
+    """Up to 64, as documented, more of them than keys among them: against one split, f32 sums in another order."""
+    import torch
+
+    for sk in (19, 640):
+        q, k, v = _rand(n_splits, 4, 2, 2, sk, hd)
+        want = _static_attention(torch, q, k, v, n_splits=1)
+        assert rel_l2(_static_attention(torch, q, k, v, n_splits=n_splits), want) < 1e-5

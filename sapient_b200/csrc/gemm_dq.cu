@@ -361,7 +361,8 @@ __device__ __forceinline__ bool dq_drain(DqBars& bars, const uint8_t* raw, int r
         __syncwarp();
         if (lane == 0) tc5_arrive(&bars.empty_r[rr.st]);
         rr.next(r_stages);
-        if (DT == T_Q4_K) ok = ok && rx.full(bars.full_x);
+        // (the warp's verdict, not each lane's: what it guards is an instruction of the whole warp)
+        if (DT == T_Q4_K) ok = __all_sync(0xFFFFFFFFu, ok && rx.full(bars.full_x));
         const uint8_t* xrow = xs + (size_t)rx.st * x_bytes + (half * NJT * 8 + g) * 32 + t * 8;
         if (DT == T_Q4_K && ok) {
 #pragma unroll

@@ -61,7 +61,8 @@ int32_t sp_cuda_dequant(const SpWeight* w, float* out_host);
 /* Y[m,n] = X[m,k] · Wᵀ, host buffers (copies inside). */
 int32_t sp_cuda_matmul_nt(const SpWeight* w, const float* x_host, int64_t m, float* y_host);
 /* Same with device buffers on `stream` (a cudaStream_t, or NULL for the default stream); the launches are not waited
- * for. The weight carries a private workspace (activation digits, and an fp16 copy of x for calls of 17 rows and
+ * for. With the default kernels and modes y may be x (n == k), and up to 16 rows overlap it in any way; with others not.
+ * The weight carries a private workspace (activation digits, and an fp16 copy of x for calls of 17 rows and
  * more), so calls on one SpWeight must be ordered on ONE stream and never run from two threads at once; use one
  * SpWeight per stream otherwise. The fp16 buffer grows on demand: the first call with a given (larger) m of 17 rows or
  * more frees and allocates device memory, which waits for all work of the device — issue one such call per weight at

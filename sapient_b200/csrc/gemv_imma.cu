@@ -1137,7 +1137,10 @@ cudaError_t launch_quant_gemv(const float* x, int ldx, ImmaArgs& a, const ActWor
     if (a.m <= 0) return cudaSuccess;
     if (a.m > imma_rows_per_pass() || a.k > ws.k_max) return cudaErrorInvalidValue;
     imma_plan(a, ws);
-    if (requantize && imma_makes_digits(a)) {
+    // (outputs may take the row's place: blocks that are done store theirs while others still read it, a launch of its own has read it all)
+    bool in_place = false;
+    for (int s = 0; s < a.nseg; ++s) in_place = in_place || (x < a.seg[s].y + a.seg[s].n && a.seg[s].y < x + a.k);
+    if (requantize && !in_place && imma_makes_digits(a)) {
         a.x = x;
         return launch_gemv_imma(a, st);
     }

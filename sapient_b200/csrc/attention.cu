@@ -512,8 +512,9 @@ attention_prefill_kernel(const float* __restrict__ q, int ldq, float* __restrict
 // softmax weights are split the same way for the second contraction. K and V are fp16 in the cache, hence exact.
 // Online softmax per page with the reference's recurrence (kernels/attention.rs:98-165); the warps' states are merged
 // through shared memory, and the block writes either the output rows (one split) or the split partials.
+// (96 coordinates: with room for three blocks an SM the compiler keeps 159 registers, left alone 128 with which ranges of many keys took 12 to 19 % longer.)
 template <int HD16, int GM_WARPS>
-__global__ void __launch_bounds__(GM_WARPS * 32)
+__global__ void __launch_bounds__(GM_WARPS * 32, HD16 == 6 ? 3 : 0)
 attention_gqa_mma_kernel(const float* __restrict__ q, int ldq, float* __restrict__ out, int ldo, int n_heads, const int32_t* __restrict__ tok_slot,
                          const int32_t* __restrict__ tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* __restrict__ part,
                          int fresh) {
@@ -676,32 +677,39 @@ bool attention_gqa_mma_supported(int n_heads, int n_kv, int head_dim) {
     return group >= 2 && group <= 8 && head_dim % 16 == 0 && head_dim >= 16 && head_dim <= 128;
 }
 
+// Four warps a block, or three where all of them then run in fewer rounds of the SMs: 512 blocks of 128 coordinates, of which an SM holds
+// three or four, 18.8 -> 13.3 us with the rotation before it (32 sequences of the 8B shape at 400 keys, two splits), 768 of 64
+// coordinates 0.91 of the time; in as many rounds three take longer, 384 blocks of 128 coordinates 1.05, 208 of 96 up to 1.3.
+template <int HD16>
+static cudaError_t launch_gqa_mma(const float* q, int ldq, float* out, int ldo, int n_tok, int n_heads, const int32_t* tok_slot, const int32_t* tok_pos,
+                                  KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st, int fresh) {
+    constexpr size_t WARP_SMEM = 4 * KV_PAGE * (16 * HD16 + 8) * sizeof(__half);
+    static PerDeviceOnce once;
+    static int held[SP_MAX_DEVICES][2];  // blocks of four and of three warps that an SM holds
+    int* const fit = held[current_device_index()];
+    cudaError_t le = once.run([&] {
+        cudaError_t e = cudaFuncSetAttribute(attention_gqa_mma_kernel<HD16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * WARP_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_gqa_mma_kernel<HD16, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * WARP_SMEM);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit[0], attention_gqa_mma_kernel<HD16, 4>, 128, 4 * WARP_SMEM);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit[1], attention_gqa_mma_kernel<HD16, 3>, 96, 3 * WARP_SMEM);
+        return e;
+    });
+    if (le != cudaSuccess) return le;
+    const int64_t blocks = (int64_t)kv.n_kv * n_tok * n_splits;
+    auto rounds = [&](int per_sm) { const int64_t at_once = (int64_t)std::max(per_sm, 1) * device_sm_count(); return (blocks + at_once - 1) / at_once; };
+    const bool narrow = rounds(fit[1]) < rounds(fit[0]);
+    const int warps = narrow ? 3 : 4;
+    return launch_pdl(narrow ? attention_gqa_mma_kernel<HD16, 3> : attention_gqa_mma_kernel<HD16, 4>, dim3(kv.n_kv, n_tok, n_splits), dim3(32 * warps),
+                      warps * WARP_SMEM, st, q, ldq, out, ldo, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, fresh);
+}
+
 cudaError_t launch_gqa_mma_phase(const float* q, int ldq, float* out, int ldo, int n_tok, int n_heads, const int32_t* tok_slot,
                                  const int32_t* tok_pos, KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st, int fresh) {
-    const int hd16 = kv.head_dim / 16;
-    const dim3 grid(kv.n_kv, n_tok, n_splits);
-    // Four warps a block while few blocks share an SM; three where they would not all fit at once (70 KB each with 128 coordinates; four blocks
-    // of three warps do): 32 sequences of the 8B shape, 512 blocks, 23.2 -> 20.4 us a layer, but 104 blocks of the 1.5B shape 6.0 -> 6.5.
-    const bool narrow = (int64_t)kv.n_kv * n_tok * n_splits > 2 * device_sm_count();
-    const int warps = narrow ? 3 : 4;
-    const size_t smem = (size_t)warps * 4 * KV_PAGE * (kv.head_dim + 8) * sizeof(__half);
-    const dim3 block(32 * warps);
-    cudaError_t le = cudaErrorInvalidValue;
-#define SP_GM(N)                                                                                                        \
-    if (hd16 == N) {                                                                                                    \
-        static PerDeviceOnce big_smem;                                                                                  \
-        if (smem > 48 * 1024) {                                                                                         \
-            le = big_smem.run([] {                                                                                      \
-                const cudaError_t e = cudaFuncSetAttribute(attention_gqa_mma_kernel<N, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024); \
-                return e != cudaSuccess ? e : cudaFuncSetAttribute(attention_gqa_mma_kernel<N, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024); \
-            });                                                                                                         \
-            if (le != cudaSuccess) return le;                                                                           \
-        }                                                                                                               \
-        le = launch_pdl(narrow ? attention_gqa_mma_kernel<N, 3> : attention_gqa_mma_kernel<N, 4>, grid, block, smem, st, q, ldq, out, ldo, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, fresh); \
-    }
-    SP_GM(1) SP_GM(2) SP_GM(3) SP_GM(4) SP_GM(5) SP_GM(6) SP_GM(7) SP_GM(8)
-#undef SP_GM
-    return le;
+    auto launch = kv.head_dim == 16 ? launch_gqa_mma<1> : kv.head_dim == 32 ? launch_gqa_mma<2> : kv.head_dim == 48 ? launch_gqa_mma<3>
+                  : kv.head_dim == 64 ? launch_gqa_mma<4> : kv.head_dim == 80 ? launch_gqa_mma<5> : kv.head_dim == 96 ? launch_gqa_mma<6>
+                  : kv.head_dim == 112 ? launch_gqa_mma<7> : kv.head_dim == 128 ? launch_gqa_mma<8> : nullptr;
+    if (!launch) return cudaErrorInvalidValue;
+    return launch(q, ldq, out, ldo, n_tok, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, st, fresh);
 }
 
 // A tile walks all its keys alone, at 50 to 76 ns each whatever the number of its rows, and up to two blocks per SM take no longer

@@ -30,7 +30,8 @@ __device__ __forceinline__ int64_t kv_off(const KvGeom& kv, int layer, int page,
 // position, page, rows. Requested as they were needed, all by size of the largest head, it was 6.1 us of a layer of the 8B shape at
 // context 517 (33 keys a block), 6.4 of Phi-2's at 645, 6.6 for 5 rows of the 1.5B shape; now 4.5, 5.0, 4.4. (Eight keys a round: 3.8,
 // 4.8, 6.3, and 3.7 against 2.5 for the 9 keys a block of the 0.5B shape at 130, where the sums over lanes of keys that are not
-// there count.)
+// there count.) Pages are looked up a round ahead of the rows, whose addresses have a base per page: with both inside the request 2000 keys of
+// 64 coordinates in one range took 107 us, 86 with nothing requested ahead, now 83.
 template <int PAIRS>
 __global__ void __launch_bounds__(ATT_WARPS * 32)
 attention_split_kernel(const float* __restrict__ q, int ldq, float* __restrict__ out, int ldo, int n_heads,
@@ -50,15 +51,19 @@ attention_split_kernel(const float* __restrict__ q, int ldq, float* __restrict__
     const int32_t* pt = kv.page_table + (int64_t)slot * kv.max_pages;
     // all K and V fragments of a round are requested before any arithmetic, so the V loads do not wait for the scores
     struct Round { __half2 k[ATT_KEYS][PAIRS], v[ATT_KEYS][PAIRS]; };
-    auto load = [&](int key0, Round& r) {
+    auto pages_of = [&](int key0) {  // of the round's first and last key (past the range: of its last one)
+        return make_int2(pt[min(key0, k_end - 1) / KV_PAGE], pt[(min(key0 + ATT_KEYS, k_end) - 1) / KV_PAGE]);
+    };
+    const int64_t of_page = (int64_t)2 * kv.n_kv * KV_PAGE * hd, to_v = (int64_t)kv.n_kv * KV_PAGE * hd;
+    const __half* const keys = kv.pool + kv_off(kv, layer, 0, 0, kv_h);
+    auto load = [&](int key0, int2 pages, Round& r) {
         const int last = min(key0 + ATT_KEYS, k_end) - 1;  // tail keys repeat the last one and get weight 0
-        const int page0 = pt[key0 / KV_PAGE], page1 = pt[last / KV_PAGE];
+        const __half *const first = keys + pages.x * of_page, *const second = keys + pages.y * of_page;
 #pragma unroll
         for (int j = 0; j < ATT_KEYS; ++j) {
             const int key = min(key0 + j, last);
-            const int page = key / KV_PAGE == key0 / KV_PAGE ? page0 : page1;
-            const __half2* kp = reinterpret_cast<const __half2*>(kv.pool + kv_off(kv, layer, page, 0, kv_h) + (int64_t)(key % KV_PAGE) * hd);
-            const __half2* vp = reinterpret_cast<const __half2*>(kv.pool + kv_off(kv, layer, page, 1, kv_h) + (int64_t)(key % KV_PAGE) * hd);
+            const __half* row = (key / KV_PAGE == key0 / KV_PAGE ? first : second) + (key % KV_PAGE) * hd;
+            const __half2 *kp = reinterpret_cast<const __half2*>(row), *vp = reinterpret_cast<const __half2*>(row + to_v);
 #pragma unroll
             for (int i = 0; i < PAIRS; ++i) {
                 const int p = lane + 32 * i;
@@ -71,10 +76,13 @@ attention_split_kernel(const float* __restrict__ q, int ldq, float* __restrict__
     constexpr int STRIDE = ATT_WARPS * ATT_KEYS;
     int key0 = k_begin + warp * ATT_KEYS;
     Round ra, rb;
+    int2 pages = make_int2(0, 0);
     const bool early = fresh >= 0 && key0 < k_end && min(key0 + ATT_KEYS, k_end) <= n_keys - fresh;
-    if (early) load(key0, ra);
+    if (early) load(key0, pages_of(key0), ra);
     if (fresh >= 0) pdl_wait();
     pdl_trigger();
+    if (!early && key0 < k_end) load(key0, pages_of(key0), ra);
+    if (key0 + STRIDE < k_end) pages = pages_of(key0 + STRIDE);  // a round ahead of its rows
     const float* qrow = q + (int64_t)t * ldq + (int64_t)h * hd;
     float2 qv[PAIRS], o[PAIRS];
 #pragma unroll
@@ -83,7 +91,6 @@ attention_split_kernel(const float* __restrict__ q, int ldq, float* __restrict__
         qv[i] = (p < npairs) ? make_float2(qrow[2 * p], qrow[2 * p + 1]) : make_float2(0.f, 0.f);
         o[i] = make_float2(0.f, 0.f);
     }
-    if (!early && key0 < k_end) load(key0, ra);
     float m = -INFINITY, l = 0.f;
     auto round = [&](int k0, const Round& r) {
         float s[ATT_KEYS];
@@ -131,10 +138,16 @@ attention_split_kernel(const float* __restrict__ q, int ldq, float* __restrict__
         m = m_new;
     };
     for (; key0 < k_end; key0 += 2 * STRIDE) {
-        if (key0 + STRIDE < k_end) load(key0 + STRIDE, rb);
+        if (key0 + STRIDE < k_end) {
+            load(key0 + STRIDE, pages, rb);
+            pages = pages_of(key0 + 2 * STRIDE);
+        }
         round(key0, ra);
         if (key0 + STRIDE >= k_end) break;
-        if (key0 + 2 * STRIDE < k_end) load(key0 + 2 * STRIDE, ra);
+        if (key0 + 2 * STRIDE < k_end) {
+            load(key0 + 2 * STRIDE, pages, ra);
+            pages = pages_of(key0 + 3 * STRIDE);
+        }
         round(key0 + STRIDE, rb);
     }
     if (lane == 0) { sh_m[warp] = m; sh_l[warp] = l; }
@@ -678,8 +691,9 @@ bool attention_gqa_mma_supported(int n_heads, int n_kv, int head_dim) {
 }
 
 // Four warps a block, or three where all of them then run in fewer rounds of the SMs: 512 blocks of 128 coordinates, of which an SM holds
-// three or four, 18.8 -> 13.3 us with the rotation before it (32 sequences of the 8B shape at 400 keys, two splits), 768 of 64
-// coordinates 0.91 of the time; in as many rounds three take longer, 384 blocks of 128 coordinates 1.05, 208 of 96 up to 1.3.
+// three or four, 17.3 -> 14.7 us with the rotation before it (32 sequences of the 8B shape at 400 keys, two splits), 768 of 64
+// coordinates 0.91 of the time; in as many rounds three take longer, 384 blocks of 128 coordinates 1.05, 320 of 96 (40 sequences at 2000
+// keys) 31.0 -> 34.7.
 template <int HD16>
 static cudaError_t launch_gqa_mma(const float* q, int ldq, float* out, int ldo, int n_tok, int n_heads, const int32_t* tok_slot, const int32_t* tok_pos,
                                   KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st, int fresh) {

@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(WARPS * 32, (NT == 1 && FMT != 0 && FMT != T_Q
                 compute_q4_k<NT>(w, BGlobal<NT>(a, at, lane), lane, acc);
             }
         };
-        constexpr bool TWO = NT <= 3;  // (a second tile in flight where registers allow)
+        constexpr bool TWO = NT <= 3 && !(NT == 1 && FMT == T_Q4_K);  // (a second tile in flight where registers allow)
         int kt = warp;
         if (kt < kts) load_q4_k<true>(base + (int64_t)kt * Q4_K_TILE_BYTES, lane, ra);
         if (TWO && kt + WARPS < kts) load_q4_k<true>(base + (int64_t)(kt + WARPS) * Q4_K_TILE_BYTES, lane, rb);
@@ -1106,11 +1106,11 @@ cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st) {
         q6_only = q6_only && a.seg[s].dtype == T_Q6_K;
         q8_only = q8_only && a.seg[s].dtype == T_Q8_0;
     }
-    // One or two rows: the 80-register single-format instances trade per-block speed for a third block per SM. Q6_K 17920 x 1536 (1120
-    // tile rows) 11.1 -> 9.7 us, 128256 x 4096 99 -> 81; with grids that fit the SMs at once a block's latency is the kernel's. Q4_K has two
-    // tiles per warp in flight without them, and few waves are worth more evenly filled: 18944 x 3584 13.6 us with two blocks, 15.4
-    // with three, 28672 x 4096 19.4 and 20.9, but 128256 x 4096 71.9 and 66.6, 151936 x 1536 58.0 and 49.8.
-    const bool deep_q4 = tiles >= 4096, deep_q6 = tiles >= 1024;
+    // One or two rows: the 80-register single-format instances, one tile per warp in flight and a third block per SM, where the grid goes
+    // over the SMs several times; with grids that fit them at once a block's latency is the kernel's. From cold weights, two blocks of
+    // two tiles and three of one: Q4_K 16400 x 256 7.5 and 6.1 us, 28672 x 4096 20.4 and 18.3, 64000 x 1024 24.8 and 18.0, 151936 x 1536 51.0 and 42.6;
+    // Q6_K 17920 x 1536 11.1 and 9.7.
+    const bool deep = tiles >= 1024;
     // Fewer tile rows than SMs: 16 warps share a row's columns, where there is a piece for more than eight. Q4_K 1536 x 8960 1 row 6.3
     // -> 5.6 us, 13 rows 14.7 -> 10.9; Q8_0 896 x 4864 5.6 -> 4.6, 13 rows 9.5 -> 7.4. (With eight pieces or fewer 2 % slower.)
     const bool wide = tiles <= device_sm_count() && a.k / (q8_only && a.seg[0].bpt > 1 ? 128 : 256) > IMMA_WARPS;
@@ -1118,8 +1118,8 @@ cudaError_t launch_gemv_imma(const ImmaArgs& a, cudaStream_t st) {
         if (!imma_makes_digits(a)) return cudaErrorInvalidValue;
         le = !wide ? launch_pdl(gemv_imma_kernel<1, 0, 8, 2>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a)
                    : launch_pdl(gemv_imma_kernel<1, 0, 16, 1>, dim3(tiles), dim3(512), 0, st, a);
-    } else if (nt == 1 && q4_only && deep_q4) le = launch_pdl(gemv_imma_kernel<1, T_Q4_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
-    else if (nt == 1 && q6_only && deep_q6) le = launch_pdl(gemv_imma_kernel<1, T_Q6_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
+    } else if (nt == 1 && q4_only && deep) le = launch_pdl(gemv_imma_kernel<1, T_Q4_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
+    else if (nt == 1 && q6_only && deep) le = launch_pdl(gemv_imma_kernel<1, T_Q6_K>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a);
 #define SP_GEMV(N)                                                                                                                   \
     else if (nt == N)                                                                                                                \
         le = !wide ? launch_pdl(q8_only ? gemv_imma_kernel<N, T_Q8_0> : gemv_imma_kernel<N, 0>, dim3(tiles), dim3(IMMA_WARPS * 32), 0, st, a) \

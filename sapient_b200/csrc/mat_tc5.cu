@@ -369,38 +369,44 @@ cudaError_t launch_mat_tc5(const MatArgs& a, int max_tiles, cudaStream_t st) {
         while (bn > 32 && ((int64_t)row_blocks * groups * ((a.m + bn - 1) / bn) < sms || bn >= 2 * a.m)) bn >>= 1;
     const int acc = a.dual ? 2 : 1;
     // More than 32 rows: low tiles fetch every weight once more, high ones leave a ring of two stages and SMs idle; a shared K range pays
-    // for partial sums that cross the cluster. The rows are dealt out evenly to 1, 2, 3 .. tiles, and height and parts are the fastest in the
-    // model below. 301 rows in two tiles of 160 where powers of two gave 256 and 45: 16512 x 2048 41.1 -> 26.8 us, 9216 x 2048 (four of 80
-    // for three of 128) 22.4 -> 17.2, 2048 x 8192 (eight parts for four) 26.3 -> 20.7; 389 rows of 12288 x 4096 63.8 -> 39.0; 33 rows of 2048 x
-    // 6144, the one that lost, 10.8 -> 11.6. K is shared with a long K and few tiles (2048 x 9216, 96 rows:
-    // 41.6 -> 15.9 us), not where a part is over before its sums are added (2048 x 512, 512 rows: 6.1, shared 11.9). Constants fitted to
-    // 3400 times of 24 matrices at 33 to 2000 rows with heights 32, 64, 128, 256 and every number of parts, 10 % off on average.
+    // for partial sums that cross the cluster. It is shared where that takes less time in the model below: with a long K and few tiles (2048 x
+    // 9216, 96 rows: 41.6 -> 15.9 us), not where a part is over before its sums are added (2048 x 512, 512 rows: 6.1, shared 11.9). Heights are
+    // powers of two, or, where the model promises a tenth, rows dealt out evenly to 1, 2, 3 .. tiles: 301 rows in two tiles of 160 where
+    // powers of two gave 256 and 45 16512 x 2048 41.1 -> 26.8 us, 9216 x 2048 (four of 80 for three of 128) 22.4 -> 17.2, 2048 x 8192 (eight
+    // parts for four) 26.3 -> 20.7; 389 rows of 12288 x 4096 63.8 -> 39.0. Over 728 sizes (26 matrices, 33 to 1500 rows) that is 0.973 of the
+    // time of powers of two alone, at worst 1.014; with any promise taken 125 of them lost 3 to 30 %, among them 2048 x 2048, 80 rows, 7.6 -> 9.7.
+    // Constants fitted to 3400 times of 24 matrices at heights 32, 64, 128, 256 and every number of parts, 10 % off on average, 14 over all
+    // heights. Gated products of several waves, whose last one the model overrates, keep powers of two (14336 x 4096, 257 rows: 98, even shares 114).
     k.parts = 1;
     if (!a.moe && a.nseg == 1 && a.m > 32) {
+        auto ctas_of = [&](int h, int p) { return (double)row_blocks * groups * ((a.m + h - 1) / h) * p; };
+        // clusters of four and eight leave SMs over
+        auto waves = [&](int h, int p) { return ceil(ctas_of(h, p) / ((p == 8 ? 0.865 : p == 4 ? 0.946 : 1.0) * 2.0 * sms)); };
         auto time = [&](int h, int p) {  // us
-            // 64 columns of K, heights 32 to 256, for a CTA alone on its SM and for two; clusters of four and eight leave SMs over
+            // 64 columns of K, heights 32 to 256, for a CTA alone on its SM and for two
             static constexpr double CHUNK[2][2][4] = {{{0.287, 0.303, 0.358, 0.539}, {0.315, 0.331, 0.385, 0.634}},
                                                       {{0.436, 0.685, 0.767, 0.767}, {0.491, 0.607, 0.843, 0.843}}};
-            const double ctas = (double)row_blocks * groups * ((a.m + h - 1) / h) * p, values = (double)h * acc;
-            const double waves = ceil(ctas / ((p == 8 ? 0.865 : p == 4 ? 0.946 : 1.0) * 2.0 * sms));
+            const double ctas = ctas_of(h, p), n_waves = waves(h, p), values = (double)h * acc;
             const bool two = ctas > sms;
             const int low = h < 64 ? 0 : h < 128 ? 1 : 2;
             const double* const at = CHUNK[a.dual][two] + low;
             const double chunk = at[0] + (at[1] - at[0]) * (h - (32 << low)) / (32 << low);
-            return 2.52 + waves * (kp_max / MT_BK) / p * chunk + 0.0168 * std::max(1.0, ctas / sms) * values +
-                   (p > 1 ? waves * (2.79 + 0.127 * p) + (two ? 2.0 * waves : 1.0) * values * 0.0589 / p : 0.0);
+            return 2.52 + n_waves * (kp_max / MT_BK) / p * chunk + 0.0168 * std::max(1.0, ctas / sms) * values +
+                   (p > 1 ? n_waves * (2.79 + 0.127 * p) + (two ? 2.0 * n_waves : 1.0) * values * 0.0589 / p : 0.0);
         };
-        const int top = a.dual ? 128 : 256;
-        double best = 0.0;
-        for (int t = (a.m + top - 1) / top, h = 0; h != 32; ++t) {
-            const int height = std::max(32, ((a.m + t - 1) / t + 15) & ~15);
-            if (height == h) continue;
-            h = height;
+        double best = time(bn, 1);
+        for (int h = 32; h <= (a.dual ? 64 : 128) && h < 2 * a.m; h *= 2)
+            for (int p = 2; p <= MT_MAX_PARTS && kp_max / MT_BK >= 4 * p; p *= 2)
+                if (const double t = time(h, p); t < best) { best = t; bn = h; k.parts = p; }
+        best *= 0.91;
+        for (int h = std::min(a.dual ? 128 : 256, (a.m + 15) & ~15); h >= 32; h -= 16) {
+            const int tiles = (a.m + h - 1) / h;
+            if (h > 32 && h != (((a.m + tiles - 1) / tiles + 15) & ~15)) continue;
             const int stage = acc * MT_A_BYTES + h * MT_BK * 2, ring = std::min(MT_MAX_STAGES, MT_SMEM / stage) * stage;
             for (int p = 1; p <= MT_MAX_PARTS; p *= 2) {
                 if (p > 1 && (kp_max / MT_BK < 4 * p || acc * h * MT_BM * 4 > ring)) break;  // (the partial tile takes the ring's place)
-                const double c = time(h, p);
-                if (best == 0.0 || c < best) { best = c; bn = h; k.parts = p; }
+                if (a.dual && waves(h, p) > 1.0) break;
+                if (const double t = time(h, p); t < best) { best = t; bn = h; k.parts = p; }
             }
         }
     }

@@ -762,31 +762,32 @@ __global__ void __launch_bounds__(DQ_THREADS, 1) gemm_dq_kernel(const DqArgs a, 
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
 }
 
-// How many clusters of `parts` blocks the device holds at once (a block fills an SM, and a cluster lies within one GPC).
-static int dq_clusters(int parts) {
-    static std::atomic<int> cache[SP_MAX_DEVICES][DQ_MAX_PARTS + 1];
-    std::atomic<int>& c = cache[current_device_index()][parts];
-    int n = c.load(std::memory_order_relaxed);
-    if (n > 0) return n;
-    n = device_sm_count() / parts;
-    if (parts > 1) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(1, 1, (unsigned)parts);
-        cfg.blockDim = dim3(DQ_THREADS);
-        cfg.dynamicSmemBytes = DQ_SMEM;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = (unsigned)parts;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int got = 0;
-        if (cudaOccupancyMaxActiveClusters(&got, gemm_dq_kernel<2>, &cfg) == cudaSuccess && got > 0) n = got;
-        else cudaGetLastError();
+// How many clusters of 1 .. DQ_MAX_PARTS blocks the device holds at once (a block fills an SM, and a cluster lies within one GPC).
+struct DqClusters { std::atomic<int> of[DQ_MAX_PARTS + 1]; };
+static const DqClusters& dq_clusters() {
+    static DqClusters cache[SP_MAX_DEVICES];
+    DqClusters& c = cache[current_device_index()];
+    for (int parts = 1; parts <= DQ_MAX_PARTS; ++parts) {  // (each for itself: another thread may be half through)
+        if (c.of[parts].load(std::memory_order_relaxed) != 0) continue;
+        int n = device_sm_count() / parts;
+        if (parts > 1) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(1, 1, (unsigned)parts);
+            cfg.blockDim = dim3(DQ_THREADS);
+            cfg.dynamicSmemBytes = DQ_SMEM;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = (unsigned)parts;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int got = 0;
+            if (cudaOccupancyMaxActiveClusters(&got, gemm_dq_kernel<2>, &cfg) == cudaSuccess && got > 0) n = got;
+            else cudaGetLastError();
+        }
+        c.of[parts].store(std::max(n, 1), std::memory_order_relaxed);
     }
-    n = std::max(n, 1);
-    c.store(n, std::memory_order_relaxed);
-    return n;
+    return c;
 }
 
 cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& in, int m, int ldy, const float* res, int ldres, cudaStream_t st) {
@@ -819,46 +820,46 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
         return cudaSuccess;
     });
     if (le != cudaSuccess) return le;
-    // How high the tiles are and how they are dealt out, by the longest SM's time. One block per SM that walks over tiles: in tenths of
-    // a span of 256 columns, a tile is its spans and 3, the walk's start 10. Clusters that share a tile's K range: every wave of them is
-    // its spans and 45 (5 less for the first, whose start lies under the kernel before). Where tiles go over whole rounds of the SMs,
-    // those that do may have a launch of their own, 30 for the launch. Fitted to forced choices over 13 shapes x 6 row counts x 3 formats,
-    // of which the rule takes the fastest or one within 4 %. In us: Q4_K 6144 x 4096, 512 rows (192 tiles) walked 74.7, clusters of two
-    // 84.5, a walk and 44 tiles shared by two 70.6; 20000 x 14336, 20 rows (157 tiles) 160, clusters of four 121, nine tiles shared by
+    // How high the tiles are and how they are dealt out, by a model of the time in us, fitted to 30,000 forced choices (21 matrices x 24 row
+    // counts x 3 formats; 4 % off). SPAN: 256 columns of a tile by its height; a low tile's take less time, if more for each row. One block per
+    // SM walks over tiles, or clusters share a tile's K range, where every wave pays for its start and for the parts that are added; where tiles
+    // go over whole rounds of the SMs, those that do may have a launch of their own. Q4_K 6144 x 4096, 512 rows (192 tiles) walked 74.7, clusters
+    // of two 84.5, a walk and 44 tiles shared by two 70.6; 20000 x 14336, 20 rows (157 tiles) 160, clusters of four 121, nine tiles shared by
     // eight 97; 8960 x 1536, 300 rows (210 tiles) 37 walked, 39 in two launches.
-    // A span of a low tile takes less time, if more for each row (SPAN: us, measured with one tile per SM): lower ones than need be are
-    // for SMs that would be idle, and taken where they promise a seventh (of less than that nothing was left). Q8_0, 389 rows: 2560 x 2560
-    // 80 tiles of 112 rows 25.4 us, 140 of 64 21.1; 2560 x 10240 71.9 and 66.1; 1152 x 896, 300 rows 10.9 and 8.6; Q4_K 2048 x 1536, 192
-    // rows 12.0 and 11.0.
-    const int all_sb = (k + 255) / 256, sms = device_sm_count();
-    auto shared = [&](int n, int& parts) {
-        long cost = 0;
-        for (int p = 1; p <= std::min(DQ_MAX_PARTS, all_sb); ++p) {
-            const long waves = (n + dq_clusters(p) - 1) / dq_clusters(p), c = waves * (10 * ((all_sb + p - 1) / p) + 45) - 5;
-            if (p == 1 || c < cost) { parts = p; cost = c; }
-        }
-        return cost;
-    };
-    auto walked = [&](int n) { return (long)((n + sms - 1) / sms) * (10 * all_sb + 3) + 10; };
+    // Tiles lower than need be are for SMs that would be idle, and taken where they promise 3 %; not in clusters that fill their places
+    // to the last, which start one after the other (3000 x 2048, 112 rows, 72 of 74 pairs 15.5, as four parts of one tile 14.1). That is 0.962 of the
+    // time of the fewest tiles over those sizes, at worst 1.05. Q8_0, 389 rows: 2560 x 2560 80 tiles of 112 rows 25.4 us, 140 of 64 21.1;
+    // 2560 x 10240 71.9 and 66.1; 1152 x 896, 300 rows 10.9 and 8.6; Q4_K 2048 x 1536, 192 rows 12.0 and 11.0.
+    const int all_sb = (k + 255) / 256, sms = device_sm_count(), fewest = (m + DQ_NB - 1) / DQ_NB;
+    const DqClusters& clusters = dq_clusters();
     int items = 0, walk = 0, parts = 1;  // tiles; those that are walked over; the rest is shared by `parts` blocks each
     double best = 0.0;
-    const int fewest = (m + DQ_NB - 1) / DQ_NB;
+    bool lower = false;
     for (int low = fewest, last = 0; last != 16; ++low) {
         const int h = ((m + low - 1) / low + 15) & ~15, m_tiles = (m + h - 1) / h, n = tiles * m_tiles;
         if (h == last) continue;
-        last = h;
-        static constexpr double SPAN[2][8] = {{1.30, 1.39, 1.50, 1.67, 1.98, 2.18, 2.33, 2.53}, {1.04, 1.13, 1.26, 1.27, 1.70, 1.77, 1.94, 2.03}};
-        const double span = (low > fewest ? 1.16 : 1.0) * (SPAN[0][h / 16 - 1] * (tiles - one_plane) + SPAN[1][h / 16 - 1] * one_plane) / tiles;
-        auto take = [&](long tenths, int w, int p) {
-            if (best == 0.0 || span * tenths < best) { best = span * tenths; a.nb = h; a.m_tiles = m_tiles; items = n; walk = w; parts = p; }
+        if (last && n > 8 * sms) break;
+        if (last && !lower) best *= 0.97;
+        lower = last != 0;
+        static constexpr double SPAN[2][8] = {{1.26, 1.35, 1.47, 1.52, 1.79, 1.82, 1.87, 1.98}, {1.12, 1.10, 1.25, 1.26, 1.64, 1.67, 1.70, 1.74}};
+        const double span = (SPAN[0][h / 16 - 1] * (tiles - one_plane) + SPAN[1][h / 16 - 1] * one_plane) / tiles;
+        const int whole = n / sms * sms;
+        auto walked = [&](int count) { return ((count + sms - 1) / sms) * (all_sb * span + 0.014 * h); };
+        auto take = [&](double us, int w, int p) {
+            if (best == 0.0 || us < best) { best = us; a.nb = h; a.m_tiles = m_tiles; items = n; walk = w; parts = p; }
         };
         take(walked(n), n, 1);
-        for (const int first : {0, n / sms * sms}) {
-            int p = 1;
-            if (first == n) continue;
-            const long c = shared(n - first, p) + (first > 0 ? walked(first) + 30 : 0);
-            take(c, first, p);
+        for (int p = 2; p <= std::min(DQ_MAX_PARTS, all_sb); ++p) {
+            const int places = clusters.of[p].load(std::memory_order_relaxed);
+            const double wave = ((all_sb + p - 1) / p) * span + 4.72 + 0.036 * h + 0.012 * p;
+            auto shared = [&](int first, double launch) {
+                const int count = n - first;
+                if (count > 0 && (!lower || count <= 0.95 * places)) take(((count + places - 1) / places) * wave + launch, first, p);
+            };
+            shared(0, -3.61);  // (its start lies under the kernel before)
+            if (whole > 0) shared(whole, walked(whole) + 0.22);
         }
+        last = h;
     }
     // shared memory: at most half for activations (each box serves 64 columns), the rest for raw tiles
     const int njt = a.nb <= 16 ? 1 : a.nb <= 32 ? 2 : a.nb <= 64 ? 4 : 8;

@@ -825,14 +825,14 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
     if (le != cudaSuccess) return le;
     // How high the tiles are and how they are dealt out, by a model of the time in us, fitted to 30,000 forced choices (21 matrices x 24 row
     // counts x 3 formats; 4 % off). SPAN: 256 columns of a tile by its height; a low tile's take less time, if more for each row. One block per
-    // SM walks over tiles, or clusters share a tile's K range, where every wave pays for its start and for the parts that are added; where tiles
-    // go over whole rounds of the SMs, those that do may have a launch of their own. Q4_K 6144 x 4096, 512 rows (192 tiles) walked 74.7, clusters
-    // of two 84.5, a walk and 44 tiles shared by two 70.6; 20000 x 14336, 20 rows (157 tiles) 160, clusters of four 121, nine tiles shared by
-    // eight 97; 8960 x 1536, 300 rows (210 tiles) 37 walked, 39 in two launches.
-    // Tiles lower than need be are for SMs that would be idle, and taken where they promise 3 %; not in clusters that fill their places
-    // to the last, which start one after the other (3000 x 2048, 112 rows, 72 of 74 pairs 15.5, as four parts of one tile 14.1). That is 0.962 of the
-    // time of the fewest tiles over those sizes, at worst 1.05. Q8_0, 389 rows: 2560 x 2560 80 tiles of 112 rows 25.4 us, 140 of 64 21.1;
-    // 2560 x 10240 71.9 and 66.1; 1152 x 896, 300 rows 10.9 and 8.6; Q4_K 2048 x 1536, 192 rows 12.0 and 11.0.
+    // SM walks over tiles, or clusters share a tile's K range, where every wave pays for its start and for the parts that are added, and the
+    // last clusters that fit start late (3000 x 2048, 112 rows, 72 of 74 pairs 15.5, as four parts of one tile 14.1); where tiles go over whole
+    // rounds of the SMs, those that do may have a launch of their own. Q4_K 6144 x 4096, 512 rows (192 tiles) walked 74.7, clusters of two 84.5, a
+    // walk and 44 tiles shared by two 70.6; 20000 x 14336, 20 rows (157 tiles) 160, clusters of four 121, nine tiles shared by eight 97; 8960 x
+    // 1536, 300 rows (210 tiles) 37 walked, 39 in two launches.
+    // Tiles lower than need be are for SMs that would be idle, and taken where they promise 3 %: 0.96 of the time of the fewest tiles over those
+    // sizes. Q8_0, 389 rows: 2560 x 2560 80 tiles of 112 rows 25.4 us, 140 of 64 21.1; 2560 x 10240 71.9 and 66.1; 1152 x 896, 300 rows 10.9
+    // and 8.6; Q4_K 2048 x 1536, 192 rows 12.0 and 11.0.
     const int all_sb = (k + 255) / 256, sms = device_sm_count(), fewest = (m + DQ_NB - 1) / DQ_NB;
     const DqClusters& clusters = dq_clusters();
     int items = 0, walk = 0, parts = 1;  // tiles; those that are walked over; the rest is shared by `parts` blocks each
@@ -844,23 +844,24 @@ cudaError_t launch_gemm_dq(const Tc5Seg* segs, int nseg, int k, const DqInput& i
         if (last && n > 8 * sms) break;
         if (last && !lower) best *= 0.97;
         lower = last != 0;
-        static constexpr double SPAN[2][8] = {{1.26, 1.35, 1.47, 1.52, 1.79, 1.82, 1.87, 1.98}, {1.12, 1.10, 1.25, 1.26, 1.64, 1.67, 1.70, 1.74}};
+        static constexpr double SPAN[2][8] = {{1.26, 1.36, 1.48, 1.54, 1.81, 1.84, 1.89, 2.00}, {1.12, 1.10, 1.26, 1.27, 1.66, 1.68, 1.72, 1.77}};
         const double span = (SPAN[0][h / 16 - 1] * (tiles - one_plane) + SPAN[1][h / 16 - 1] * one_plane) / tiles;
         const int whole = n / sms * sms;
-        auto walked = [&](int count) { return ((count + sms - 1) / sms) * (all_sb * span + 0.014 * h); };
+        auto walked = [&](int count) { return ((count + sms - 1) / sms) * (all_sb * span + 0.013 * h); };
         auto take = [&](double us, int w, int p) {
             if (best == 0.0 || us < best) { best = us; a.nb = h; a.m_tiles = m_tiles; items = n; walk = w; parts = p; }
         };
         take(walked(n), n, 1);
         for (int p = 2; p <= std::min(DQ_MAX_PARTS, all_sb); ++p) {
             const int places = clusters.of[p].load(std::memory_order_relaxed);
-            const double wave = ((all_sb + p - 1) / p) * span + 4.72 + 0.036 * h + 0.012 * p;
+            const double wave = ((all_sb + p - 1) / p) * span + 3.92 + 0.037 * h - 0.017 * p;
             auto shared = [&](int first, double launch) {
                 const int count = n - first;
-                if (count > 0 && (!lower || count <= 0.95 * places)) take(((count + places - 1) / places) * wave + launch, first, p);
+                const double filled = std::min(1.0, (double)count / places), late = filled * filled;
+                if (count > 0) take(((count + places - 1) / places) * wave + 1.37 * late * late + launch, first, p);
             };
-            shared(0, -3.61);  // (its start lies under the kernel before)
-            if (whole > 0) shared(whole, walked(whole) + 0.22);
+            shared(0, -3.05);  // (its start lies under the kernel before)
+            if (whole > 0) shared(whole, walked(whole) + 0.80);
         }
         last = h;
     }

@@ -699,19 +699,22 @@ static cudaError_t launch_gqa_mma(const float* q, int ldq, float* out, int ldo, 
                                   KvGeom kv, int layer, float scale, int n_splits, float* scratch, cudaStream_t st, int fresh) {
     constexpr size_t WARP_SMEM = 4 * KV_PAGE * (16 * HD16 + 8) * sizeof(__half);
     static PerDeviceOnce once;
-    static int held[SP_MAX_DEVICES][2];  // blocks of four and of three warps that an SM holds
-    int* const fit = held[current_device_index()];
+    static std::atomic<int> held[SP_MAX_DEVICES][2];  // blocks of four and of three warps that an SM holds
+    std::atomic<int>* const fit = held[current_device_index()];
     cudaError_t le = once.run([&] {
+        int four = 0, three = 0;
         cudaError_t e = cudaFuncSetAttribute(attention_gqa_mma_kernel<HD16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * WARP_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_gqa_mma_kernel<HD16, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * WARP_SMEM);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit[0], attention_gqa_mma_kernel<HD16, 4>, 128, 4 * WARP_SMEM);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit[1], attention_gqa_mma_kernel<HD16, 3>, 96, 3 * WARP_SMEM);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&four, attention_gqa_mma_kernel<HD16, 4>, 128, 4 * WARP_SMEM);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&three, attention_gqa_mma_kernel<HD16, 3>, 96, 3 * WARP_SMEM);
+        fit[0].store(four);
+        fit[1].store(three);
         return e;
     });
     if (le != cudaSuccess) return le;
     const int64_t blocks = (int64_t)kv.n_kv * n_tok * n_splits;
     auto rounds = [&](int per_sm) { const int64_t at_once = (int64_t)std::max(per_sm, 1) * device_sm_count(); return (blocks + at_once - 1) / at_once; };
-    const bool narrow = rounds(fit[1]) < rounds(fit[0]);
+    const bool narrow = rounds(fit[1].load()) < rounds(fit[0].load());
     const int warps = narrow ? 3 : 4;
     return launch_pdl(narrow ? attention_gqa_mma_kernel<HD16, 3> : attention_gqa_mma_kernel<HD16, 4>, dim3(kv.n_kv, n_tok, n_splits), dim3(32 * warps),
                       warps * WARP_SMEM, st, q, ldq, out, ldo, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, fresh);

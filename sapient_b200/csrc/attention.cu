@@ -729,17 +729,16 @@ cudaError_t launch_gqa_mma_phase(const float* q, int ldq, float* out, int ldo, i
     return launch(q, ldq, out, ldo, n_tok, n_heads, tok_slot, tok_pos, kv, layer, scale, n_splits, scratch, st, fresh);
 }
 
-// A tile walks all its keys alone, at 50 to 76 ns each whatever the number of its rows, and up to two blocks per SM take no longer
-// than one. With a token per block the same keys cost every (token, cached head) pair -- (token, query head) where no kernel
-// shares cached rows -- its own pass: so tiles are for many pairs, and the later a portion of a prompt stands in its
-// context the more pairs it takes. Whole steps of four-layer models, us, a token per block / tiles:
-//   32 heads on 8 cached, 128 coordinates   128 tokens at position 0: 874 / 849, at 1000: 1085 / 1164, at 8000: 2558 / 3284
-//                                           300 tokens at position 0: 1849 / 1782, at 1000: 2283 / 2099, at 8000: 5279 / 4252
-//   12 on 2, 128                            300 tokens at position 0: 662 / 675, at 8000: 1795 / 2459
-//   14 on 2, 64                             300 tokens at position 0: 412 / 445, at 8000: 1022 / 2196
-//   32 unshared, 80                         24 tokens at position 0: 369 / 373, at 200: 468 / 407; 300 at 8000: 39048 / 3018
-// Both times are lines through 168 such pairs (these models, 17 to 300 tokens, positions 0 to 8000). The choice is the faster side's in
-// all but a few, by up to 8 us a layer; more than 600 pairs at any position, the rule before, cost up to 180.
+// A tile's keys are one chain (or two halves of it, launch_attention_prefill), and up to two blocks per SM take no longer than one. With a
+// token per block the same keys cost every (token, cached head) pair -- (token, query head) where no kernel shares cached rows --
+// its own pass: so tiles are for many pairs, and the later a portion of a prompt stands in its context the more pairs it takes.
+// The constants are lines through 168 times of whole steps (17 to 300 tokens, positions 0 to 8000, these models), taken when a tile walked
+// its keys alone at 50 to 76 ns each. Since two blocks share them tiles take down to half of that, which the rule leaves. Rotation and
+// attention, us, a token per block / tiles, * what it chooses:
+//   32 heads on 8 cached, 128 coordinates   150 tokens at position 1000: 76* / 49, at 7600: 449* / 279; 389 at 7600: 1095 / 550*
+//   12 on 2, 128                            512 tokens at position 1000: 82* / 59; 300 at 7600: 282* / 280
+//   14 on 2, 64                             512 tokens at position 7600: 214* / 250; 17 at 200: 13* / 11
+//   32 unshared, 80                         24 tokens at position 0: 7.9* / 7.9; 389 at 7600: 8900 / 465*
 bool attention_takes_tiles(int n_tok, int pos0, int n_heads, int n_kv, int head_dim) {
     if (n_tok < 16) return false;
     const bool shared = attention_gqa_mma_supported(n_heads, n_kv, head_dim);
@@ -761,8 +760,10 @@ cudaError_t launch_attention_prefill(const float* q, int ldq, float* out, int ld
     if (!attention_prefill_supported(kv.head_dim)) return cudaErrorInvalidValue;
     const int hd16 = kv.head_dim / 16;
     const size_t smem = (size_t)4 * FA_KEYS * (kv.head_dim + 8) * sizeof(__half);  // two (K, V) tile buffers
-    // The longest tile's chain of keys is what a launch takes, some 4 us for 64 of them: two blocks share it while SMs have room for them
-    // (389 tokens of Phi-2 29.6 -> 22.7 us a layer, 512 of the 8B shape 39.2 -> 36.5, most of it from pages that are looked up a tile ahead).
+    // The longest tile's chain of keys is what a launch takes, some 4 us for 64 of them: two blocks share it while SMs have room for them.
+    // With the rotation before it, one block / two, exact operands: 389 tokens of Phi-2 29.1 / 24.6 us, 256 of the 8B shape 24.8 / 18.9; from 149
+    // to 296 tiles of 128 coordinates, whose halves then take a second round, 512 tokens 41.2 / 38.8, rounded operands 33.4 / 33.9; up to
+    // 128 keys two take longer (24 tokens at position 0 8.1 / 11.0).
     const int row_tiles = (n_tok + FA_ROWS - 1) / FA_ROWS;
     const int parts = pos0 + n_tok > 2 * FA_KEYS && (int64_t)n_heads * row_tiles <= 2 * device_sm_count() ? 2 : 1;
     const dim3 grid(n_heads, row_tiles, parts), block(FA_WARPS * 32);

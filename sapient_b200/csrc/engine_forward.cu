@@ -144,11 +144,11 @@ int Engine::enqueue_decode_step(int T) {
 
 // The first n floats of logits_ to host memory of the caller's, through the pinned buffer. From four megabytes on several threads
 // copy out of it while the device still fills it: a lone one takes longer to write a caller's fresh pages (32 rows of 128256 logits:
-// 1.6 ms) than the device to make them. (Five rows of 151936, three megabytes, take 100 us longer so: threads wake slowly.) The device's copies are few, for each costs it
-// three microseconds and a short one runs slower (16.4 MB: one copy 293 us, 8 318, 32 404, with their events 496); threads take a quarter of a
-// megabyte at a time of what has arrived, and ask the driver, where they would queue, only for copies that none has seen done (24 rows of
-// 51200: a step of two layers 561 us, each asking for each, 501). This thread waits for the first copy alone; the engine's helpers, which sleep until then, are
-// woken for what is left. Returns with the stream's work done.
+// 1.6 ms) than the device to make them. (Five rows of 151936, three megabytes, take 100 us longer so: threads wake slowly.) The device's
+// copies are few, for each costs it three microseconds and a short one runs slower (16.4 MB: one copy 293 us, 8 318, 32 404, with their
+// events 496); threads take a quarter of a megabyte at a time of what has arrived, and ask the driver, where they would queue, only for
+// copies that none has seen done (24 rows of 51200: a step of two layers 561 us, each asking for each, 501). This thread waits for the
+// first copy alone; the engine's helpers, which sleep until then, are woken for what is left. Returns with the stream's work done.
 int Engine::fetch_logits(float* out, size_t n) {
     constexpr size_t SLICE = (size_t)1 << 16;  // floats that a thread takes
     const int slices = (int)((n + SLICE - 1) / SLICE);

@@ -32,11 +32,7 @@
 // 31.0 -> 29.3; Q4_K 17920 x 1536 192 rows 29.7 -> 28.0; Q8_0 28672 x 4096 32 rows 49.8 -> 48.5, 10240 x 2560 389 rows 60.2 -> 60.0.
 // Without effect: a second group of eight producers, two warps that issue products for accumulators in turn, a ring of 3 or 5
 // activation stages instead of 4, waits that ask without looking first.
-// Measured against the kernel before (matmul with its split of activations), us: Q4_K 28672 x 4096, 32 rows 101 -> 51, 512 rows 285 -> 230;
-// 4096 x 14336 Q6_K, 37 rows 54.6 -> 35; Q4_K 4096 x 4096, 512 rows 85 -> 44; Q8_0 17920 x 1536, 192 rows 32.5 -> 33.5, 512 rows 71.7 ->
-// 68. That kernel took 256 activation rows per tile, one pass over the weights where two are made here, which still tells at the
-// largest products of little more than a tile's rows: Q6_K 20000 x 14336, 130 rows 237 -> 267, 192 rows 267 -> 286; of 210 products (three
-// formats, 1000 x 1024 to 20000 x 14336, 17 to 512 rows) 15 take longer than on that kernel, all together 0.67 of its time. Error against float64 at K = 14336: 1.3e-5 -> 5e-7.
+// Error against float64 at K = 14336: 5e-7.
 // The K range of a tile is shared by the blocks of a cluster when tiles alone leave SMs idle; they meet in distributed shared
 // memory and add in part order, so results do not vary from run to run. Every wait on an mbarrier is bounded; after one that ran out
 // nothing more is issued, the warps that did issue wait (bounded) for their copies and products in flight, y is left alone.
